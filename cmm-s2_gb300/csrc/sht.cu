@@ -9,6 +9,8 @@
 //      zero padding, Z2Z 4L inverse);
 //   3. Legendre analysis with Clenshaw-Curtis weights in cos(theta), exact
 //      for the degree <= 2L-1 products: f_lm = sum_j w_j F'_m(j) Pbar_lm(j).
+//   With Pbar tables 2 and 3 are one contraction with the table of the
+//   combined weights W_lm(t) on the L+1 rings (build_w_kernel).
 // Inverse (pyssht.inverse in project_stream, :84-91): Legendre synthesis on
 // the L+1 rings, then inverse real FFTs (cuFFT Z2D).
 // Pbar_lm are orthonormal with the Condon-Shortley phase and come from the
@@ -309,6 +311,93 @@ __global__ void ladder2_kernel(double2* __restrict__ fields, int L) {
   }
 }
 
+// The velocity's coefficient fields in the FP64 form, from the analysis a
+// (lap: psi = D_inv a, cmm_s2/core/spherical_simulations.py:195-198) or
+// the stream function itself.  With A_k = iL_k (ladder above) u_i = A_i psi
+// and the 9 gradients A_k u_i need only six Legendre sums:
+//   psi, u_x, u_y, A_x u_x, A_x u_y, A_y u_y;
+// A_z is the factor i m on a ring spectrum (u_z, A_z u_x, A_z u_y, A_z u_z),
+// and the commutators A_x A_y - A_y A_x = -A_z (and cyclic) give the rest on
+// the grid: A_y u_x = A_x u_y + u_z, A_x u_z = A_z u_x + u_y, A_y u_z = A_z u_y
+// - u_x.  One pass over a (neighbouring orders m-2..m+2) in place of the
+// inverse Laplacian and two ladder passes over 12 fields, and half of the
+// Legendre synthesis, which is FP64-bound.  Velocity inversion, with the
+// analysis weights below: 207 -> 103 us at L = 128, 2.99 -> 1.61 ms at L = 512.
+__device__ __forceinline__ double2 order_value(const double2* __restrict__ a, int L, int l, int mm, double d) {
+  const int k = mm < 0 ? -mm : mm;
+  if (k > l) return make_double2(0.0, 0.0);
+  const double2 v = cmul(a[(int64_t)k * L + l], d);
+  if (mm >= 0) return v;   // a_{l,-k} = (-1)^k conj(a_{l,k})
+  return (k & 1) ? make_double2(-v.x, v.y) : make_double2(v.x, -v.y);
+}
+
+__global__ void __launch_bounds__(128) velocity_fields_kernel(const double2* __restrict__ a, int L, int lap,
+                                                              double2* __restrict__ fields) {
+  const int l = blockIdx.x * blockDim.x + threadIdx.x, m = blockIdx.y;
+  if (l >= L) return;
+  const int64_t fs = (int64_t)L * L, i = (int64_t)m * L + l;
+  if (l < m) {
+#pragma unroll
+    for (int f = 0; f < 6; ++f) fields[f * fs + i] = make_double2(0.0, 0.0);
+    return;
+  }
+  const double ll = (double)l * (double)(l + 1);
+  const double d = lap ? (l == 0 ? 0.0 : -1.0 / ll) : 1.0;
+  double2 v[5];   // psi at orders m-2 .. m+2
+#pragma unroll
+  for (int k = 0; k < 5; ++k) v[k] = order_value(a, L, l, m - 2 + k, d);
+  double c[4];    // sqrt(l(l+1) - k(k-1)) / 2 at k = m-1 .. m+2
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const double q = (double)(m - 1 + k);
+    c[k] = 0.5 * sqrt(fmax(ll - q * (q - 1.0), 0.0));
+  }
+  // X = (up + dn) / 2 and Y = (up - dn) / 2 at orders m-1, m, m+1: u_x = i X,
+  // u_y = Y
+  double2 X[3], Y[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const double2 up = cmul(v[k], c[k]), dn = cmul(v[k + 2], c[k + 1]);
+    X[k] = make_double2(up.x + dn.x, up.y + dn.y);
+    Y[k] = make_double2(up.x - dn.x, up.y - dn.y);
+  }
+  const double cu = c[1], cd = c[2];
+  fields[i] = v[2];
+  fields[fs + i] = make_double2(-X[1].y, X[1].x);
+  fields[2 * fs + i] = Y[1];
+  // A_x f = i (cu f_{m-1} + cd f_{m+1}) / 2, A_y f = (cu f_{m-1} - cd f_{m+1}) / 2
+  fields[3 * fs + i] = make_double2(-(cu * X[0].x + cd * X[2].x), -(cu * X[0].y + cd * X[2].y));
+  fields[4 * fs + i] = make_double2(-(cu * Y[0].y + cd * Y[2].y), cu * Y[0].x + cd * Y[2].x);
+  fields[5 * fs + i] = make_double2(cu * Y[0].x - cd * Y[2].x, cu * Y[0].y - cd * Y[2].y);
+}
+
+// The nine ring spectra (and grid fields) of the velocity in the FP64 form:
+// u_x, u_y, u_z, A_x u_x, A_x u_y, A_y u_y, A_z u_x, A_z u_y, A_z u_z.
+constexpr int kVelLegendre = 6, kVelSpectra = 9;
+
+// Spectra of Legendre field f (velocity_fields_kernel's order) at (t, m),
+// value v, into S (9, L+1, L+1); the m = L column is zeroed beside m = 0
+// (an out-of-place C2R transform may overwrite its input).
+__device__ __forceinline__ void store_velocity_spectra(double2* __restrict__ S, int L, int f, int t, int m,
+                                                       double2 v) {
+  const int64_t row = L + 1, fs = (int64_t)(L + 1) * row, at = (int64_t)t * row + m;
+  const double2 z = make_double2(-(double)m * v.y, (double)m * v.x);   // i m v
+  const double2 zero = make_double2(0.0, 0.0);
+  const int64_t ny = (int64_t)t * row + L;
+  if (f == 0) {          // psi: u_z = i m psi, A_z u_z = -m^2 psi
+    S[2 * fs + at] = z;
+    S[8 * fs + at] = make_double2(-(double)m * z.y, (double)m * z.x);
+    if (m == 0) S[2 * fs + ny] = S[8 * fs + ny] = zero;
+  } else if (f <= 2) {   // u_x, u_y and their A_z
+    S[(f - 1) * fs + at] = v;
+    S[(f + 5) * fs + at] = z;
+    if (m == 0) S[(f - 1) * fs + ny] = S[(f + 5) * fs + ny] = zero;
+  } else {
+    S[f * fs + at] = v;
+    if (m == 0) S[f * fs + ny] = zero;
+  }
+}
+
 // power[l] = sum over all orders -l..l of |a_lm|^2 = |a_l0|^2 + 2 sum_{m>0}
 // |a_lm|^2 (real field); one block per degree.  The summand of
 // energy_spectrum (cmm_s2/core/spherical_harmonic_tools.py:157-163).
@@ -367,7 +456,8 @@ __global__ void scalar_jets_kernel(const double* __restrict__ fld, int L, const 
 // Legendre synthesis of nf fields: block (m, ring-pair tile); each thread
 // one ring pair (t, L-t).  Out: spectra S[f][t][m] (nf, L+1, L+1), m = L
 // column zero (written by the caller's memset).
-template <int NF>
+// VEL: the six fields of velocity_fields_kernel -> the nine spectra.
+template <int NF, bool VEL = false>
 __global__ void __launch_bounds__(kSynthBlock) synthesis_kernel(const double2* __restrict__ alm, int L,
                                                                 const double* __restrict__ ct,
                                                                 const double* __restrict__ pmm,
@@ -423,6 +513,14 @@ __global__ void __launch_bounds__(kSynthBlock) synthesis_kernel(const double2* _
     }
   }
   if (!active) return;
+  if (VEL) {
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+      store_velocity_spectra(S, L, f, t, m, make_double2(E[f].x + O[f].x, E[f].y + O[f].y));
+      if (L - t != t) store_velocity_spectra(S, L, f, L - t, m, make_double2(E[f].x - O[f].x, E[f].y - O[f].y));
+    }
+    return;
+  }
   const int64_t row = L + 1;
 #pragma unroll
   for (int f = 0; f < NF; ++f) {
@@ -436,11 +534,12 @@ __global__ void __launch_bounds__(kSynthBlock) synthesis_kernel(const double2* _
 // At small L the recurrence kernels above run a few warps per SM (one
 // block per m, one thread per ring pair) and are latency-bound, and the
 // analysis spends 3 FP64 operations of recurrence per 2 of contraction.
-// With tables the Pbar_lm values are computed once per plan (FP64, the same
-// recurrence) and both Legendre stages become table contractions with one
-// thread per (m, l) (analysis) or per (m, ring pair, field group)
-// (synthesis): L^3/2 and L^3/4 doubles, 68 + 34 MB at L = 256, 0.54 + 0.27
-// GB at L = 512, 4.3 + 2.2 GB at L = 1024.  By default (cmm_sht_set_tables)
+// With tables the Pbar_lm values (synthesis) and the analysis weights are
+// computed once per plan (FP64, the same recurrence) and both Legendre
+// stages become table contractions with one thread per (m, l) and slice
+// (analysis) or per (m, ring pair, field group) (synthesis): L^3/4 doubles
+// each, 34 + 34 MB at L = 256, 0.27 + 0.27 GB at L = 512, 2.2 + 2.2 GB at
+// L = 1024.  By default (cmm_sht_set_tables)
 // plans with L <= kTabMaxL use them.
 constexpr int kTabMaxL = 512;
 constexpr int kTabShared = 1024;   // largest L the analysis kernel's shared arrays hold
@@ -450,17 +549,16 @@ __device__ __host__ __forceinline__ int64_t tab_off(int m, int L, int nj) {
   return (int64_t)nj * ((int64_t)m * L - (int64_t)m * (m - 1) / 2);
 }
 
-// One thread per (m, ring j): Pbar_{l,m}(theta_j), l = m..L-1.  lmajor:
-// layout [m][l-m][j] (synthesis) else [m][j][l-m] (analysis).
-__global__ void build_pbar_kernel(int L, int nj, const double* __restrict__ ct, const double* __restrict__ pmm,
-                                  int pmm_stride, const double* __restrict__ ra, const double* __restrict__ rb,
-                                  bool lmajor, double* __restrict__ tab) {
+// One thread per (m, ring j): Pbar_{l,m}(theta_{j0 + dj j}), l = m..L-1, j <
+// nj, in the layout [m][l-m][j].
+__global__ void build_pbar_kernel(int L, int nj, int j0, int dj, const double* __restrict__ ct,
+                                  const double* __restrict__ pmm, int pmm_stride, const double* __restrict__ ra,
+                                  const double* __restrict__ rb, double* __restrict__ tab) {
   const int m = blockIdx.y, j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= nj) return;
-  const double x = ct[j];
-  double p0 = pmm[(int64_t)m * pmm_stride + j], p1 = 0.0;
+  const double x = ct[j0 + dj * j];
+  double p0 = pmm[(int64_t)m * pmm_stride + j0 + dj * j], p1 = 0.0;
   double* base = tab + tab_off(m, L, nj);
-  const int nl = L - m;
   for (int l = m; l < L; ++l) {
     double P;
     if (l == m) {
@@ -474,53 +572,157 @@ __global__ void build_pbar_kernel(int L, int nj, const double* __restrict__ ct, 
       p1 = p0;
       p0 = P;
     }
-    const int i = l - m;
-    base[lmajor ? (int64_t)i * nj + j : (int64_t)j * nl + i] = P;
+    base[(int64_t)(l - m) * nj + j] = P;
   }
 }
 
-// Analysis from the table: block (m, tile of 64 degrees), thread l; the
-// weighted even/odd ring spectra of order m staged in shared memory.
+// Analysis weights.  The forward transform's resampling (the torus
+// extension of the ring spectra, its trigonometric interpolant with the
+// Nyquist term split evenly, read on the 2L+1 fine rings) and the
+// quadrature are linear in the L+1 ring values of each order, so with
+// R_m(j, t) the interpolant's matrix
+//   a_lm = sum_t W_lm(t) F_m(t),  W_lm(t) = (pi/L) sum_j w_j Pbar_lm(theta'_j) R_m(j, t):
+// one contraction over L/2+1 ring pairs (W_lm(L-t) = (-1)^(l-m) W_lm(t)) in
+// place of two transforms per order, a padding pass and a contraction over
+// L+1 pairs.  R is the identity on the even fine rings (they are the rings),
+// and on the odd ones the Dirichlet kernel sin(L x) cot(x/2) / 2L of x =
+// theta'_j - theta_t, plus (-1)^m that of the mirrored ring 2L-t (0 < t < L).
+// odd_kernel_kernel: Kp[v][jj][t] = (pi/L) w_j (R_m(j, t) + s R_m(2L-j, t)),
+// j = 2 jj + 1 <= L (unpaired at j = L), with v = 2 (m odd) + (l-m odd) and s
+// = (-1)^(l-m), the odd fine rings' weight of the pair.
+__global__ void odd_kernel_kernel(int L, const double* __restrict__ w, double* __restrict__ Kp) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, jj = blockIdx.y, v = blockIdx.z;
+  const int npair = L / 2 + 1, npo = (L + 1) / 2;
+  if (t >= npair) return;
+  const double mm = (v & 2) ? -1.0 : 1.0, sl = (v & 1) ? -1.0 : 1.0;
+  auto R = [&](int j) {
+    double s, c, r;
+    sincospi((double)(j - 2 * t) / (4.0 * L), &s, &c);
+    r = c / s;
+    if (t > 0 && t < L) {
+      sincospi((double)(j + 2 * t) / (4.0 * L), &s, &c);
+      r += mm * (c / s);
+    }
+    return ((((j - 1) / 2 - t) & 1) ? -r : r) / (2.0 * L);
+  };
+  const int j = 2 * jj + 1;
+  double k = R(j);
+  if (j < L) k += sl * R(2 * L - j);
+  Kp[((int64_t)v * npo + jj) * npair + t] = M_PI / L * w[j] * k;
+}
+
+// W of order m = blockIdx.y from Pbar on the odd fine rings (po, [m][l-m][jj])
+// and on the rings (ps, [m][l-m][t]): 32 degrees of one parity (blockIdx.z
+// & 1) x 64 ring pairs per block, layout [m][t][l-m].  Set-up work, once per
+// table.
+__global__ void __launch_bounds__(256) build_w_kernel(int L, const double* __restrict__ po,
+                                                      const double* __restrict__ ps, const double* __restrict__ Kp,
+                                                      const double* __restrict__ w, double* __restrict__ W) {
+  const int npair = L / 2 + 1, npo = (L + 1) / 2;
+  const int m = blockIdx.y, par = blockIdx.z & 1, i0 = (blockIdx.z >> 1) * 32, t0 = blockIdx.x * 64;
+  const int nl = L - m;
+  if (2 * i0 + par >= nl) return;   // uniform for the block
+  __shared__ double A[32][17], B[16][65];
+  const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;   // ring pair; 8 degrees each
+  const double* P = po + tab_off(m, L, npo);
+  const double* K = Kp + (int64_t)(2 * (m & 1) + par) * npo * npair;
+  double acc[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) acc[q] = 0.0;
+  // towards the poles Pbar_lm falls off exponentially and grows with l: the
+  // leading tiles of rings where the block's two highest degrees are below
+  // 1e-30 add nothing (about a third of the products)
+  int k_first = 0;
+  const int itop = min(nl - 1, 2 * (i0 + 31) + 1);
+  for (; k_first + 16 < npo; k_first += 16) {
+    const double a = P[(int64_t)itop * npo + k_first + 15], b = itop > 0 ? P[(int64_t)(itop - 1) * npo + k_first + 15] : 0.0;
+    if (!(fabs(a) < 1e-30 && fabs(b) < 1e-30)) break;
+  }
+  for (int k0 = k_first; k0 < npo; k0 += 16) {
+    for (int e = threadIdx.x; e < 32 * 16; e += 256) {
+      const int r = e >> 4, k = e & 15, i = 2 * (i0 + r) + par;
+      A[r][k] = (i < nl && k0 + k < npo) ? P[(int64_t)i * npo + k0 + k] : 0.0;
+    }
+    for (int e = threadIdx.x; e < 16 * 64; e += 256) {
+      const int k = e >> 6, t = e & 63;
+      B[k][t] = (k0 + k < npo && t0 + t < npair) ? K[(int64_t)(k0 + k) * npair + t0 + t] : 0.0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      const double b = B[k][tx];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) acc[q] += A[8 * ty + q][k] * b;
+    }
+    __syncthreads();
+  }
+  const int t = t0 + tx;
+  if (t >= npair) return;
+  const double we = M_PI / L * w[2 * t];   // the even fine ring 2t is ring t
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int i = 2 * (i0 + 8 * ty + q) + par;
+    if (i < nl)
+      W[tab_off(m, L, npair) + (int64_t)t * nl + i] = acc[q] + we * ps[tab_off(m, L, npair) + (int64_t)i * npair + t];
+  }
+}
+
+// Analysis from the table: block (m, tile of 64 degrees), 64 threads (one
+// degree each) x 4 slices of the ring pairs; the parity-folded ring values
+// of order m staged in shared memory, the slices added at the end.  FP64:
+// two multiply-adds per table entry, each entry (8 B) read once.  The
+// slices shorten the serial chain where L is small (65 pairs at L = 128).
+// F: ring spectra (L+1, L+1).
 constexpr int kTabBlock = 64;
-__global__ void __launch_bounds__(kTabBlock) analysis_tab_kernel(const double2* __restrict__ fine, int L,
-                                                                 const double* __restrict__ w,
-                                                                 const double* __restrict__ tab,
-                                                                 double2* __restrict__ alm) {
-  __shared__ double2 E[kTabShared + 1], O[kTabShared + 1];
-  const int m = blockIdx.x, l = m + blockIdx.y * kTabBlock + threadIdx.x;
-  if (m + (int)blockIdx.y * kTabBlock >= L) return;   // the whole tile is past l = L-1
-  const int npair = L + 1;
-  for (int j = threadIdx.x; j < npair; j += blockDim.x) {
-    const double2 a = fine[(int64_t)m * 4 * L + j];
-    double2 e, o;
-    if (j < L) {
-      const double2 b = fine[(int64_t)m * 4 * L + 2 * L - j];
+constexpr int kAnaSlices = 4;
+__global__ void __launch_bounds__(kTabBlock * kAnaSlices) analysis_w_kernel(const double2* __restrict__ F, int L,
+                                                                            const double* __restrict__ W,
+                                                                            double2* __restrict__ alm) {
+  constexpr int kMaxPair = kTabShared / 2 + 1;
+  __shared__ double2 E[kMaxPair], O[kMaxPair];
+  const int m = blockIdx.x, tid = threadIdx.x;
+  const int lane = tid % kTabBlock, slice = tid / kTabBlock;
+  const int i = blockIdx.y * kTabBlock + lane, nl = L - m, npair = L / 2 + 1;
+  if ((int)blockIdx.y * kTabBlock >= nl) return;   // the whole tile is past l = L-1
+  for (int t = tid; t < npair; t += blockDim.x) {
+    const double2 a = F[(int64_t)t * (L + 1) + m];
+    double2 e = a, o = make_double2(0.0, 0.0);
+    if (t < L - t) {
+      const double2 b = F[(int64_t)(L - t) * (L + 1) + m];
       e = make_double2(a.x + b.x, a.y + b.y);
       o = make_double2(a.x - b.x, a.y - b.y);
-    } else {
-      e = a;
-      o = make_double2(0.0, 0.0);
     }
-    E[j] = cmul(e, w[j]);
-    O[j] = cmul(o, w[j]);
+    E[t] = e;
+    O[t] = o;
   }
   __syncthreads();
-  if (l >= L) return;
-  const int nl = L - m, i = l - m;
-  const double* P = tab + tab_off(m, L, npair) + i;
-  const double2* V = (i & 1) == 0 ? E : O;
   double2 acc = make_double2(0.0, 0.0);
-  for (int j = 0; j < npair; ++j) {
-    const double pj = __ldg(P + (int64_t)j * nl);
-    acc.x += pj * V[j].x;
-    acc.y += pj * V[j].y;
+  if (i < nl) {
+    const double* P = W + tab_off(m, L, npair) + i;
+    const double2* V = (i & 1) == 0 ? E : O;
+#pragma unroll 4
+    for (int t = slice; t < npair; t += kAnaSlices) {
+      const double p = __ldg(P + (int64_t)t * nl);
+      acc.x += p * V[t].x;
+      acc.y += p * V[t].y;
+    }
   }
-  alm[(int64_t)m * L + l] = acc;
+  __shared__ double2 red[kAnaSlices - 1][kTabBlock];
+  if (slice) red[slice - 1][lane] = acc;
+  __syncthreads();
+  if (slice || i >= nl) return;
+#pragma unroll
+  for (int q = 0; q < kAnaSlices - 1; ++q) {
+    acc.x += red[q][lane].x;
+    acc.y += red[q][lane].y;
+  }
+  alm[(int64_t)m * L + m + i] = acc;
 }
 
 // Synthesis from the table: block (m, tile of ring pairs, group of G
-// fields); each thread one ring pair (t, L-t) and G fields.
-template <int G>
+// fields); each thread one ring pair (t, L-t) and G fields.  VEL: the six
+// fields of velocity_fields_kernel (two groups of 3) -> the nine spectra.
+template <int G, bool VEL = false>
 __global__ void __launch_bounds__(kTabBlock) synthesis_tab_kernel(const double2* __restrict__ alm, int L,
                                                                   const double* __restrict__ tab,
                                                                   double2* __restrict__ S) {
@@ -560,6 +762,15 @@ __global__ void __launch_bounds__(kTabBlock) synthesis_tab_kernel(const double2*
     }
   }
   if (!active) return;
+  if (VEL) {
+#pragma unroll
+    for (int f = 0; f < G; ++f) {
+      store_velocity_spectra(S, L, f0 + f, t, m, make_double2(E[f].x + O[f].x, E[f].y + O[f].y));
+      if (L - t != t)
+        store_velocity_spectra(S, L, f0 + f, L - t, m, make_double2(E[f].x - O[f].x, E[f].y - O[f].y));
+    }
+    return;
+  }
   const int64_t row = L + 1;
 #pragma unroll
   for (int f = 0; f < G; ++f) {
@@ -573,9 +784,9 @@ __global__ void __launch_bounds__(kTabBlock) synthesis_tab_kernel(const double2*
 // the 12 synthesised fields on the grid: vals[i][0] = u_i and, with
 // g = (iLx, iLy, iLz) u_i, vals[c][1+i] = (g x X - ((g x X).X/|X|) X)_c;
 // poles from sample 0 of the first and last rings.
-// jets_f (nullable): the same values as floats (exact for R = float).
-template <typename R>
-__global__ void jets_kernel(const R* __restrict__ fld, int L, const double* __restrict__ grid,
+// Split-BF16 form: FP32 samples and arithmetic; jets_f: the same values as
+// floats.
+__global__ void jets_kernel(const float* __restrict__ fld, int L, const double* __restrict__ grid,
                             double* __restrict__ jets, float* __restrict__ jets_f) {
   const int N = 2 * L;
   const int64_t nv = 2 + (int64_t)(L - 1) * N;
@@ -589,21 +800,49 @@ __global__ void jets_kernel(const R* __restrict__ fld, int L, const double* __re
   else
     node = N + (v - 1);
   const int64_t fs = (int64_t)(L + 1) * N;
-  // arithmetic in the samples' precision (FP32 in the mixed form)
-  const R X0 = (R)grid[4 * node], X1 = (R)grid[4 * node + 1], X2 = (R)grid[4 * node + 2];
-  const R nX = sqrt(X0 * X0 + X1 * X1 + X2 * X2);
+  const float X0 = (float)grid[4 * node], X1 = (float)grid[4 * node + 1], X2 = (float)grid[4 * node + 2];
+  const float nX = sqrt(X0 * X0 + X1 * X1 + X2 * X2);
   for (int i = 0; i < 3; ++i) {
-    const R g0 = fld[(3 + 3 * i) * fs + node], g1 = fld[(4 + 3 * i) * fs + node],
+    const float g0 = fld[(3 + 3 * i) * fs + node], g1 = fld[(4 + 3 * i) * fs + node],
             g2 = fld[(5 + 3 * i) * fs + node];
-    const R c0 = g1 * X2 - g2 * X1, c1 = g2 * X0 - g0 * X2, c2 = g0 * X1 - g1 * X0;
-    const R sc = (c0 * X0 + c1 * X1 + c2 * X2) / nX;
-    const R val[4] = {fld[i * fs + node], c0 - sc * X0, c1 - sc * X1, c2 - sc * X2};
+    const float c0 = g1 * X2 - g2 * X1, c1 = g2 * X0 - g0 * X2, c2 = g0 * X1 - g1 * X0;
+    const float sc = (c0 * X0 + c1 * X1 + c2 * X2) / nX;
+    const float val[4] = {fld[i * fs + node], c0 - sc * X0, c1 - sc * X1, c2 - sc * X2};
     const int64_t slot[4] = {i * 4, 0 * 4 + 1 + i, 1 * 4 + 1 + i, 2 * 4 + 1 + i};
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       jets[slot[k] * nv + v] = (double)val[k];
-      if (jets_f) jets_f[slot[k] * nv + v] = (float)val[k];
+      jets_f[slot[k] * nv + v] = val[k];
     }
+  }
+}
+
+// The same jets in the FP64 form from the nine grid fields of
+// store_velocity_spectra; g x X is tangent by itself (the gradients are
+// angular-momentum images, X . (L f) = 0), so the projection of jets_kernel,
+// which removes a rounding residue, is left out.  FP64-bound otherwise
+// (68 us at L = 512 with it).
+__global__ void __launch_bounds__(128) velocity_jets_kernel(const double* __restrict__ fld, int L,
+                                                            const double* __restrict__ grid,
+                                                            double* __restrict__ jets) {
+  const int N = 2 * L;
+  const int64_t nv = 2 + (int64_t)(L - 1) * N;
+  const int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (v >= nv) return;
+  const int64_t node = v == 0 ? 0 : (v == nv - 1 ? (int64_t)L * N : N + (v - 1));
+  const int64_t fs = (int64_t)(L + 1) * N;
+  const double X0 = grid[4 * node], X1 = grid[4 * node + 1], X2 = grid[4 * node + 2];
+  double f[kVelSpectra];
+#pragma unroll
+  for (int k = 0; k < kVelSpectra; ++k) f[k] = fld[k * fs + node];
+  const double ux = f[0], uy = f[1], uz = f[2], xx = f[3], xy = f[4], yy = f[5], zx = f[6], zy = f[7], zz = f[8];
+  const double g[3][3] = {{xx, xy + uz, zx}, {xy, yy, zy}, {zx + uy, zy - ux, zz}};   // [i][k] = A_k u_i
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    jets[(int64_t)(4 * i) * nv + v] = f[i];
+    jets[(int64_t)(1 + i) * nv + v] = g[i][1] * X2 - g[i][2] * X1;
+    jets[(int64_t)(5 + i) * nv + v] = g[i][2] * X0 - g[i][0] * X2;
+    jets[(int64_t)(9 + i) * nv + v] = g[i][0] * X1 - g[i][1] * X0;
   }
 }
 
@@ -972,16 +1211,16 @@ int check_launch(const char* what) {
 struct cmm_sht {
   int L = 0;
   int precision = CMM_SHT_FP64;
-  cufftHandle ring_fwd = 0, torus_fwd = 0, pad_inv = 0, ring_inv = 0;
-  bool have_plans[4] = {false, false, false, false};
+  cufftHandle ring_fwd = 0, torus_fwd = 0, pad_inv = 0, ring_inv = 0, ring_inv9 = 0;
+  bool have_plans[5] = {false, false, false, false, false};
   // FP64 forward on order-major rows (torus_t_kernel / pad_t_kernel)
   cufftHandle torus_fwd_t = 0, pad_inv_t = 0;
   bool have_tplans[2] = {false, false};
   cmm::DeviceBuffer ct_rings, ct_fine, w_fine, pmm_rings, pmm_fine, ra, rb;
-  // Pbar tables of the FP64 stages (analysis a, synthesis s); plans of one
-  // band-limit may hold the same tables (cmm_sht_share_tables)
+  // tables of the FP64 stages (analysis weights w, synthesis Pbar s); plans
+  // of one band-limit may hold the same tables (cmm_sht_share_tables)
   struct PbarTables {
-    cmm::DeviceBuffer a, s;
+    cmm::DeviceBuffer w, s;
   };
   std::shared_ptr<PbarTables> tab;
   int tab_mode = 0;                 // cmm_sht_set_tables: 0 auto, 1 always, -1 never
@@ -1021,6 +1260,7 @@ cmm_sht::~cmm_sht() {
     if (have_plans[1]) cufftDestroy(torus_fwd);
     if (have_plans[2]) cufftDestroy(pad_inv);
     if (have_plans[3]) cufftDestroy(ring_inv);
+    if (have_plans[4]) cufftDestroy(ring_inv9);
     if (have_tplans[0]) cufftDestroy(torus_fwd_t);
     if (have_tplans[1]) cufftDestroy(pad_inv_t);
     if (have_fplans[0]) cufftDestroy(f_ring_fwd);
@@ -1140,6 +1380,10 @@ int sht_create(int L, cmm_sht** out) {
   r = cufftPlanMany(&p->ring_inv, 1, n2, cin, 1, L + 1, rout, 1, 2 * L, CUFFT_Z2D, kFields * (L + 1));
   if (r != CUFFT_SUCCESS) return fail(cufft_fail(r, "cufftPlanMany(ring_inv)"));
   p->have_plans[3] = true;
+  // and the velocity's kVelSpectra*(L+1) rows in the FP64 form
+  r = cufftPlanMany(&p->ring_inv9, 1, n2, cin, 1, L + 1, rout, 1, 2 * L, CUFFT_Z2D, kVelSpectra * (L + 1));
+  if (r != CUFFT_SUCCESS) return fail(cufft_fail(r, "cufftPlanMany(ring_inv9)"));
+  p->have_plans[4] = true;
   r = cufftPlanMany(&p->torus_fwd_t, 1, n2, tn, 1, 2 * L, tn, 1, 2 * L, CUFFT_Z2Z, L);
   if (r != CUFFT_SUCCESS) return fail(cufft_fail(r, "cufftPlanMany(torus_fwd_t)"));
   p->have_tplans[0] = true;
@@ -1158,9 +1402,8 @@ static int set_streams(cmm_sht* p, cudaStream_t s) {
     cufftResult r = cufftSetStream(h[k], s);
     if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftSetStream");
   }
-  cufftHandle ht[2] = {p->torus_fwd_t, p->pad_inv_t};
-  for (int k = 0; k < 2; ++k) {
-    if (!p->have_tplans[k]) continue;
+  cufftHandle ht[3] = {p->torus_fwd_t, p->pad_inv_t, p->ring_inv9};
+  for (int k = 0; k < 3; ++k) {
     cufftResult r = cufftSetStream(ht[k], s);
     if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftSetStream");
   }
@@ -1185,24 +1428,31 @@ static int ensure_tables(cmm_sht* p, cudaStream_t s, bool* ok) {
   }
   if (cs != cudaStreamCaptureStatusNone) return CMM_OK;
   const int64_t tri = (int64_t)L * (L + 1) / 2;
-  const int na = L + 1, ns = L / 2 + 1;
+  const int ns = L / 2 + 1, npo = (L + 1) / 2;
   int rc;
   auto tab = std::make_shared<cmm_sht::PbarTables>();
-  if ((rc = tab->a.alloc((size_t)tri * na * 8)) || (rc = tab->s.alloc((size_t)tri * ns * 8))) return rc;
-  build_pbar_kernel<<<dim3((na + 127) / 128, L), 128, 0, s>>>(L, na, (const double*)p->ct_fine.p,
-                                                              (const double*)p->pmm_fine.p, 2 * L + 1,
-                                                              (const double*)p->ra.p, (const double*)p->rb.p,
-                                                              false, (double*)tab->a.p);
+  DeviceBuffer po, kp;   // Pbar on the odd fine rings and their weights, for the build only
+  if ((rc = tab->w.alloc((size_t)tri * ns * 8)) || (rc = tab->s.alloc((size_t)tri * ns * 8)) ||
+      (rc = po.alloc((size_t)tri * npo * 8)) || (rc = kp.alloc((size_t)4 * npo * ns * 8)))
+    return rc;
+  const double *ra = (const double*)p->ra.p, *rb = (const double*)p->rb.p, *w = (const double*)p->w_fine.p;
+  build_pbar_kernel<<<dim3((ns + 127) / 128, L), 128, 0, s>>>(L, ns, 0, 1, (const double*)p->ct_rings.p,
+                                                              (const double*)p->pmm_rings.p, L + 1, ra, rb,
+                                                              (double*)tab->s.p);
   if ((rc = check_launch("build_pbar_kernel"))) return rc;
-  build_pbar_kernel<<<dim3((ns + 127) / 128, L), 128, 0, s>>>(L, ns, (const double*)p->ct_rings.p,
-                                                              (const double*)p->pmm_rings.p, L + 1,
-                                                              (const double*)p->ra.p, (const double*)p->rb.p,
-                                                              true, (double*)tab->s.p);
+  build_pbar_kernel<<<dim3((npo + 127) / 128, L), 128, 0, s>>>(L, npo, 1, 2, (const double*)p->ct_fine.p,
+                                                               (const double*)p->pmm_fine.p, 2 * L + 1, ra, rb,
+                                                               (double*)po.p);
   if ((rc = check_launch("build_pbar_kernel"))) return rc;
+  odd_kernel_kernel<<<dim3((ns + 127) / 128, npo, 4), 128, 0, s>>>(L, w, (double*)kp.p);
+  if ((rc = check_launch("odd_kernel_kernel"))) return rc;
+  build_w_kernel<<<dim3((ns + 63) / 64, L, 2 * (((L + 1) / 2 + 31) / 32)), 256, 0, s>>>(
+      L, (const double*)po.p, (const double*)tab->s.p, (const double*)kp.p, w, (double*)tab->w.p);
+  if ((rc = check_launch("build_w_kernel"))) return rc;
   // published only once built: a later call of this plan on another
   // stream, unordered with s, must not read a partly written table
   cudaError_t e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return cuda_fail(e, "build_pbar_kernel");
+  if (e != cudaSuccess) return cuda_fail(e, "build_w_kernel");
   p->tab = std::move(tab);
   *ok = true;
   return CMM_OK;
@@ -1286,6 +1536,13 @@ int sht_forward(cmm_sht* p, const double* samples, double2* out, cudaStream_t s)
   }
   cufftResult r = cufftExecD2Z(p->ring_fwd, (cufftDoubleReal*)samples, (cufftDoubleComplex*)p->spec.p);
   if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftExecD2Z");
+  bool tab;
+  if ((rc = ensure_tables(p, s, &tab))) return rc;
+  if (tab) {
+    analysis_w_kernel<<<dim3(L, (L + kTabBlock - 1) / kTabBlock), kTabBlock * kAnaSlices, 0, s>>>(
+        (const double2*)p->spec.p, L, (const double*)p->tab->w.p, out);
+    return check_launch("analysis_w_kernel");
+  }
   torus_t_kernel<<<g1, b, 0, s>>>((const double2*)p->spec.p, L, (double2*)p->torus.p);
   if ((rc = check_launch("torus_t_kernel"))) return rc;
   r = cufftExecZ2Z(p->torus_fwd_t, (cufftDoubleComplex*)p->torus.p, (cufftDoubleComplex*)p->torus.p,
@@ -1298,13 +1555,6 @@ int sht_forward(cmm_sht* p, const double* samples, double2* out, cudaStream_t s)
   if (L + 1 > 8 * 256) {
     set_last_error("sht_forward: L too large for the analysis kernel");
     return CMM_ERR_UNSUPPORTED;
-  }
-  bool tab;
-  if ((rc = ensure_tables(p, s, &tab))) return rc;
-  if (tab) {
-    analysis_tab_kernel<<<dim3(L, (L + kTabBlock - 1) / kTabBlock), kTabBlock, 0, s>>>(
-        (const double2*)p->pad.p, L, (const double*)p->w_fine.p, (const double*)p->tab->a.p, out);
-    return check_launch("analysis_tab_kernel");
   }
   analysis_kernel<<<L, 256, 0, s>>>((const double2*)p->pad.p, L, (const double*)p->w_fine.p,
                                     (const double*)p->ct_fine.p, (const double*)p->pmm_fine.p,
@@ -1378,29 +1628,65 @@ int sht_inverse(cmm_sht* p, const double2* alm, int nf, double* samples, cudaStr
   return CMM_OK;
 }
 
-// The stream function's 12 velocity/jet fields, their synthesis and the
-// jets at the velocity mesh's vertices.
+// Split-BF16 form: the stream function's 12 velocity/jet fields, their
+// synthesis and the jets at the velocity mesh's vertices.
 static int velocity_from_psi(cmm_sht* p, const cmm_mesh* vm, const double2* psi, double* jets,
                              cudaStream_t s);
+
+static int velocity_fp64(cmm_sht* p, const cmm_mesh* vm, const double2* a, bool lap, double2* psi_out,
+                         double* jets, cudaStream_t s);
 
 int sht_velocity(cmm_sht* p, const cmm_mesh* vm, const double* omega, double2* psi_out,
                  double* jets, cudaStream_t s) {
   const int L = p->L;
   double2* psi = (double2*)p->alm.p;
   int rc;
-  dim3 b(128), g((L + 127) / 128, L);
+  if (omega && (rc = sht_forward(p, omega, psi, s))) return rc;
+  if (!omega) {   // stream function given by the caller
+    psi = psi_out;
+    psi_out = nullptr;
+  }
+  if (p->precision == CMM_SHT_FP64) return velocity_fp64(p, vm, psi, omega != nullptr, psi_out, jets, s);
   if (omega) {
-    if ((rc = sht_forward(p, omega, psi, s))) return rc;
-    dinv_kernel<<<g, b, 0, s>>>(psi, L);
+    dinv_kernel<<<dim3((L + 127) / 128, L), 128, 0, s>>>(psi, L);
     if ((rc = check_launch("dinv_kernel"))) return rc;
     if (psi_out) {
       cudaError_t e = cudaMemcpyAsync(psi_out, psi, (size_t)L * L * sizeof(double2), cudaMemcpyDeviceToDevice, s);
       if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync(psi)");
     }
-  } else {
-    psi = psi_out;  // stream function given by the caller
   }
   return velocity_from_psi(p, vm, psi, jets, s);
+}
+
+// The FP64 form from the analysis a (lap) or the stream function: six
+// Legendre fields, nine ring spectra, the jets.
+static int velocity_fp64(cmm_sht* p, const cmm_mesh* vm, const double2* a, bool lap, double2* psi_out,
+                         double* jets, cudaStream_t s) {
+  const int L = p->L, npair = L / 2 + 1;
+  int rc = set_streams(p, s);
+  if (rc || (rc = ensure_fp64_inverse(p))) return rc;
+  double2 *F = (double2*)p->fields.p, *S = (double2*)p->synth.p;
+  velocity_fields_kernel<<<dim3((L + 127) / 128, L), 128, 0, s>>>(a, L, lap, F);
+  if ((rc = check_launch("velocity_fields_kernel"))) return rc;
+  if (psi_out) {
+    cudaError_t e = cudaMemcpyAsync(psi_out, F, (size_t)L * L * sizeof(double2), cudaMemcpyDeviceToDevice, s);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync(psi)");
+  }
+  bool tab;
+  if ((rc = ensure_tables(p, s, &tab))) return rc;
+  if (tab)
+    synthesis_tab_kernel<3, true><<<dim3(L, (npair + kTabBlock - 1) / kTabBlock, kVelLegendre / 3), kTabBlock, 0, s>>>(
+        F, L, (const double*)p->tab->s.p, S);
+  else
+    synthesis_kernel<kVelLegendre, true><<<dim3(L, (npair + kSynthBlock - 1) / kSynthBlock), kSynthBlock, 0, s>>>(
+        F, L, (const double*)p->ct_rings.p, (const double*)p->pmm_rings.p, (const double*)p->ra.p,
+        (const double*)p->rb.p, S);
+  if ((rc = check_launch("synthesis (velocity)"))) return rc;
+  cufftResult r = cufftExecZ2D(p->ring_inv9, (cufftDoubleComplex*)S, (cufftDoubleReal*)p->samples.p);
+  if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftExecZ2D(velocity)");
+  const int64_t nv = 2 + (int64_t)(L - 1) * 2 * L;
+  velocity_jets_kernel<<<(int)((nv + 127) / 128), 128, 0, s>>>((const double*)p->samples.p, L, vm->view.grid, jets);
+  return check_launch("velocity_jets_kernel");
 }
 
 // Batched form of sht_velocity(p, vm, omega, NULL, jets): the forward
@@ -1530,12 +1816,8 @@ static int velocity_from_psi(cmm_sht* p, const cmm_mesh* vm, const double2* psi,
   if ((rc = check_launch("ladder2_kernel"))) return rc;
   if ((rc = sht_inverse(p, F, kFields, nullptr, s))) return rc;
   const int64_t nv = 2 + (int64_t)(L - 1) * 2 * L;
-  if (p->precision == CMM_SHT_SPLIT_BF16)
-    jets_kernel<float><<<(int)((nv + 127) / 128), 128, 0, s>>>((const float*)p->f_samples.p, L,
-                                                                vm->view.grid, jets, (float*)p->f_jets.p);
-  else
-    jets_kernel<double><<<(int)((nv + 127) / 128), 128, 0, s>>>((const double*)p->samples.p, L,
-                                                                 vm->view.grid, jets, nullptr);
+  jets_kernel<<<(int)((nv + 127) / 128), 128, 0, s>>>((const float*)p->f_samples.p, L, vm->view.grid, jets,
+                                                      (float*)p->f_jets.p);
   return check_launch("jets_kernel");
 }
 
