@@ -50,6 +50,7 @@ struct MeshView {
   const int* root_adj;      // 20 x 3: face across edge ab, bc, ca
   const double* node_n;     // hierarchy nodes x 9: normals n0,n1,n2 (levels 0..level-1)
   const float* node_nf;     // same, FP32, unit normals
+  const float4* coarse_nf;  // node_nf of levels 0 .. min(level, 4)-1, one float4 per normal
   const int* leaf_row;      // (nt) hierarchical leaf -> reference row
   // walk location (locate_row): per row kWalkStride floats -- for each edge
   // (v0v1, v1v2, v2v0) its inward unit normal (FP32) and the row across it
@@ -135,7 +136,7 @@ struct DeviceBuffer {
 
 struct cmm_mesh {
   cmm::MeshView view;
-  cmm::DeviceBuffer verts, tri_v, tri_loc, tri_asm, root, root_f, root_adj, node_n, node_nf, leaf_row,
+  cmm::DeviceBuffer verts, tri_v, tri_loc, tri_asm, root, root_f, root_adj, node_n, node_nf, coarse_nf, leaf_row,
       status, theta, phi, grid, cos_theta, tri_asm_f, tri_loc_f, sh_ab, sh_fm, walk_f, walk_d, jump, ring_n,
       diag_n;
 };

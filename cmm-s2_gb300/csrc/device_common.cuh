@@ -150,18 +150,28 @@ __device__ __forceinline__ float edge_dot(float4 e, float fx, float fy, float fz
   return fmaf(e.x, fx, fmaf(e.y, fy, e.z * fz));
 }
 
-__device__ __forceinline__ bool edge_out(const MeshView& m, int t, int k, float d, double x, double y, double z) {
+// The point of a location, as FP64 values asked for only where the FP32
+// filter cannot decide: here in registers (a fixed-point composition makes
+// them on demand).
+struct PointD {
+  double x, y, z;
+  __device__ __forceinline__ PointD fp64() const { return *this; }
+};
+
+template <class Pt>
+__device__ __forceinline__ bool edge_out(const MeshView& m, int t, int k, float d, const Pt& pt) {
   if (fabsf(d) > kFilter) return d < 0.0f;
   const double* n = m.walk_d + (int64_t)t * kWalkStride + 3 * k;
-  return n[0] * x + n[1] * y + n[2] * z < 0.0;
+  const PointD q = pt.fp64();
+  return n[0] * q.x + n[1] * q.y + n[2] * q.z < 0.0;
 }
 
 // Walk from the jump-table row of q's cube-map cell across the first edge
 // that q lies outside of until q is inside all three (a handful of steps:
 // the cells are smaller than the triangles).  Returns the row, with the
 // three FP32 edge values of the final row in d, or -1 after kWalkMax steps.
-__device__ __forceinline__ int walk_locate(const MeshView& m, double x, double y, double z, float fx, float fy,
-                                           float fz, float* d) {
+template <class Pt>
+__device__ __forceinline__ int walk_locate(const MeshView& m, const Pt& pt, float fx, float fy, float fz, float* d) {
   int t = __ldg(m.jump + jump_cell(m.jump_res, fx, fy, fz));
   for (int it = 0; it < kWalkMax; ++it) {
     const float4* r = reinterpret_cast<const float4*>(m.walk_f + (int64_t)t * kWalkStride);
@@ -169,11 +179,11 @@ __device__ __forceinline__ int walk_locate(const MeshView& m, double x, double y
     d[0] = edge_dot(e0, fx, fy, fz);
     d[1] = edge_dot(e1, fx, fy, fz);
     d[2] = edge_dot(e2, fx, fy, fz);
-    if (edge_out(m, t, 0, d[0], x, y, z))
+    if (edge_out(m, t, 0, d[0], pt))
       t = __float_as_int(e0.w);
-    else if (edge_out(m, t, 1, d[1], x, y, z))
+    else if (edge_out(m, t, 1, d[1], pt))
       t = __float_as_int(e1.w);
-    else if (edge_out(m, t, 2, d[2], x, y, z))
+    else if (edge_out(m, t, 2, d[2], pt))
       t = __float_as_int(e2.w);
     else
       return t;
@@ -186,11 +196,19 @@ __device__ __forceinline__ int walk_locate(const MeshView& m, double x, double y
 // not ended after kWalkMax steps.  Both are exact containment tests, so
 // they agree except for queries within rounding distance of an edge,
 // where either neighbour contains the query.
+template <class Pt>
+__device__ __forceinline__ int locate_row_f(const MeshView& m, const Pt& pt, float fx, float fy, float fz) {
+  if (m.jump) {
+    float d[3];
+    const int t = walk_locate(m, pt, fx, fy, fz, d);
+    if (t >= 0) return t;
+  }
+  const PointD q = pt.fp64();
+  return locate_descent(m, q.x, q.y, q.z);
+}
+
 __device__ __forceinline__ int locate_row(const MeshView& m, double x, double y, double z) {
-  if (!m.jump) return locate_descent(m, x, y, z);
-  float d[3];
-  const int t = walk_locate(m, x, y, z, to_f32_trunc(x), to_f32_trunc(y), to_f32_trunc(z), d);
-  return t >= 0 ? t : locate_descent(m, x, y, z);
+  return locate_row_f(m, PointD{x, y, z}, to_f32_trunc(x), to_f32_trunc(y), to_f32_trunc(z));
 }
 
 struct Bcc {
@@ -240,11 +258,12 @@ __device__ __forceinline__ Split split_of(const Bcc& b) {
 // the sum of their FP32 error bounds (s_i kFilter); otherwise -- and when
 // the walk fell back to the descent -- the FP64 barycentrics R q decide,
 // with split_of's rule.  Either way the choice is split_of(R q)'s.
-__device__ __forceinline__ int locate_split(const MeshView& m, double x, double y, double z, Split* sp) {
+template <class Pt>
+__device__ __forceinline__ int locate_split(const MeshView& m, const Pt& pt, float fx, float fy, float fz, Split* sp) {
   int t = -1;
   if (m.jump) {
     float d[3];
-    t = walk_locate(m, x, y, z, to_f32_trunc(x), to_f32_trunc(y), to_f32_trunc(z), d);
+    t = walk_locate(m, pt, fx, fy, fz, d);
     if (t >= 0) {
       const float4 sc = __ldg(reinterpret_cast<const float4*>(m.walk_f + (int64_t)t * kWalkStride) + 3);
       const float b0 = sc.x * d[1], b1 = sc.y * d[2], b2 = sc.z * d[0];
@@ -257,12 +276,13 @@ __device__ __forceinline__ int locate_split(const MeshView& m, double x, double 
       }
     }
   }
-  if (t < 0) t = locate_descent(m, x, y, z);
+  const PointD q = pt.fp64();
+  if (t < 0) t = locate_descent(m, q.x, q.y, q.z);
   const double* L = m.tri_loc + (int64_t)t * kLocStride;
   double R[9];
 #pragma unroll
   for (int k = 0; k < 9; ++k) R[k] = __ldg(L + k);
-  *sp = split_of(bcc_of(R, x, y, z));
+  *sp = split_of(bcc_of(R, q.x, q.y, q.z));
   return t;
 }
 

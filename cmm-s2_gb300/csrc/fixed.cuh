@@ -1,0 +1,88 @@
+// Fixed-point arithmetic on the integer pipes, for the points of a
+// composition through map forms.
+//
+// GB300 runs one warp FP64 instruction in the time of 64 issue slots of a
+// scheduler, so a product of two 60-bit fixed-point numbers (three 32 x 32 ->
+// 64 bit multiply-adds) costs a small fraction of an FP64 multiply-add, and
+// points and forms of a map are O(1) with absolute accuracy all that matters:
+// 2^-58 steps carry them more exactly than FP64's 2^-53 roundings.
+//
+// A number is an int64 in units of 2^-58 or, to be multiplied, two limbs
+// h 2^-29 + l 2^-59 with |l| < 2^30.  A product of limbs is h h' (units
+// 2^-58) plus h l' + l h' (2^-88); l l' (below 2^-58) is dropped.
+#pragma once
+#include <cuda_runtime.h>
+
+#include "ff.cuh"
+
+namespace cmm {
+namespace dev {
+
+constexpr double kFxUnit = 3.469446951953614e-18;   // 2^-58
+
+struct Limbs {
+  int h, l;
+};
+
+// X (units of 2^-58), |X| < 4 in value
+__device__ __forceinline__ Limbs fx_limbs(long long X) {
+  return Limbs{(int)(X >> 29), (int)(((unsigned)X << 1) & 0x3fffffffu)};
+}
+
+// The running sums of products: hi in units of 2^-58, lo in 2^-88.  Within
+// |lo| < 2^63 for up to 12 cross products of |h| < 2^30 and |l| < 2^30 whose
+// h are not all at their bound (|point|^2 < 1.4, |form entry| < 2).
+struct FxSum {
+  long long hi, lo;
+  __device__ __forceinline__ void add(Limbs a, Limbs b) {
+    hi += (long long)a.h * b.h;
+    lo += (long long)a.h * b.l;
+    lo += (long long)a.l * b.h;
+  }
+  __device__ __forceinline__ long long value() const { return hi + (lo >> 30); }
+};
+
+// A form entry |q| < 2 as limbs (2^-59 steps, toward zero), from the
+// double's bits; where |q| >= 2 or q is not finite the sign bit of `bad` is
+// set (the limbs are then meaningless).
+__device__ __forceinline__ Limbs fx_entry(double q, int& bad) {
+  const int hi = __double2hiint(q);
+  const unsigned lo = (unsigned)__double2loint(q);
+  const int e = 1023 - (int)(((unsigned)hi << 1) >> 21);   // right shift of the 53-bit significand << 7
+  bad |= e;
+  const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;
+  unsigned long long T = ((((unsigned long long)mh) << 32) | lo) << 7;
+  asm("shr.u64 %0, %1, %2;" : "=l"(T) : "l"(T), "r"(e));   // 0 from a shift of 64 on
+  const int sg = (hi >> 31) | 1;
+  return Limbs{(int)(T >> 30) * sg, (int)((unsigned)T & 0x3fffffffu) * sg};
+}
+
+// x, |x| < 16, in units of 2^-58 (toward zero)
+__device__ __forceinline__ long long fx_of(double x) {
+  const int hi = __double2hiint(x);
+  const unsigned lo = (unsigned)__double2loint(x);
+  const int e = 1028 - (int)(((unsigned)hi << 1) >> 21);   // right shift of the 53-bit significand << 11
+  const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;
+  unsigned long long T = ((((unsigned long long)mh) << 32) | lo) << 11;
+  asm("shr.u64 %0, %1, %2;" : "=l"(T) : "l"(T), "r"(e));
+  return hi < 0 ? -(long long)T : (long long)T;
+}
+
+// X as a float: its high word, rounded (within 2^-25 of |x| <= 1)
+__device__ __forceinline__ float fx_f32(long long X) { return __fmul_rn((float)(int)(X >> 32), 1.4901161193847656e-08f); }
+
+// X (|x| < 16) as a float-float: 26 + 23 + 15 bits converted exactly, the
+// first two added without error, the last joining the low part.
+__device__ __forceinline__ ff fx_ff(long long X) {
+  const float a = __fmul_rn((float)(int)(X >> 38), 9.5367431640625e-07f);   // 2^-20 units
+  // 0x4b000000 | n is the float 2^23 + n for n < 2^23
+  const float b = fmaf(__uint_as_float(0x4b000000u | ((unsigned)(X >> 15) & 0x7fffffu)), 1.1368683772161603e-13f,
+                       -9.5367431640625e-07f);                               // 2^-43 units
+  const float c = fmaf(__uint_as_float(0x4b000000u | ((unsigned)X & 0x7fffu)), 3.469446951953614e-18f,
+                       -2.9103830456733704e-11f);                            // 2^-58 units
+  const float s = __fadd_rn(a, b);
+  return ff{s, __fadd_rn(__fsub_rn(b, __fsub_rn(s, a)), c)};
+}
+
+}  // namespace dev
+}  // namespace cmm

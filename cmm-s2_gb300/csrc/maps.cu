@@ -27,6 +27,7 @@
 #include "dd.cuh"
 #include "device_common.cuh"
 #include "ff.cuh"
+#include "fixed.cuh"
 
 namespace cmm {
 
@@ -35,21 +36,20 @@ using namespace dev;
 namespace {
 
 constexpr int kBlock = 256;
-// The composition normalises the point every kNormEvery submaps (a power
-// of two); queries whose FP32 squared norm is outside [1/4, 4] are
-// normalised first, so the unnormalised chain stays far from overflow.
+// The composition through coefficient records normalises the point every
+// kNormEvery submaps (a power of two); queries whose FP32 squared norm is
+// outside [1/4, 4] are normalised first, so the unnormalised chain stays far
+// from overflow.
 constexpr int kNormEvery = 8;
 // default register budgets of the compositions, as resident 256-thread
-// blocks per SM (measured at level 7, 2^24 queries, 8 submaps, map forms,
-// cell order, normalising every fourth submap: Jacobians 12.8 / 13.6 /
-// 13.2 ms at 4 / 3 / 2 blocks; points only 7.5 ms at 4 or 6 blocks, and
-// 10.2 against 13.5 ms in caller order); the autotuner may set others
+// blocks per SM; the autotuner may set others
 constexpr int kComposeJacBlocks = 4;
-// with the low floats of the forms' split loaded (fewer live values):
-// 10.83 / 11.02 / 11.59 ms at 3 / 4 / 2 blocks, same workload; normalising
-// every eighth submap, 10.56 / 10.72 / 11.93 ms
-constexpr int kComposeJacBlocksFF = 3;
+constexpr int kComposeJacBlocksFF = 4;   // with the forms' low floats
 constexpr int kComposeBlocks = 4;
+constexpr int kFormsCallerBlocks = 3;   // points only through forms, in caller order
+// Submaps listed in the kernel parameters of the usual calls (768 bytes);
+// longer lists take the 24 KB form, whose upload alone costs microseconds.
+constexpr int kShortList = 32;
 
 // Submap lists: by value in the kernel parameters (host calls), or a
 // device table whose length comes from a device-driven step's state.
@@ -58,10 +58,11 @@ constexpr int kComposeBlocks = 4;
 // A submap with a form record may also have the low floats of its
 // float-float split (the Jacobian pushes then load them instead of
 // extracting them from the doubles on the integer pipe).
+template <int N>
 struct SubmapPtrs {
-  const double* p[CMM_MAX_SUBMAPS];
-  const double* f[CMM_MAX_SUBMAPS];
-  const float* g[CMM_MAX_SUBMAPS];
+  const double* p[N];
+  const double* f[N];
+  const float* g[N];
   int S;
   __device__ __forceinline__ int count() const { return S; }
   __device__ __forceinline__ const double* at(int s, int) const { return p[s]; }
@@ -116,7 +117,7 @@ struct Pushes {
   }
 };
 
-// 2^m as a double, from its bit pattern (0 <= m <= kNormEvery here)
+// 2^m as a double, from its bit pattern
 __device__ __forceinline__ double pow2(int m) { return __longlong_as_double((long long)(1023 + m) << 52); }
 
 __global__ void __launch_bounds__(kBlock) locate_kernel(MeshView m, const double* __restrict__ q,
@@ -376,12 +377,188 @@ __global__ void to_f32_kernel(const double* __restrict__ a, int64_t n, float* __
   if (i < n) b[i] = (float)a[i];
 }
 
+// One submap from its coefficient record at p, in triangle t: the
+// un-normalised image P and, with JAC, the two pushes (half derivatives).
+template <bool JAC>
+__device__ __forceinline__ void record_eval(const MeshView& m, const double* __restrict__ recs, int t,
+                                            const double* p, Pushes w, double* P) {
+  double Lr[13];
+  load_loc(m, t, Lr);
+  const Bcc b = bcc_of(Lr, p[0], p[1], p[2]);
+  const Split sp = split_of(b);
+  const Gam g = gamma_of(Lr, b, sp);
+  const double* rec = recs + (int64_t)t * kCoeffStride3;
+  if (JAC) {
+            // The patch is the quadratic form P_c = gamma^T M_c gamma of the
+            // symmetric ordinate matrix M_c; its half gradient M_c gamma (FP64)
+            // gives the value with three more operations per component and
+            // serves the two tangent pushes: half derivatives along the
+            // barycentric directions dgamma = T Minv w, formed in float-float
+            // from the FP64 location record.
+            // the pushes' sub-triangle barycentric directions, ff values 6..11
+            // of the thread's shared-memory slots
+            {
+              ff d1[3], d2[3];
+              // the inverse vertex rows re-read (L1) rather than held in
+              // registers from the value path
+              const double* Lp = m.tri_loc + (int64_t)t * kLocStride;
+    #pragma unroll
+              for (int r = 0; r < 3; ++r) {
+                const ff m0 = ff_of(__ldg(Lp + 3 * r)), m1 = ff_of(__ldg(Lp + 3 * r + 1)),
+                         m2 = ff_of(__ldg(Lp + 3 * r + 2));
+                d1[r] = ff_dot3(m0, w.get(0), m1, w.get(1), m2, w.get(2));
+                d2[r] = ff_dot3(m0, w.get(3), m1, w.get(4), m2, w.get(5));
+              }
+              const ff en = ff_of(edge_norm(Lr, sp.hi, sp.mid)), ec = ff_of(Lr[9]);
+              const ff l1 = pick_ff(d1, sp.lo), m1 = pick_ff(d1, sp.mid), h1 = pick_ff(d1, sp.hi);
+              const ff l2 = pick_ff(d2, sp.lo), m2 = pick_ff(d2, sp.mid), h2 = pick_ff(d2, sp.hi);
+              w.set(6, ff_sub(h1, m1));
+              w.set(7, ff_mul(en, ff_sub(m1, l1)));
+              w.set(8, ff_mul(ec, l1));
+              w.set(9, ff_sub(h2, m2));
+              w.set(10, ff_mul(en, ff_sub(m2, l2)));
+              w.set(11, ff_mul(ec, l2));
+            }
+            const int* id = kSplitOrd[sp.lo][sp.hi];
+    #pragma unroll
+            for (int c = 0; c < 3; ++c) {
+              double o[6];
+    #pragma unroll
+              for (int k = 0; k < 6; ++k) o[k] = __ldg(rec + 3 * id[k] + c);
+              const double pV = g.V * o[0] + g.E * o[3] + g.C * o[5];
+              const double pE = g.E * o[1] + g.V * o[3] + g.C * o[4];
+              const double pC = g.C * o[2] + g.E * o[4] + g.V * o[5];
+              P[c] = g.V * pV + g.E * pE + g.C * pC;
+              const ff fV = ff_of(pV), fE = ff_of(pE), fC = ff_of(pC);
+              w.set(c, ff_dot3(fV, w.get(6), fE, w.get(7), fC, w.get(8)));
+              w.set(3 + c, ff_dot3(fV, w.get(9), fE, w.get(10), fC, w.get(11)));
+            }
+  } else {
+    Ords<3> o;
+    load_ords<3>(rec, sp, o);
+    sbb<3>(o, g, P);
+  }
+}
+
+// One submap from its map form: P_c = p^T Q_c p of the sub-triangle's
+// quadratic form (24 FP64 operations for the three components) and the
+// pushes' half derivatives (Q_c p) . w in float-float.  q: the form's 18
+// doubles; g (FF): the low floats of their split, else converted here to the
+// same pairs.  One component at a time: unrolled, the three copies overflow
+// the instruction cache (a quarter of the issue slots lost).
+template <bool FF>
+__device__ __forceinline__ void form_push(const double* __restrict__ q, const float* __restrict__ g, const double* p,
+                                          Pushes w, double* P) {
+  const double2* qf = reinterpret_cast<const double2*>(q);
+  const float2* qg = reinterpret_cast<const float2*>(g);
+  const double xx = p[0] * p[0], yy = p[1] * p[1], zz = p[2] * p[2];
+  const double xy = p[0] * p[1], xz = p[0] * p[2], yz = p[1] * p[2];
+  const ff u0 = ff_of(p[0]), u1 = ff_of(p[1]), u2 = ff_of(p[2]);
+  const ff a0 = w.get(0), a1 = w.get(1), a2 = w.get(2), c0 = w.get(3), c1 = w.get(4), c2 = w.get(5);
+#pragma unroll 1
+  for (int c = 0; c < 3; ++c) {
+    const double2 q01 = __ldg(qf + 3 * c), q23 = __ldg(qf + 3 * c + 1), q45 = __ldg(qf + 3 * c + 2);
+    const double v = q01.x * xx + q01.y * yy + q23.x * zz + q23.y * xy + q45.x * xz + q45.y * yz;
+    ff Q00, Q11, Q22, Q01, Q02, Q12;
+    if (FF) {   // the stored low floats; the high floats from the doubles' bits
+      const float2 ga = __ldg(qg + 3 * c), gb = __ldg(qg + 3 * c + 1), gc = __ldg(qg + 3 * c + 2);
+      Q00 = ff{ff_hi(q01.x), ga.x};
+      Q11 = ff{ff_hi(q01.y), ga.y};
+      Q22 = ff{ff_hi(q23.x), gb.x};
+      Q01 = ff{__fmul_rn(0.5f, ff_hi(q23.y)), gb.y};
+      Q02 = ff{__fmul_rn(0.5f, ff_hi(q45.x)), gc.x};
+      Q12 = ff{__fmul_rn(0.5f, ff_hi(q45.y)), gc.y};
+    } else {
+      Q00 = ff_of(q01.x);
+      Q11 = ff_of(q01.y);
+      Q22 = ff_of(q23.x);
+      const ff h01 = ff_of(q23.y), h02 = ff_of(q45.x), h12 = ff_of(q45.y);
+      Q01 = ff{__fmul_rn(0.5f, h01.h), __fmul_rn(0.5f, h01.l)};
+      Q02 = ff{__fmul_rn(0.5f, h02.h), __fmul_rn(0.5f, h02.l)};
+      Q12 = ff{__fmul_rn(0.5f, h12.h), __fmul_rn(0.5f, h12.l)};
+    }
+    const ff g0 = ff_dot3(Q00, u0, Q01, u1, Q02, u2);
+    const ff g1 = ff_dot3(Q01, u0, Q11, u1, Q12, u2);
+    const ff g2 = ff_dot3(Q02, u0, Q12, u1, Q22, u2);
+    w.set(c, ff_dot3(g0, a0, g1, a1, g2, a2));
+    w.set(3 + c, ff_dot3(g0, c0, g1, c1, g2, c2));
+    P[0] = c == 0 ? v : P[0];
+    P[1] = c == 1 ? v : P[1];
+    P[2] = c == 2 ? v : P[2];
+  }
+}
+
+// The pushes brought to the normalised point p: their components along p
+// removed, scaled by sc.
+__device__ __forceinline__ void project_pushes(const double* p, double scale, Pushes w) {
+  const ff sc = ff_of(scale);
+  const ff u0 = ff_of(p[0]), u1 = ff_of(p[1]), u2 = ff_of(p[2]);
+  const ff d1 = ff_dot3(u0, w.get(0), u1, w.get(1), u2, w.get(2));
+  const ff d2 = ff_dot3(u0, w.get(3), u1, w.get(4), u2, w.get(5));
+  const ff u[3] = {u0, u1, u2};
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    w.set(c, ff_mul(ff_sub(w.get(c), ff_mul(u[c], d1)), sc));
+    w.set(3 + c, ff_mul(ff_sub(w.get(3 + c), ff_mul(u[c], d2)), sc));
+  }
+}
+
+// A query's point, normalised first where its FP32 squared norm is outside
+// [1/4, 4]; false where it is not finite.
+__device__ __forceinline__ bool load_query(const double* __restrict__ q, int64_t i, double* p) {
+  p[0] = q[3 * i];
+  p[1] = q[3 * i + 1];
+  p[2] = q[3 * i + 2];
+  const float f0 = to_f32_trunc(p[0]), f1 = to_f32_trunc(p[1]), f2 = to_f32_trunc(p[2]);
+  const float n2 = f0 * f0 + f1 * f1 + f2 * f2;
+  if (!(n2 > 0.25f && n2 < 4.f)) {   // also NaN / inf
+    const double inv = rsqrt(p[0] * p[0] + p[1] * p[1] + p[2] * p[2]);
+    p[0] *= inv;
+    p[1] *= inv;
+    p[2] *= inv;
+  }
+  return finite3(p[0], p[1], p[2]);
+}
+
+// The outputs of a query without a finite image: NaN points and Jacobians,
+// ids -1 from submap s (the first not evaluated) on.
+template <bool JAC>
+__device__ __forceinline__ void store_nan(const MeshView& m, int64_t i, int64_t n, int s, int S,
+                                          double* __restrict__ out, int32_t* __restrict__ tri,
+                                          int32_t* __restrict__ tri_all, double* __restrict__ jac) {
+  flag(m, CMM_FLAG_NONFINITE);
+  out[3 * i] = out[3 * i + 1] = out[3 * i + 2] = nan("");
+  if (tri && s == S - 1) tri[i] = -1;
+  if (tri_all)
+    for (; s >= 0; --s) tri_all[(int64_t)s * n + i] = -1;
+  if (JAC)
+    for (int k = 0; k < 9; ++k) jac[9 * i + k] = nan("");
+}
+
+// The Jacobian from the pushes and the tangent basis at the query (formed
+// again from q: cheaper than keeping it in registers across the submaps).
+__device__ __forceinline__ void store_jacobian(const double* __restrict__ q, int64_t i, Pushes w,
+                                               double* __restrict__ jac) {
+  const double q0[3] = {q[3 * i], q[3 * i + 1], q[3 * i + 2]};
+  ff t1[3], t2[3];
+  tangent_basis_ff(q0, t1, t2);
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+#pragma unroll
+    for (int b2 = 0; b2 < 3; ++b2)
+      jac[9 * i + 3 * a + b2] = ff_to_double(ff_dot2(w.get(a), t1[b2], w.get(3 + a), t2[b2]));
+}
+
+// Composition in FP64 with the Jacobian's pushes in float-float: through
+// coefficient records and, with JAC, through map forms.  (The fixed-point
+// evaluation of compose_forms_kernel does not pay with Jacobians: the pushes
+// fill the issue slots that it takes; 2.63 against 2.42 ms per 2^22 queries.)
+// FF: every submap with a form record also has the low floats of its split.
 // perm (nullable): process the queries in this order (grouped by coarse
 // cell, cmm_query_order) so that neighbouring threads gather neighbouring
 // records; every query's own arithmetic and output slot are unchanged.
 // MINB: resident 256-thread blocks per SM the register allocation must
-// allow (the register budget; cmm_mesh_set_variant).  FF: every submap
-// with a form record also has the low floats of its float-float split.
+// allow (the register budget; cmm_mesh_set_variant).
 template <bool JAC, class Src, int MINB, bool FF = false>
 __global__ void __launch_bounds__(kBlock, MINB) compose_kernel(MeshView m, Src cp,
                                                          const double* __restrict__ q, int64_t n,
@@ -390,6 +567,12 @@ __global__ void __launch_bounds__(kBlock, MINB) compose_kernel(MeshView m, Src c
                                                          int32_t* __restrict__ tri_all,
                                                          double* __restrict__ jac,
                                                          const int32_t* __restrict__ perm) {
+  // Jacobian: two tangent vectors pushed through the chain in float-float
+  // on the FP32 pipe (points, location predicates, barycentrics and patch
+  // values stay FP64).  They live in shared memory, [value][thread], not in
+  // registers: with them the loop exceeds the register budget of four
+  // resident blocks and spills to local memory, whose traffic thrashes the
+  // L1 that the gathers need.
   __shared__ float push_smem[JAC ? 24 * kBlock : 1];
   const int S = cp.count();
   for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n;
@@ -399,34 +582,11 @@ __global__ void __launch_bounds__(kBlock, MINB) compose_kernel(MeshView m, Src c
       flag(m, CMM_FLAG_INDEX);
       continue;
     }
-    double p[3] = {q[3 * i], q[3 * i + 1], q[3 * i + 2]};
-    {
-      const float f0 = to_f32_trunc(p[0]), f1 = to_f32_trunc(p[1]), f2 = to_f32_trunc(p[2]);
-      const float n2 = f0 * f0 + f1 * f1 + f2 * f2;
-      if (!(n2 > 0.25f && n2 < 4.f)) {   // also NaN / inf: then the check below flags it
-        const double inv = rsqrt(p[0] * p[0] + p[1] * p[1] + p[2] * p[2]);
-        p[0] *= inv;
-        p[1] *= inv;
-        p[2] *= inv;
-      }
-    }
-    if (!finite3(p[0], p[1], p[2])) {
-      flag(m, CMM_FLAG_NONFINITE);
-      out[3 * i] = out[3 * i + 1] = out[3 * i + 2] = nan("");
-      if (tri) tri[i] = -1;
-      if (tri_all)
-        for (int s = 0; s < S; ++s) tri_all[(int64_t)s * n + i] = -1;
-      if (JAC)
-        for (int k = 0; k < 9; ++k) jac[9 * i + k] = nan("");
+    double p[3];
+    if (!load_query(q, i, p)) {
+      store_nan<JAC>(m, i, n, S - 1, S, out, tri, tri_all, jac);
       continue;
     }
-    // Jacobian: two tangent vectors pushed through the chain in
-    // float-float on the FP32 pipe (the points, the location predicates,
-    // the barycentrics and the patch values stay FP64)
-    // The pushes live in shared memory, [value][thread], not in
-    // registers: with them the loop exceeds the register budget of four
-    // resident blocks and spills to local memory, whose traffic thrashes
-    // the L1 that the gathers need.
     Pushes w{push_smem + threadIdx.x, (int)blockDim.x};
     int since = 0;   // submaps pushed since the last normalisation
     if (JAC) {   // pushed from the tangent basis at q
@@ -440,124 +600,21 @@ __global__ void __launch_bounds__(kBlock, MINB) compose_kernel(MeshView m, Src c
     }
     for (int s = S - 1; s >= 0; --s) {
       double P[3];
-      const double* fr = cp.form(s, S);
-      if (fr) {
-        // map-form record: P_c = p^T Q_c p of the sub-triangle's quadratic
-        // form (24 FP64 operations for the three components); the half
-        // derivative along w is (Q_c p) . w, formed in float-float
-        Split sp;
-        const int t = locate_split(m, p[0], p[1], p[2], &sp);
-        if (s == S - 1 && tri) tri[i] = t;
-        if (tri_all) tri_all[(int64_t)s * n + i] = t;
-        const double2* qf =
-            reinterpret_cast<const double2*>(fr + (int64_t)t * kFormStride + 18 * kSubIndex[sp.lo][sp.hi]);
-        const double xx = p[0] * p[0], yy = p[1] * p[1], zz = p[2] * p[2];
-        const double xy = p[0] * p[1], xz = p[0] * p[2], yz = p[1] * p[2];
-        if (JAC) {
-          const ff u0 = ff_of(p[0]), u1 = ff_of(p[1]), u2 = ff_of(p[2]);
-          const ff a0 = w.get(0), a1 = w.get(1), a2 = w.get(2), c0 = w.get(3), c1 = w.get(4), c2 = w.get(5);
-          const float2* qg =
-              FF ? reinterpret_cast<const float2*>(cp.form_ff(s, S) + (int64_t)t * kFormFFStride +
-                                                   18 * kSubIndex[sp.lo][sp.hi])
-                 : nullptr;
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            const double2 q01 = __ldg(qf + 3 * c), q23 = __ldg(qf + 3 * c + 1), q45 = __ldg(qf + 3 * c + 2);
-            P[c] = q01.x * xx + q01.y * yy + q23.x * zz + q23.y * xy + q45.x * xz + q45.y * yz;
-            ff Q00, Q11, Q22, Q01, Q02, Q12;
-            if (FF) {   // the stored low floats; the high floats from the doubles' bits
-              const float2 ga = __ldg(qg + 3 * c), gb = __ldg(qg + 3 * c + 1), gc = __ldg(qg + 3 * c + 2);
-              Q00 = ff{ff_hi(q01.x), ga.x};
-              Q11 = ff{ff_hi(q01.y), ga.y};
-              Q22 = ff{ff_hi(q23.x), gb.x};
-              Q01 = ff{__fmul_rn(0.5f, ff_hi(q23.y)), gb.y};
-              Q02 = ff{__fmul_rn(0.5f, ff_hi(q45.x)), gc.x};
-              Q12 = ff{__fmul_rn(0.5f, ff_hi(q45.y)), gc.y};
-            } else {   // the same pairs converted here
-              Q00 = ff_of(q01.x);
-              Q11 = ff_of(q01.y);
-              Q22 = ff_of(q23.x);
-              const ff h01 = ff_of(q23.y), h02 = ff_of(q45.x), h12 = ff_of(q45.y);
-              Q01 = ff{__fmul_rn(0.5f, h01.h), __fmul_rn(0.5f, h01.l)};
-              Q02 = ff{__fmul_rn(0.5f, h02.h), __fmul_rn(0.5f, h02.l)};
-              Q12 = ff{__fmul_rn(0.5f, h12.h), __fmul_rn(0.5f, h12.l)};
-            }
-            const ff g0 = ff_dot3(Q00, u0, Q01, u1, Q02, u2);
-            const ff g1 = ff_dot3(Q01, u0, Q11, u1, Q12, u2);
-            const ff g2 = ff_dot3(Q02, u0, Q12, u1, Q22, u2);
-            w.set(c, ff_dot3(g0, a0, g1, a1, g2, a2));
-            w.set(3 + c, ff_dot3(g0, c0, g1, c1, g2, c2));
-          }
-          ++since;
-        } else {
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            const double2 q01 = __ldg(qf + 3 * c), q23 = __ldg(qf + 3 * c + 1), q45 = __ldg(qf + 3 * c + 2);
-            P[c] = q01.x * xx + q01.y * yy + q23.x * zz + q23.y * xy + q45.x * xz + q45.y * yz;
-          }
-        }
-      } else {
-      const int t = locate_row(m, p[0], p[1], p[2]);
+      const double* fr = JAC ? cp.form(s, S) : nullptr;
+      const PointD pt{p[0], p[1], p[2]};
+      const float fx = to_f32_trunc(p[0]), fy = to_f32_trunc(p[1]), fz = to_f32_trunc(p[2]);
+      Split sp;
+      const int t = fr ? locate_split(m, pt, fx, fy, fz, &sp) : locate_row_f(m, pt, fx, fy, fz);
       if (s == S - 1 && tri) tri[i] = t;
       if (tri_all) tri_all[(int64_t)s * n + i] = t;
-      double Lr[13];
-      load_loc(m, t, Lr);
-      const Bcc b = bcc_of(Lr, p[0], p[1], p[2]);
-      const Split sp = split_of(b);
-      const Gam g = gamma_of(Lr, b, sp);
-      const double* rec = cp.at(s, S) + (int64_t)t * kCoeffStride3;
-      if (JAC) {
-        // The patch is the quadratic form P_c = gamma^T M_c gamma of the
-        // symmetric ordinate matrix M_c; its half gradient M_c gamma (FP64)
-        // gives the value with three more operations per component and
-        // serves the two tangent pushes: half derivatives along the
-        // barycentric directions dgamma = T Minv w, formed in float-float
-        // from the FP64 location record.
-        // the pushes' sub-triangle barycentric directions, ff values 6..11
-        // of the thread's shared-memory slots
-        {
-          ff d1[3], d2[3];
-          // the inverse vertex rows re-read (L1) rather than held in
-          // registers from the value path
-          const double* Lp = m.tri_loc + (int64_t)t * kLocStride;
-#pragma unroll
-          for (int r = 0; r < 3; ++r) {
-            const ff m0 = ff_of(__ldg(Lp + 3 * r)), m1 = ff_of(__ldg(Lp + 3 * r + 1)),
-                     m2 = ff_of(__ldg(Lp + 3 * r + 2));
-            d1[r] = ff_dot3(m0, w.get(0), m1, w.get(1), m2, w.get(2));
-            d2[r] = ff_dot3(m0, w.get(3), m1, w.get(4), m2, w.get(5));
-          }
-          const ff en = ff_of(edge_norm(Lr, sp.hi, sp.mid)), ec = ff_of(Lr[9]);
-          const ff l1 = pick_ff(d1, sp.lo), m1 = pick_ff(d1, sp.mid), h1 = pick_ff(d1, sp.hi);
-          const ff l2 = pick_ff(d2, sp.lo), m2 = pick_ff(d2, sp.mid), h2 = pick_ff(d2, sp.hi);
-          w.set(6, ff_sub(h1, m1));
-          w.set(7, ff_mul(en, ff_sub(m1, l1)));
-          w.set(8, ff_mul(ec, l1));
-          w.set(9, ff_sub(h2, m2));
-          w.set(10, ff_mul(en, ff_sub(m2, l2)));
-          w.set(11, ff_mul(ec, l2));
-        }
-        const int* id = kSplitOrd[sp.lo][sp.hi];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          double o[6];
-#pragma unroll
-          for (int k = 0; k < 6; ++k) o[k] = __ldg(rec + 3 * id[k] + c);
-          const double pV = g.V * o[0] + g.E * o[3] + g.C * o[5];
-          const double pE = g.E * o[1] + g.V * o[3] + g.C * o[4];
-          const double pC = g.C * o[2] + g.E * o[4] + g.V * o[5];
-          P[c] = g.V * pV + g.E * pE + g.C * pC;
-          const ff fV = ff_of(pV), fE = ff_of(pE), fC = ff_of(pC);
-          w.set(c, ff_dot3(fV, w.get(6), fE, w.get(7), fC, w.get(8)));
-          w.set(3 + c, ff_dot3(fV, w.get(9), fE, w.get(10), fC, w.get(11)));
-        }
-        ++since;
+      if (fr) {
+        const int sub = 18 * kSubIndex[sp.lo][sp.hi];
+        form_push<FF>(fr + (int64_t)t * kFormStride + sub, FF ? cp.form_ff(s, S) + (int64_t)t * kFormFFStride + sub : nullptr,
+                      p, w, P);
       } else {
-        Ords<3> o;
-        load_ords<3>(rec, sp, o);
-        sbb<3>(o, g, P);
+        record_eval<JAC>(m, cp.at(s, S), t, p, w, P);
       }
-      }
+      ++since;
       // Location, barycentrics and sub-triangle choice are invariant under
       // p -> lambda p (lambda > 0) and the patch is homogeneous of degree 2,
       // so the projection onto the sphere can wait: normalising every
@@ -579,35 +636,156 @@ __global__ void __launch_bounds__(kBlock, MINB) compose_kernel(MeshView m, Src c
       p[1] = P[1] * inv_n;
       p[2] = P[2] * inv_n;
       if (JAC) {
-        const ff sc = ff_of(inv_n * pow2(since));
+        project_pushes(p, inv_n * pow2(since), w);
         since = 0;
-        const ff u0 = ff_of(p[0]), u1 = ff_of(p[1]), u2 = ff_of(p[2]);
-        const ff d1 = ff_dot3(u0, w.get(0), u1, w.get(1), u2, w.get(2));
-        const ff d2 = ff_dot3(u0, w.get(3), u1, w.get(4), u2, w.get(5));
-        const ff u[3] = {u0, u1, u2};
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          w.set(c, ff_mul(ff_sub(w.get(c), ff_mul(u[c], d1)), sc));
-          w.set(3 + c, ff_mul(ff_sub(w.get(3 + c), ff_mul(u[c], d2)), sc));
-        }
       }
     }
     if (!finite3(p[0], p[1], p[2])) flag(m, CMM_FLAG_NONFINITE);
     out[3 * i] = p[0];
     out[3 * i + 1] = p[1];
     out[3 * i + 2] = p[2];
-    if (JAC) {
-      // the basis again, from q re-read (cheaper than keeping it in
-      // registers across the submap loop)
-      const double q0[3] = {q[3 * i], q[3 * i + 1], q[3 * i + 2]};
-      ff t1[3], t2[3];
-      tangent_basis_ff(q0, t1, t2);
-#pragma unroll
-      for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int b2 = 0; b2 < 3; ++b2)
-          jac[9 * i + 3 * a + b2] = ff_to_double(ff_dot2(w.get(a), t1[b2], w.get(3 + a), t2[b2]));
+    if (JAC) store_jacobian(q, i, w, jac);
+  }
+}
+
+// The point of the fixed-point composition as a location's argument: FP64
+// values on demand.
+struct PointX {
+  const long long* X;
+  __device__ __forceinline__ PointD fp64() const {
+    return PointD{(double)X[0] * kFxUnit, (double)X[1] * kFxUnit, (double)X[2] * kFxUnit};
+  }
+};
+
+// Points-only composition through map forms (submaps without one through
+// their coefficient records).  The point is kept in fixed point (fixed.cuh)
+// and every form P_c = p^T Q_c p evaluated on the integer pipes: in FP64 its
+// 24 operations per map bound the kernel on GB300 (89 % of the FP64 pipe, 25
+// FP64 instructions per evaluation; now ~5 beside ~960 others).  Errors are
+// below FP64's roundings: entries to 2^-59, sums to ~2^-57.  A form with an
+// entry of 2 or more (a map stretching by more than about 2) goes through
+// FP64; a point outside (0.5, 1.4) in squared norm is normalised first.
+template <class Src, int MINB>
+__global__ void __launch_bounds__(kBlock, MINB) compose_forms_kernel(MeshView m, Src cp,
+                                                                     const double* __restrict__ q, int64_t n,
+                                                                     double* __restrict__ out,
+                                                                     int32_t* __restrict__ tri,
+                                                                     int32_t* __restrict__ tri_all,
+                                                                     const int32_t* __restrict__ perm) {
+  const int S = cp.count();
+  for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n;
+       j += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = perm ? (int64_t)__ldg(perm + j) : j;
+    if ((uint64_t)i >= (uint64_t)n) {   // a bad permutation entry
+      flag(m, CMM_FLAG_INDEX);
+      continue;
     }
+    long long X[3];   // the point, units of 2^-58
+    int t;
+    Split sp;
+    {
+      double p[3];
+      if (!load_query(q, i, p)) {
+        store_nan<false>(m, i, n, S - 1, S, out, tri, tri_all, nullptr);
+        continue;
+      }
+      // the first location from the query's own FP64 values
+      t = locate_split(m, PointD{p[0], p[1], p[2]}, to_f32_trunc(p[0]), to_f32_trunc(p[1]), to_f32_trunc(p[2]), &sp);
+      if (tri) tri[i] = t;
+      if (tri_all) tri_all[(int64_t)(S - 1) * n + i] = t;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) X[c] = fx_of(p[c]);
+    }
+    bool lost = false;   // no finite image
+    int s = S - 1;
+    float f0 = fx_f32(X[0]), f1 = fx_f32(X[1]), f2 = fx_f32(X[2]);
+    while (true) {
+      const float n2 = fmaf(f0, f0, fmaf(f1, f1, f2 * f2));
+      if (!(n2 > 0.5f && n2 < 1.4f)) {
+        // rare: back to the unit sphere (the direction, and so the location
+        // above, stays)
+        PointD p = PointX{X}.fp64();
+        const double inv_n = rsqrt(p.x * p.x + p.y * p.y + p.z * p.z);
+        lost = !finite3(p.x * inv_n, p.y * inv_n, p.z * inv_n);
+        if (lost) break;
+        X[0] = fx_of(p.x * inv_n);
+        X[1] = fx_of(p.y * inv_n);
+        X[2] = fx_of(p.z * inv_n);
+      }
+      const double* fr = cp.form(s, S);
+      bool wide = fr == nullptr;
+      if (fr) {
+        const double2* qf = reinterpret_cast<const double2*>(fr + (int64_t)t * kFormStride + 18 * kSubIndex[sp.lo][sp.hi]);
+        double2 Q[9];   // all in flight together where the registers hold them
+#pragma unroll
+        for (int k = 0; k < 9; ++k) Q[k] = __ldg(qf + k);
+        const Limbs x = fx_limbs(X[0]), y = fx_limbs(X[1]), z = fx_limbs(X[2]);
+        auto prod = [](Limbs a, Limbs b) {
+          FxSum v{0, 0};
+          v.add(a, b);
+          return fx_limbs(v.value());
+        };
+        const Limbs xx = prod(x, x), yy = prod(y, y), zz = prod(z, z);
+        const Limbs xy = prod(x, y), xz = prod(x, z), yz = prod(y, z);
+        int bad = 0;
+        long long Y[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          FxSum r{0, 0};
+          r.add(fx_entry(Q[3 * c].x, bad), xx);
+          r.add(fx_entry(Q[3 * c].y, bad), yy);
+          r.add(fx_entry(Q[3 * c + 1].x, bad), zz);
+          r.add(fx_entry(Q[3 * c + 1].y, bad), xy);
+          r.add(fx_entry(Q[3 * c + 2].x, bad), xz);
+          r.add(fx_entry(Q[3 * c + 2].y, bad), yz);
+          Y[c] = r.value();
+        }
+        wide = bad < 0;
+        if (!wide) {
+#pragma unroll
+          for (int c = 0; c < 3; ++c) X[c] = Y[c];
+        }
+      }
+      if (wide) {   // in FP64: a coefficient record, or a form out of range
+        const PointD u = PointX{X}.fp64();
+        double p[3] = {u.x, u.y, u.z}, P[3];
+        if (fr) {
+          const double* Q = fr + (int64_t)t * kFormStride + 18 * kSubIndex[sp.lo][sp.hi];
+          for (int c = 0; c < 3; ++c)
+            P[c] = Q[6 * c] * p[0] * p[0] + Q[6 * c + 1] * p[1] * p[1] + Q[6 * c + 2] * p[2] * p[2] +
+                   Q[6 * c + 3] * p[0] * p[1] + Q[6 * c + 4] * p[0] * p[2] + Q[6 * c + 5] * p[1] * p[2];
+        } else {
+          record_eval<false>(m, cp.at(s, S), t, p, Pushes{nullptr, 0}, P);
+        }
+        const double r2 = P[0] * P[0] + P[1] * P[1] + P[2] * P[2];
+        if (!(r2 > 0.5 && r2 < 1.4)) {
+          const double inv_n = rsqrt(r2);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) P[c] *= inv_n;
+          lost = !finite3(P[0], P[1], P[2]);
+          if (lost) break;
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) X[c] = fx_of(P[c]);
+      }
+      if (--s < 0) break;
+      f0 = fx_f32(X[0]);
+      f1 = fx_f32(X[1]);
+      f2 = fx_f32(X[2]);
+      t = locate_split(m, PointX{X}, f0, f1, f2, &sp);
+      if (tri_all) tri_all[(int64_t)s * n + i] = t;
+    }
+    double p[3] = {(double)X[0], (double)X[1], (double)X[2]};   // the units drop out
+    const double inv_n = rsqrt(p[0] * p[0] + p[1] * p[1] + p[2] * p[2]);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) p[c] *= inv_n;
+    if (lost || !finite3(p[0], p[1], p[2])) {
+      store_nan<false>(m, i, n, s - 1, S, out, tri, tri_all, nullptr);
+      continue;
+    }
+    out[3 * i] = p[0];
+    out[3 * i + 1] = p[1];
+    out[3 * i + 2] = p[2];
   }
 }
 
@@ -646,55 +824,79 @@ __global__ void __launch_bounds__(kBlock) stencil_kernel(MeshView m, const doubl
 // kOrderLevel containing the query, FP32 descent, no FP64 filter: any
 // cell is a valid bucket) in four passes without global atomics:
 // per-block histograms, a scan along each cell's row of blocks, a scan of
-// the cell totals, a scatter.
+// the cell totals, a scatter.  A fifth pass groups each cell's queries by
+// cube-map cell (64 bins of 1/128): a warp of the composition then gathers
+// the records of a few triangles instead of 32, and stays with neighbours
+// through the whole stack (the gathers took 78 % of the L1 throughput with
+// the coarse cells alone; 2^22 queries through 8 level-7 maps 1.44 -> 1.33
+// ms points only, 2.66 -> 2.28 ms with Jacobians).
 constexpr int kOrderLevel = 4;          // 20 * 4^4 = 5120 cells
 constexpr int kOrderCells = 20 << (2 * kOrderLevel);
 constexpr int kOrderBlock = 1024;       // threads per block of passes 1 and 3
-constexpr int kOrderPer = 16;           // queries per thread
+constexpr int kOrderPer = 16;           // most queries per thread
+constexpr int kOrderFine = 3;           // bits of each cube-map coordinate in the fifth pass
+constexpr int kOrderSpan = 4096;        // most queries grouped by one block of it
+// fewer queries: the pass costs more than it gives (375,000 on a level-7
+// mesh, one a triangle: the composition 177 us without it, 174 with)
+constexpr int64_t kOrderFineMin = 1 << 20;
 
-__device__ __forceinline__ int coarse_cell(const MeshView& m, double x, double y, double z) {
-  const float fx = (float)x, fy = (float)y, fz = (float)z;
-  const float* rf = m.root_f;
-  int f = 0;
-  float best = -4.0f;
-  for (int g = 0; g < 20; ++g) {
-    const float d = fmaf(rf[12 * g], fx, fmaf(rf[12 * g + 1], fy, rf[12 * g + 2] * fz));
-    if (d > best) {
-      best = d;
-      f = g;
-    }
-  }
-  int64_t off = 0, cnt = 20;
-  const int lv = m.level < kOrderLevel ? m.level : kOrderLevel;
-  for (int j = 0; j < lv; ++j) {
-    const float* nf = m.node_nf + 9 * (off + f);
-    int c;
-    if (plane_f(nf, fx, fy, fz) > 0.f) c = 0;
-    else if (plane_f(nf + 3, fx, fy, fz) > 0.f) c = 1;
-    else if (plane_f(nf + 6, fx, fy, fz) > 0.f) c = 2;
-    else c = 3;
-    off += cnt;
-    cnt *= 4;
-    f = 4 * f + c;
-  }
-  return f << (2 * (kOrderLevel - lv));
+// Queries per thread of passes 1 and 4: as many blocks as SMs before more
+// than one query each (the descent is a serial chain; 10^5 queries in
+// blocks of 16 per thread ran on 7 SMs).
+int order_per(int64_t n) {
+  const int64_t per = (n + (int64_t)kOrderBlock * kNumSMs - 1) / ((int64_t)kOrderBlock * kNumSMs);
+  return (int)std::min<int64_t>(kOrderPer, std::max<int64_t>(1, per));
 }
 
-// pass 1: keys and per-block histograms hist[cell * nblk + block]
+// pass 1: keys and per-block histograms hist[cell * nblk + block].  key:
+// (cell << 2 fine) | interleaved low bits of the query's cube-map cell.  A
+// node's three normals are three aligned float4, loaded together: as nine
+// scalars, one test after the other, their L1 gathers took 0.62 of the sort's
+// 0.69 ms at 2^24 queries.  (In shared memory the table makes the SMs change
+// their L1 split between this kernel and the composition, which stalls a
+// pipeline of several streams.)
 __global__ void __launch_bounds__(kOrderBlock) order_count_kernel(MeshView m, const double* __restrict__ q,
-                                                                  int64_t n, int32_t* __restrict__ key,
+                                                                  int64_t n, int per, int fine,
+                                                                  int32_t* __restrict__ key,
                                                                   int32_t* __restrict__ hist) {
   __shared__ int h[kOrderCells];
+  const int lv = m.level < kOrderLevel ? m.level : kOrderLevel;
   for (int k = threadIdx.x; k < kOrderCells; k += blockDim.x) h[k] = 0;
   __syncthreads();
-  const int64_t base = (int64_t)blockIdx.x * kOrderBlock * kOrderPer;
-  for (int r = 0; r < kOrderPer; ++r) {
+  const int64_t base = (int64_t)blockIdx.x * kOrderBlock * per;
+  for (int r = 0; r < per; ++r) {
     const int64_t i = base + (int64_t)r * kOrderBlock + threadIdx.x;
-    if (i < n) {
-      const int c = coarse_cell(m, q[3 * i], q[3 * i + 1], q[3 * i + 2]);
-      key[i] = c;
-      atomicAdd(&h[c], 1);
+    if (i >= n) break;
+    const float fx = (float)q[3 * i], fy = (float)q[3 * i + 1], fz = (float)q[3 * i + 2];
+    int f = 0;
+    float best = -4.0f;
+#pragma unroll 4
+    for (int g = 0; g < 20; ++g) {
+      const float4 c = __ldg(reinterpret_cast<const float4*>(m.root_f + 12 * g));
+      const float d = fmaf(c.x, fx, fmaf(c.y, fy, c.z * fz));
+      if (d > best) {
+        best = d;
+        f = g;
+      }
     }
+    int off = 0, cnt = 20;
+    for (int j = 0; j < lv; ++j) {
+      const float4* nf = m.coarse_nf + 3 * (off + f);
+      const float4 n0 = __ldg(nf), n1 = __ldg(nf + 1), n2 = __ldg(nf + 2);
+      const int c = edge_dot(n0, fx, fy, fz) > 0.f ? 0 : (edge_dot(n1, fx, fy, fz) > 0.f ? 1 : (edge_dot(n2, fx, fy, fz) > 0.f ? 2 : 3));
+      off += cnt;
+      cnt *= 4;
+      f = 4 * f + c;
+    }
+    f <<= 2 * (kOrderLevel - lv);
+    atomicAdd(&h[f], 1);
+    int sub = 0;
+    if (fine) {   // 256 cells along a cube edge: about 8 across a coarse cell
+      const int cell = jump_cell(256, fx, fy, fz);
+      for (int b = 0; b < fine; ++b)   // bits kOrderFine-1 down to kOrderFine-fine of u and v
+        sub = (sub << 2) | (((cell >> (8 + kOrderFine - 1 - b)) & 1) << 1) | ((cell >> (kOrderFine - 1 - b)) & 1);
+    }
+    key[i] = (f << (2 * fine)) | sub;
   }
   __syncthreads();
   for (int k = threadIdx.x; k < kOrderCells; k += blockDim.x) hist[(int64_t)k * gridDim.x + blockIdx.x] = h[k];
@@ -748,8 +950,10 @@ __global__ void __launch_bounds__(1024) order_cellscan_kernel(int32_t* __restric
     }
 }
 
-// pass 4: scatter the query ids into their cells' ranges
-__global__ void __launch_bounds__(kOrderBlock) order_scatter_kernel(const int32_t* __restrict__ key, int64_t n,
+// pass 4: scatter the query ids into their cells' ranges, the cube-map bin
+// (2 fine bits) packed above the id for the fifth pass
+__global__ void __launch_bounds__(kOrderBlock) order_scatter_kernel(const int32_t* __restrict__ key, int64_t n, int per,
+                                                                    int fine,
                                                                     const int32_t* __restrict__ hist,
                                                                     const int32_t* __restrict__ cbase,
                                                                     int32_t* __restrict__ perm) {
@@ -757,10 +961,79 @@ __global__ void __launch_bounds__(kOrderBlock) order_scatter_kernel(const int32_
   for (int k = threadIdx.x; k < kOrderCells; k += blockDim.x)
     h[k] = cbase[k] + hist[(int64_t)k * gridDim.x + blockIdx.x];
   __syncthreads();
-  const int64_t base = (int64_t)blockIdx.x * kOrderBlock * kOrderPer;
-  for (int r = 0; r < kOrderPer; ++r) {
+  const int64_t base = (int64_t)blockIdx.x * kOrderBlock * per;
+  for (int r = 0; r < per; ++r) {
     const int64_t i = base + (int64_t)r * kOrderBlock + threadIdx.x;
-    if (i < n) perm[atomicAdd(&h[key[i]], 1)] = (int32_t)i;
+    if (i < n) {
+      const int k = key[i];
+      const unsigned sub = fine ? (unsigned)k << (32 - 2 * fine) : 0u;   // the low 2 fine bits, at the top
+      perm[atomicAdd(&h[k >> (2 * fine)], 1)] = (int32_t)(sub | (unsigned)i);
+    }
+  }
+}
+
+// pass 5: group by cube-map bin inside each cell, in place.  The array is cut
+// at the cells' starts and at the multiples of kOrderSpan (so that queries
+// crowded into one cell are shared out too): block c < kOrderCells takes the
+// piece from cell c's start, block kOrderCells + w the one from w kOrderSpan
+// if that lies inside a cell.
+__global__ void __launch_bounds__(256) order_group_kernel(const int32_t* __restrict__ cbase, int64_t n, int fine,
+                                                          int32_t* __restrict__ perm) {
+  constexpr int kPer = kOrderSpan / 256;
+  __shared__ int cur[1 << (2 * kOrderFine)];
+  const int tid = threadIdx.x, nb = 1 << (2 * fine), shift = 32 - 2 * fine;
+  int c;
+  int64_t lo;
+  if (blockIdx.x < kOrderCells) {
+    c = blockIdx.x;
+    lo = cbase[c];
+  } else {
+    lo = (int64_t)(blockIdx.x - kOrderCells) * kOrderSpan;
+    int a = 0, b = kOrderCells;   // the last cell starting at or before lo
+    while (b - a > 1) {
+      const int mid = (a + b) / 2;
+      if (cbase[mid] <= lo) a = mid;
+      else b = mid;
+    }
+    c = a;
+    if (cbase[c] == lo) return;   // block c's piece
+  }
+  const int64_t cell_end = c + 1 < kOrderCells ? cbase[c + 1] : n;
+  const int64_t hi = min(cell_end, (lo / kOrderSpan + 1) * kOrderSpan);
+  const int cnt = (int)(hi - lo);
+  if (cnt <= 0) return;
+  for (int k = tid; k < nb; k += 256) cur[k] = 0;
+  __syncthreads();
+  int val[kPer];   // in registers: all are read before any is written back
+#pragma unroll
+  for (int r = 0; r < kPer; ++r) {
+    const int k = r * 256 + tid;
+    if (k < cnt) {
+      val[r] = perm[lo + k];
+      atomicAdd(&cur[(unsigned)val[r] >> shift], 1);
+    }
+  }
+  __syncthreads();
+  if (tid < 32) {   // exclusive scan of the nb <= 64 bins, two per lane
+    const int k = 2 * tid;
+    const int a = k < nb ? cur[k] : 0, b = k + 1 < nb ? cur[k + 1] : 0;
+    int inc = a + b;
+    for (int d = 1; d < 32; d <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, inc, d);
+      if (tid >= d) inc += u;
+    }
+    if (k < nb) cur[k] = inc - a - b;
+    if (k + 1 < nb) cur[k + 1] = inc - b;
+  }
+  __syncthreads();
+  const unsigned mask = (1u << shift) - 1u;
+#pragma unroll
+  for (int r = 0; r < kPer; ++r) {
+    const int k = r * 256 + tid;
+    if (k < cnt) {
+      const unsigned v = (unsigned)val[r];
+      perm[lo + atomicAdd(&cur[v >> shift], 1)] = (int32_t)(v & mask);
+    }
   }
 }
 
@@ -828,39 +1101,53 @@ int launch_compose(const MeshView& m, const double* const* coeffs, int S, const 
                    cudaStream_t s, const int32_t* perm, const double* const* forms,
                    const float* const* forms_ff) {
   if (n == 0) return CMM_OK;
-  SubmapPtrs cp;
-  cp.S = S;
-  // the float-float copies are used when every submap with a form record
-  // has one
+  // the low floats are used when every submap with a form record has them
   bool ff = forms_ff != nullptr;
-  for (int k = 0; k < S; ++k) {
-    cp.p[k] = coeffs[k];
-    cp.f[k] = forms ? forms[k] : nullptr;
-    cp.g[k] = forms && forms[k] && forms_ff ? forms_ff[k] : nullptr;
-    if (cp.f[k] && !cp.g[k]) ff = false;
-  }
+  for (int k = 0; forms && k < S; ++k)
+    if (forms[k] && !(forms_ff && forms_ff[k])) ff = false;
+  // by the argument alone, as the device-driven step chooses (their results
+  // are bitwise equal, also while a run's stack is still empty)
+  const bool any = forms != nullptr;
   const int b = block_for(m, kTuneCompose, kBlock, n);
-  const int g = grid_for(n, b);
-  if (jac) {
-    const int v = m.variant[CMM_VARIANT_COMPOSE_JAC] ? m.variant[CMM_VARIANT_COMPOSE_JAC]
-                                                    : (ff ? kComposeJacBlocksFF : kComposeJacBlocks);
-    if (v == 2 && ff)
-      compose_kernel<true, SubmapPtrs, 2, true><<<g, b, 0, s>>>(m, cp, q, n, out, tri, tri_all, jac, perm);
-    else if (v == 2)
-      compose_kernel<true, SubmapPtrs, 2><<<g, b, 0, s>>>(m, cp, q, n, out, tri, tri_all, jac, perm);
-    else if (v == 3 && ff)
-      compose_kernel<true, SubmapPtrs, 3, true><<<g, b, 0, s>>>(m, cp, q, n, out, tri, tri_all, jac, perm);
-    else if (v == 3)
-      compose_kernel<true, SubmapPtrs, 3><<<g, b, 0, s>>>(m, cp, q, n, out, tri, tri_all, jac, perm);
-    else if (ff)
-      compose_kernel<true, SubmapPtrs, 4, true><<<g, b, 0, s>>>(m, cp, q, n, out, tri, tri_all, jac, perm);
-    else
-      compose_kernel<true, SubmapPtrs, 4><<<g, b, 0, s>>>(m, cp, q, n, out, tri, tri_all, jac, perm);
-  } else if ((m.variant[CMM_VARIANT_COMPOSE] ? m.variant[CMM_VARIANT_COMPOSE] : kComposeBlocks) == 4) {
-    compose_kernel<false, SubmapPtrs, 4><<<g, b, 0, s>>>(m, cp, q, n, out, tri, tri_all, jac, perm);
-  } else {
-    compose_kernel<false, SubmapPtrs, 6><<<g, b, 0, s>>>(m, cp, q, n, out, tri, tri_all, jac, perm);
-  }
+  const int vj = m.variant[CMM_VARIANT_COMPOSE_JAC], v = m.variant[CMM_VARIANT_COMPOSE];
+  auto run = [&](auto list) {
+    using Src = decltype(list);
+    list.S = S;
+    for (int k = 0; k < S; ++k) {
+      list.p[k] = coeffs[k];
+      list.f[k] = forms ? forms[k] : nullptr;
+      list.g[k] = forms && forms[k] && forms_ff ? forms_ff[k] : nullptr;
+    }
+    auto go = [&](auto kernel) { kernel<<<grid_for(n, b), b, 0, s>>>(m, list, q, n, out, tri, tri_all, jac, perm); };
+    constexpr bool tuned = sizeof(list.p) <= kShortList * sizeof(double*);   // variants for the usual lists only
+    constexpr int J2 = tuned ? 2 : kComposeJacBlocks, J3 = tuned ? 3 : kComposeJacBlocks;
+    constexpr int F2 = tuned ? 2 : kComposeJacBlocksFF, F3 = tuned ? 3 : kComposeJacBlocksFF;
+    constexpr int V6 = tuned ? 6 : kComposeBlocks;
+    if (jac && forms && ff) {
+      if (vj == 2) go(compose_kernel<true, Src, F2, true>);
+      else if (vj == 3) go(compose_kernel<true, Src, F3, true>);
+      else go(compose_kernel<true, Src, kComposeJacBlocksFF, true>);
+    } else if (jac) {
+      if (vj == 2) go(compose_kernel<true, Src, J2>);
+      else if (vj == 3) go(compose_kernel<true, Src, J3>);
+      else go(compose_kernel<true, Src, kComposeJacBlocks>);
+    } else if (any) {
+      auto gof = [&](auto kernel) { kernel<<<grid_for(n, b), b, 0, s>>>(m, list, q, n, out, tri, tri_all, perm); };
+      // in caller order the gathers may be scattered: 80 registers hold a
+      // form's nine loads in flight (2^22 random queries 2.53 against 2.95
+      // ms; grouped ones 1.45 against 1.35, a sample grid 287 against 270 us)
+      if (v == 6) gof(compose_forms_kernel<Src, V6>);
+      else if (v == 4 || perm) gof(compose_forms_kernel<Src, kComposeBlocks>);
+      else gof(compose_forms_kernel<Src, kFormsCallerBlocks>);
+    } else {
+      if (v == 6) go(compose_kernel<false, Src, V6>);
+      else go(compose_kernel<false, Src, kComposeBlocks>);
+    }
+  };
+  if (S <= kShortList)
+    run(SubmapPtrs<kShortList>{});
+  else
+    run(SubmapPtrs<CMM_MAX_SUBMAPS>{});
   return check_launch("compose_kernel");
 }
 
@@ -917,26 +1204,33 @@ int build_jump_table(cmm_mesh* mesh) {
 }
 
 int64_t order_workspace(int64_t n) {
-  const int64_t nblk = (n + (int64_t)kOrderBlock * kOrderPer - 1) / ((int64_t)kOrderBlock * kOrderPer);
+  const int64_t span = (int64_t)kOrderBlock * order_per(n), nblk = (n + span - 1) / span;
   return n + (int64_t)kOrderCells * ((nblk < 1 ? 1 : nblk) + 1);
 }
 
 int launch_query_order(const MeshView& m, const double* q, int64_t n, int32_t* perm, int32_t* work,
                        cudaStream_t s) {
   if (n == 0) return CMM_OK;
-  const int64_t nblk = (n + (int64_t)kOrderBlock * kOrderPer - 1) / ((int64_t)kOrderBlock * kOrderPer);
+  const int per = order_per(n);
+  const int64_t nblk = (n + (int64_t)kOrderBlock * per - 1) / ((int64_t)kOrderBlock * per);
   int32_t* key = work;
   int32_t* hist = work + n;
   int32_t* total = hist + (int64_t)kOrderCells * nblk;
-  order_count_kernel<<<(int)nblk, kOrderBlock, 0, s>>>(m, q, n, key, hist);
+  // bins of the fifth pass: as far as the packed ids leave bits, and for
+  // enough queries
+  int fine = kOrderFine;
+  while (fine > 0 && (n < kOrderFineMin || n > (1LL << (32 - 2 * fine)))) --fine;
+  order_count_kernel<<<(int)nblk, kOrderBlock, 0, s>>>(m, q, n, per, fine, key, hist);
   int rc = check_launch("order_count_kernel");
   if (rc) return rc;
   order_rowscan_kernel<<<kOrderCells / 8, 256, 0, s>>>(hist, (int)nblk, total);
   if ((rc = check_launch("order_rowscan_kernel"))) return rc;
   order_cellscan_kernel<<<1, 1024, 0, s>>>(total);
   if ((rc = check_launch("order_cellscan_kernel"))) return rc;
-  order_scatter_kernel<<<(int)nblk, kOrderBlock, 0, s>>>(key, n, hist, total, perm);
-  return check_launch("order_scatter_kernel");
+  order_scatter_kernel<<<(int)nblk, kOrderBlock, 0, s>>>(key, n, per, fine, hist, total, perm);
+  if ((rc = check_launch("order_scatter_kernel")) || !fine) return rc;
+  order_group_kernel<<<kOrderCells + (int)((n + kOrderSpan - 1) / kOrderSpan), 256, 0, s>>>(total, n, fine, perm);
+  return check_launch("order_group_kernel");
 }
 
 int launch_compose_dev(const MeshView& m, const double* const* table, const BveState* st,
@@ -945,12 +1239,15 @@ int launch_compose_dev(const MeshView& m, const double* const* table, const BveS
   if (n == 0) return CMM_OK;
   DevSubmaps cp{table, ftable, st, last};
   const int b = block_for(m, kTuneCompose, kBlock, n);
-  if ((m.variant[CMM_VARIANT_COMPOSE] ? m.variant[CMM_VARIANT_COMPOSE] : kComposeBlocks) == 4)
-    compose_kernel<false, DevSubmaps, 4><<<grid_for(n, b), b, 0, s>>>(m, cp, q, n, out, nullptr, nullptr,
-                                                                      nullptr, nullptr);
+  const bool six = m.variant[CMM_VARIANT_COMPOSE] == 6;
+  auto go = [&](auto kernel) {
+    kernel<<<grid_for(n, b), b, 0, s>>>(m, cp, q, n, out, nullptr, nullptr, nullptr, nullptr);
+  };
+  auto gof = [&](auto kernel) { kernel<<<grid_for(n, b), b, 0, s>>>(m, cp, q, n, out, nullptr, nullptr, nullptr); };
+  if (ftable)
+    six ? gof(compose_forms_kernel<DevSubmaps, 6>) : gof(compose_forms_kernel<DevSubmaps, kComposeBlocks>);
   else
-    compose_kernel<false, DevSubmaps, 6><<<grid_for(n, b), b, 0, s>>>(m, cp, q, n, out, nullptr, nullptr,
-                                                                      nullptr, nullptr);
+    six ? go(compose_kernel<false, DevSubmaps, 6>) : go(compose_kernel<false, DevSubmaps, kComposeBlocks>);
   return check_launch("compose_kernel");
 }
 

@@ -373,6 +373,13 @@ int upload_mesh(const HostMesh& h, cmm_mesh* m) {
   if ((rc = m->root_adj.upload(h.root_adj.data(), h.root_adj.size() * 4))) return rc;
   if ((rc = m->node_n.upload(h.node_n.data(), h.node_n.size() * 8))) return rc;
   if ((rc = m->node_nf.upload(h.node_nf.data(), h.node_nf.size() * 4))) return rc;
+  {
+    // levels 0..3 of the FP32 normals with a float4 each (the query sort)
+    const size_t nn = std::min<size_t>(h.node_nf.size() / 3, 3 * 20 * ((1 << 8) - 1) / 3);
+    std::vector<float4> cf(std::max<size_t>(nn, 1));
+    for (size_t k = 0; k < nn; ++k) cf[k] = make_float4(h.node_nf[3 * k], h.node_nf[3 * k + 1], h.node_nf[3 * k + 2], 0.f);
+    if ((rc = m->coarse_nf.upload(cf.data(), cf.size() * sizeof(float4)))) return rc;
+  }
   if ((rc = m->leaf_row.upload(h.leaf_row.data(), h.leaf_row.size() * 4))) return rc;
   if ((rc = m->walk_f.upload(h.walk_f.data(), h.walk_f.size() * 4))) return rc;
   if ((rc = m->walk_d.upload(h.walk_d.data(), h.walk_d.size() * 8))) return rc;
@@ -391,6 +398,7 @@ int upload_mesh(const HostMesh& h, cmm_mesh* m) {
   v.root_adj = (const int*)m->root_adj.p;
   v.node_n = (const double*)m->node_n.p;
   v.node_nf = (const float*)m->node_nf.p;
+  v.coarse_nf = (const float4*)m->coarse_nf.p;
   v.leaf_row = (const int*)m->leaf_row.p;
   v.walk_f = (const float*)m->walk_f.p;
   v.walk_d = (const double*)m->walk_d.p;

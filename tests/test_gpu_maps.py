@@ -403,3 +403,63 @@ def test_map_forms_match_coefficient_records(nat):
     assert torch.isnan(Xn[3]).all() and int(tn[3]) == -1 and torch.isfinite(Xn[4:]).all()
     assert m.status(clear=True) == nat.FLAG_NONFINITE
     assert m.status() == 0
+
+
+@pytest.mark.parametrize("scale", [1.0, 1.9, 2.3, 40.0])
+@pytest.mark.parametrize("radius", [1.0, 0.51, 1.7, 1e-3, 1e4])
+def test_fixed_point_forms_at_the_ends_of_their_range(nat, scale, radius):
+    """The points-only composition through map forms (fixed point) against
+    the same submaps' coefficient records in FP64: jets scaled by `scale` make
+    forms with entries on both sides of 2 (the bound of the fixed-point
+    entries; the images are normalised, so the composed map stays the same),
+    queries of norm `radius` lie inside and outside the range kept
+    unnormalised, and a submap without a form record sits in the stack.  Same
+    triangles, points to 1e-13."""
+    from cmm_gpu.meshgen import icosahedral_mesh, random_sphere_points
+    from cmm_gpu.workloads import submap_stack
+    verts, tris = icosahedral_mesh(4)
+    tan, s_pts = OG.stencil_points(verts)
+    jets = submap_stack(s_pts, tan, 4, seed=8)
+    jets[1] *= scale
+    jets[3] /= scale
+    m = nat.Mesh(verts, tris, 4)
+    cs = [m.assemble(dev(j)) for j in jets]
+    fs = [m.assemble_forms(c) for c in cs]
+    fs[2] = None
+    q = dev(random_sphere_points(4099, seed=9) * radius)
+    Xr, tr, tar, _ = m.compose(cs, q, want_tri=True, want_tri_all=True)
+    Xf, tf, taf, _ = m.compose(cs, q, want_tri=True, want_tri_all=True, forms=fs)
+    assert torch.equal(tr, tf) and torch.equal(tar, taf)
+    assert float((Xf - Xr).abs().max()) < 1e-13
+    for v in (4, 6):
+        m.set_variant(nat.Mesh.VARIANT_COMPOSE, v)
+        assert torch.equal(m.compose(cs, q, forms=fs)[0], Xf)
+    # a form that is not finite: NaN images, the flag, later ids -1
+    bad = fs[3].clone()
+    bad[:, :6] = float("nan")
+    Xn, tn, tan_, _ = m.compose(cs, q, want_tri=True, want_tri_all=True, forms=fs[:3] + [bad])
+    hit = torch.isnan(Xn).any(dim=1)
+    assert hit.any() and not hit.all() and torch.equal(tn, tf)
+    assert torch.equal(Xn[~hit], Xf[~hit]) and bool((tan_[:3, hit] == -1).all())
+    assert m.status(clear=True) == nat.FLAG_NONFINITE
+
+
+@pytest.mark.parametrize("n,spread", [(1, 2.0), (1023, 2.0), (155649, 2.0), ((1 << 20) - 1, 2.0), (1 << 20, 2.0),
+                                      ((1 << 20) + 4097, 1e-3), ((1 << 20) + 4097, 0.2)])
+def test_query_order_is_a_permutation(nat, n, spread):
+    """cmm_query_order either side of its fifth pass and of a block's span,
+    with the queries over the whole sphere, within a few cells, and all in
+    one or two cells."""
+    from cmm_gpu.meshgen import icosahedral_mesh
+    verts, tris = icosahedral_mesh(3 if n < 2000 else 5)
+    m = nat.Mesh(verts, tris, 3 if n < 2000 else 5)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    q = torch.randn((n, 3), dtype=torch.float64, device="cuda", generator=g)
+    if spread < 2.0:
+        q = spread * q + torch.tensor([0.3, -0.5, 0.8], dtype=torch.float64, device="cuda")
+    q = (q / q.norm(dim=1, keepdim=True)).contiguous()
+    perm = m.query_order(q)
+    assert torch.equal(torch.sort(perm.long())[0], torch.arange(n, device="cuda"))
+    if spread == 2.0 and n > 1 << 17:
+        p = q[perm.long()]
+        assert float((p[1:] - p[:-1]).norm(dim=1).median()) < 0.1
