@@ -321,7 +321,12 @@ int tc_plan_create(int L, const double* ct_rings, const double* pmm_rings, const
 void tc_plan_destroy(TcPlan* p);
 int tc_plan_share(const TcPlan* src, TcPlan** out);
 size_t tc_plan_bytes(const TcPlan* p);
-int tc_synthesis(TcPlan* p, const double2* fields, float2* S, int* status, cudaStream_t s);
+// The synthesis' data tiles from 12 coefficient fields (12, L, L), or the
+// velocity's 12 fields straight from the analysis (lap) or stream function
+// a (L, L); then the synthesis of the tiles.
+int tc_field_tiles(TcPlan* p, const double2* fields, cudaStream_t s);
+int tc_velocity_tiles(TcPlan* p, const double2* a, bool lap, cudaStream_t s);
+int tc_synthesis(TcPlan* p, float2* S, int* status, cudaStream_t s);
 void tc_set_schedule(TcPlan* p, int schedule);
 int sht_set_schedule(cmm_sht* p, int schedule);
 int tc_analysis(TcPlan* p, const float2* fine, const double* w, double2* alm, int* status,

@@ -39,20 +39,18 @@ constexpr int kSynthBlock = 64;
 constexpr int kLChunk = 32;
 
 __device__ __forceinline__ double2 cmul(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
-__device__ __forceinline__ float2 cmul(float2 a, double s) {
-  return make_float2(a.x * (float)s, a.y * (float)s);
-}
+__device__ __forceinline__ float2 cmul(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
 
 // ----------------------------------------------------------------- forward
-// C = double2 (FP64 form) or float2 (ring FFTs of the split-BF16 form).
-// F (L+1, L+1) ring spectra -> torus columns G (2L, L): G[t][m].
-template <typename C>
-__global__ void torus_kernel(const C* __restrict__ F, int L, C* __restrict__ G) {
+// Split-BF16 form: ring spectra F (L+1, L+1) -> torus columns G (2L, L),
+// G[t][m], scaled by s = pi/L.  (The scale comes from the host: a division
+// and a conversion in each thread on the FP64 pipe took 34 of the kernel's
+// 40 us at L = 1024, and 40 of pad_kernel's 54.)
+__global__ void torus_kernel(const float2* __restrict__ F, int L, float s, float2* __restrict__ G) {
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   const int t = blockIdx.y;
   if (m >= L || t >= 2 * L) return;
-  const double s = M_PI / L;
-  C v;
+  float2 v;
   if (t <= L) {
     v = F[(int64_t)t * (L + 1) + m];
   } else {
@@ -65,20 +63,17 @@ __global__ void torus_kernel(const C* __restrict__ F, int L, C* __restrict__ G) 
   G[(int64_t)t * L + m] = cmul(v, s);
 }
 
-// Torus spectrum Gh (2L, L) -> zero-padded H (4L, L), Nyquist split.
-template <typename C>
-__global__ void pad_kernel(const C* __restrict__ Gh, int L, C* __restrict__ H) {
+// Torus spectrum Gh (2L, L) -> zero-padded H (4L, L), Nyquist split, scaled
+// by s = 1/2L.
+__global__ void pad_kernel(const float2* __restrict__ Gh, int L, float s, float2* __restrict__ H) {
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   const int k = blockIdx.y;  // 0..4L-1
   if (m >= L || k >= 4 * L) return;
-  const double s = 1.0 / (2 * L);
-  C v;
-  v.x = 0;
-  v.y = 0;
+  float2 v = make_float2(0.f, 0.f);
   if (k < L) {
     v = Gh[(int64_t)k * L + m];
   } else if (k == L || k == 3 * L) {
-    v = cmul(Gh[(int64_t)L * L + m], 0.5);
+    v = cmul(Gh[(int64_t)L * L + m], 0.5f);
   } else if (k > 3 * L) {
     v = Gh[(int64_t)(k - 2 * L) * L + m];
   }
@@ -88,12 +83,11 @@ __global__ void pad_kernel(const C* __restrict__ Gh, int L, C* __restrict__ H) {
 // The FP64 form keeps the torus and padded spectra order-major, G[m][t]
 // (L, 2L) and H[m][k] (L, 4L), so that cuFFT transforms L contiguous rows
 // (the strided column transforms of the layout above run a few blocks at
-// small L).  Same values as torus_kernel / pad_kernel.
-__global__ void torus_t_kernel(const double2* __restrict__ F, int L, double2* __restrict__ G) {
+// small L).  Same values as torus_kernel / pad_kernel in FP64.
+__global__ void torus_t_kernel(const double2* __restrict__ F, int L, double s, double2* __restrict__ G) {
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   const int t = blockIdx.y;
   if (m >= L || t >= 2 * L) return;
-  const double s = M_PI / L;
   double2 v;
   if (t <= L) {
     v = F[(int64_t)t * (L + 1) + m];
@@ -107,11 +101,10 @@ __global__ void torus_t_kernel(const double2* __restrict__ F, int L, double2* __
   G[(int64_t)m * 2 * L + t] = cmul(v, s);
 }
 
-__global__ void pad_t_kernel(const double2* __restrict__ Gh, int L, double2* __restrict__ H) {
+__global__ void pad_t_kernel(const double2* __restrict__ Gh, int L, double s, double2* __restrict__ H) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;  // 0..4L-1
   const int m = blockIdx.y;
   if (k >= 4 * L || m >= L) return;
-  const double s = 1.0 / (2 * L);
   const double2* g = Gh + (int64_t)m * 2 * L;
   double2 v = make_double2(0.0, 0.0);
   if (k < L) {
@@ -286,31 +279,6 @@ __device__ __forceinline__ void ladder(const double2* __restrict__ a, int L, int
   o[2] = make_double2(-(double)m * am.y, (double)m * am.x);           // i m a
 }
 
-// fields[f] (f = 0..11): 0..2 = u_i = iL_i psi; 3 + 3i + k = iL_k u_i.
-__global__ void ladder1_kernel(const double2* __restrict__ psi, int L, double2* __restrict__ fields) {
-  const int l = blockIdx.x * blockDim.x + threadIdx.x, m = blockIdx.y;
-  if (l >= L) return;
-  const int64_t fs = (int64_t)L * L, i = (int64_t)m * L + l;
-  if (l < m) {
-    for (int f = 0; f < 3; ++f) fields[f * fs + i] = make_double2(0.0, 0.0);
-    return;
-  }
-  double2 o[3];
-  ladder(psi, L, l, m, o);
-  for (int f = 0; f < 3; ++f) fields[f * fs + i] = o[f];
-}
-
-__global__ void ladder2_kernel(double2* __restrict__ fields, int L) {
-  const int l = blockIdx.x * blockDim.x + threadIdx.x, m = blockIdx.y;
-  if (l >= L) return;
-  const int64_t fs = (int64_t)L * L, i = (int64_t)m * L + l;
-  for (int u = 0; u < 3; ++u) {
-    double2 o[3] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
-    if (l >= m) ladder(fields + u * fs, L, l, m, o);
-    for (int k = 0; k < 3; ++k) fields[(3 + 3 * u + k) * fs + i] = o[k];
-  }
-}
-
 // The velocity's coefficient fields in the FP64 form, from the analysis a
 // (lap: psi = D_inv a, cmm_s2/core/spherical_simulations.py:195-198) or
 // the stream function itself.  With A_k = iL_k (ladder above) u_i = A_i psi
@@ -327,6 +295,7 @@ __device__ __forceinline__ double2 order_value(const double2* __restrict__ a, in
   const int k = mm < 0 ? -mm : mm;
   if (k > l) return make_double2(0.0, 0.0);
   const double2 v = cmul(a[(int64_t)k * L + l], d);
+  if (k == 0) return make_double2(v.x, 0.0);   // a real field's: an imaginary part means nothing
   if (mm >= 0) return v;   // a_{l,-k} = (-1)^k conj(a_{l,k})
   return (k & 1) ? make_double2(-v.x, v.y) : make_double2(v.x, -v.y);
 }
@@ -785,7 +754,23 @@ __global__ void __launch_bounds__(kTabBlock) synthesis_tab_kernel(const double2*
 // g = (iLx, iLy, iLz) u_i, vals[c][1+i] = (g x X - ((g x X).X/|X|) X)_c;
 // poles from sample 0 of the first and last rings.
 // Split-BF16 form: FP32 samples and arithmetic; jets_f: the same values as
-// floats.
+// floats.  The conversions between the two widths are made from the bits:
+// 15 per vertex on the FP64 pipe took most of the kernel's 75 us at L = 1024.
+__device__ __forceinline__ double widen(float x) {
+  const unsigned b = __float_as_uint(x), e = (b >> 23) & 255u;
+  if (e - 1u >= 254u) return (double)x;   // zero, subnormal, infinite, NaN
+  return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + (896u << 20))), (int)(b << 29));
+}
+
+__device__ __forceinline__ float narrow(double x) {   // round to nearest even
+  const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x), e = (h >> 20) & 2047u;
+  if (e - 897u >= 253u) return (float)x;   // zero, outside FP32's normal range (or next to its end), NaN
+  unsigned f = (((h & 0x7fffffffu) - (896u << 20)) << 3) | (l >> 29);
+  const unsigned r = l & 0x1fffffffu;
+  f += (r > 0x10000000u || (r == 0x10000000u && (f & 1u))) ? 1u : 0u;
+  return __uint_as_float((h & 0x80000000u) | f);
+}
+
 __global__ void jets_kernel(const float* __restrict__ fld, int L, const double* __restrict__ grid,
                             double* __restrict__ jets, float* __restrict__ jets_f) {
   const int N = 2 * L;
@@ -800,7 +785,7 @@ __global__ void jets_kernel(const float* __restrict__ fld, int L, const double* 
   else
     node = N + (v - 1);
   const int64_t fs = (int64_t)(L + 1) * N;
-  const float X0 = (float)grid[4 * node], X1 = (float)grid[4 * node + 1], X2 = (float)grid[4 * node + 2];
+  const float X0 = narrow(grid[4 * node]), X1 = narrow(grid[4 * node + 1]), X2 = narrow(grid[4 * node + 2]);
   const float nX = sqrt(X0 * X0 + X1 * X1 + X2 * X2);
   for (int i = 0; i < 3; ++i) {
     const float g0 = fld[(3 + 3 * i) * fs + node], g1 = fld[(4 + 3 * i) * fs + node],
@@ -811,7 +796,7 @@ __global__ void jets_kernel(const float* __restrict__ fld, int L, const double* 
     const int64_t slot[4] = {i * 4, 0 * 4 + 1 + i, 1 * 4 + 1 + i, 2 * 4 + 1 + i};
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      jets[slot[k] * nv + v] = (double)val[k];
+      jets[slot[k] * nv + v] = widen(val[k]);
       jets_f[slot[k] * nv + v] = val[k];
     }
   }
@@ -1512,11 +1497,11 @@ static int forward_rings_f32(cmm_sht* p, const double* samples, cudaStream_t s) 
   if ((rc = check_launch("to_float_kernel"))) return rc;
   cufftResult r = cufftExecR2C(p->f_ring_fwd, (cufftReal*)p->f_in.p, (cufftComplex*)p->f_spec.p);
   if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftExecR2C");
-  torus_kernel<float2><<<g1, b, 0, s>>>((const float2*)p->f_spec.p, L, (float2*)p->f_torus.p);
+  torus_kernel<<<g1, b, 0, s>>>((const float2*)p->f_spec.p, L, (float)(M_PI / L), (float2*)p->f_torus.p);
   if ((rc = check_launch("torus_kernel"))) return rc;
   r = cufftExecC2C(p->f_torus_fwd, (cufftComplex*)p->f_torus.p, (cufftComplex*)p->f_torus.p, CUFFT_FORWARD);
   if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftExecC2C(torus)");
-  pad_kernel<float2><<<g2, b, 0, s>>>((const float2*)p->f_torus.p, L, (float2*)p->f_pad.p);
+  pad_kernel<<<g2, b, 0, s>>>((const float2*)p->f_torus.p, L, (float)(1.0 / (2 * L)), (float2*)p->f_pad.p);
   if ((rc = check_launch("pad_kernel"))) return rc;
   r = cufftExecC2C(p->f_pad_inv, (cufftComplex*)p->f_pad.p, (cufftComplex*)p->f_pad.p, CUFFT_INVERSE);
   if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftExecC2C(pad)");
@@ -1543,12 +1528,13 @@ int sht_forward(cmm_sht* p, const double* samples, double2* out, cudaStream_t s)
         (const double2*)p->spec.p, L, (const double*)p->tab->w.p, out);
     return check_launch("analysis_w_kernel");
   }
-  torus_t_kernel<<<g1, b, 0, s>>>((const double2*)p->spec.p, L, (double2*)p->torus.p);
+  torus_t_kernel<<<g1, b, 0, s>>>((const double2*)p->spec.p, L, M_PI / L, (double2*)p->torus.p);
   if ((rc = check_launch("torus_t_kernel"))) return rc;
   r = cufftExecZ2Z(p->torus_fwd_t, (cufftDoubleComplex*)p->torus.p, (cufftDoubleComplex*)p->torus.p,
                    CUFFT_FORWARD);
   if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftExecZ2Z(torus)");
-  pad_t_kernel<<<dim3((4 * L + 127) / 128, L), b, 0, s>>>((const double2*)p->torus.p, L, (double2*)p->pad.p);
+  pad_t_kernel<<<dim3((4 * L + 127) / 128, L), b, 0, s>>>((const double2*)p->torus.p, L, 1.0 / (2 * L),
+                                                                 (double2*)p->pad.p);
   if ((rc = check_launch("pad_t_kernel"))) return rc;
   r = cufftExecZ2Z(p->pad_inv_t, (cufftDoubleComplex*)p->pad.p, (cufftDoubleComplex*)p->pad.p, CUFFT_INVERSE);
   if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftExecZ2Z(pad)");
@@ -1562,6 +1548,8 @@ int sht_forward(cmm_sht* p, const double* samples, double2* out, cudaStream_t s)
   return check_launch("analysis_kernel");
 }
 
+static int synthesis_split(cmm_sht* p, cudaStream_t s);
+
 // nf fields (nf, L, L) m-major -> samples (nf, L+1, 2L).
 int sht_inverse(cmm_sht* p, const double2* alm, int nf, double* samples, cudaStream_t s) {
   const int L = p->L;
@@ -1569,12 +1557,7 @@ int sht_inverse(cmm_sht* p, const double2* alm, int nf, double* samples, cudaStr
   if (rc) return rc;
   if (nf == kFields && p->precision == CMM_SHT_SPLIT_BF16) {
     // tensor-core synthesis into FP32 spectra, FP32 ring FFTs
-    const int nrows = kFields * (L + 1);
-    zero_nyquist_kernel<<<(nrows + 255) / 256, 256, 0, s>>>((float2*)p->f_synth.p, L, nrows);
-    if ((rc = check_launch("zero_nyquist_kernel"))) return rc;
-    if ((rc = tc_synthesis(p->tc, alm, (float2*)p->f_synth.p, (int*)p->status.p, s))) return rc;
-    cufftResult r = cufftExecC2R(p->f_ring_inv, (cufftComplex*)p->f_synth.p, (cufftReal*)p->f_samples.p);
-    if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftExecC2R");
+    if ((rc = tc_field_tiles(p->tc, alm, s)) || (rc = synthesis_split(p, s))) return rc;
     if (samples) {
       const int64_t ns = (int64_t)nf * (L + 1) * 2 * L;
       to_double_kernel<<<(int)((ns + 255) / 256), 256, 0, s>>>((const float*)p->f_samples.p, ns, samples);
@@ -1628,10 +1611,11 @@ int sht_inverse(cmm_sht* p, const double2* alm, int nf, double* samples, cudaStr
   return CMM_OK;
 }
 
-// Split-BF16 form: the stream function's 12 velocity/jet fields, their
-// synthesis and the jets at the velocity mesh's vertices.
-static int velocity_from_psi(cmm_sht* p, const cmm_mesh* vm, const double2* psi, double* jets,
-                             cudaStream_t s);
+// Split-BF16 form from the analysis a (lap) or the stream function: the
+// 12 velocity/jet fields, their synthesis and the jets at the velocity
+// mesh's vertices.
+static int velocity_split(cmm_sht* p, const cmm_mesh* vm, const double2* a, bool lap, double* jets,
+                          cudaStream_t s);
 
 static int velocity_fp64(cmm_sht* p, const cmm_mesh* vm, const double2* a, bool lap, double2* psi_out,
                          double* jets, cudaStream_t s);
@@ -1647,15 +1631,13 @@ int sht_velocity(cmm_sht* p, const cmm_mesh* vm, const double* omega, double2* p
     psi_out = nullptr;
   }
   if (p->precision == CMM_SHT_FP64) return velocity_fp64(p, vm, psi, omega != nullptr, psi_out, jets, s);
-  if (omega) {
-    dinv_kernel<<<dim3((L + 127) / 128, L), 128, 0, s>>>(psi, L);
+  if (psi_out) {
+    cudaError_t e = cudaMemcpyAsync(psi_out, psi, (size_t)L * L * sizeof(double2), cudaMemcpyDeviceToDevice, s);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync(psi)");
+    dinv_kernel<<<dim3((L + 127) / 128, L), 128, 0, s>>>(psi_out, L);
     if ((rc = check_launch("dinv_kernel"))) return rc;
-    if (psi_out) {
-      cudaError_t e = cudaMemcpyAsync(psi_out, psi, (size_t)L * L * sizeof(double2), cudaMemcpyDeviceToDevice, s);
-      if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync(psi)");
-    }
   }
-  return velocity_from_psi(p, vm, psi, jets, s);
+  return velocity_split(p, vm, psi, omega != nullptr, jets, s);
 }
 
 // The FP64 form from the analysis a (lap) or the stream function: six
@@ -1705,13 +1687,8 @@ int sht_velocity_pre(cmm_sht* p, const double* omega, cudaStream_t s) {
 
 // ... and after the batch's analysis (which wrote p->alm), the rest.
 int sht_velocity_post(cmm_sht* p, const cmm_mesh* vm, double* jets, cudaStream_t s) {
-  const int L = p->L;
-  int rc = set_streams(p, s);
-  if (rc) return rc;
-  double2* psi = (double2*)p->alm.p;
-  dinv_kernel<<<dim3((L + 127) / 128, L), 128, 0, s>>>(psi, L);
-  if ((rc = check_launch("dinv_kernel"))) return rc;
-  return velocity_from_psi(p, vm, psi, jets, s);
+  const int rc = set_streams(p, s);
+  return rc ? rc : velocity_split(p, vm, (const double2*)p->alm.p, true, jets, s);
 }
 
 int sht_batch_create(cmm_sht* const* plans, int n, cmm_sht_batch** out) {
@@ -1804,17 +1781,21 @@ int sht_batch_forward(cmm_sht_batch* bt, const double* const* samples, double2* 
   return sht_batch_analysis(bt, alm, s);
 }
 
-static int velocity_from_psi(cmm_sht* p, const cmm_mesh* vm, const double2* psi, double* jets,
-                             cudaStream_t s) {
+// Ring FFTs of the tensor-core synthesis' spectra, whose data tiles are made.
+static int synthesis_split(cmm_sht* p, cudaStream_t s) {
+  const int nrows = kFields * (p->L + 1);
+  zero_nyquist_kernel<<<(nrows + 255) / 256, 256, 0, s>>>((float2*)p->f_synth.p, p->L, nrows);
+  int rc = check_launch("zero_nyquist_kernel");
+  if (rc || (rc = tc_synthesis(p->tc, (float2*)p->f_synth.p, (int*)p->status.p, s))) return rc;
+  cufftResult r = cufftExecC2R(p->f_ring_inv, (cufftComplex*)p->f_synth.p, (cufftReal*)p->f_samples.p);
+  return r == CUFFT_SUCCESS ? CMM_OK : cufft_fail(r, "cufftExecC2R");
+}
+
+static int velocity_split(cmm_sht* p, const cmm_mesh* vm, const double2* a, bool lap, double* jets,
+                          cudaStream_t s) {
   const int L = p->L;
-  int rc;
-  dim3 b(128), g((L + 127) / 128, L);
-  double2* F = (double2*)p->fields.p;
-  ladder1_kernel<<<g, b, 0, s>>>(psi, L, F);
-  if ((rc = check_launch("ladder1_kernel"))) return rc;
-  ladder2_kernel<<<g, b, 0, s>>>(F, L);
-  if ((rc = check_launch("ladder2_kernel"))) return rc;
-  if ((rc = sht_inverse(p, F, kFields, nullptr, s))) return rc;
+  int rc = set_streams(p, s);
+  if (rc || (rc = tc_velocity_tiles(p->tc, a, lap, s)) || (rc = synthesis_split(p, s))) return rc;
   const int64_t nv = 2 + (int64_t)(L - 1) * 2 * L;
   jets_kernel<<<(int)((nv + 127) / 128), 128, 0, s>>>((const float*)p->f_samples.p, L, vm->view.grid, jets,
                                                       (float*)p->f_jets.p);

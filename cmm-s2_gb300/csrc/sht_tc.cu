@@ -36,6 +36,7 @@
 
 #include "cmm_internal.h"
 #include "device_common.cuh"
+#include "ff.cuh"
 
 namespace cmm {
 
@@ -248,6 +249,162 @@ __global__ void build_atab_kernel(TcGeometry g, const double2* __restrict__ fiel
     const int off = tile_offset(n, k);
     *(__nv_bfloat16*)(rec + (2 * par) * kATile + off) = h;
     *(__nv_bfloat16*)(rec + (2 * par + 1) * kATile + off) = lo;
+  }
+}
+
+// The velocity's 12 fields u_i = A_i psi and A_k u_i (A_k = iL_k; column 2f,
+// 2f + 1 with f = i and 3 + 3i + k) from the analysis a (lap: psi = D_inv a) or
+// the stream function, straight into the A tiles: one thread per (m, l) reads
+// the orders m-2 .. m+2 and works in float-float (the FP64 pipe made the
+// inverse Laplacian, two ladder passes over FP64 fields and the tile builder
+// 197 us at L = 1024; 2^-47 is far inside the tiles' split, 2^-17).  psi at
+// negative orders from a_{l,-k} = (-1)^k conj(a_lk).  The tiles hold the FP64
+// values truncated to FP32: where a float-float value sits on a truncation
+// boundary to its rounding level (m / (l (l+1)) and c_m^2 often make the exact
+// value one of 24 bits) the FP64 arithmetic decides.
+struct ffc {
+  dev::ff x, y;
+};
+
+__device__ __forceinline__ ffc c_scale(ffc a, dev::ff s) { return ffc{dev::ff_mul(a.x, s), dev::ff_mul(a.y, s)}; }
+__device__ __forceinline__ ffc c_add(ffc a, ffc b) { return ffc{dev::ff_add(a.x, b.x), dev::ff_add(a.y, b.y)}; }
+__device__ __forceinline__ ffc c_sub(ffc a, ffc b) { return ffc{dev::ff_sub(a.x, b.x), dev::ff_sub(a.y, b.y)}; }
+__device__ __forceinline__ ffc c_i(ffc a) { return ffc{dev::ff_neg(a.y), a.x}; }   // i a
+// i n a for an integer n < 2^24
+__device__ __forceinline__ ffc c_im(ffc a, float n) { return c_scale(c_i(a), dev::ff{n, 0.f}); }
+
+// h + l truncated to 24 bits toward zero (h its rounding); on_edge: l within
+// 2^-42 |h|, above the arithmetic's rounding level (~2^-44).
+__device__ __forceinline__ bool on_edge(dev::ff a) { return a.h != 0.f && fabsf(a.l) <= 2.3e-13f * fabsf(a.h); }
+__device__ __forceinline__ float ff_trunc(dev::ff a) {
+  const bool back = a.l != 0.f && ((__float_as_uint(a.h) ^ __float_as_uint(a.l)) >> 31);
+  return back ? __uint_as_float(__float_as_uint(a.h) - 1u) : a.h;
+}
+
+// i(L_x, L_y, L_z) of the coefficients get(k) of degree l at order m, in FP64.
+template <class Get>
+__device__ __forceinline__ void ladder_at(const Get& get, int l, int m, double2* o) {
+  const double ll = (double)l * (double)(l + 1);
+  double2 am1, ap1;
+  if (m == 0) {
+    am1 = (l >= 1) ? get(1) : make_double2(0.0, 0.0);
+    am1 = make_double2(-am1.x, am1.y);  // -conj
+  } else {
+    am1 = get(m - 1);
+  }
+  ap1 = (m + 1 <= l) ? get(m + 1) : make_double2(0.0, 0.0);
+  const double cu = sqrt(ll - (double)m * (double)(m - 1));
+  const double cd = sqrt(ll - (double)m * (double)(m + 1));
+  const double2 up = make_double2(cu * am1.x, cu * am1.y);
+  const double2 dn = make_double2(cd * ap1.x, cd * ap1.y);
+  const double2 sx = make_double2((up.x + dn.x) / 2, (up.y + dn.y) / 2);
+  o[0] = make_double2(-sx.y, sx.x);                                   // i * sx
+  o[1] = make_double2((up.x - dn.x) / 2, (up.y - dn.y) / 2);
+  const double2 am = get(m);
+  o[2] = make_double2(-(double)m * am.y, (double)m * am.x);           // i m a
+}
+
+// The 12 fields at (m, l) in FP64 (rarely needed).
+__device__ __noinline__ void velocity_fields_fp64(const double2* __restrict__ a, int L, int l, int m, int lap, float* w) {
+  const double d = lap ? (l == 0 ? 0.0 : -1.0 / ((double)l * (double)(l + 1))) : 1.0;
+  auto psi = [&](int k) {
+    const double2 z = a[(int64_t)k * L + l];
+    return make_double2(z.x * d, z.y * d);
+  };
+  double2 u[3][3];   // u_i at orders m-1 (or 1 for m = 0), m, m+1
+  for (int q = 0; q < 3; ++q) {
+    const int k = q == 0 ? (m > 0 ? m - 1 : 1) : m - 1 + q;
+    double2 o[3] = {};
+    if (k <= l) ladder_at(psi, l, k, o);
+    for (int i = 0; i < 3; ++i) u[i][q] = o[i];
+  }
+  for (int i = 0; i < 3; ++i) {
+    auto ui = [&](int k) { return u[i][k == m ? 1 : (k == m + 1 ? 2 : 0)]; };
+    double2 o[3];
+    ladder_at(ui, l, m, o);
+    w[2 * i] = dev::to_f32_trunc(u[i][1].x);
+    w[2 * i + 1] = dev::to_f32_trunc(u[i][1].y);
+    for (int k = 0; k < 3; ++k) {
+      w[2 * (3 + 3 * i + k)] = dev::to_f32_trunc(o[k].x);
+      w[2 * (3 + 3 * i + k) + 1] = dev::to_f32_trunc(o[k].y);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(128) build_velocity_atab_kernel(TcGeometry g, const double2* __restrict__ a, int lap,
+                                                                  unsigned char* __restrict__ atab) {
+  using dev::ff;
+  const int l = blockIdx.x * blockDim.x + threadIdx.x, m = blockIdx.y, L = g.L;
+  if (l >= L || l < m) return;
+  ff d{1.f, 0.f};
+  const float ll = (float)(l * (l + 1));   // exact: L <= 4096
+  if (lap) {
+    d = ff{0.f, 0.f};
+    if (l > 0) {   // -1 / (l (l+1)), one Newton step beyond the FP32 reciprocal
+      const float r = __frcp_rn(ll);
+      d = dev::two_sum(-r, -__fmul_rn(r, fmaf(-r, ll, 1.f)));
+    }
+  }
+  ffc v[5];   // psi at orders m-2 .. m+2
+#pragma unroll
+  for (int q = 0; q < 5; ++q) {
+    const int mm = m - 2 + q, k = mm < 0 ? -mm : mm;
+    ffc w{ff{0.f, 0.f}, ff{0.f, 0.f}};
+    if (k <= l) {
+      const double2 z = a[(int64_t)k * L + l];
+      w = c_scale(ffc{dev::ff_of(z.x), dev::ff_of(z.y)}, d);
+      if (mm < 0) w = (k & 1) ? ffc{dev::ff_neg(w.x), w.y} : ffc{w.x, dev::ff_neg(w.y)};
+    }
+    v[q] = w;
+  }
+  ff c[4];   // sqrt(l(l+1) - k(k-1)) / 2 at k = m-1 .. m+2
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int k = m - 1 + q, n = l * (l + 1) - k * (k - 1);
+    c[q] = ff{0.f, 0.f};
+    if (n > 0) {
+      const float f = (float)n, r = __fsqrt_rn(f);   // f exact (n < 2^24 + ...: L <= 4096)
+      const float e = __fdividef(fmaf(-r, r, f), r + r);
+      const ff t = dev::two_sum(r, e);
+      c[q] = ff{__fmul_rn(0.5f, t.h), __fmul_rn(0.5f, t.l)};
+    }
+  }
+  ffc ux[3], uy[3];   // at orders m-1, m, m+1
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const ffc up = c_scale(v[q], c[q]), dn = c_scale(v[q + 2], c[q + 1]);
+    ux[q] = c_i(c_add(up, dn));
+    uy[q] = c_sub(up, dn);
+  }
+  if (m == 0) {   // order -1 of a real field from order 1 (the rounding residue in a_l0's imaginary part drops out)
+    ux[0] = ffc{dev::ff_neg(ux[2].x), ux[2].y};
+    uy[0] = ffc{dev::ff_neg(uy[2].x), uy[2].y};
+  }
+  const float fm = (float)m;
+  const ffc x = ux[1], y = uy[1], z = c_im(v[2], fm);
+  auto Ax = [&](const ffc* f) { return c_i(c_add(c_scale(f[0], c[1]), c_scale(f[2], c[2]))); };
+  auto Ay = [&](const ffc* f) { return c_sub(c_scale(f[0], c[1]), c_scale(f[2], c[2])); };
+  const ffc xx = Ax(ux), yx = Ay(ux), xy = Ax(uy), yy = Ay(uy);   // A_x u_x, A_y u_x, A_x u_y, A_y u_y
+  const ffc zx = c_im(x, fm), zy = c_im(y, fm), zz = c_im(z, fm);
+  // A_x u_z = A_z u_x + u_y, A_y u_z = A_z u_y - u_x
+  const ffc f[12] = {x, y, z, xx, yx, zx, xy, yy, zy, c_add(zx, y), c_sub(zy, x), zz};
+  float w[kNUsed];
+  bool edge = false;
+#pragma unroll
+  for (int n = 0; n < kNUsed; ++n) {
+    const ff u = (n & 1) ? f[n >> 1].y : f[n >> 1].x;
+    w[n] = ff_trunc(u);
+    edge = edge || on_edge(u);
+  }
+  if (edge) velocity_fields_fp64(a, L, l, m, lap, w);
+  const int par = (l - m) & 1, j = (l - m) >> 1, k = j % kKc;
+  unsigned char* rec = atab + (int64_t)(g.cbase[m] + j / kKc) * kARecord + 2 * par * kATile;
+#pragma unroll
+  for (int n = 0; n < kNUsed; ++n) {
+    const __nv_bfloat16 h = __float2bfloat16_rn(w[n]);
+    const int off = tile_offset(n, k);
+    *(__nv_bfloat16*)(rec + off) = h;
+    *(__nv_bfloat16*)(rec + kATile + off) = __float2bfloat16_rn(w[n] - __bfloat162float(h));
   }
 }
 
@@ -689,36 +846,52 @@ __global__ void build_ftab_kernel(TcFwdGeometry g, const double* __restrict__ ct
 // ring FFTs, rows 0..2L used.
 // slot: the field's column pair (2 slot, 2 slot + 1) of the 16-column data
 // tiles (0 for a plan's own tiles; a batch's member index in shared tiles).
-__global__ void build_xtab_kernel(TcFwdGeometry g, const float2* __restrict__ fine,
-                                  const double* __restrict__ w, unsigned char* __restrict__ xtab,
-                                  int slot) {
-  const int m = blockIdx.y;
-  const int L = g.L;
-  // only the field's 2 columns (re, im); the other columns are zeroed once
-  // when the tiles are made and written only by the other slots' fields
-  const int total = g.nck * 2 * 2 * kKc;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
-    const int c = e / (2 * 2 * kKc), r = e % (2 * 2 * kKc);
-    const int par = r / (2 * kKc), n = (r / kKc) % 2, k = r % kKc;
-    const int j = c * kKc + k;
-    float v = 0.f;
-    if (j <= L) {   // FP32 throughout: the samples are FP32, the split keeps 2^-17
+// One block makes the tiles of 16 orders for one chunk: the rings are read
+// along the orders (16 of them: 128-byte rows), folded, and turned in shared
+// memory so that eight ring pairs of a column go out as one 16-byte store.
+constexpr int kXm = 16;
+
+__global__ void __launch_bounds__(256) build_xtab_kernel(TcFwdGeometry g, const float2* __restrict__ fine,
+                                                         const double* __restrict__ w,
+                                                         unsigned char* __restrict__ xtab, int slot) {
+  __shared__ float v[4][kXm][kKc + 1];   // (parity, re/im), order, ring pair
+  const int c = blockIdx.x, m0 = blockIdx.y * kXm, L = g.L;
+  for (int e = threadIdx.x; e < kXm * kKc; e += 256) {
+    const int dm = e % kXm, k = e / kXm, m = m0 + dm, j = c * kKc + k;
+    float2 ev = make_float2(0.f, 0.f), od = ev;
+    if (j <= L && m < L) {   // FP32 throughout: the samples are FP32, the split keeps 2^-17
       const float2 a = fine[(int64_t)j * L + m];
-      float2 s;
+      const float wj = dev::to_f32_trunc(w[j]);
+      ev = a;
       if (j < L) {
         const float2 b = fine[(int64_t)(2 * L - j) * L + m];
-        s = par == 0 ? make_float2(a.x + b.x, a.y + b.y) : make_float2(a.x - b.x, a.y - b.y);
-      } else {
-        s = par == 0 ? a : make_float2(0.f, 0.f);
+        ev = make_float2(a.x + b.x, a.y + b.y);
+        od = make_float2(a.x - b.x, a.y - b.y);
       }
-      v = dev::to_f32_trunc(w[j]) * (n == 0 ? s.x : s.y);
+      ev = make_float2(wj * ev.x, wj * ev.y);
+      od = make_float2(wj * od.x, wj * od.y);
     }
-    const __nv_bfloat16 h = __float2bfloat16_rn(v);
-    const __nv_bfloat16 lo = __float2bfloat16_rn(v - __bfloat162float(h));
-    unsigned char* rec = xtab + ((int64_t)m * g.nck + c) * kXRecord;
-    const int off = tile_offset(2 * slot + n, k);
-    *(__nv_bfloat16*)(rec + (2 * par) * kXTile + off) = h;
-    *(__nv_bfloat16*)(rec + (2 * par + 1) * kXTile + off) = lo;
+    v[0][dm][k] = ev.x;
+    v[1][dm][k] = ev.y;
+    v[2][dm][k] = od.x;
+    v[3][dm][k] = od.y;
+  }
+  __syncthreads();
+  // (order, parity, re/im, group of 8 pairs) per thread
+  for (int e = threadIdx.x; e < kXm * 4 * (kKc / 8); e += 256) {
+    const int kg = e % (kKc / 8), pn = (e / (kKc / 8)) % 4, dm = e / (4 * (kKc / 8)), m = m0 + dm;
+    if (m >= L) continue;
+    __align__(16) __nv_bfloat16 hi[8], lo[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const float x = v[pn][dm][8 * kg + q];
+      hi[q] = __float2bfloat16_rn(x);
+      lo[q] = __float2bfloat16_rn(x - __bfloat162float(hi[q]));
+    }
+    unsigned char* rec = xtab + ((int64_t)m * g.nck + c) * kXRecord + 2 * (pn >> 1) * kXTile;
+    const int off = tile_offset(2 * slot + (pn & 1), 8 * kg);
+    *(uint4*)(rec + off) = *(const uint4*)hi;
+    *(uint4*)(rec + kXTile + off) = *(const uint4*)lo;
   }
 }
 
@@ -1003,11 +1176,20 @@ int tc_wait_timeout_probe(long long polls, int* status, cudaStream_t s) {
 
 void tc_set_schedule(TcPlan* p, int schedule) { p->schedule = schedule; }
 
-int tc_synthesis(TcPlan* p, const double2* fields, float2* S, int* status, cudaStream_t s) {
+int tc_field_tiles(TcPlan* p, const double2* fields, cudaStream_t s) {
   TcGeometry g{p->L, p->npair, p->nrb, (const int*)p->tab->cbase.p};
   build_atab_kernel<<<dim3(16, p->L), 256, 0, s>>>(g, fields, (unsigned char*)p->atab.p);
-  int rc = check("build_atab_kernel");
-  if (rc) return rc;
+  return check("build_atab_kernel");
+}
+
+int tc_velocity_tiles(TcPlan* p, const double2* a, bool lap, cudaStream_t s) {
+  TcGeometry g{p->L, p->npair, p->nrb, (const int*)p->tab->cbase.p};
+  build_velocity_atab_kernel<<<dim3((p->L + 127) / 128, p->L), 128, 0, s>>>(g, a, lap, (unsigned char*)p->atab.p);
+  return check("build_velocity_atab_kernel");
+}
+
+int tc_synthesis(TcPlan* p, float2* S, int* status, cudaStream_t s) {
+  TcGeometry g{p->L, p->npair, p->nrb, (const int*)p->tab->cbase.p};
   const int nitems = p->L * p->nrb;
   const int grid = std::min(nitems, std::max(p->sms, 1));
   if (p->schedule == 1) {
@@ -1035,7 +1217,7 @@ int tc_analysis_tiles(TcPlan* p, const float2* fine, const double* w, unsigned c
                       cudaStream_t s) {
   const int L = p->L;
   TcFwdGeometry g{L, p->nck, (const int*)p->tab->lbase.p};
-  build_xtab_kernel<<<dim3(8, L), 256, 0, s>>>(g, fine, w, xtab, slot);
+  build_xtab_kernel<<<dim3(p->nck, (L + kXm - 1) / kXm), 256, 0, s>>>(g, fine, w, xtab, slot);
   return check("build_xtab_kernel");
 }
 

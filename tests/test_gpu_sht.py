@@ -431,3 +431,32 @@ def test_velocity_jets_of_six_fields_against_oracle(nat, L, mode):
     vm = nat.VelMesh(L, theta, phi, g, verts)
     got = nat.Sht(L).set_tables(mode).velocity(vm, dev(om)).cpu().numpy()
     assert np.abs(got - ref).max() < 1e-12 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("L", [32, 65, 200])
+def test_split_velocity_tiles_match_the_field_route(nat, L):
+    """The split-BF16 velocity's data tiles, made straight from the analysis
+    in float-float, against the twelve FP64 coefficient fields of the same
+    analysis put through the synthesis (cmm_sht_inverse): the tiles hold the
+    FP64 values truncated to FP32, so the value jets u_i away from the poles
+    agree but for values next to a truncation boundary (2^-40 of them; a
+    whole FP32 unit is 6e-8)."""
+    theta, phi, g, verts, Phi, The = grid(L)
+    rng = np.random.default_rng(L)
+    om = 3 * np.cos(The) ** 3 + np.sin(The) ** 2 * np.sin(2 * Phi) + 0.1 * rng.standard_normal(Phi.shape)
+    om[0], om[-1] = om[0, 0], om[-1, 0]
+    vm = nat.VelMesh(L, theta, phi, g, verts)
+    tc = nat.Sht(L).set_precision(nat.Sht.SPLIT_BF16)
+    jets = tc.velocity(vm, dev(om)).cpu().numpy()
+    a = tc.forward(dev(om)).cpu().numpy().T                       # [l, m]
+    psi = S.shifted_from_vec(S.full_from_half(a), L) * S.inverse_laplacian_diag(L)[:, None]
+    lp, lm, lz = S.ladder_operators(L)
+    u = S.angular_momentum(psi, lp, lm, lz)
+    fields = list(u) + [f for x in u for f in S.angular_momentum(x, lp, lm, lz)]
+    half = [S.half_from_full(S.vec_from_shifted(f, L), L).T for f in fields]
+    smp = tc.inverse(dev(np.stack([np.triu(h) for h in half]))).cpu().numpy()
+    scale = np.abs(jets[:, 0]).max()
+    for i in range(3):
+        got, ref = jets[i, 0, 1:-1], smp[i, 1:-1].reshape(-1)
+        assert np.abs(got - ref).max() < 1e-6 * scale
+    assert tc.status() == 0
