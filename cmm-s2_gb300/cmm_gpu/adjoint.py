@@ -26,26 +26,28 @@ def _s(dev):
 
 
 # ------------------------------------------------------ SH coefficient maps
+def _lm(lmax):
+    """l, m of the half layout [l, m] and its mask m <= l."""
+    l, m = np.arange(lmax + 1)[:, None], np.arange(lmax + 1)[None]
+    return l, m, m <= l
+
+
 def real_to_complex(a):
     """Real series (lmax+1, 2 lmax+1) (column l+m; m > 0 sqrt2 cos, m < 0
     sqrt2 sin) -> complex half layout c[l, m] (m >= 0) of the same field."""
-    lmax = a.shape[0] - 1
-    c = np.zeros((lmax + 1, lmax + 1), dtype=complex)
-    for l in range(lmax + 1):
-        c[l, 0] = a[l, l]
-        for m in range(1, l + 1):
-            c[l, m] = (a[l, l + m] - 1j * a[l, l - m]) / np.sqrt(2)
-    return c
+    l, m, half = _lm(a.shape[0] - 1)
+    c = (np.take_along_axis(a, l + np.where(half, m, 0), 1)
+         - 1j * np.take_along_axis(a, l - np.where(half, m, 0), 1)) / np.sqrt(2)
+    c[:, 0] = a[l[:, 0], l[:, 0]]
+    return np.where(half, c, 0.0)
 
 
 def complex_to_real(c):
     lmax = c.shape[0] - 1
     a = np.zeros((lmax + 1, 2 * lmax + 1))
-    for l in range(lmax + 1):
-        a[l, l] = c[l, 0].real
-        for m in range(1, l + 1):
-            a[l, l + m] = np.sqrt(2) * c[l, m].real
-            a[l, l - m] = -np.sqrt(2) * c[l, m].imag
+    l, m = np.nonzero(_lm(lmax)[2])
+    a[l, l - m] = -np.sqrt(2) * c[l, m].imag
+    a[l, l + m] = np.where(m == 0, 1.0, np.sqrt(2)) * c[l, m].real
     return a
 
 
@@ -55,19 +57,22 @@ def il_series(a):
     a_{l,-1} = -conj(a_{l,1}) for a real field); the tangent gradient of f
     at a unit point x is -x cross (iL f)(x).  Returns (3, lmax+1, 2 lmax+1)."""
     c = real_to_complex(np.asarray(a, dtype=np.float64))
-    lmax = c.shape[0] - 1
-    out = [np.zeros_like(c) for _ in range(3)]
-    for l in range(lmax + 1):
-        ll = l * (l + 1.0)
-        for m in range(0, l + 1):
-            am1 = -np.conj(c[l, 1]) if m == 0 and l >= 1 else (c[l, m - 1] if m >= 1 else 0.0)
-            ap1 = c[l, m + 1] if m + 1 <= l else 0.0
-            up = np.sqrt(ll - m * (m - 1.0)) * am1
-            dn = np.sqrt(ll - m * (m + 1.0)) * ap1
-            out[0][l, m] = 1j * (up + dn) / 2
-            out[1][l, m] = (up - dn) / 2
-            out[2][l, m] = 1j * m * c[l, m]
-    return np.stack([complex_to_real(o) for o in out])
+    l, m, half = _lm(c.shape[0] - 1)
+    ll = l * (l + 1.0)
+    am1, ap1 = np.zeros_like(c), np.zeros_like(c)
+    am1[:, 1:] = c[:, :-1]
+    ap1[:, :-1] = c[:, 1:]
+    if c.shape[0] > 1:
+        am1[:, 0] = -np.conj(c[:, 1])
+    up = np.sqrt(np.maximum(ll - m * (m - 1.0), 0.0)) * am1
+    dn = np.sqrt(np.maximum(ll - m * (m + 1.0), 0.0)) * ap1
+    return np.stack([complex_to_real(np.where(half, o, 0.0))
+                     for o in (1j * (up + dn) / 2, (up - dn) / 2, 1j * m * c)])
+
+
+def il_series_of(sh):
+    """il_series of a device series, on its device (one copy each way)."""
+    return torch.from_numpy(il_series(sh.detach().cpu().numpy())).to(sh.device)
 
 
 # ------------------------------------------------------- autograd Functions
@@ -119,26 +124,29 @@ class Compose(torch.autograd.Function):
 
 class Vorticity(torch.autograd.Function):
     """omega (L+1, 2L) at the back-traced points X (Q,3) from the real
-    series sh and the planetary term (cmm_vorticity_eval, kind NONE)."""
+    series sh and the planetary term (cmm_vorticity_eval, kind NONE).
+    dsh: il_series_of(sh) where the caller has it (the backward pass makes it
+    otherwise, which waits for the device)."""
 
     @staticmethod
-    def forward(ctx, X, sh, vm, rot):
+    def forward(ctx, X, sh, vm, rot, dsh=None):
         ctx.vm, ctx.rot = vm, rot
-        ctx.save_for_backward(X, sh)
+        ctx.save_for_backward(X, sh, dsh)
         return vm.vorticity(native.VORT_NONE, [], X.detach(), rot, sh=sh.detach())
 
     @staticmethod
     def backward(ctx, gw):
-        X, sh = ctx.saved_tensors
+        X, sh, dsh = ctx.saved_tensors
         vm = ctx.vm
         lmax = sh.shape[0] - 1
-        dsh = torch.from_numpy(il_series(sh.detach().cpu().numpy())).to(X.device)
+        if dsh is None:
+            dsh = il_series_of(sh)
         gX = torch.zeros_like(X)
         gsh = torch.zeros_like(sh)
         native.check(native.lib.cmm_vorticity_bwd(vm.h, native._ptr(dsh), lmax, ctx.rot, native._ptr(X),
                                                   native._ptr(gw.contiguous()), native._ptr(gX),
                                                   native._ptr(gsh), _s(X.device)), "cmm_vorticity_bwd")
-        return gX, gsh, None, None
+        return gX, gsh, None, None, None
 
 
 class Velocity(torch.autograd.Function):
@@ -226,8 +234,8 @@ class BVEGradient:
         self.empty = torch.empty(0, dtype=torch.float64, device=dev)
 
     # pieces
-    def _project(self, X, sh, rot):
-        om = Vorticity.apply(X, sh, self.vm, rot)
+    def _project(self, X, sh, rot, dsh):
+        om = Vorticity.apply(X, sh, self.vm, rot, dsh)
         return Assemble.apply(Velocity.apply(om, self.sht, self.vm), self.vm), om
 
     def _advect(self, prev, vel, nvs, ts0, scheme, t):
@@ -243,21 +251,23 @@ class BVEGradient:
         """Vorticity (L+1, 2L) on the grid at the end of the run."""
         dt, ts0 = self.dt, float(self.tspan[0])
         E, IE, RK = native.EULER, native.IMPROVED_EULER, native.RK4
+        # the series' angular-momentum images, once for every step's backward
+        dsh = il_series_of(sh) if torch.is_grad_enabled() and sh.requires_grad else None
         # bootstrap (spherical_simulations.py:216-261)
-        v0, _ = self._project(self.sample, sh, 0.0)
+        v0, _ = self._project(self.sample, sh, 0.0, dsh)
         c = self._advect(None, [v0], 1, ts0, E, 0.0)
-        v1, _ = self._project(self._sample([c]), sh, self.rot)
+        v1, _ = self._project(self._sample([c]), sh, self.rot, dsh)
         c = self._advect(None, [v0, v1], 2, ts0, IE, 0.0)
-        v1, _ = self._project(self._sample([c]), sh, self.rot)
+        v1, _ = self._project(self._sample([c]), sh, self.rot, dsh)
         c = self._advect(c, [v0, v1], 2, ts0, RK, dt)
-        v2, om = self._project(self._sample([c]), sh, self.rot)
+        v2, om = self._project(self._sample([c]), sh, self.rot, dsh)
         state = dict(c=c, vel=[v0, v1, v2], stack=[], identity=False, count=2, ts0=ts0, k=2, om=om)
         while state["count"] < self.Nt:
             nsteps = min(self.block, self.Nt - state["count"])
-            state = self._run_block(state, sh, nsteps)
+            state = self._run_block(state, sh, dsh, nsteps)
         return state["om"]
 
-    def _steps(self, nsteps, k0, count0, ts00, identity0, nstack, sh, c, v0, v1, v2, *stack):
+    def _steps(self, nsteps, k0, count0, ts00, identity0, nstack, sh, dsh, c, v0, v1, v2, *stack):
         """nsteps main-loop steps (spherical_simulations.py:263-294) as a
         pure function of tensors (for checkpointing)."""
         vel, stack, identity, count, ts0 = [v0, v1, v2], list(stack), identity0, count0, ts00
@@ -266,7 +276,7 @@ class BVEGradient:
             t = float(self.tspan[k0 + j])
             c = self._advect(None if identity else c, vel, 3, ts0, native.RK4, t)
             X = self._sample(stack + [c])
-            vn, om = self._project(X, sh, self.rot)
+            vn, om = self._project(X, sh, self.rot, dsh)
             vel = [vel[1], vel[2], vn]
             ts0 += self.dt
             count += 1
@@ -276,9 +286,9 @@ class BVEGradient:
                 identity = True
         return (c, *vel, om, *stack[nstack:])
 
-    def _run_block(self, st, sh, nsteps):
+    def _run_block(self, st, sh, dsh, nsteps):
         ns_before = len(st["stack"])
-        args = (nsteps, st["k"], st["count"], st["ts0"], st["identity"], ns_before, sh, st["c"], *st["vel"],
+        args = (nsteps, st["k"], st["count"], st["ts0"], st["identity"], ns_before, sh, dsh, st["c"], *st["vel"],
                 *st["stack"])
         out = checkpoint(self._steps, *args, use_reentrant=False)
         c, v0, v1, v2, om, *new = out
