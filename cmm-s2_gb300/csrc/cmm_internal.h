@@ -12,7 +12,8 @@ namespace cmm {
 
 // Per-triangle location record (doubles): rows r1,r2,r3 of the inverse of
 // the vertex matrix [v1 v2 v3] (bcc_i = r_i . q), then |v1+v2+v3|,
-// |v1+v2|, |v2+v3|, |v3+v1|, 3 doubles of padding.
+// |v1+v2|, |v2+v3|, |v3+v1|, then 3 doubles: v1 on a lat-lon mesh, padding
+// on an icosahedral one.
 constexpr int kLocStride = 16;
 // Per-triangle assembly factors (doubles): for each of the 9 gradient
 // ordinates 3..11 (a_x, a_y, a_z, b) with c = a . grad f(v) - b f(v);
@@ -75,13 +76,14 @@ struct MeshView {
   const double* ring_n;
   const double* diag_n;
   double dphi, dthe;
+  int loc_exp;              // every entry of the inverse vertex rows is below 2^loc_exp
   // velocity records (ncomp = 3) in FP32 (cmm_velmesh_set_records):
   // (nt, 64) floats, assembled from the FP32 copy of the factors
   int rec32;
   const float* tri_asm_f;   // (kAsmFactors, nt), factor-major, when rec32
   int field32;              // analytic initial vorticity fields in FP32
   const float* tri_loc_f;   // (nt, kLocStride) FP32 copy of the location records, when rec32
-  float phi0_f, dphi_f, the0_f, dthe_f;   // FP32 copies of phi[0], dphi, theta[0], dthe
+  float phi0_f, idphi_f, the0_f, idthe_f;   // FP32 copies of phi[0], 1/dphi, theta[0], 1/dthe
   // recurrence table of the orthonormal associated Legendre functions for
   // real SH series of degree <= kShTableMax: sh_ab[2 (m (kShTableMax+1) + l)]
   // = (a_lm, b_lm), sh_fm[m] = sqrt((2m+1)/(2m))

@@ -522,46 +522,79 @@ static __device__ __noinline__ int latlon_locate_exact(const MeshView& m, double
   return N + 2 * (N * (theta_l - 1) + phi_l) + s;
 }
 
+// Sign of n.q for a tabulated side-test normal: FP32 where the value is
+// beyond its error bound (both factors truncated to 2^-23, four roundings:
+// below 5e-7 of the sum |n_i| at |q_i| <= 1), else FP64; 0 where the FP64
+// value is within tiny.
+__device__ __forceinline__ int side_sign(const D3 n, const PointD& q, float fx, float fy, float fz, double tiny) {
+  const float nx = to_f32_trunc(n.x), ny = to_f32_trunc(n.y), nz = to_f32_trunc(n.z);
+  const float d = fmaf(nx, fx, fmaf(ny, fy, nz * fz));
+  const float big = fmaxf(1.f, fmaxf(fabsf(fx), fmaxf(fabsf(fy), fabsf(fz))));
+  if (fabsf(d) > 1e-6f * big * (fabsf(nx) + fabsf(ny) + fabsf(nz)) && fabsf(d) > 1e-12f) return d > 0.f ? 1 : -1;
+  const double e = n.x * q.x + n.y * q.y + n.z * q.z;
+  return fabs(e) <= tiny ? 0 : (e > 0.0 ? 1 : -1);
+}
+
 // The same location with the angles taken in FP32 (FP64 atan2/fmod cost
-// ~100 FP64 instructions on a part whose FP64 rate is 1/58 of FP32): the
-// cell indices and the row-correction thresholds are read off the FP32
-// angles when every fractional part is farther than the FP32 error bound
-// (2e-6 rad, scaled to cell units) from a decision boundary; the sign tests
-// then run in FP64 against q and are trusted when |n.q| > 1e-13 (the
-// re-synthesised point q0 of the reference differs from q by ~1e-16).
-// Otherwise the exact FP64 path decides, so both give the same triangle.
+// ~250 FP64 instructions on a part whose FP64 rate is 1/58 of FP32): the
+// cell indices are read off the FP32 angles when every fractional part is
+// farther than the FP32 error bound (2.5e-6 rad, scaled to cell units) from a
+// cell boundary; next to a boundary (1e-3 of the queries at L = 512, so a
+// twentieth of the warps) the side of that meridian or parallel is taken from
+// its tabulated ring points in FP64.  The row-correction tests run against q
+// (side_sign); whether one is made at fv ~ 0.03 or 0.85 does not matter where
+// the great circles bulge less than that off their parallels (L >= 32: by
+// pi/16L of a row), else an undecided threshold goes to the exact path.  All
+// sign tests are trusted beyond 1e-13 (the re-synthesised point q0 of the
+// reference differs from q by ~1e-16); within it the exact FP64 path decides,
+// so both give the same triangle.
 __device__ __forceinline__ int latlon_locate(const MeshView& m, double x, double y, double z) {
   const int N = 2 * m.L, M = m.L + 1;
   const float xf = to_f32_trunc(x), yf = to_f32_trunc(y), zf = to_f32_trunc(z);
   float phif = atan2f(yf, xf);
   if (phif < 0.f) phif += 6.28318530717958647692f;
   const float thef = atan2f(sqrtf(xf * xf + yf * yf), zf);
-  const float u = (phif - m.phi0_f) / m.dphi_f;
-  const float v = (thef - m.the0_f) / m.dthe_f;
-  const float du = 2e-6f / m.dphi_f, dv = 2e-6f / m.dthe_f;
+  const float u = (phif - m.phi0_f) * m.idphi_f;
+  const float v = (thef - m.the0_f) * m.idthe_f;
+  const float du = 2.5e-6f * m.idphi_f, dv = 2.5e-6f * m.idthe_f;   // the factors' rounding included
   const float uf = floorf(u), vf = floorf(v);
-  const float fu = u - uf, fv = v - vf;
-  const int phi_l = (int)uf;
-  int theta_l = (int)vf;
-  if (!(fu > du && fu < 1.f - du && fv > dv && fv < 1.f - dv && fabsf(fv - 0.03f) > dv &&
-        fabsf(fv - 0.85f) > dv && phi_l >= 0 && phi_l < N && theta_l >= 0 && theta_l <= M - 2))
+  const float fu = u - uf;
+  float fv = v - vf;
+  int phi_l = (int)uf, theta_l = (int)vf;
+  if (!(u >= -1.f && u <= N + 1.f && v >= -1.f && v <= M && du < 0.25f && dv < 0.25f))   // also NaN
     return latlon_locate_exact(m, x, y, z);
-  const D3 q = D3{x, y, z};
+  if (!(fu > du && fu < 1.f - du)) {
+    int k = (int)rintf(u);
+    k = k >= N ? k - N : (k < 0 ? k + N : k);
+    const double2 g = __ldg(reinterpret_cast<const double2*>(m.grid + 4 * ((int64_t)(m.L / 2) * N + k)));
+    const double s = g.x * y - g.y * x;   // on the side of sector k
+    if (!(fabs(s) > 1e-13)) return latlon_locate_exact(m, x, y, z);
+    phi_l = s > 0.0 ? k : (k == 0 ? N - 1 : k - 1);
+  }
+  if (!(fv > dv && fv < 1.f - dv)) {
+    const int k = min(max((int)rintf(v), 0), M - 1);
+    const double* g = m.grid + 4 * (int64_t)k * N;
+    const double gx = __ldg(g), gy = __ldg(g + 1), gz = __ldg(g + 2);
+    const double s = sqrt(x * x + y * y) * gz - z * sqrt(gx * gx + gy * gy);   // south of ring k
+    if (!(fabs(s) > 1e-13)) return latlon_locate_exact(m, x, y, z);
+    theta_l = s > 0.0 ? k : k - 1;
+    fv = s > 0.0 ? 0.f : 1.f;
+  } else if (m.L < 32 && !(fabsf(fv - 0.03f) > dv && fabsf(fv - 0.85f) > dv)) {
+    return latlon_locate_exact(m, x, y, z);
+  }
+  if (!(phi_l >= 0 && phi_l < N && theta_l >= 0 && theta_l <= M - 2)) return latlon_locate_exact(m, x, y, z);
+  const PointD q{x, y, z};
   const bool row_lo = fv <= 0.03f && theta_l != 0;
   const bool row_hi = !row_lo && fv > 0.85f && theta_l != M - 2;
-  if (row_lo) {
-    const double d = dot(ring_normal(m, theta_l, phi_l), q);
-    if (fabs(d) <= 1e-13) return latlon_locate_exact(m, x, y, z);
-    if (d > 0.0) theta_l -= 1;
-  } else if (row_hi) {
-    const double d = -dot(ring_normal(m, theta_l + 1, phi_l), q);
-    if (fabs(d) <= 1e-13) return latlon_locate_exact(m, x, y, z);
-    if (d > 0.0) theta_l += 1;
+  if (row_lo || row_hi) {
+    const int sg = side_sign(ring_normal(m, row_lo ? theta_l : theta_l + 1, phi_l), q, xf, yf, zf, 1e-13);
+    if (sg == 0) return latlon_locate_exact(m, x, y, z);
+    if (row_lo && sg > 0) theta_l -= 1;
+    if (row_hi && sg < 0) theta_l += 1;
   }
   if (theta_l == 0) return phi_l;
   if (theta_l == M - 2) return 2 * N * (M - 2) - N + phi_l;
-  const D3 n = diag_normal(m, theta_l, phi_l);
-  const int s = (-dot(n, q) > 0.0) ? 1 : 0;
+  const int s = side_sign(diag_normal(m, theta_l, phi_l), q, xf, yf, zf, 0.0) < 0 ? 1 : 0;
   return N + 2 * (N * (theta_l - 1) + phi_l) + s;
 }
 

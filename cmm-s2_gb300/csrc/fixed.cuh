@@ -42,19 +42,37 @@ struct FxSum {
   __device__ __forceinline__ long long value() const { return hi + (lo >> 30); }
 };
 
-// A form entry |q| < 2 as limbs (2^-59 steps, toward zero), from the
-// double's bits; where |q| >= 2 or q is not finite the sign bit of `bad` is
-// set (the limbs are then meaningless).
-__device__ __forceinline__ Limbs fx_entry(double q, int& bad) {
-  const int hi = __double2hiint(q);
-  const unsigned lo = (unsigned)__double2loint(q);
-  const int e = 1023 - (int)(((unsigned)hi << 1) >> 21);   // right shift of the 53-bit significand << 7
+// v / 2^(eb - 1022), at most 1 in magnitude where eb is the largest biased
+// exponent met, as limbs (2^-59 steps, toward zero), from the double's bits;
+// where v is larger (its exponent above eb) or not finite the sign bit of
+// `bad` is set and the limbs are meaningless.
+__device__ __forceinline__ Limbs fx_scaled(double v, int eb, int& bad) {
+  const int hi = __double2hiint(v);
+  const unsigned lo = (unsigned)__double2loint(v);
+  const int e = eb + 1 - (int)(((unsigned)hi << 1) >> 21);   // right shift of the 53-bit significand << 7
   bad |= e;
   const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;
   unsigned long long T = ((((unsigned long long)mh) << 32) | lo) << 7;
   asm("shr.u64 %0, %1, %2;" : "=l"(T) : "l"(T), "r"(e));   // 0 from a shift of 64 on
   const int sg = (hi >> 31) | 1;
   return Limbs{(int)(T >> 30) * sg, (int)((unsigned)T & 0x3fffffffu) * sg};
+}
+
+// A form entry |q| < 2 as limbs.
+__device__ __forceinline__ Limbs fx_entry(double q, int& bad) { return fx_scaled(q, 1022, bad); }
+
+// Biased exponent of a double.
+__device__ __forceinline__ int fx_exponent(double v) { return (int)(((unsigned)__double2hiint(v) << 1) >> 21); }
+
+// X 2^(eb - 1022 - 58) as a double (truncated toward zero, 59 <= eb < 2000),
+// from the bits: the conversion and the scaling would take the FP64 pipe.
+__device__ __forceinline__ double fx_to_double(long long X, int eb) {
+  unsigned long long M = X < 0 ? (unsigned long long)-X : (unsigned long long)X;
+  const int n = __clzll(M);
+  if (n == 64) return 0.0;
+  M <<= n;   // leading bit at 63: value 2^(63 - n)
+  const unsigned hi = ((unsigned)(M >> 43) & 0xfffffu) | ((unsigned)(eb - 1080 + 1023 + 63 - n) << 20);
+  return __hiloint2double((int)(hi | (X < 0 ? 0x80000000u : 0u)), (int)(unsigned)(M >> 11));
 }
 
 // x, |x| < 16, in units of 2^-58 (toward zero)

@@ -17,6 +17,7 @@
 
 #include "cmm_internal.h"
 #include "device_common.cuh"
+#include "fixed.cuh"
 #include "geom.h"
 #include "integrators.cuh"
 
@@ -36,15 +37,127 @@ struct W3 {
   double a, b, c;
 };
 
-__device__ __forceinline__ W3 stage(const TimeWeights& tw, int s) {
+// The stage's weights from the kernel parameters or (st) a device-driven
+// step's state.
+__device__ __forceinline__ W3 stage(const TimeWeights& tw, int s, const BveState* st = nullptr) {
+  if (st) return W3{__ldg(&st->tw.w[s][0]), __ldg(&st->tw.w[s][1]), __ldg(&st->tw.w[s][2])};
   return W3{tw.w[s][0], tw.w[s][1], tw.w[s][2]};
+}
+
+// FP64 records in FP64: points off the unit sphere, weights of 2 or more,
+// ordinates near the ends of the exponent range.
+__device__ __noinline__ void velocity_wide(const MeshView& m, const VelPtrs& vc, int nvs, const W3 w, int t, double x,
+                                           double y, double z, double* V) {
+  V[0] = V[1] = V[2] = 0.0;
+  double Lr[13];
+  load_loc(m, t, Lr);
+  const Bcc b = bcc_of(Lr, x, y, z);
+  const Split sp = split_of(b);
+  const Gam g = gamma_of(Lr, b, sp);
+#pragma unroll
+  for (int l = 0; l < 3; ++l) {
+    if (l >= nvs) break;
+    const double wl = l == 0 ? w.a : (l == 1 ? w.b : w.c);
+    Ords<3> o;
+    load_ords<3>(vc.p[l] + (int64_t)t * kCoeffStride3, sp, o);
+    double P[3];
+    sbb<3>(o, g, P);
+    V[0] += wl * P[0];
+    V[1] += wl * P[1];
+    V[2] += wl * P[2];
+  }
+}
+
+
+// FP64 records in fixed point (fixed.cuh).  In FP64 an evaluation's ~110
+// operations bind the RK4 foot points on GB300 (82 % of the FP64 pipe); here
+// the FP64 pipe forms p - v1 only.  The barycentrics b = R (p - v1) + (1,0,0)
+// carry no cancellation (R p loses the triangle's inverse size, ~1/h, in
+// FP64's last places), the Bernstein weights and each level's six ordinates
+// (relative to the level's largest) go through 2^-58 steps, and the levels are
+// combined in the largest one's scale: every result is within a few 2^-57 of
+// the largest ordinate, where the FP64 sum rounds at 2^-53 per term.
+__device__ __forceinline__ void velocity_fixed(const MeshView& m, const VelPtrs& vc, int nvs, const W3 w, int t,
+                                               double x, double y, double z, double* V) {
+  const double* L = m.tri_loc + (int64_t)t * kLocStride;   // R (9), norms (4), v1 (3)
+  int bad = 0;
+  const Limbs d0 = fx_limbs(fx_of(x - __ldg(L + 13))), d1 = fx_limbs(fx_of(y - __ldg(L + 14))),
+              d2 = fx_limbs(fx_of(z - __ldg(L + 15)));
+  const int ke = m.loc_exp;   // |R| < 2^ke
+  long long b[3];
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+    FxSum v{0, 0};
+    v.add(fx_scaled(__ldg(L + 3 * r), 1022 + ke, bad), d0);
+    v.add(fx_scaled(__ldg(L + 3 * r + 1), 1022 + ke, bad), d1);
+    v.add(fx_scaled(__ldg(L + 3 * r + 2), 1022 + ke, bad), d2);
+    b[r] = (v.hi << ke) + (v.lo >> (30 - ke));
+  }
+  b[0] += 1LL << 58;
+  // argmin / argmax with the first-index rule (split_of)
+  int lo = 0, hi = 0;
+  long long bl = b[0], bh = b[0];
+  if (b[1] < bl) { bl = b[1]; lo = 1; }
+  if (b[2] < bl) { bl = b[2]; lo = 2; }
+  if (b[1] > bh) { bh = b[1]; hi = 1; }
+  if (b[2] > bh) { bh = b[2]; hi = 2; }
+  if (lo == hi) { lo = 1; hi = 0; }
+  const int mid = 3 - lo - hi;
+  const long long bm = mid == 0 ? b[0] : (mid == 1 ? b[1] : b[2]);
+  auto prod = [](Limbs p, Limbs q) {
+    FxSum v{0, 0};
+    v.add(p, q);
+    return v.value();
+  };
+  // sub-triangle barycentrics; the norms (at most 3) enter as quarters
+  const Limbs gV = fx_limbs(bh - bm);
+  const int es = hi + mid;
+  const double ne = __ldg(L + (es == 1 ? 10 : (es == 3 ? 11 : 12)));
+  const Limbs gE = fx_limbs(prod(fx_scaled(ne, 1024, bad), fx_limbs(bm - bl)) << 2);
+  const Limbs gC = fx_limbs(prod(fx_scaled(__ldg(L + 9), 1024, bad), fx_limbs(bl)) << 2);
+  const Limbs B[6] = {fx_limbs(prod(gV, gV)), fx_limbs(prod(gE, gE)), fx_limbs(prod(gC, gC)),
+                      fx_limbs(prod(gV, gE) << 1), fx_limbs(prod(gE, gC) << 1), fx_limbs(prod(gV, gC) << 1)};
+  const int* id = kSplitOrd[lo][hi];
+  // the levels' patches times their weights (halved, |w| < 2), in the scale
+  // 2^(em - 1022) of the largest ordinate so far; one level's code (three
+  // unrolled overflow the instruction cache)
+  long long U[3] = {0, 0, 0};
+  int em = 0;
+#pragma unroll 1
+  for (int l = 0; l < nvs; ++l) {
+    const double* rec = (l == 0 ? vc.p[0] : (l == 1 ? vc.p[1] : vc.p[2])) + (int64_t)t * kCoeffStride3;
+    double o[6][3];
+    int eb = 0, unused = 0;   // no ordinate is above the largest exponent
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        o[k][c] = __ldg(rec + 3 * id[k] + c);
+        eb = max(eb, fx_exponent(o[k][c]));
+      }
+    const Limbs wl = fx_scaled(l == 0 ? w.a : (l == 1 ? w.b : w.c), 1023, bad);
+    const int up = min(max(eb - em, 0), 63), dn = min(max(em - eb, 0), 63);
+    em = max(em, eb);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      FxSum v{0, 0};
+#pragma unroll
+      for (int k = 0; k < 6; ++k) v.add(fx_scaled(o[k][c], eb, unused), B[k]);
+      U[c] = (U[c] >> up) + (prod(wl, fx_limbs(v.value())) >> dn);
+    }
+  }
+  if (bad < 0 || em < 100 || em > 1900) {
+    velocity_wide(m, vc, nvs, w, t, x, y, z, V);
+    return;
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) V[c] = fx_to_double(U[c], em + 1);
 }
 
 __device__ __forceinline__ void velocity_at(const MeshView& m, const VelPtrs& vc, int nvs,
                                             const W3 w, double x, double y, double z,
                                             double* V) {
   const int t = latlon_locate(m, x, y, z);
-  V[0] = V[1] = V[2] = 0.0;
   if (m.rec32) {  // FP32 records: barycentrics, patches and time combination in FP32
     const float* Lf = m.tri_loc_f + (int64_t)t * kLocStride;
     float Lr[13];
@@ -73,41 +186,42 @@ __device__ __forceinline__ void velocity_at(const MeshView& m, const VelPtrs& vc
     V[2] = Vf[2];
     return;
   }
-  double Lr[13];
-  load_loc(m, t, Lr);
-  const Bcc b = bcc_of(Lr, x, y, z);
-  const Split sp = split_of(b);
-  const Gam g = gamma_of(Lr, b, sp);
-#pragma unroll
-  for (int l = 0; l < 3; ++l) {
-    if (l >= nvs) break;
-    const double wl = l == 0 ? w.a : (l == 1 ? w.b : w.c);
-    Ords<3> o;
-    load_ords<3>(vc.p[l] + (int64_t)t * kCoeffStride3, sp, o);
-    double P[3];
-    sbb<3>(o, g, P);
-    V[0] += wl * P[0];
-    V[1] += wl * P[1];
-    V[2] += wl * P[2];
-  }
+  const float xf = to_f32_trunc(x), yf = to_f32_trunc(y), zf = to_f32_trunc(z);
+  const float n2 = fmaf(xf, xf, fmaf(yf, yf, zf * zf));
+  if (n2 > 0.9f && n2 < 1.1f)
+    velocity_fixed(m, vc, nvs, w, t, x, y, z, V);
+  else
+    velocity_wide(m, vc, nvs, w, t, x, y, z, V);
 }
 
-// The spline velocity as the integrators' velocity source: stage s uses
-// the Lagrange weights of the scheme's s-th evaluation time.
-struct SplineVel {
-  const MeshView& m;
-  const VelPtrs& vc;
-  int nvs;
-  const TimeWeights& tw;
-  __device__ __forceinline__ void operator()(int s, double x, double y, double z, double* V) const {
-    velocity_at(m, vc, nvs, stage(tw, s), x, y, z, V);
-  }
-};
-
+// Backward foot point of x under the spline velocity: integrate_back's
+// schemes (integrators.cuh) with one copy of the velocity evaluation, whose
+// four inlined copies overflow the instruction cache.
 __device__ __forceinline__ void integrate_point(const MeshView& m, const VelPtrs& vc, int nvs,
                                                 const TimeWeights& tw, int scheme, double dt,
-                                                double* x) {
-  integrate_back(SplineVel{m, vc, nvs, tw}, scheme, dt, x);
+                                                double* x, const BveState* st = nullptr) {
+  const int n = scheme == CMM_EULER ? 1 : (scheme == CMM_RK4 ? 4 : 2);
+  double s[3] = {x[0], x[1], x[2]}, acc[3] = {0.0, 0.0, 0.0};
+#pragma unroll 1
+  for (int k = 0; k < n; ++k) {
+    double v[3];
+    velocity_at(m, vc, nvs, stage(tw, k, st), s[0], s[1], s[2], v);
+    // the stages' sum v1 + 2 v2 + 2 v3 + v4 (RK4), v1 + v2 (improved Euler),
+    // the last one alone (Euler, RK2)
+    const double f = scheme == CMM_RK4 && (k == 1 || k == 2) ? 2.0 : 1.0;
+    const bool add = scheme == CMM_RK4 || scheme == CMM_IMPROVED_EULER;
+    for (int c = 0; c < 3; ++c) acc[c] = add ? acc[c] + f * v[c] : v[c];
+    const bool last = k == n - 1;
+    // the next stage's point, or the foot point
+    double a = dt;
+    if (last)
+      a = scheme == CMM_RK4 ? dt / 6 : (scheme == CMM_IMPROVED_EULER ? dt / 2 : dt);
+    else if (scheme == CMM_RK2 || (scheme == CMM_RK4 && k < 2))
+      a = dt / 2;
+    for (int c = 0; c < 3; ++c) s[c] = x[c] - a * (last ? acc[c] : v[c]);
+    sphere_proj(s);
+  }
+  for (int c = 0; c < 3; ++c) x[c] = s[c];
 }
 
 __global__ void __launch_bounds__(kBlock) latlon_locate_kernel(MeshView m, const double* __restrict__ q,
@@ -134,7 +248,7 @@ __global__ void __launch_bounds__(kBlock) latlon_locate_kernel(MeshView m, const
 }
 
 // x, out: (3,n) component-major, as the reference's (3,N) arrays.
-__global__ void __launch_bounds__(kBlock) velocity_kernel(MeshView m, VelPtrs vc, int nvs,
+__global__ void __launch_bounds__(kBlock, 4) velocity_kernel(MeshView m, VelPtrs vc, int nvs,
                                                           TimeWeights tw, const double* __restrict__ x,
                                                           int64_t n, double* __restrict__ out) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
@@ -151,7 +265,7 @@ __global__ void __launch_bounds__(kBlock) velocity_kernel(MeshView m, VelPtrs vc
   }
 }
 
-__global__ void __launch_bounds__(kBlock) integrate_kernel(MeshView m, VelPtrs vc, int nvs,
+__global__ void __launch_bounds__(kBlock, 4) integrate_kernel(MeshView m, VelPtrs vc, int nvs,
                                                            TimeWeights tw, int scheme, double dt,
                                                            const double* __restrict__ x, int64_t n,
                                                            double* __restrict__ out) {
@@ -171,43 +285,42 @@ __global__ void __launch_bounds__(kBlock) integrate_kernel(MeshView m, VelPtrs v
 }
 
 // Foot points of the mesh vertices and of their stencil points
-// (advect, cmm_s2/core/evolution_functions.py:117-133).  Point i < nv is
-// vertex i, point nv + k*nv + v is stencil point k of vertex v.  work:
-// yn (3,nv) followed by the stencil foot points (3,4,nv).  Register cap
-// for 3 blocks of 256 (6 of 128) per SM: 80 registers and a few spills
-// beat 120 registers at 16 warps by 4-6 %.
-__global__ void __launch_bounds__(kMaxBlock, 3) advect_points_kernel(MeshView mesh, MeshView vm, VelPtrs vc,
+// (advect, cmm_s2/core/evolution_functions.py:117-133).  Five neighbouring
+// threads take a vertex and its four stencil points, 1e-5 away: they gather
+// the same records at every stage.  work: yn (3,nv) followed by the stencil
+// foot points (3,4,nv).  Level 6 / L = 512: 253 us in FP64 with the points
+// in array order, ~150 now (issue- and latency-bound: ~3000 instructions per
+// velocity, two thirds of them converting the 54 ordinates).
+__global__ void __launch_bounds__(kMaxBlock, 2) advect_points_kernel(MeshView mesh, MeshView vm, VelPtrs vc,
                                                                int nvs, TimeWeights tw, int scheme,
                                                                double dt,
                                                                const double* __restrict__ s_pts,
                                                                double* __restrict__ work,
                                                                const BveState* __restrict__ st) {
-  if (st) {
-    vc = VelPtrs{{st->vel[0], st->vel[1], st->vel[2]}};
-    tw = st->tw;
-  }
+  if (st) vc = VelPtrs{{st->vel[0], st->vel[1], st->vel[2]}};
   const int64_t nv = mesh.nv, n = 5 * nv;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t v = i / 5;
+    const int k = (int)(i - 5 * v) - 1;   // -1: the vertex, else stencil point k
+    const int64_t j = k * nv + v;         // within the (3, 4nv) stencil array
     double p[3];
-    if (i < nv) {
-      p[0] = mesh.verts[4 * i];
-      p[1] = mesh.verts[4 * i + 1];
-      p[2] = mesh.verts[4 * i + 2];
+    if (k < 0) {
+      p[0] = mesh.verts[4 * v];
+      p[1] = mesh.verts[4 * v + 1];
+      p[2] = mesh.verts[4 * v + 2];
     } else {
-      const int64_t j = i - nv;  // k*nv + v within the (3, 4nv) stencil array
       p[0] = s_pts[j];
       p[1] = s_pts[4 * nv + j];
       p[2] = s_pts[8 * nv + j];
     }
-    integrate_point(vm, vc, nvs, tw, scheme, dt, p);
+    integrate_point(vm, vc, nvs, tw, scheme, dt, p, st);
     if (!finite3(p[0], p[1], p[2])) flag(vm, CMM_FLAG_NONFINITE);
-    if (i < nv) {
-      work[i] = p[0];
-      work[nv + i] = p[1];
-      work[2 * nv + i] = p[2];
+    if (k < 0) {
+      work[v] = p[0];
+      work[nv + v] = p[1];
+      work[2 * nv + v] = p[2];
     } else {
-      const int64_t j = i - nv;
       double* sn = work + 3 * nv;
       sn[j] = p[0];
       sn[4 * nv + j] = p[1];

@@ -194,3 +194,65 @@ def test_fp32_velocity_records(nat):
     f64 = host(vm64.integrate(c64, 0.0, 2, 0.05, 0.1, dev(x)))
     f32 = host(vm32.integrate(c32, 0.0, 2, 0.05, 0.1, dev(x)))
     assert np.abs(f32 - f64).max() < 0.1 * 1e-6 * scale
+
+
+@pytest.mark.parametrize("L", [8, 40, 512])
+def test_latlon_locate_next_to_cell_boundaries(nat, L):
+    """Triangle ids of points 1e-4 .. 1e-12 rad off the rings and meridians
+    (inside the FP32 angles' error bound from 2e-6 rad on), and off the 0.03 and
+    0.85 thresholds of the row corrections, against the reference's rule."""
+    rng = np.random.default_rng(L)
+    n = 4000
+    off = rng.choice([-1.0, 1.0], n) * 10.0 ** rng.uniform(-12, -4, n)
+    theta, phi = rng.uniform(0.02, np.pi - 0.02, n), rng.uniform(0, 2 * np.pi, n)
+    h = np.pi / L
+    ring = (np.rint(theta / h) + rng.choice([0.0, 0.03, 0.85], n)) * h
+    pts = [(ring + off, phi), (theta, np.rint(phi / h) * h + off), (ring + off, np.rint(phi / h) * h - off[::-1])]
+    q = np.concatenate([np.stack([np.sin(t) * np.cos(p), np.sin(t) * np.sin(p), np.cos(t)], 1) for t, p in pts])
+    vm, _ = velmesh(nat, L)
+    tri = host(vm.locate(dev(q))[0])
+    mu = OG.LatLonMesh(L)
+    _, ref, _ = mu.query(q)
+    diff = tri != ref
+    assert (OG.edge_distance(mu.vertices, mu.simplices, ref[diff], q[diff]) <= 1e-13).all()
+    assert diff.mean() < 0.02
+
+
+@pytest.mark.parametrize("nvs", [1, 2, 3])
+def test_velocity_scales_exactly_and_at_its_limits(nat, nvs):
+    """The velocity evaluation works relative to the largest ordinate of a
+    patch, so a power of two in the jets comes out exactly; zero jets, jets
+    beyond the scaled range, weights beyond 2 (times far from the levels) and
+    points off the unit sphere take the FP64 evaluation.  Against the oracle
+    within 1e-12 of max |u| throughout."""
+    from cmm_gpu.meshgen import random_sphere_points
+    d = golden("velocity_L8.npz")
+    vm, _ = velmesh(nat, 8)
+    vals = d["vals"][:nvs]
+    vc = [vm.assemble(dev(v)) for v in vals]
+    x = dev(np.ascontiguousarray(random_sphere_points(5003, seed=3).T))
+    V = vm.velocity(vc, 0.0, 0.05, 0.1, x)
+    for k in (-300, -40, 7, 300):
+        s = [vm.assemble(dev(v * 2.0 ** k)) for v in vals]
+        assert torch.equal(vm.velocity(s, 0.0, 0.05, 0.1, x), V * 2.0 ** k)
+    scale = float(V.abs().max())
+    tiny = [vm.assemble(dev(v * 2.0 ** -1000)) for v in vals]
+    assert float((vm.velocity(tiny, 0.0, 0.05, 0.1, x) * 2.0 ** 1000 - V).abs().max()) < 1e-12 * scale
+    assert not vm.velocity([torch.zeros_like(c) for c in vc], 0.0, 0.05, 0.1, x).any()
+    # a level of another magnitude beside the others
+    if nvs > 1:
+        mixed = [vc[0] * 2.0 ** -80] + vc[1:]
+        z = [torch.zeros_like(vc[0])] + vc[1:]
+        a, b = vm.velocity(mixed, 0.0, 0.05, 0.1, x), vm.velocity(z, 0.0, 0.05, 0.1, x)
+        assert float((a - b).abs().max()) < 1e-15 * scale
+    # weights beyond 2: the same combination of the levels' own velocities
+    t = 0.93
+    w = {1: [1.0], 2: [1 - t / 0.1, t / 0.1],
+         3: [(t - 0.1) * (t - 0.2) / 0.02, -t * (t - 0.2) / 0.01, t * (t - 0.1) / 0.02]}[nvs]
+    far = vm.velocity(vc, 0.0, t, 0.1, x)
+    ref = sum(c * vm.velocity([v], 0.0, 0.0, 0.1, x) for c, v in zip(w, vc))
+    assert float((far - ref).abs().max()) < 1e-12 * scale * max(abs(c) for c in w)
+    # off the sphere: homogeneous of degree 2
+    out = vm.velocity(vc, 0.0, 0.05, 0.1, 1.5 * x)
+    assert float((out / 2.25 - V).abs().max()) < 1e-12 * scale
+    assert vm.status() == 0
