@@ -3,6 +3,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -343,4 +344,15 @@ int tc_analysis_tiles(TcPlan* p, const float2* fine, const double* w, unsigned c
 int tc_analysis_batch(TcPlan* p, const unsigned char* xtab, double2* const* alm, int n, int* status,
                       cudaStream_t s);
 int tc_wait_timeout_probe(long long polls, int* status, cudaStream_t s);
+
+// FP64 velocity synthesis by digits on the tensor cores (sht_digits.cu), L <=
+// kDigitMaxL: the digit table from the FP64 table tab[m][l - m][t] (t =
+// 0..L/2), a plan's own data tiles and column scales, and the fields (from
+// the analysis, lap, or the stream function) -> the nine ring spectra S.
+constexpr int kDigitMaxL = 1024;
+struct DigitTables;
+int digit_tables_build(int L, const double* tab, std::shared_ptr<DigitTables>* out, cudaStream_t s);
+int digit_workspace(int L, DeviceBuffer* tiles, DeviceBuffer* aexp);
+int digit_velocity(const DigitTables& t, const double* tab, const double2* a, bool lap, double2* psi_out,
+                   void* tiles, void* aexp, double2* S, int* status, cudaStream_t s);
 }  // namespace cmm

@@ -29,17 +29,17 @@
 #include <vector>
 
 #include "cmm_internal.h"
+#include "sht_fields.cuh"
 
 namespace cmm {
+
+using namespace sht;
 
 namespace {
 
 constexpr int kFields = 12;   // 3 velocity components + 3x3 gradients
 constexpr int kSynthBlock = 64;
 constexpr int kLChunk = 32;
-
-__device__ __forceinline__ double2 cmul(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
-__device__ __forceinline__ float2 cmul(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
 
 // ----------------------------------------------------------------- forward
 // Split-BF16 form: ring spectra F (L+1, L+1) -> torus columns G (2L, L),
@@ -289,17 +289,8 @@ __device__ __forceinline__ void ladder(const double2* __restrict__ a, int L, int
 // the grid: A_y u_x = A_x u_y + u_z, A_x u_z = A_z u_x + u_y, A_y u_z = A_z u_y
 // - u_x.  One pass over a (neighbouring orders m-2..m+2) in place of the
 // inverse Laplacian and two ladder passes over 12 fields, and half of the
-// Legendre synthesis, which is FP64-bound.  Velocity inversion, with the
-// analysis weights below: 207 -> 103 us at L = 128, 2.99 -> 1.61 ms at L = 512.
-__device__ __forceinline__ double2 order_value(const double2* __restrict__ a, int L, int l, int mm, double d) {
-  const int k = mm < 0 ? -mm : mm;
-  if (k > l) return make_double2(0.0, 0.0);
-  const double2 v = cmul(a[(int64_t)k * L + l], d);
-  if (k == 0) return make_double2(v.x, 0.0);   // a real field's: an imaginary part means nothing
-  if (mm >= 0) return v;   // a_{l,-k} = (-1)^k conj(a_{l,k})
-  return (k & 1) ? make_double2(-v.x, v.y) : make_double2(v.x, -v.y);
-}
-
+// Legendre synthesis.  This kernel serves plans without tables; with them
+// velocity_digits_kernel makes the fields.
 __global__ void __launch_bounds__(128) velocity_fields_kernel(const double2* __restrict__ a, int L, int lap,
                                                               double2* __restrict__ fields) {
   const int l = blockIdx.x * blockDim.x + threadIdx.x, m = blockIdx.y;
@@ -312,59 +303,16 @@ __global__ void __launch_bounds__(128) velocity_fields_kernel(const double2* __r
   }
   const double ll = (double)l * (double)(l + 1);
   const double d = lap ? (l == 0 ? 0.0 : -1.0 / ll) : 1.0;
-  double2 v[5];   // psi at orders m-2 .. m+2
-#pragma unroll
-  for (int k = 0; k < 5; ++k) v[k] = order_value(a, L, l, m - 2 + k, d);
   double c[4];    // sqrt(l(l+1) - k(k-1)) / 2 at k = m-1 .. m+2
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const double q = (double)(m - 1 + k);
     c[k] = 0.5 * sqrt(fmax(ll - q * (q - 1.0), 0.0));
   }
-  // X = (up + dn) / 2 and Y = (up - dn) / 2 at orders m-1, m, m+1: u_x = i X,
-  // u_y = Y
-  double2 X[3], Y[3];
+  double2 f[kVelLegendre];
+  velocity_fields_at(a, L, l, m, d, c, f);
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const double2 up = cmul(v[k], c[k]), dn = cmul(v[k + 2], c[k + 1]);
-    X[k] = make_double2(up.x + dn.x, up.y + dn.y);
-    Y[k] = make_double2(up.x - dn.x, up.y - dn.y);
-  }
-  const double cu = c[1], cd = c[2];
-  fields[i] = v[2];
-  fields[fs + i] = make_double2(-X[1].y, X[1].x);
-  fields[2 * fs + i] = Y[1];
-  // A_x f = i (cu f_{m-1} + cd f_{m+1}) / 2, A_y f = (cu f_{m-1} - cd f_{m+1}) / 2
-  fields[3 * fs + i] = make_double2(-(cu * X[0].x + cd * X[2].x), -(cu * X[0].y + cd * X[2].y));
-  fields[4 * fs + i] = make_double2(-(cu * Y[0].y + cd * Y[2].y), cu * Y[0].x + cd * Y[2].x);
-  fields[5 * fs + i] = make_double2(cu * Y[0].x - cd * Y[2].x, cu * Y[0].y - cd * Y[2].y);
-}
-
-// The nine ring spectra (and grid fields) of the velocity in the FP64 form:
-// u_x, u_y, u_z, A_x u_x, A_x u_y, A_y u_y, A_z u_x, A_z u_y, A_z u_z.
-constexpr int kVelLegendre = 6, kVelSpectra = 9;
-
-// Spectra of Legendre field f (velocity_fields_kernel's order) at (t, m),
-// value v, into S (9, L+1, L+1); the m = L column is zeroed beside m = 0
-// (an out-of-place C2R transform may overwrite its input).
-__device__ __forceinline__ void store_velocity_spectra(double2* __restrict__ S, int L, int f, int t, int m,
-                                                       double2 v) {
-  const int64_t row = L + 1, fs = (int64_t)(L + 1) * row, at = (int64_t)t * row + m;
-  const double2 z = make_double2(-(double)m * v.y, (double)m * v.x);   // i m v
-  const double2 zero = make_double2(0.0, 0.0);
-  const int64_t ny = (int64_t)t * row + L;
-  if (f == 0) {          // psi: u_z = i m psi, A_z u_z = -m^2 psi
-    S[2 * fs + at] = z;
-    S[8 * fs + at] = make_double2(-(double)m * z.y, (double)m * z.x);
-    if (m == 0) S[2 * fs + ny] = S[8 * fs + ny] = zero;
-  } else if (f <= 2) {   // u_x, u_y and their A_z
-    S[(f - 1) * fs + at] = v;
-    S[(f + 5) * fs + at] = z;
-    if (m == 0) S[(f - 1) * fs + ny] = S[(f + 5) * fs + ny] = zero;
-  } else {
-    S[f * fs + at] = v;
-    if (m == 0) S[f * fs + ny] = zero;
-  }
+  for (int k = 0; k < kVelLegendre; ++k) fields[k * fs + i] = f[k];
 }
 
 // power[l] = sum over all orders -l..l of |a_lm|^2 = |a_l0|^2 + 2 sum_{m>0}
@@ -508,15 +456,12 @@ __global__ void __launch_bounds__(kSynthBlock) synthesis_kernel(const double2* _
 // stages become table contractions with one thread per (m, l) and slice
 // (analysis) or per (m, ring pair, field group) (synthesis): L^3/4 doubles
 // each, 34 + 34 MB at L = 256, 0.27 + 0.27 GB at L = 512, 2.2 + 2.2 GB at
-// L = 1024.  By default (cmm_sht_set_tables)
+// L = 1024, beside the velocity synthesis' digit table (sht_digits.cu) of 1.5
+// times one of them.  By default (cmm_sht_set_tables)
 // plans with L <= kTabMaxL use them.
 constexpr int kTabMaxL = 512;
 constexpr int kTabShared = 1024;   // largest L the analysis kernel's shared arrays hold
-
-// offset of order m in a table with nj entries per (m, l): nj sum_{m'<m} (L - m')
-__device__ __host__ __forceinline__ int64_t tab_off(int m, int L, int nj) {
-  return (int64_t)nj * ((int64_t)m * L - (int64_t)m * (m - 1) / 2);
-}
+static_assert(kTabShared <= kDigitMaxL, "tables come with the digit tables");
 
 // One thread per (m, ring j): Pbar_{l,m}(theta_{j0 + dj j}), l = m..L-1, j <
 // nj, in the layout [m][l-m][j].
@@ -689,9 +634,8 @@ __global__ void __launch_bounds__(kTabBlock * kAnaSlices) analysis_w_kernel(cons
 }
 
 // Synthesis from the table: block (m, tile of ring pairs, group of G
-// fields); each thread one ring pair (t, L-t) and G fields.  VEL: the six
-// fields of velocity_fields_kernel (two groups of 3) -> the nine spectra.
-template <int G, bool VEL = false>
+// fields); each thread one ring pair (t, L-t) and G fields.
+template <int G>
 __global__ void __launch_bounds__(kTabBlock) synthesis_tab_kernel(const double2* __restrict__ alm, int L,
                                                                   const double* __restrict__ tab,
                                                                   double2* __restrict__ S) {
@@ -731,15 +675,6 @@ __global__ void __launch_bounds__(kTabBlock) synthesis_tab_kernel(const double2*
     }
   }
   if (!active) return;
-  if (VEL) {
-#pragma unroll
-    for (int f = 0; f < G; ++f) {
-      store_velocity_spectra(S, L, f0 + f, t, m, make_double2(E[f].x + O[f].x, E[f].y + O[f].y));
-      if (L - t != t)
-        store_velocity_spectra(S, L, f0 + f, L - t, m, make_double2(E[f].x - O[f].x, E[f].y - O[f].y));
-    }
-    return;
-  }
   const int64_t row = L + 1;
 #pragma unroll
   for (int f = 0; f < G; ++f) {
@@ -1206,8 +1141,10 @@ struct cmm_sht {
   // of one band-limit may hold the same tables (cmm_sht_share_tables)
   struct PbarTables {
     cmm::DeviceBuffer w, s;
+    std::shared_ptr<cmm::DigitTables> digits;   // of s, for the velocity's synthesis
   };
   std::shared_ptr<PbarTables> tab;
+  cmm::DeviceBuffer dig_tiles, dig_exp;   // this plan's data tiles for tab->digits
   int tab_mode = 0;                 // cmm_sht_set_tables: 0 auto, 1 always, -1 never
   cmm::DeviceBuffer spec, torus, pad, alm, fields, synth, samples, status;
   cmm::TcPlan* tc = nullptr;
@@ -1402,7 +1339,7 @@ static int ensure_tables(cmm_sht* p, cudaStream_t s, bool* ok) {
   *ok = false;
   const int L = p->L;
   if (p->tab_mode < 0 || (p->tab_mode == 0 && L > kTabMaxL) || L > kTabShared) return CMM_OK;
-  if (p->tab) {
+  if (p->tab && p->dig_tiles.p) {
     *ok = true;
     return CMM_OK;
   }
@@ -1412,9 +1349,14 @@ static int ensure_tables(cmm_sht* p, cudaStream_t s, bool* ok) {
     return CMM_OK;
   }
   if (cs != cudaStreamCaptureStatusNone) return CMM_OK;
+  int rc;
+  if (!p->dig_tiles.p && (rc = digit_workspace(L, &p->dig_tiles, &p->dig_exp))) return rc;
+  if (p->tab) {
+    *ok = true;
+    return CMM_OK;
+  }
   const int64_t tri = (int64_t)L * (L + 1) / 2;
   const int ns = L / 2 + 1, npo = (L + 1) / 2;
-  int rc;
   auto tab = std::make_shared<cmm_sht::PbarTables>();
   DeviceBuffer po, kp;   // Pbar on the odd fine rings and their weights, for the build only
   if ((rc = tab->w.alloc((size_t)tri * ns * 8)) || (rc = tab->s.alloc((size_t)tri * ns * 8)) ||
@@ -1434,6 +1376,7 @@ static int ensure_tables(cmm_sht* p, cudaStream_t s, bool* ok) {
   build_w_kernel<<<dim3((ns + 63) / 64, L, 2 * (((L + 1) / 2 + 31) / 32)), 256, 0, s>>>(
       L, (const double*)po.p, (const double*)tab->s.p, (const double*)kp.p, w, (double*)tab->w.p);
   if ((rc = check_launch("build_w_kernel"))) return rc;
+  if ((rc = digit_tables_build(L, (const double*)tab->s.p, &tab->digits, s))) return rc;
   // published only once built: a later call of this plan on another
   // stream, unordered with s, must not read a partly written table
   cudaError_t e = cudaStreamSynchronize(s);
@@ -1647,23 +1590,26 @@ static int velocity_fp64(cmm_sht* p, const cmm_mesh* vm, const double2* a, bool 
   const int L = p->L, npair = L / 2 + 1;
   int rc = set_streams(p, s);
   if (rc || (rc = ensure_fp64_inverse(p))) return rc;
-  double2 *F = (double2*)p->fields.p, *S = (double2*)p->synth.p;
-  velocity_fields_kernel<<<dim3((L + 127) / 128, L), 128, 0, s>>>(a, L, lap, F);
-  if ((rc = check_launch("velocity_fields_kernel"))) return rc;
-  if (psi_out) {
-    cudaError_t e = cudaMemcpyAsync(psi_out, F, (size_t)L * L * sizeof(double2), cudaMemcpyDeviceToDevice, s);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync(psi)");
-  }
+  double2* S = (double2*)p->synth.p;
   bool tab;
   if ((rc = ensure_tables(p, s, &tab))) return rc;
-  if (tab)
-    synthesis_tab_kernel<3, true><<<dim3(L, (npair + kTabBlock - 1) / kTabBlock, kVelLegendre / 3), kTabBlock, 0, s>>>(
-        F, L, (const double*)p->tab->s.p, S);
-  else
+  if (tab) {
+    if ((rc = digit_velocity(*p->tab->digits, (const double*)p->tab->s.p, a, lap, psi_out, p->dig_tiles.p,
+                             p->dig_exp.p, S, (int*)p->status.p, s)))
+      return rc;
+  } else {
+    double2* F = (double2*)p->fields.p;
+    velocity_fields_kernel<<<dim3((L + 127) / 128, L), 128, 0, s>>>(a, L, lap, F);
+    if ((rc = check_launch("velocity_fields_kernel"))) return rc;
+    if (psi_out) {
+      cudaError_t e = cudaMemcpyAsync(psi_out, F, (size_t)L * L * sizeof(double2), cudaMemcpyDeviceToDevice, s);
+      if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync(psi)");
+    }
     synthesis_kernel<kVelLegendre, true><<<dim3(L, (npair + kSynthBlock - 1) / kSynthBlock), kSynthBlock, 0, s>>>(
         F, L, (const double*)p->ct_rings.p, (const double*)p->pmm_rings.p, (const double*)p->ra.p,
         (const double*)p->rb.p, S);
-  if ((rc = check_launch("synthesis (velocity)"))) return rc;
+    if ((rc = check_launch("synthesis_kernel (velocity)"))) return rc;
+  }
   cufftResult r = cufftExecZ2D(p->ring_inv9, (cufftDoubleComplex*)S, (cufftDoubleReal*)p->samples.p);
   if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftExecZ2D(velocity)");
   const int64_t nv = 2 + (int64_t)(L - 1) * 2 * L;
@@ -1982,7 +1928,7 @@ int sht_share_tables(cmm_sht* p, cmm_sht* src) {
     }
     p->tab = src->tab;
     p->tab_mode = src->tab_mode;
-    return CMM_OK;
+    return p->dig_tiles.p ? CMM_OK : digit_workspace(p->L, &p->dig_tiles, &p->dig_exp);
   }
   if (!src->tc) {
     set_last_error("cmm_sht_share_tables: source plan without split-BF16 tables");
@@ -2007,6 +1953,8 @@ int sht_trim(cmm_sht* p) {
   p->synth.release();
   p->samples.release();
   p->tab.reset();
+  p->dig_tiles.release();
+  p->dig_exp.release();
   return CMM_OK;
 }
 

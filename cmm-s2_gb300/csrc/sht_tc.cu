@@ -37,10 +37,16 @@
 #include "cmm_internal.h"
 #include "device_common.cuh"
 #include "ff.cuh"
+#include "tc.cuh"
 
 namespace cmm {
 
+using namespace tc;
+
 namespace {
+
+// descriptors of the 64-deep tiles (tile_offset)
+__device__ __forceinline__ uint64_t tile_desc(uint32_t saddr) { return smem_desc(saddr, 128u, 1024u); }
 
 constexpr int kM = 128;                  // ring pairs per CTA (MMA M)
 constexpr int kN = 32;                   // real columns per MMA (24 used)
@@ -51,7 +57,6 @@ constexpr int kATile = kN * kKc * 2;     // 4 KiB
 constexpr int kPRecord = 4 * kPTile;     // E_hi, E_lo, O_hi, O_lo
 constexpr int kARecord = 4 * kATile;
 constexpr int kThreads = 128;
-constexpr long long kSpinLimit = 1LL << 26;
 
 // Byte offset of element (row, k) in a K-major no-swizzle tile image with
 // 8x8 core matrices: core (row/8, k/8) at (row/8 * (K/8) + k/8) * 128,
@@ -59,53 +64,6 @@ constexpr long long kSpinLimit = 1LL << 26;
 // k-group stride (LBO) = 128.
 __host__ __device__ __forceinline__ int tile_offset(int row, int k) {
   return ((row >> 3) * (kKc >> 3) + (k >> 3)) * 128 + (row & 7) * 16 + (k & 7) * 2;
-}
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-               : "memory");
-}
-
-__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-// Bounded wait; false on timeout.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long long limit = kSpinLimit) {
-  for (long long i = 0; i < limit; ++i)
-    if (mbar_test(bar, parity)) return true;
-  return false;
-}
-
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-          smem_u32(dst)),
-      "l"(src), "r"(bytes), "r"(smem_u32(bar))
-      : "memory");
-}
-
-__device__ __forceinline__ void tc_fence_before() {
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tc_fence_after() {
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
 // Compensated (Kahan) FP32 accumulation of the per-chunk partial sums:
@@ -121,58 +79,6 @@ struct KahanF {
   __device__ __forceinline__ double value() const { return (double)s - (double)c; }
   __device__ __forceinline__ float valuef() const { return s - c; }
 };
-
-// Shared-memory matrix descriptor: start, leading (k-group) and stride
-// (row-group) byte offsets, descriptor version 1, no swizzle.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
-  d |= (uint64_t)((128u >> 4) & 0x3FFFu) << 16;    // LBO: next core matrix along K
-  d |= (uint64_t)((1024u >> 4) & 0x3FFFu) << 32;   // SBO: next 8-row group
-  d |= (uint64_t)1 << 46;
-  return d;
-}
-
-// Instruction descriptor of kind::f16: D f32, A and B bf16, both K-major,
-// N = 32, M = 128.
-__device__ __forceinline__ uint32_t mma_idesc() {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kN >> 3) << 17) | ((uint32_t)(kM >> 4) << 24);
-}
-
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc,
-                                         uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   smem_u32(bar))
-               : "memory");
-}
-
-// 32 lanes x 32 consecutive 32-bit columns -> this thread's 32 values.
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
-  uint32_t r[32];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
-        "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
-        "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr)
-      : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
 
 struct TcGeometry {
   int L, npair, nrb;
@@ -457,10 +363,10 @@ __device__ __forceinline__ void syn_mma(uint32_t stage, uint32_t d, uint32_t ide
   const uint32_t p0 = stage, a0 = stage + kPRecord;
   for (int ks = 0; ks < kKc / 16; ++ks)
     for (int par = 0; par < 2; ++par) {
-      const uint64_t ph = smem_desc(p0 + (2 * par) * kPTile + ks * 256);
-      const uint64_t pl = smem_desc(p0 + (2 * par + 1) * kPTile + ks * 256);
-      const uint64_t ah = smem_desc(a0 + (2 * par) * kATile + ks * 256);
-      const uint64_t al = smem_desc(a0 + (2 * par + 1) * kATile + ks * 256);
+      const uint64_t ph = tile_desc(p0 + (2 * par) * kPTile + ks * 256);
+      const uint64_t pl = tile_desc(p0 + (2 * par + 1) * kPTile + ks * 256);
+      const uint64_t ah = tile_desc(a0 + (2 * par) * kATile + ks * 256);
+      const uint64_t al = tile_desc(a0 + (2 * par + 1) * kATile + ks * 256);
       const uint32_t dd = d + par * kN;
       mma_bf16(dd, ph, ah, idesc, ks > 0 ? 1u : 0u);
       mma_bf16(dd, ph, al, idesc, 1u);
@@ -498,7 +404,7 @@ __global__ void __launch_bounds__(kThreads, 1) synth_tc_kernel(TcGeometry g, int
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_base_s;
-  const uint32_t idesc = mma_idesc();
+  const uint32_t idesc = mma_idesc(kN);
   const uint32_t s0 = smem_u32(smem);
   SynCursor dr;   // next chunk to drain (all threads)
   bool have = syn_set(dr, blockIdx.x, nitems, g);
@@ -623,15 +529,6 @@ __global__ void __launch_bounds__(kThreads, 1) synth_tc_kernel(TcGeometry g, int
 constexpr int kSynWarps2 = 6;
 constexpr int kSynStages2 = 2;
 
-__device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort) {
-  for (long long i = 0; i < kSpinLimit; ++i) {
-    if (mbar_test(bar, parity)) return true;
-    if ((i & 255) == 255 && *abort) return false;
-  }
-  *abort = 1;
-  return false;
-}
-
 __global__ void __launch_bounds__(32 * kSynWarps2, 1) synth_tc2_kernel(TcGeometry g, int nitems,
                                                                        const unsigned char* __restrict__ ptab,
                                                                        const unsigned char* __restrict__ atab,
@@ -690,7 +587,7 @@ __global__ void __launch_bounds__(32 * kSynWarps2, 1) synth_tc2_kernel(TcGeometr
     }
   } else if (warp == 5 && lane == 0) {
     // MMA issuer: chunk j of this CTA's stream into accumulator pair j & 1
-    const uint32_t idesc = mma_idesc();
+    const uint32_t idesc = mma_idesc(kN);
     const uint32_t s0 = smem_u32(smem);
     long long j = 0;
     bool committed = false;
@@ -786,25 +683,6 @@ struct TcFwdGeometry {
 __device__ __forceinline__ int nlblocks(int L, int m) {
   const int kmax = (L - m + 1) / 2;
   return (kmax + kM - 1) / kM;
-}
-
-__device__ __forceinline__ uint32_t mma_idesc_n16() {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kNA >> 3) << 17) | ((uint32_t)(kM >> 4) << 24);
-}
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
 // One thread per (m, fine ring pair j): Pbar_lm(theta'_j), l = m..L-1.
@@ -938,7 +816,7 @@ __global__ void __launch_bounds__(kThreads) analysis_tc_kernel(TcFwdGeometry g,
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_base_s;
-  const uint32_t idesc = mma_idesc_n16();
+  const uint32_t idesc = mma_idesc(kNA);
   KahanF aE[2 * NB], aO[2 * NB];
   uint32_t ph_load = 0, ph_mma = 0;
   for (int c = 0; c < g.nck; ++c) {
@@ -957,10 +835,10 @@ __global__ void __launch_bounds__(kThreads) analysis_tc_kernel(TcFwdGeometry g,
         const uint32_t p0 = smem_u32(sP), x0 = smem_u32(sX);
         for (int ks = 0; ks < kKc / 16; ++ks)
           for (int par = 0; par < 2; ++par) {
-            const uint64_t ph = smem_desc(p0 + (2 * par) * kPTile + ks * 256);
-            const uint64_t pl = smem_desc(p0 + (2 * par + 1) * kPTile + ks * 256);
-            const uint64_t xh = smem_desc(x0 + (2 * par) * kXTile + ks * 256);
-            const uint64_t xl = smem_desc(x0 + (2 * par + 1) * kXTile + ks * 256);
+            const uint64_t ph = tile_desc(p0 + (2 * par) * kPTile + ks * 256);
+            const uint64_t pl = tile_desc(p0 + (2 * par + 1) * kPTile + ks * 256);
+            const uint64_t xh = tile_desc(x0 + (2 * par) * kXTile + ks * 256);
+            const uint64_t xl = tile_desc(x0 + (2 * par + 1) * kXTile + ks * 256);
             const uint32_t d = tmem + par * kNA;
             mma_bf16(d, ph, xh, idesc, ks > 0 ? 1u : 0u);
             mma_bf16(d, ph, xl, idesc, 1u);

@@ -433,6 +433,28 @@ def test_velocity_jets_of_six_fields_against_oracle(nat, L, mode):
     assert np.abs(got - ref).max() < 1e-12 * np.abs(ref).max()
 
 
+@pytest.mark.parametrize("L", [3, 33, 130, 258, 523])
+def test_digit_velocity_matches_the_recurrence(nat, L):
+    """The table form of the FP64 velocity (digits on the tensor cores) where
+    its tiles end (groups of 16 degrees of a parity, chunks of 64, blocks of
+    128 ring pairs), on generic samples, against the recurrence kernels:
+    1e-12 of the largest jet (two FP64 transforms of up to 523 degrees, whose
+    recurrences lose about L ulps each).  Its scales are powers of two, so
+    scaling the input by one scales the result exactly; a NaN reaches it."""
+    theta, phi, g, verts, Phi, The = grid(L)
+    rng = np.random.default_rng(L)
+    om = np.cos(The) ** 3 * np.sin(2 * Phi) + 0.1 * rng.standard_normal(Phi.shape)
+    om[0], om[-1] = om[0, 0], om[-1, 0]
+    vm = nat.VelMesh(L, theta, phi, g, verts)
+    tab, rec = nat.Sht(L).set_tables(1), nat.Sht(L).set_tables(-1)
+    got, ref = (p.velocity(vm, dev(om)).cpu().numpy() for p in (tab, rec))
+    assert np.abs(got - ref).max() < 1e-12 * np.abs(ref).max()
+    np.testing.assert_array_equal(tab.velocity(vm, dev(om * 2.0**-300)).cpu().numpy() * 2.0**300, got)
+    om[L // 2, 1] = np.nan
+    assert not np.isfinite(tab.velocity(vm, dev(om)).cpu().numpy()).all()
+    assert tab.status() == 0
+
+
 @pytest.mark.parametrize("L", [32, 65, 200])
 def test_split_velocity_tiles_match_the_field_route(nat, L):
     """The split-BF16 velocity's data tiles, made straight from the analysis
