@@ -355,4 +355,13 @@ int digit_tables_build(int L, const double* tab, std::shared_ptr<DigitTables>* o
 int digit_workspace(int L, DeviceBuffer* tiles, DeviceBuffer* aexp);
 int digit_velocity(const DigitTables& t, const double* tab, const double2* a, bool lap, double2* psi_out,
                    void* tiles, void* aexp, double2* S, int* status, cudaStream_t s);
+
+// Inverse ring transforms by digits (ring_digits.cu), L <= kDigitMaxL: tables
+// for `fields` fields of L+1 rings, a plan's own data workspace, and the
+// transform of the spectra S (fields, L+1, L+1; m = L taken as zero) ->
+// x (fields, L+1, 2L).
+struct RingTables;
+int ring_tables_build(int L, int fields, std::shared_ptr<RingTables>* out, cudaStream_t s);
+int ring_workspace(int L, int fields, DeviceBuffer* data);
+int ring_inverse(const RingTables& t, int fields, const double2* S, void* data, double* x, int* status, cudaStream_t s);
 }  // namespace cmm

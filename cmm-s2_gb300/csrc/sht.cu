@@ -1142,9 +1142,10 @@ struct cmm_sht {
   struct PbarTables {
     cmm::DeviceBuffer w, s;
     std::shared_ptr<cmm::DigitTables> digits;   // of s, for the velocity's synthesis
+    std::shared_ptr<cmm::RingTables> ring;      // for its ring transforms
   };
   std::shared_ptr<PbarTables> tab;
-  cmm::DeviceBuffer dig_tiles, dig_exp;   // this plan's data tiles for tab->digits
+  cmm::DeviceBuffer dig_tiles, dig_exp, ring_data;   // this plan's data digits for them
   int tab_mode = 0;                 // cmm_sht_set_tables: 0 auto, 1 always, -1 never
   cmm::DeviceBuffer spec, torus, pad, alm, fields, synth, samples, status;
   cmm::TcPlan* tc = nullptr;
@@ -1332,6 +1333,20 @@ static int set_streams(cmm_sht* p, cudaStream_t s) {
   return CMM_OK;
 }
 
+// Least L whose velocity takes the ring transforms by digits (ring_digits.cu):
+// below, their few work items leave the chip idle and the fast transform is
+// short (velocity inversion at L = 128: 71 us by digits, 66 by the FFT; 160: 93
+// and 92; 192: 107 and 117; 256: 138 and 172; 512: 466 and 681).
+constexpr int kRingMinL = 160;
+
+// The digit forms' data workspaces of a plan with tables.
+static int ensure_digits(cmm_sht* p) {
+  if (p->dig_tiles.p) return CMM_OK;
+  int rc = CMM_OK;
+  if (p->L >= kRingMinL) rc = ring_workspace(p->L, kVelSpectra, &p->ring_data);
+  return rc ? rc : digit_workspace(p->L, &p->dig_tiles, &p->dig_exp);
+}
+
 // Pbar tables of the FP64 Legendre stages at L <= kTabMaxL, built at their
 // first use on `s` (a call inside a stream capture keeps the recurrence
 // kernels, since a capture cannot allocate); released by cmm_sht_trim.
@@ -1350,7 +1365,7 @@ static int ensure_tables(cmm_sht* p, cudaStream_t s, bool* ok) {
   }
   if (cs != cudaStreamCaptureStatusNone) return CMM_OK;
   int rc;
-  if (!p->dig_tiles.p && (rc = digit_workspace(L, &p->dig_tiles, &p->dig_exp))) return rc;
+  if ((rc = ensure_digits(p))) return rc;
   if (p->tab) {
     *ok = true;
     return CMM_OK;
@@ -1377,6 +1392,7 @@ static int ensure_tables(cmm_sht* p, cudaStream_t s, bool* ok) {
       L, (const double*)po.p, (const double*)tab->s.p, (const double*)kp.p, w, (double*)tab->w.p);
   if ((rc = check_launch("build_w_kernel"))) return rc;
   if ((rc = digit_tables_build(L, (const double*)tab->s.p, &tab->digits, s))) return rc;
+  if (L >= kRingMinL && (rc = ring_tables_build(L, kVelSpectra, &tab->ring, s))) return rc;
   // published only once built: a later call of this plan on another
   // stream, unordered with s, must not read a partly written table
   cudaError_t e = cudaStreamSynchronize(s);
@@ -1594,9 +1610,9 @@ static int velocity_fp64(cmm_sht* p, const cmm_mesh* vm, const double2* a, bool 
   bool tab;
   if ((rc = ensure_tables(p, s, &tab))) return rc;
   if (tab) {
-    if ((rc = digit_velocity(*p->tab->digits, (const double*)p->tab->s.p, a, lap, psi_out, p->dig_tiles.p,
-                             p->dig_exp.p, S, (int*)p->status.p, s)))
-      return rc;
+    rc = digit_velocity(*p->tab->digits, (const double*)p->tab->s.p, a, lap, psi_out, p->dig_tiles.p, p->dig_exp.p, S,
+                        (int*)p->status.p, s);
+    if (rc) return rc;
   } else {
     double2* F = (double2*)p->fields.p;
     velocity_fields_kernel<<<dim3((L + 127) / 128, L), 128, 0, s>>>(a, L, lap, F);
@@ -1610,8 +1626,13 @@ static int velocity_fp64(cmm_sht* p, const cmm_mesh* vm, const double2* a, bool 
         (const double*)p->rb.p, S);
     if ((rc = check_launch("synthesis_kernel (velocity)"))) return rc;
   }
-  cufftResult r = cufftExecZ2D(p->ring_inv9, (cufftDoubleComplex*)S, (cufftDoubleReal*)p->samples.p);
-  if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftExecZ2D(velocity)");
+  if (tab && p->tab->ring) {
+    rc = ring_inverse(*p->tab->ring, kVelSpectra, S, p->ring_data.p, (double*)p->samples.p, (int*)p->status.p, s);
+    if (rc) return rc;
+  } else {
+    cufftResult r = cufftExecZ2D(p->ring_inv9, (cufftDoubleComplex*)S, (cufftDoubleReal*)p->samples.p);
+    if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftExecZ2D(velocity)");
+  }
   const int64_t nv = 2 + (int64_t)(L - 1) * 2 * L;
   velocity_jets_kernel<<<(int)((nv + 127) / 128), 128, 0, s>>>((const double*)p->samples.p, L, vm->view.grid, jets);
   return check_launch("velocity_jets_kernel");
@@ -1928,7 +1949,7 @@ int sht_share_tables(cmm_sht* p, cmm_sht* src) {
     }
     p->tab = src->tab;
     p->tab_mode = src->tab_mode;
-    return p->dig_tiles.p ? CMM_OK : digit_workspace(p->L, &p->dig_tiles, &p->dig_exp);
+    return ensure_digits(p);
   }
   if (!src->tc) {
     set_last_error("cmm_sht_share_tables: source plan without split-BF16 tables");
@@ -1955,6 +1976,7 @@ int sht_trim(cmm_sht* p) {
   p->tab.reset();
   p->dig_tiles.release();
   p->dig_exp.release();
+  p->ring_data.release();
   return CMM_OK;
 }
 

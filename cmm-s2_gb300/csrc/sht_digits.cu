@@ -36,19 +36,19 @@
 
 #include "cmm_internal.h"
 #include "device_common.cuh"
+#include "digits.cuh"
 #include "sht_fields.cuh"
 #include "tc.cuh"
 
 namespace cmm {
 
+using namespace dig;
 using namespace sht;
 using namespace tc;
 
 namespace {
 
 constexpr int kRows = 128;              // ring pairs per work item (MMA M)
-constexpr int kDigits = 6;
-constexpr int kLevels = 7;
 constexpr int kCols = 12;               // real columns (16 with padding)
 constexpr int kChunkGroups = 4;         // groups of 16 degrees per chunk
 constexpr int kRowGroupBytes = kDigits * 2 * 128;          // one 8-row group of one degree group
@@ -65,49 +65,7 @@ struct DigGeometry {
   const int* gbase;       // (L+1) prefix sums of the degree groups per m
 };
 
-__host__ __device__ __forceinline__ int groups16(int n) { return (n + 15) / 16; }
-
-// ---------------------------------------------------------------- digits
-// x 2^(1075 - e) rounded to nearest, e the biased exponent of the scale's
-// binade (>= that of x, >= 1): |result| < 2^53.
-__device__ __forceinline__ long long to_fixed(double x, int e) {
-  const long long b = __double_as_longlong(x);
-  int ex = (int)((b >> 52) & 2047);
-  long long v = b & 0xfffffffffffffLL;
-  if (ex)
-    v |= 0x10000000000000LL;
-  else
-    ex = 1;
-  const int sh = e - ex;
-  if (sh > 54) return 0;
-  if (sh > 0) v = (v + (1LL << (sh - 1))) >> sh;
-  return b < 0 ? -v : v;
-}
-
-// The six digits of eight entries as bf16 vectors, highest first.
-__device__ __forceinline__ void digits8(const long long* v, uint4* out) {
-  uint32_t w[kDigits][4];
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    long long r = v[q];
-#pragma unroll
-    for (int i = kDigits - 1; i >= 0; --i) {
-      int d = (int)r;
-      if (i > 0) {
-        d = (int)(((unsigned)d + 256u) & 511u) - 256;
-        r = (r - d) >> 9;
-      }
-      const uint32_t f = __float_as_uint((float)d) >> 16;   // at most 8 significant bits: exact
-      if (q & 1)
-        w[i][q >> 1] |= f << 16;
-      else
-        w[i][q >> 1] = f;
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < kDigits; ++i) out[i] = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
-}
-
+// ----------------------------------------------------------- tables, data
 // Block (row block, m): the digit table of its rows from the FP64 table
 // tab[m][l - m][t], one thread per row; scales in pexp[m][t - 1].
 __global__ void __launch_bounds__(kRows) build_digits_kernel(DigGeometry g, const double* __restrict__ tab,
@@ -458,12 +416,15 @@ __global__ void __launch_bounds__(kSynThreads, 1) synth_digits_kernel(DigGeometr
           const int pe = pexp[(int64_t)u.m * g.rows + t - 1] - 2096;
           // value = (hi + lo) 2^54 2^(pe + ae - 2150), (hi + lo) 2^54 the
           // integers' products, the scales' exponents biased
+          int ae_[kCols];   // all loads before the stores
+#pragma unroll
+          for (int k = 0; k < kCols; ++k) ae_[k] = aexp[u.m * kCols + k];
 #pragma unroll
           for (int f = 0; f < kVelLegendre; ++f) {
             double v[2][2];
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
-              const int k = 2 * f + r, ae = aexp[u.m * kCols + k];
+              const int k = 2 * f + r, ae = ae_[k];
               v[0][r] = scale2((double)(E[k] + acc[k]) + (double)(El[k] + accl[k]), pe + ae);
               v[1][r] = scale2((double)(E[k] - acc[k]) + (double)(El[k] - accl[k]), pe + ae);
               if (ae == kNonFinite) v[0][r] = v[1][r] = __longlong_as_double(0x7ff8000000000000LL);

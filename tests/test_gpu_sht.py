@@ -433,12 +433,12 @@ def test_velocity_jets_of_six_fields_against_oracle(nat, L, mode):
     assert np.abs(got - ref).max() < 1e-12 * np.abs(ref).max()
 
 
-@pytest.mark.parametrize("L", [3, 33, 130, 258, 523])
+@pytest.mark.parametrize("L", [3, 33, 130, 258, 523, 1024])
 def test_digit_velocity_matches_the_recurrence(nat, L):
     """The table form of the FP64 velocity (digits on the tensor cores) where
     its tiles end (groups of 16 degrees of a parity, chunks of 64, blocks of
     128 ring pairs), on generic samples, against the recurrence kernels:
-    1e-12 of the largest jet (two FP64 transforms of up to 523 degrees, whose
+    1e-12 of the largest jet (two FP64 transforms of up to 1024 degrees, whose
     recurrences lose about L ulps each).  Its scales are powers of two, so
     scaling the input by one scales the result exactly; a NaN reaches it."""
     theta, phi, g, verts, Phi, The = grid(L)
