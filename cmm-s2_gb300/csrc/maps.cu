@@ -144,77 +144,72 @@ __global__ void __launch_bounds__(kBlock) locate_kernel(MeshView m, const double
   }
 }
 
-// One triangle per thread: the 19 ordinates of each component from the
-// jets of its three vertices (assemble_coefficients,
-// cmm_s2/core/spherical_spline.py:300-337) using the per-triangle factors
-// (factor-major, coalesced loads).  The block's records are staged in
-// shared memory (rows padded to stride+1 doubles against bank conflicts)
-// and written out as one contiguous, coalesced range, record padding
-// included (zeros).
-constexpr int kAsmTri = 64;   // triangles (threads) per block
+// The 19 ordinates of each component from the jets of a triangle's three
+// vertices (assemble_coefficients, cmm_s2/core/spherical_spline.py:300-337)
+// using the per-triangle factors (factor-major, coalesced loads).  Three
+// threads per triangle: first one per corner (its value and its three
+// ordinates, for all components), then one per component (the inner ordinates
+// from the corners').  The block's records are staged in shared memory (rows
+// padded to stride+1 doubles against bank conflicts) and written out as one
+// contiguous, coalesced range, record padding included (zeros).  FP64-bound
+// (153 per triangle); one thread per triangle held 166 registers and left
+// four warps per SM at level 5 (17 us; level 6: 38 us).
+constexpr int kAsmTri = 64;   // triangles per block
 
 template <int NC>
-__global__ void __launch_bounds__(kAsmTri) assemble_kernel(MeshView m, const double* __restrict__ jets,
-                                                           double* __restrict__ coeffs,
-                                                           const BveState* __restrict__ st) {
+__global__ void __launch_bounds__(3 * kAsmTri) assemble_kernel(MeshView m, const double* __restrict__ jets,
+                                                               double* __restrict__ coeffs,
+                                                               const BveState* __restrict__ st) {
   if (st) coeffs = st->vel[0];
   constexpr int kStride = NC == 3 ? kCoeffStride3 : kCoeffStride1;
   constexpr int kRow = kStride + 1;
   __shared__ double rec[kAsmTri * kRow];
   const int t0 = blockIdx.x * kAsmTri;
   const int nblk = min(kAsmTri, m.nt - t0);
-  const int tl = threadIdx.x, t = t0 + tl;
+  const int tl = threadIdx.x % kAsmTri, part = threadIdx.x / kAsmTri, t = t0 + tl;   // part: corner, then component
   double* out = rec + tl * kRow;
+  const int nv = m.nv, nt = m.nt;
+  const double* A = m.tri_asm + t;   // factor j at A[j * nt]
   if (tl < nblk) {
-    const int nv = m.nv, nt = m.nt;
     const int4 tv = m.tri_v[t];
-    const int vid[3] = {tv.x, tv.y, tv.z};
-    const double* A = m.tri_asm + t;   // factor j at A[j * nt]
-    const int corner[9] = {0, 0, 0, 1, 1, 1, 2, 2, 2};
+    const int v = part == 0 ? tv.x : (part == 1 ? tv.y : tv.z);
+    double a[3][4];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) a[i][j] = __ldg(A + (int64_t)(4 * (3 * part + i) + j) * nt);
 #pragma unroll
     for (int k = 0; k < NC; ++k) {
-      double f[3], c[19];
+      const double f = __ldg(jets + (int64_t)(k * 4) * nv + v);
+      // d_j f_k = jets[j][1+k] (three components), jets[1+j] (scalar)
+      const int g0 = NC == 3 ? 1 + k : 1, dg = NC == 3 ? 4 : 1;
+      const double gx = __ldg(jets + (int64_t)g0 * nv + v), gy = __ldg(jets + (int64_t)(g0 + dg) * nv + v),
+                   gz = __ldg(jets + (int64_t)(g0 + 2 * dg) * nv + v);
+      out[NC * part + k] = f;
 #pragma unroll
-      for (int v = 0; v < 3; ++v) f[v] = __ldg(jets + (int64_t)(k * 4) * nv + vid[v]);
-      c[0] = f[0];
-      c[1] = f[1];
-      c[2] = f[2];
-#pragma unroll
-      for (int o = 0; o < 9; ++o) {
-        const int v = vid[corner[o]];
-        double gx, gy, gz;
-        if (NC == 3) {  // d_j f_k = jets[j][1+k]
-          gx = __ldg(jets + (int64_t)(0 * 4 + 1 + k) * nv + v);
-          gy = __ldg(jets + (int64_t)(1 * 4 + 1 + k) * nv + v);
-          gz = __ldg(jets + (int64_t)(2 * 4 + 1 + k) * nv + v);
-        } else {  // scalar: d_j f = jets[1+j]
-          gx = __ldg(jets + (int64_t)1 * nv + v);
-          gy = __ldg(jets + (int64_t)2 * nv + v);
-          gz = __ldg(jets + (int64_t)3 * nv + v);
-        }
-        const double a0 = __ldg(A + (int64_t)(4 * o) * nt), a1 = __ldg(A + (int64_t)(4 * o + 1) * nt),
-                     a2 = __ldg(A + (int64_t)(4 * o + 2) * nt), a3 = __ldg(A + (int64_t)(4 * o + 3) * nt);
-        c[3 + o] = a0 * gx + a1 * gy + a2 * gz - a3 * f[corner[o]];
-      }
-      double e[9];
-#pragma unroll
-      for (int j = 0; j < 9; ++j) e[j] = __ldg(A + (int64_t)(36 + j) * nt);
-      c[12] = e[0] * c[3] + e[1] * c[8];
-      c[13] = e[2] * c[6] + e[3] * c[11];
-      c[14] = e[5] * c[9] + e[4] * c[5];
-      c[15] = e[0] * c[4] + e[1] * c[7];
-      c[16] = e[2] * c[7] + e[3] * c[10];
-      c[17] = e[4] * c[4] + e[5] * c[10];
-      c[18] = e[6] * c[4] + e[7] * c[7] + e[8] * c[10];
-#pragma unroll
-      for (int o = 0; o < 19; ++o) out[NC * o + k] = c[o];
+      for (int i = 0; i < 3; ++i)
+        out[NC * (3 + 3 * part + i) + k] = a[i][0] * gx + a[i][1] * gy + a[i][2] * gz - a[i][3] * f;
     }
+    for (int j = 19 * NC + part; j < kStride; j += 3) out[j] = 0.0;
+  }
+  __syncthreads();
+  if (tl < nblk && part < NC) {
+    double e[9], c[12];
 #pragma unroll
-    for (int j = 19 * NC; j < kStride; ++j) out[j] = 0.0;
+    for (int j = 0; j < 9; ++j) e[j] = __ldg(A + (int64_t)(36 + j) * nt);
+#pragma unroll
+    for (int o = 3; o < 12; ++o) c[o] = out[NC * o + part];
+    out[NC * 12 + part] = e[0] * c[3] + e[1] * c[8];
+    out[NC * 13 + part] = e[2] * c[6] + e[3] * c[11];
+    out[NC * 14 + part] = e[5] * c[9] + e[4] * c[5];
+    out[NC * 15 + part] = e[0] * c[4] + e[1] * c[7];
+    out[NC * 16 + part] = e[2] * c[7] + e[3] * c[10];
+    out[NC * 17 + part] = e[4] * c[4] + e[5] * c[10];
+    out[NC * 18 + part] = e[6] * c[4] + e[7] * c[7] + e[8] * c[10];
   }
   __syncthreads();
   double* dst = coeffs + (int64_t)t0 * kStride;
-  for (int i = tl; i < nblk * kStride; i += kAsmTri) dst[i] = rec[(i / kStride) * kRow + i % kStride];
+  for (int i = threadIdx.x; i < nblk * kStride; i += 3 * kAsmTri) dst[i] = rec[(i / kStride) * kRow + i % kStride];
 }
 
 // FP32 velocity records (velmesh with rec32, ncomp = 3): the same
@@ -1080,9 +1075,9 @@ int launch_assemble(const MeshView& m, const double* jets, int ncomp, double* co
   if (ncomp == 3 && m.rec32)
     assemble_f32_kernel<double><<<blocks, kAsmTri, 0, s>>>(m, jets, (float*)coeffs, st);
   else if (ncomp == 3)
-    assemble_kernel<3><<<blocks, kAsmTri, 0, s>>>(m, jets, coeffs, st);
+    assemble_kernel<3><<<blocks, 3 * kAsmTri, 0, s>>>(m, jets, coeffs, st);
   else
-    assemble_kernel<1><<<blocks, kAsmTri, 0, s>>>(m, jets, coeffs, st);
+    assemble_kernel<1><<<blocks, 3 * kAsmTri, 0, s>>>(m, jets, coeffs, st);
   return check_launch("assemble_kernel");
 }
 

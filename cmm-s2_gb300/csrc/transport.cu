@@ -49,20 +49,19 @@ __device__ __forceinline__ void rotate3(const double* L, double x, double y, dou
   o[2] = L[6] * x + L[7] * y + L[8] * z;
 }
 
-// utils.cross(a, b) with b = (bx, by, bz)
-__device__ __forceinline__ void cross3(double ax, double ay, double az, double bx, double by, double bz,
-                                       double* o) {
-  o[0] = ay * bz - az * by;
-  o[1] = az * bx - ax * bz;
-  o[2] = ax * by - ay * bx;
-}
-
+// cross((x, y, z), (wx, 0, wz)), without the products with zero (:18-22)
 __device__ __forceinline__ void u_sbr(const FlowSpec& f, double x, double y, double z, double* V) {
-  cross3(x, y, z, f.wx, 0.0, f.wz, V);  // :18-22
+  V[0] = y * f.wz;
+  V[1] = z * f.wx - x * f.wz;
+  V[2] = -y * f.wx;
 }
 
+// cross((x, y, z), (0, c1 y, 0)) (:24-30)
 __device__ __forceinline__ void u_deform(double c1, double x, double y, double z, double* V) {
-  cross3(x, y, z, 0.0 * x, c1 * y, 0.0 * z, V);  // :24-30
+  const double w = c1 * y;
+  V[0] = -z * w;
+  V[1] = 0.0;
+  V[2] = x * w;
 }
 
 // omega_r (:48-55): angular speed of the static vortex at colatitude theta
@@ -103,7 +102,7 @@ __device__ void flow_at(const FlowSpec& f, int s, double x, double y, double z, 
       double r[3], u[3], w[3];
       rotate3(g.fwd, x, y, z, r);
       u_deform(g.c1, r[0], r[1], r[2], u);
-      rotate3(g.back, u[0], u[1], u[2], w);
+      for (int c = 0; c < 3; ++c) w[c] = g.back[3 * c] * u[0] + g.back[3 * c + 2] * u[2];   // u[1] = 0
       u_sbr(f, x, y, z, V);
       V[0] = w[0] + V[0];
       V[1] = w[1] + V[1];

@@ -333,62 +333,68 @@ __global__ void __launch_bounds__(kMaxBlock, 2) advect_points_kernel(MeshView me
 // cmm_s2/core/evolution_functions.py:90-113); with a previous map, the
 // images are the previous map evaluated at the stencil foot points in the
 // sub-triangle of the vertex foot point, un-normalised (stencil_eval,
-// cmm_s2/core/spherical_spline.py:268-298).
+// cmm_s2/core/spherical_spline.py:268-298).  Four neighbouring lanes take a
+// vertex: lane k evaluates stencil point k, then (k < 3) component k's mean and
+// differences and the gradients' slot k.  FP64- and latency-bound: one thread
+// per vertex left two warps per SM at level 5 (18 us; level 6: 40 us), a
+// quarter of its FP64 work in nine divisions.
 __global__ void __launch_bounds__(kBlock) project_jets_kernel(MeshView m, const double* __restrict__ prev,
                                                               const double* __restrict__ yn,
                                                               const double* __restrict__ sn,
                                                               const double* __restrict__ tan,
-                                                              double eps, double* __restrict__ jets,
+                                                              double inv4eps, double* __restrict__ jets,
                                                               const BveState* __restrict__ st) {
   const int64_t nv = m.nv;
-  const int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (v >= nv) return;
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int k = (int)(i & 3);
+  const bool active = (i >> 2) < nv;
+  const int64_t v = active ? i >> 2 : nv - 1;   // every lane of the warp takes part in the exchange
   if (st && st->identity) prev = nullptr;
-  double S[4][3];
+  double P[3];
 #pragma unroll
-  for (int k = 0; k < 4; ++k)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) S[k][c] = sn[(c * 4 + k) * nv + v];
+  for (int c = 0; c < 3; ++c) P[c] = sn[(c * 4 + k) * nv + v];
+  bool ok = true;
   if (prev) {
     const double x = yn[v], y = yn[nv + v], z = yn[2 * nv + v];
-    if (!finite3(x, y, z)) {
-      flag(m, CMM_FLAG_NONFINITE);
-      for (int k = 0; k < 12; ++k) jets[k * nv + v] = nan("");
-      return;
-    }
-    const int t = locate_row(m, x, y, z);
-    double Lr[13];
-    load_loc(m, t, Lr);
-    const Split sp = split_of(bcc_of(Lr, x, y, z));
-    Ords<3> o;
-    load_ords<3>(prev + (int64_t)t * kCoeffStride3, sp, o);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const Gam g = gamma_of(Lr, bcc_of(Lr, S[k][0], S[k][1], S[k][2]), sp);
-      double P[3];
+    ok = finite3(x, y, z);
+    if (ok) {
+      const int t = locate_row(m, x, y, z);
+      double Lr[13];
+      load_loc(m, t, Lr);
+      const Split sp = split_of(bcc_of(Lr, x, y, z));
+      Ords<3> o;
+      load_ords<3>(prev + (int64_t)t * kCoeffStride3, sp, o);
+      const Gam g = gamma_of(Lr, bcc_of(Lr, P[0], P[1], P[2]), sp);
       sbb<3>(o, g, P);
-      S[k][0] = P[0];
-      S[k][1] = P[1];
-      S[k][2] = P[2];
     }
   }
-  double mv[3], d1[3], d2[3];
+  // component k of the four images (lane 3 repeats component 2)
+  double S[4];
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    mv[c] = (S[0][c] + S[1][c] + S[2][c] + S[3][c]) / 4;
-    d1[c] = (S[1][c] - S[0][c] + S[3][c] - S[2][c]) / (4 * eps);
-    d2[c] = (S[2][c] - S[0][c] + S[3][c] - S[1][c]) / (4 * eps);
+  for (int q = 0; q < 4; ++q) {
+    const double a = __shfl_sync(0xffffffffu, P[0], q, 4), b = __shfl_sync(0xffffffffu, P[1], q, 4),
+                 c = __shfl_sync(0xffffffffu, P[2], q, 4);
+    S[q] = k == 0 ? a : (k == 1 ? b : c);
   }
-  const double nm = sqrt(mv[0] * mv[0] + mv[1] * mv[1] + mv[2] * mv[2]);
+  const double mv = (S[0] + S[1] + S[2] + S[3]) * 0.25;
+  const double d1 = (S[1] - S[0] + S[3] - S[2]) * inv4eps;
+  const double d2 = (S[2] - S[0] + S[3] - S[1]) * inv4eps;
+  const double m0 = __shfl_sync(0xffffffffu, mv, 0, 4), m1 = __shfl_sync(0xffffffffu, mv, 1, 4),
+               m2 = __shfl_sync(0xffffffffu, mv, 2, 4);
+  if (!active || k == 3) return;
+  if (!ok) {
+    if (k == 0) flag(m, CMM_FLAG_NONFINITE);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) jets[(c * 4 + 1 + k) * nv + v] = nan("");
+    jets[(k * 4) * nv + v] = nan("");
+    return;
+  }
   const double* a1 = tan + 3 * v;
   const double* a2 = tan + 3 * (nv + v);
+  jets[(k * 4) * nv + v] = mv * rsqrt(m0 * m0 + m1 * m1 + m2 * m2);
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    jets[(c * 4 + 0) * nv + v] = mv[c] / nm;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) jets[(c * 4 + 1 + k) * nv + v] = d1[k] * a1[c] + d2[k] * a2[c];
-  }
-  if (!finite3(mv[0], mv[1], mv[2])) flag(m, CMM_FLAG_NONFINITE);
+  for (int c = 0; c < 3; ++c) jets[(c * 4 + 1 + k) * nv + v] = d1 * a1[c] + d2 * a2[c];
+  if (!isfinite(mv)) flag(m, CMM_FLAG_NONFINITE);
 }
 
 int check_launch(const char* what) {
@@ -486,8 +492,9 @@ int launch_project_jets(const MeshView& mesh, const double* prev_coeffs, const d
                         const double* sn, const double* tan, double eps, double* jets,
                         cudaStream_t s, const BveState* st) {
   const int64_t nv = mesh.nv;
-  const int b = small_block(nv, kBlock);
-  project_jets_kernel<<<(int)((nv + b - 1) / b), b, 0, s>>>(mesh, prev_coeffs, yn, sn, tan, eps, jets, st);
+  const int b = small_block(4 * nv, kBlock);
+  project_jets_kernel<<<(int)((4 * nv + b - 1) / b), b, 0, s>>>(mesh, prev_coeffs, yn, sn, tan, 1.0 / (4.0 * eps),
+                                                                jets, st);
   return check_launch("project_jets_kernel");
 }
 
