@@ -356,6 +356,12 @@ int digit_workspace(int L, DeviceBuffer* tiles, DeviceBuffer* aexp);
 int digit_velocity(const DigitTables& t, const double* tab, const double2* a, bool lap, double2* psi_out,
                    void* tiles, void* aexp, double2* S, int* status, cudaStream_t s);
 
+// The analysis weights W[m][t][l-m] by digits (weight_digits.cu) from Pbar on the
+// odd fine rings po[m][l-m][jj] and the rings ps[m][l-m][t], their matrix
+// Kp[v][jj][t] and the quadrature weights w; synchronises s.
+int digit_weights(int L, const double* po, const double* ps, const double* Kp, const double* w, double* W,
+                  cudaStream_t s);
+
 // Inverse ring transforms by digits (ring_digits.cu), L <= kDigitMaxL: tables
 // for `fields` fields of L+1 rings, a plan's own data workspace, and the
 // transform of the spectra S (fields, L+1, L+1; m = L taken as zero) ->

@@ -413,7 +413,10 @@ __global__ void __launch_bounds__(kRingThreads, 1)
   }
   tc_fence_before();
   __syncthreads();
-  if (tid == 0 && abort_s) atomicOr(status, drain_fail_s ? CMM_FLAG_TIMEOUT | CMM_FLAG_DRAIN_TIMEOUT : CMM_FLAG_TIMEOUT);
+  if (tid == 0 && abort_s) {   // beside the status, a NaN: the velocity is seen to be unusable
+    atomicOr(status, drain_fail_s ? CMM_FLAG_TIMEOUT | CMM_FLAG_DRAIN_TIMEOUT : CMM_FLAG_TIMEOUT);
+    x[2 * L] = __longlong_as_double(0x7ff8000000000000LL);
+  }
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols)
                  : "memory");

@@ -1339,6 +1339,10 @@ static int set_streams(cmm_sht* p, cudaStream_t s) {
 // and 92; 192: 107 and 117; 256: 138 and 172; 512: 466 and 681).
 constexpr int kRingMinL = 160;
 
+// Least L whose analysis weights are made by digits (weight_digits.cu); below,
+// the FP64 contraction takes less time than their set-up.
+constexpr int kDigitWeightsMinL = 256;
+
 // The digit forms' data workspaces of a plan with tables.
 static int ensure_digits(cmm_sht* p) {
   if (p->dig_tiles.p) return CMM_OK;
@@ -1388,9 +1392,14 @@ static int ensure_tables(cmm_sht* p, cudaStream_t s, bool* ok) {
   if ((rc = check_launch("build_pbar_kernel"))) return rc;
   odd_kernel_kernel<<<dim3((ns + 127) / 128, npo, 4), 128, 0, s>>>(L, w, (double*)kp.p);
   if ((rc = check_launch("odd_kernel_kernel"))) return rc;
-  build_w_kernel<<<dim3((ns + 63) / 64, L, 2 * (((L + 1) / 2 + 31) / 32)), 256, 0, s>>>(
-      L, (const double*)po.p, (const double*)tab->s.p, (const double*)kp.p, w, (double*)tab->w.p);
-  if ((rc = check_launch("build_w_kernel"))) return rc;
+  if (L >= kDigitWeightsMinL) {
+    if ((rc = digit_weights(L, (const double*)po.p, (const double*)tab->s.p, (const double*)kp.p, w, (double*)tab->w.p, s)))
+      return rc;
+  } else {
+    build_w_kernel<<<dim3((ns + 63) / 64, L, 2 * (((L + 1) / 2 + 31) / 32)), 256, 0, s>>>(
+        L, (const double*)po.p, (const double*)tab->s.p, (const double*)kp.p, w, (double*)tab->w.p);
+    if ((rc = check_launch("build_w_kernel"))) return rc;
+  }
   if ((rc = digit_tables_build(L, (const double*)tab->s.p, &tab->digits, s))) return rc;
   if (L >= kRingMinL && (rc = ring_tables_build(L, kVelSpectra, &tab->ring, s))) return rc;
   // published only once built: a later call of this plan on another

@@ -445,7 +445,10 @@ __global__ void __launch_bounds__(kSynThreads, 1) synth_digits_kernel(DigGeometr
   }
   tc_fence_before();
   __syncthreads();
-  if (tid == 0 && abort_s) atomicOr(status, drain_fail_s ? CMM_FLAG_TIMEOUT | CMM_FLAG_DRAIN_TIMEOUT : CMM_FLAG_TIMEOUT);
+  if (tid == 0 && abort_s) {   // beside the status, a NaN on a ring: the velocity is seen to be unusable
+    atomicOr(status, drain_fail_s ? CMM_FLAG_TIMEOUT | CMM_FLAG_DRAIN_TIMEOUT : CMM_FLAG_TIMEOUT);
+    S[L + 1] = make_double2(__longlong_as_double(0x7ff8000000000000LL), 0.0);
+  }
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols)
                  : "memory");
