@@ -691,6 +691,73 @@ __device__ __forceinline__ void sh_series_n(const MeshView& vm, const double* __
   }
 }
 
+// The same with four neighbouring lanes per point, lane g taking the orders
+// g, g+4, ...: the sums' chains are a quarter as long where there are too few
+// points to hide them (all four lanes must call; each gets the sums).  The
+// order's start values advance four orders at a time, by cos/sin(4 phi) and
+// sin^4(theta).
+constexpr int kShLanes = 4;
+// Points below which the series takes four lanes each: a thread per point then
+// leaves at most 8 warps per SM.
+constexpr int64_t kShLanesMaxQ = 152LL * 8 * 32;
+
+template <int NS>
+__device__ __forceinline__ void sh_series_lanes(const MeshView& vm, const double* __restrict__ c, int lmax,
+                                                const ShPoint& pt, int g, double* out) {
+  const int T = kShTableMax + 1;
+  const int w = 2 * lmax + 1;
+  const int64_t K = (int64_t)(lmax + 1) * w;
+#pragma unroll
+  for (int k = 0; k < NS; ++k) out[k] = 0.0;
+  const double c2 = pt.cp * pt.cp - pt.sp * pt.sp, s2 = 2.0 * pt.cp * pt.sp;
+  const double c4 = c2 * c2 - s2 * s2, s4 = 2.0 * c2 * s2;
+  const double st2 = pt.st * pt.st, st4 = st2 * st2;
+  double pmm = 0.28209479177387814;   // sqrt(1/(4 pi))
+  double cm = 1.0, sm = 0.0;          // cos(m phi), sin(m phi)
+  for (int m = 1; m <= g && m <= lmax; ++m) {
+    pmm = -pmm * __ldg(vm.sh_fm + m) * pt.st;
+    const double t = cm * pt.cp - sm * pt.sp;
+    sm = sm * pt.cp + cm * pt.sp;
+    cm = t;
+  }
+  for (int m = g; m <= lmax; m += kShLanes) {
+    const double* ab = vm.sh_ab + 2 * (int64_t)m * T;
+    double p1 = 0.0, p = pmm;
+    double ac[NS], as[NS];
+#pragma unroll
+    for (int k = 0; k < NS; ++k) ac[k] = as[k] = 0.0;
+    for (int l = m; l <= lmax; ++l) {
+      if (l > m) {   // b = 0 at l = m + 1
+        const double pn = __ldg(ab + 2 * l) * (pt.ct * p - (l > m + 1 ? __ldg(ab + 2 * l + 1) : 0.0) * p1);
+        p1 = p;
+        p = pn;
+      }
+      const int64_t i = (int64_t)l * w + l;
+#pragma unroll
+      for (int k = 0; k < NS; ++k) {
+        ac[k] += __ldg(c + k * K + i + m) * p;
+        if (m > 0) as[k] += __ldg(c + k * K + i - m) * p;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < NS; ++k)
+      out[k] += m == 0 ? ac[k] : 1.4142135623730951 * (ac[k] * cm + as[k] * sm);
+    if (m + kShLanes <= lmax) {
+      pmm *= (__ldg(vm.sh_fm + m + 1) * __ldg(vm.sh_fm + m + 2)) * (__ldg(vm.sh_fm + m + 3) * __ldg(vm.sh_fm + m + 4)) *
+             st4;
+      const double t = cm * c4 - sm * s4;
+      sm = sm * c4 + cm * s4;
+      cm = t;
+    }
+  }
+  const unsigned quad = 0xfu << (threadIdx.x & 28u);
+#pragma unroll
+  for (int k = 0; k < NS; ++k) {
+    out[k] += __shfl_xor_sync(quad, out[k], 1);
+    out[k] += __shfl_xor_sync(quad, out[k], 2);
+  }
+}
+
 // The scalar spline in FP32 (mixed form, field32 with FP32 location
 // records): FP32 barycentrics and patch from the FP64 ordinates.
 __device__ __forceinline__ double latlon_scalar_f(const MeshView& m, const double* __restrict__ coeffs,

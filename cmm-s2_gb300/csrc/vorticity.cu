@@ -178,6 +178,27 @@ __global__ void __launch_bounds__(256) vorticity_kernel(VortParams vp, const dou
   }
 }
 
+// A series alone (no analytic field, no spline) at few points: four lanes per
+// point (sh_series_lanes).  Latency-bound: 18.6k points, degrees to 16: 76 us
+// with a thread per point, 50 so.
+__global__ void __launch_bounds__(256) vorticity_series_kernel(const double* __restrict__ sh, int lmax, MeshView vm,
+                                                               double rot, const double* __restrict__ X, int64_t Q,
+                                                               int npr, const double* __restrict__ cos_ring,
+                                                               double* __restrict__ omega) {
+  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < kShLanes * Q;
+       k += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = k / kShLanes;
+    const int g = (int)(k % kShLanes);
+    const double x = X[3 * i], y = X[3 * i + 1], z = X[3 * i + 2];
+    double v;
+    sh_series_lanes<1>(vm, sh, lmax, sh_point(x, y, z), g, &v);
+    const double r = v + 2 * rot * (z * rsqrt(x * x + y * y + z * z)) - 2 * rot * cos_ring[i / npr];
+    if (g) continue;
+    if (!isfinite(r)) atomicOr(vm.status, CMM_FLAG_NONFINITE);
+    omega[i] = r;
+  }
+}
+
 }  // namespace
 
 int launch_vorticity(int kind, const double* params, int nparams, const double* sh, int lmax,
@@ -187,6 +208,12 @@ int launch_vorticity(int kind, const double* params, int nparams, const double* 
   vp.kind = kind;
   for (int k = 0; k < nparams && k < 12; ++k) vp.p[k] = params[k];
   const int b = block_for(vm, kTuneVorticity, 128, Q);
+  if (sh && kind == CMM_VORT_NONE && !spline && Q <= kShLanesMaxQ) {
+    vorticity_series_kernel<<<grid_for(kShLanes * Q, b), b, 0, s>>>(sh, lmax, vm, rot, X, Q, npr, cos_ring, omega);
+    note_launch();
+    cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? CMM_OK : cuda_fail(e, "vorticity_series_kernel");
+  }
   vorticity_kernel<<<grid_for(Q, b), b, 0, s>>>(vp, sh, lmax, vm, spline, rot, X, Q, npr,
                                                     cos_ring, omega);
   note_launch();

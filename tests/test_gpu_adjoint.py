@@ -330,3 +330,31 @@ def test_bve_gradient_matches_whole_run_restatement(mods):
     assert e_om < 1e-10
     assert abs(J - Jt) < 1e-9 * Jt
     assert e_norm < 1e-8 and e_max < 1e-8
+
+
+@pytest.mark.parametrize("lmax", [0, 1, 2, 3, 4, 7, 33, 128])
+def test_series_in_four_lanes_matches_one(mods, lmax):
+    """The series and its point gradient at few points (four lanes per point)
+    against a thread per point: the same points at the head of a grid above
+    the limit.  Degrees around the four orders a round takes, and the largest:
+    1e-12 of the largest value ((lmax + 1) ulps of the recurrences)."""
+    native, adj, meshgen, _ = mods
+    rng = np.random.default_rng(lmax)
+    sh = torch.from_numpy(rng.standard_normal((lmax + 1, 2 * lmax + 1)) / (1 + np.arange(lmax + 1))[:, None]).cuda()
+    dsh = adj.il_series_of(sh)
+    X = rng.standard_normal((161 * 320, 3))
+    X /= np.linalg.norm(X, axis=1)[:, None]
+    X[:2] = [[0, 0, 1], [0, 0, -1]]
+    out = []
+    for L in (24, 160):
+        theta, phi, grid, verts = meshgen.latlon_mesh_arrays(L)
+        vm = native.VelMesh(L, theta, phi, grid, verts)
+        x = torch.from_numpy(X[:(L + 1) * 2 * L].copy()).cuda()
+        om = vm.vorticity(native.VORT_NONE, [], x, 0.0, sh=sh)
+        gX = torch.zeros_like(x)
+        native.check(native.lib.cmm_vorticity_bwd(vm.h, native._ptr(dsh), lmax, 0.7, native._ptr(x),
+                                                  native._ptr(torch.ones_like(om)), native._ptr(gX), None,
+                                                  native._stream()), "bwd")
+        out.append((om.reshape(-1)[:1200], gX[:1200]))
+    for a, b in zip(*out):
+        assert float((a - b).abs().max()) < 1e-12 * float(b.abs().max())
