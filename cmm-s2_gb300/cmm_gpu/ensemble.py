@@ -83,8 +83,10 @@ class SharedResources:
 # the triangles by more than this factor: assembling a submap's forms costs
 # 6.1 ms per 327,680 triangles (18.6 ns per triangle, double-double on the
 # FP64 pipe), and each evaluation through a form instead of a coefficient
-# record saves ~20 FP64 instructions (26.8 against 46.5), 32 ps at the
-# measured 0.63 x 10^12 FP64 instructions/s.
+# record saves at least 32 ps (20 FP64 instructions of 46.5 at the measured
+# 0.63 x 10^12/s for the FP64 form; the fixed-point form of the points-only
+# composition takes half of a record's time, 1.35 -> 0.65 ms per 2.1 M points
+# through 8 submaps).
 FORMS_EVALS_PER_TRIANGLE = 582
 
 

@@ -89,18 +89,5 @@ __device__ __forceinline__ long long fx_of(double x) {
 // X as a float: its high word, rounded (within 2^-25 of |x| <= 1)
 __device__ __forceinline__ float fx_f32(long long X) { return __fmul_rn((float)(int)(X >> 32), 1.4901161193847656e-08f); }
 
-// X (|x| < 16) as a float-float: 26 + 23 + 15 bits converted exactly, the
-// first two added without error, the last joining the low part.
-__device__ __forceinline__ ff fx_ff(long long X) {
-  const float a = __fmul_rn((float)(int)(X >> 38), 9.5367431640625e-07f);   // 2^-20 units
-  // 0x4b000000 | n is the float 2^23 + n for n < 2^23
-  const float b = fmaf(__uint_as_float(0x4b000000u | ((unsigned)(X >> 15) & 0x7fffffu)), 1.1368683772161603e-13f,
-                       -9.5367431640625e-07f);                               // 2^-43 units
-  const float c = fmaf(__uint_as_float(0x4b000000u | ((unsigned)X & 0x7fffu)), 3.469446951953614e-18f,
-                       -2.9103830456733704e-11f);                            // 2^-58 units
-  const float s = __fadd_rn(a, b);
-  return ff{s, __fadd_rn(__fsub_rn(b, __fsub_rn(s, a)), c)};
-}
-
 }  // namespace dev
 }  // namespace cmm
