@@ -491,9 +491,13 @@ int ring_workspace(int L, int fields, DeviceBuffer* data) {
   size_t a, b;
   int rc = data->alloc(data_bytes(L, fields, &a, &b));
   if (rc) return rc;
-  // the rows past the last ring of its block are never written
+  // the rows past the last ring of its block are never written; complete
+  // before the caller's stream, which may not wait for this one, uses them
   cudaError_t e = cudaMemset(data->p, 0, data->bytes);
-  return e == cudaSuccess ? CMM_OK : cuda_fail(e, "cudaMemset(ring data)");
+  if (e == cudaSuccess) e = cudaStreamSynchronize(0);
+  if (e == cudaSuccess) return CMM_OK;
+  data->release();
+  return cuda_fail(e, "cudaMemset(ring data)");
 }
 
 int ring_inverse(const RingTables& t, int fields, const double2* S, void* data, double* x, int* status, cudaStream_t s) {

@@ -490,7 +490,9 @@ int digit_tables_build(int L, const double* tab, std::shared_ptr<DigitTables>* o
       (rc = t->pexp.alloc((size_t)L * rows * sizeof(int))) ||
       (rc = t->ladder.alloc((size_t)(L + 3) * L * sizeof(double))))
     return rc;
-  cudaError_t e = cudaFuncSetAttribute(synth_digits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStages * kStage);
+  cudaError_t e = cudaStreamSynchronize(0);   // the upload, before s reads it
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(synth_digits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStages * kStage);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(velocity_digits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              kDigitMaxL * kFieldStride * (int)sizeof(double));
@@ -508,11 +510,15 @@ int digit_tables_build(int L, const double* tab, std::shared_ptr<DigitTables>* o
 
 int digit_workspace(int L, DeviceBuffer* tiles, DeviceBuffer* aexp) {
   int rc;
-  if ((rc = tiles->alloc((size_t)total_groups(L) * kAGroup)) || (rc = aexp->alloc((size_t)L * kCols * sizeof(int))))
+  if ((rc = aexp->alloc((size_t)L * kCols * sizeof(int))) || (rc = tiles->alloc((size_t)total_groups(L) * kAGroup)))
     return rc;
-  // the padding columns and the zero block are never written
+  // the padding columns and the zero block are never written; complete before
+  // the caller's stream, which may not wait for this one, uses the tiles
   cudaError_t e = cudaMemset(tiles->p, 0, tiles->bytes);
-  return e == cudaSuccess ? CMM_OK : cuda_fail(e, "cudaMemset(digit tiles)");
+  if (e == cudaSuccess) e = cudaStreamSynchronize(0);
+  if (e == cudaSuccess) return CMM_OK;
+  tiles->release();
+  return cuda_fail(e, "cudaMemset(digit tiles)");
 }
 
 int digit_velocity(const DigitTables& t, const double* tab, const double2* a, bool lap, double2* psi_out,

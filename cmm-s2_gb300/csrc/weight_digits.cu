@@ -287,7 +287,8 @@ int digit_weights(int L, const double* po, const double* ps, const double* Kp, c
       (rc = table.alloc((size_t)4 * ntile * G * kBGroup)) || (rc = cexp.alloc((size_t)4 * npair * sizeof(int))) ||
       (rc = fail.upload(&failed, sizeof(int))))
     return rc;
-  cudaError_t e = cudaMemsetAsync(table.p, 0, table.bytes, s);   // the zero blocks
+  cudaError_t e = cudaStreamSynchronize(0);   // the uploads, before s reads them
+  if (e == cudaSuccess) e = cudaMemsetAsync(table.p, 0, table.bytes, s);   // the zero blocks
   const size_t row_smem = (size_t)8 * (16 * G + 2) * sizeof(double);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(w_product_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStages * kStage);
