@@ -113,12 +113,12 @@ __global__ void ladder_table_kernel(int L, double* __restrict__ c) {
 }
 
 // Per call: the six coefficient fields of one order m (velocity_fields_at), in
-// shared memory, their column scales and digits (FP64-bound: 32 us at L = 512
+// shared memory, their column scales and digits (FP64-bound: 27 us at L = 512
 // where the fields alone took 38).  Also what the contraction
 // leaves out: the spectra of the two poles (zero but for m = 0), and the stream
 // function where it is asked for.  The ladder factors come from a table: their
 // square roots and the division were two thirds of the FP64 work.
-constexpr int kFieldThreads = 256;
+constexpr int kFieldThreads = 384;        // 256: 5 us more at L = 512, 128: 10
 constexpr int kFieldStride = kCols + 1;   // doubles per degree (no bank conflicts)
 
 __global__ void __launch_bounds__(kFieldThreads) velocity_digits_kernel(
