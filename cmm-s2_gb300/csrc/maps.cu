@@ -1198,9 +1198,15 @@ int build_jump_table(cmm_mesh* mesh) {
   return CMM_OK;
 }
 
+// Non-decreasing in n, so that a workspace for the largest call serves every
+// smaller one: the block count itself falls wherever order_per steps up, so
+// the histogram is sized for the most blocks of any call of up to n queries
+// (one query per thread until each SM has a block, never more blocks than SMs
+// until kOrderPer queries per thread).
 int64_t order_workspace(int64_t n) {
-  const int64_t span = (int64_t)kOrderBlock * order_per(n), nblk = (n + span - 1) / span;
-  return n + (int64_t)kOrderCells * ((nblk < 1 ? 1 : nblk) + 1);
+  const int64_t one = (n + kOrderBlock - 1) / kOrderBlock, last = (one + kOrderPer - 1) / kOrderPer;
+  const int64_t nblk = std::max<int64_t>({1, last, std::min<int64_t>(one, kNumSMs)});
+  return n + (int64_t)kOrderCells * (nblk + 1);
 }
 
 int launch_query_order(const MeshView& m, const double* q, int64_t n, int32_t* perm, int32_t* work,

@@ -166,7 +166,8 @@ int cmm_tracer_eval(const cmm_mesh* mesh, int tracer, double t, const double* X,
  * sort; the order inside a cell is unspecified), so that neighbouring threads of the
  * composition gather neighbouring coefficient records and share them in
  * L1/L2 instead of re-reading DRAM.  work: cmm_query_order_workspace(n)
- * int32 device scratch.  n <= INT32_MAX.  No counterpart in the reference
+ * int32 device scratch; the size never falls as n grows, so that scratch for
+ * the largest call serves every smaller one.  n <= INT32_MAX.  No counterpart in the reference
  * (its queries are processed in caller order by numpy). */
 int64_t cmm_query_order_workspace(int64_t n);
 int cmm_query_order(const cmm_mesh* mesh, const double* q, int64_t n, int32_t* perm,

@@ -463,3 +463,25 @@ def test_query_order_is_a_permutation(nat, n, spread):
     if spread == 2.0 and n > 1 << 17:
         p = q[perm.long()]
         assert float((p[1:] - p[:-1]).norm(dim=1).median()) < 0.1
+
+
+def test_host_pipeline_last_chunk_and_reused_scratch(nat):
+    """compose_host with a last chunk on the other side of a step of the
+    query sort's block count (n = 8 x 155,649 - 7), then a smaller call in the
+    same scratch, whose chunks sort in more blocks: both bitwise
+    Mesh.compose's."""
+    from cmm_gpu.meshgen import icosahedral_mesh
+    from cmm_gpu.workloads import submap_stack
+    verts, tris = icosahedral_mesh(3)
+    tan, s_pts = OG.stencil_points(verts)
+    m = nat.Mesh(verts, tris, 3)
+    cs = [m.assemble(dev(j)) for j in submap_stack(s_pts, tan, 2, seed=3)]
+    n = 1_245_185
+    q = torch.randn((n, 3), dtype=torch.float64, generator=torch.Generator().manual_seed(4)).pin_memory()
+    out = torch.empty_like(q).pin_memory()
+    scratch = streams = None
+    for k in (n, 600_000):
+        scratch, streams = nat.compose_host(m, cs, q[:k], out[:k], streams=streams, scratch=scratch)
+        torch.cuda.synchronize()
+        assert torch.equal(out[:k], m.compose(cs, dev(q[:k].numpy()))[0].cpu())
+    assert m.status(clear=True) == 0

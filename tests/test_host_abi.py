@@ -127,3 +127,19 @@ def test_batch_and_form_entry_points_reject_bad_arguments(native):
     assert lib.cmm_bve_step_post(None, None) == ERR_ARG
     assert lib.cmm_forms_ff(None, None, None, None) == ERR_ARG
     assert native.Mesh.FORM_FF_STRIDE == 112 and native.ShtBatch.MAX == 8
+
+
+def test_query_order_workspace_never_falls(native):
+    """A query-sort workspace for n queries serves every smaller call (the
+    host pipeline's shorter last chunk, a scratch kept for smaller calls):
+    its size never falls, over all n to 4e6 in steps and around every multiple
+    of 155,648 (a query more per thread), and holds the histograms of the
+    blocks of 1024 x queries-per-thread queries."""
+    ws = native.lib.cmm_query_order_workspace
+    ns = sorted(set(range(1, 4_000_000, 97)) | {k * 155_648 + d for k in range(1, 40) for d in range(-8, 9)})
+    sizes = [ws(n) for n in ns]
+    assert all(b > a for a, b in zip(sizes, sizes[1:]))
+    for n, w in zip(ns, sizes):
+        per = min(16, max(1, -(-n // 155_648)))
+        assert w >= n + 5120 * (-(-n // (1024 * per)) + 1)
+    assert ws(0) > 0 and ws(2**31 - 1) >= ws(2**31 - 2) and ws(-1) == -1
