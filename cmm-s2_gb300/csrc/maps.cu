@@ -41,12 +41,12 @@ constexpr int kBlock = 256;
 // outside [1/4, 4] are normalised first, so the unnormalised chain stays far
 // from overflow.
 constexpr int kNormEvery = 8;
-// default register budgets of the compositions, as resident 256-thread
-// blocks per SM; the autotuner may set others
+// default register budgets of the compositions through records, as resident
+// 256-thread blocks per SM; the autotuner may set others
 constexpr int kComposeJacBlocks = 4;
-constexpr int kComposeJacBlocksFF = 4;   // with the forms' low floats
 constexpr int kComposeBlocks = 4;
-constexpr int kFormsCallerBlocks = 3;   // points only through forms, in caller order
+constexpr int64_t kBlockWave = (int64_t)kBlock * kNumSMs;   // queries of one block per SM
+constexpr int64_t kL2Bytes = 129LL << 20;
 // Submaps listed in the kernel parameters of the usual calls (768 bytes);
 // longer lists take the 24 KB form, whose upload alone costs microseconds.
 constexpr int kShortList = 32;
@@ -435,13 +435,19 @@ __device__ __forceinline__ void record_eval(const MeshView& m, const double* __r
   }
 }
 
+// A composition's submaps: coefficient records only, some with map forms, all
+// forms with their low floats.  (Apart: the form code beside the records' cost
+// the Jacobians through records 4 %.)
+constexpr int kNoForms = 0, kForms = 1, kFormsFF = 2;
+
 // One submap from its map form: P_c = p^T Q_c p of the sub-triangle's
 // quadratic form (24 FP64 operations for the three components) and the
 // pushes' half derivatives (Q_c p) . w in float-float.  q: the form's 18
 // doubles; g (FF): the low floats of their split, else converted here to the
-// same pairs.  One component at a time: unrolled, the three copies overflow
-// the instruction cache (a quarter of the issue slots lost).
-template <bool FF>
+// same pairs.  ROLL: one component at a time; unrolled, the three copies
+// overflow the instruction cache (a quarter of the issue slots lost), but a
+// lone warp's three components overlap.  Same operations either way.
+template <bool FF, bool ROLL>
 __device__ __forceinline__ void form_push(const double* __restrict__ q, const float* __restrict__ g, const double* p,
                                           Pushes w, double* P) {
   const double2* qf = reinterpret_cast<const double2*>(q);
@@ -450,7 +456,7 @@ __device__ __forceinline__ void form_push(const double* __restrict__ q, const fl
   const double xy = p[0] * p[1], xz = p[0] * p[2], yz = p[1] * p[2];
   const ff u0 = ff_of(p[0]), u1 = ff_of(p[1]), u2 = ff_of(p[2]);
   const ff a0 = w.get(0), a1 = w.get(1), a2 = w.get(2), c0 = w.get(3), c1 = w.get(4), c2 = w.get(5);
-#pragma unroll 1
+#pragma unroll ROLL ? 1 : 3
   for (int c = 0; c < 3; ++c) {
     const double2 q01 = __ldg(qf + 3 * c), q23 = __ldg(qf + 3 * c + 1), q45 = __ldg(qf + 3 * c + 2);
     const double v = q01.x * xx + q01.y * yy + q23.x * zz + q23.y * xy + q45.x * xz + q45.y * yz;
@@ -548,13 +554,12 @@ __device__ __forceinline__ void store_jacobian(const double* __restrict__ q, int
 // coefficient records and, with JAC, through map forms.  (The fixed-point
 // evaluation of compose_forms_kernel does not pay with Jacobians: the pushes
 // fill the issue slots that it takes; 2.63 against 2.42 ms per 2^22 queries.)
-// FF: every submap with a form record also has the low floats of its split.
 // perm (nullable): process the queries in this order (grouped by coarse
 // cell, cmm_query_order) so that neighbouring threads gather neighbouring
 // records; every query's own arithmetic and output slot are unchanged.
 // MINB: resident 256-thread blocks per SM the register allocation must
 // allow (the register budget; cmm_mesh_set_variant).
-template <bool JAC, class Src, int MINB, bool FF = false>
+template <bool JAC, class Src, int MINB, int FORMS = kNoForms, bool ROLL = false>
 __global__ void __launch_bounds__(kBlock, MINB) compose_kernel(MeshView m, Src cp,
                                                          const double* __restrict__ q, int64_t n,
                                                          double* __restrict__ out,
@@ -595,7 +600,7 @@ __global__ void __launch_bounds__(kBlock, MINB) compose_kernel(MeshView m, Src c
     }
     for (int s = S - 1; s >= 0; --s) {
       double P[3];
-      const double* fr = JAC ? cp.form(s, S) : nullptr;
+      const double* fr = FORMS != kNoForms ? cp.form(s, S) : nullptr;
       const PointD pt{p[0], p[1], p[2]};
       const float fx = to_f32_trunc(p[0]), fy = to_f32_trunc(p[1]), fz = to_f32_trunc(p[2]);
       Split sp;
@@ -604,8 +609,9 @@ __global__ void __launch_bounds__(kBlock, MINB) compose_kernel(MeshView m, Src c
       if (tri_all) tri_all[(int64_t)s * n + i] = t;
       if (fr) {
         const int sub = 18 * kSubIndex[sp.lo][sp.hi];
-        form_push<FF>(fr + (int64_t)t * kFormStride + sub, FF ? cp.form_ff(s, S) + (int64_t)t * kFormFFStride + sub : nullptr,
-                      p, w, P);
+        constexpr bool FF = FORMS == kFormsFF;
+        form_push<FF, ROLL>(fr + (int64_t)t * kFormStride + sub,
+                            FF ? cp.form_ff(s, S) + (int64_t)t * kFormFFStride + sub : nullptr, p, w, P);
       } else {
         record_eval<JAC>(m, cp.at(s, S), t, p, w, P);
       }
@@ -660,60 +666,101 @@ struct PointX {
 // below FP64's roundings: entries to 2^-59, sums to ~2^-57.  A form with an
 // entry of 2 or more (a map stretching by more than about 2) goes through
 // FP64; a point outside (0.5, 1.4) in squared norm is normalised first.
-template <class Src, int MINB>
+//
+// GATHER: a warp fetches its 32 forms together, nine neighbouring lanes' 16
+// bytes a form, through shared memory.  Its loads touch two lines a form
+// where every lane's own nine touch nine times 32, and all are in flight
+// without a register: scattered queries are bound by the lines (2^22 random
+// points through 8 level-7 maps 2.98 ms with own loads at 64 registers, 2.54
+// at 80, 1.82 so; in FP64 2.48).  Grouped queries share lines through the L1,
+// of which the staging takes 144 KB: 1.35 own, 1.48 so.  All lanes of a warp
+// stay in the loop; `live` marks those with a query and a finite image.
+template <class Src, int MINB, bool GATHER>
 __global__ void __launch_bounds__(kBlock, MINB) compose_forms_kernel(MeshView m, Src cp,
                                                                      const double* __restrict__ q, int64_t n,
                                                                      double* __restrict__ out,
                                                                      int32_t* __restrict__ tri,
                                                                      int32_t* __restrict__ tri_all,
                                                                      const int32_t* __restrict__ perm) {
-  const int S = cp.count();
-  for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n;
+  __shared__ double2 stage[GATHER ? 9 * kBlock : 1];
+  const int S = cp.count(), lane = threadIdx.x & 31;
+  for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; GATHER ? j - lane < n : j < n;
        j += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = perm ? (int64_t)__ldg(perm + j) : j;
-    if ((uint64_t)i >= (uint64_t)n) {   // a bad permutation entry
+    bool live = !GATHER || j < n;
+    int64_t i = j;
+    if (live && perm) i = (int64_t)__ldg(perm + j);
+    if (live && (uint64_t)i >= (uint64_t)n) {   // a bad permutation entry
       flag(m, CMM_FLAG_INDEX);
-      continue;
+      if (!GATHER) continue;
+      live = false;
     }
     long long X[3];   // the point, units of 2^-58
     int t;
     Split sp;
-    {
-      double p[3];
-      if (!load_query(q, i, p)) {
-        store_nan<false>(m, i, n, S - 1, S, out, tri, tri_all, nullptr);
-        continue;
-      }
-      // the first location from the query's own FP64 values
-      t = locate_split(m, PointD{p[0], p[1], p[2]}, to_f32_trunc(p[0]), to_f32_trunc(p[1]), to_f32_trunc(p[2]), &sp);
-      if (tri) tri[i] = t;
-      if (tri_all) tri_all[(int64_t)(S - 1) * n + i] = t;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) X[c] = fx_of(p[c]);
+    if (GATHER) {     // of a lane that has no query
+      X[0] = X[1] = X[2] = 0;
+      t = 0;
+      sp = Split{0, 2, 1};
     }
-    bool lost = false;   // no finite image
+    if (live) {
+      double p[3];
+      live = load_query(q, i, p);
+      if (!live) {
+        store_nan<false>(m, i, n, S - 1, S, out, tri, tri_all, nullptr);
+        if (!GATHER) continue;
+      } else {
+        // the first location from the query's own FP64 values
+        t = locate_split(m, PointD{p[0], p[1], p[2]}, to_f32_trunc(p[0]), to_f32_trunc(p[1]), to_f32_trunc(p[2]), &sp);
+        if (tri) tri[i] = t;
+        if (tri_all) tri_all[(int64_t)(S - 1) * n + i] = t;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) X[c] = fx_of(p[c]);
+      }
+    }
     int s = S - 1;
     float f0 = fx_f32(X[0]), f1 = fx_f32(X[1]), f2 = fx_f32(X[2]);
     while (true) {
       const float n2 = fmaf(f0, f0, fmaf(f1, f1, f2 * f2));
-      if (!(n2 > 0.5f && n2 < 1.4f)) {
+      if (live && !(n2 > 0.5f && n2 < 1.4f)) {
         // rare: back to the unit sphere (the direction, and so the location
         // above, stays)
         PointD p = PointX{X}.fp64();
         const double inv_n = rsqrt(p.x * p.x + p.y * p.y + p.z * p.z);
-        lost = !finite3(p.x * inv_n, p.y * inv_n, p.z * inv_n);
-        if (lost) break;
-        X[0] = fx_of(p.x * inv_n);
-        X[1] = fx_of(p.y * inv_n);
-        X[2] = fx_of(p.z * inv_n);
+        live = finite3(p.x * inv_n, p.y * inv_n, p.z * inv_n);
+        if (live) {
+          X[0] = fx_of(p.x * inv_n);
+          X[1] = fx_of(p.y * inv_n);
+          X[2] = fx_of(p.z * inv_n);
+        } else {
+          store_nan<false>(m, i, n, s - 1, S, out, tri, tri_all, nullptr);
+          if (!GATHER) break;
+        }
       }
       const double* fr = cp.form(s, S);
       bool wide = fr == nullptr;
       if (fr) {
-        const double2* qf = reinterpret_cast<const double2*>(fr + (int64_t)t * kFormStride + 18 * kSubIndex[sp.lo][sp.hi]);
-        double2 Q[9];   // all in flight together where the registers hold them
+        const int sub = 18 * kSubIndex[sp.lo][sp.hi];
+        const double2* mine = stage + (GATHER ? 9 * threadIdx.x : 0);
+        double2 Q[9];
+        if (GATHER) {
+          const double2* qf = reinterpret_cast<const double2*>(fr);
+          double2* warp = stage + 9 * (threadIdx.x & ~31u);
+          const int off = (t * kFormStride + sub) / 2;
+          __syncwarp();   // the last map's forms are read
 #pragma unroll
-        for (int k = 0; k < 9; ++k) Q[k] = __ldg(qf + k);
+          for (int k = 0; k < 9; ++k) {
+            const int c = 32 * k + lane, r = c / 9;   // double2 c of the warp's, of lane r's form
+            const int o = __shfl_sync(0xffffffffu, off, r) + c - 9 * r;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(
+                             (unsigned)__cvta_generic_to_shared(warp + c)),
+                         "l"(qf + o)
+                         : "memory");
+          }
+        } else {   // all in flight together where the registers hold them
+          const double2* qf = reinterpret_cast<const double2*>(fr + (int64_t)t * kFormStride + sub);
+#pragma unroll
+          for (int k = 0; k < 9; ++k) Q[k] = __ldg(qf + k);
+        }
         const Limbs x = fx_limbs(X[0]), y = fx_limbs(X[1]), z = fx_limbs(X[2]);
         auto prod = [](Limbs a, Limbs b) {
           FxSum v{0, 0};
@@ -724,15 +771,21 @@ __global__ void __launch_bounds__(kBlock, MINB) compose_forms_kernel(MeshView m,
         const Limbs xy = prod(x, y), xz = prod(x, z), yz = prod(y, z);
         int bad = 0;
         long long Y[3];
+        if (GATHER) {
+          asm volatile("cp.async.wait_all;" ::: "memory");
+          __syncwarp();
+        }
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
           FxSum r{0, 0};
-          r.add(fx_entry(Q[3 * c].x, bad), xx);
-          r.add(fx_entry(Q[3 * c].y, bad), yy);
-          r.add(fx_entry(Q[3 * c + 1].x, bad), zz);
-          r.add(fx_entry(Q[3 * c + 1].y, bad), xy);
-          r.add(fx_entry(Q[3 * c + 2].x, bad), xz);
-          r.add(fx_entry(Q[3 * c + 2].y, bad), yz);
+          const double2 q0 = GATHER ? mine[3 * c] : Q[3 * c], q1 = GATHER ? mine[3 * c + 1] : Q[3 * c + 1],
+                        q2 = GATHER ? mine[3 * c + 2] : Q[3 * c + 2];
+          r.add(fx_entry(q0.x, bad), xx);
+          r.add(fx_entry(q0.y, bad), yy);
+          r.add(fx_entry(q1.x, bad), zz);
+          r.add(fx_entry(q1.y, bad), xy);
+          r.add(fx_entry(q2.x, bad), xz);
+          r.add(fx_entry(q2.y, bad), yz);
           Y[c] = r.value();
         }
         wide = bad < 0;
@@ -741,7 +794,7 @@ __global__ void __launch_bounds__(kBlock, MINB) compose_forms_kernel(MeshView m,
           for (int c = 0; c < 3; ++c) X[c] = Y[c];
         }
       }
-      if (wide) {   // in FP64: a coefficient record, or a form out of range
+      if (live && wide) {   // in FP64: a coefficient record, or a form out of range
         const PointD u = PointX{X}.fp64();
         double p[3] = {u.x, u.y, u.z}, P[3];
         if (fr) {
@@ -757,24 +810,30 @@ __global__ void __launch_bounds__(kBlock, MINB) compose_forms_kernel(MeshView m,
           const double inv_n = rsqrt(r2);
 #pragma unroll
           for (int c = 0; c < 3; ++c) P[c] *= inv_n;
-          lost = !finite3(P[0], P[1], P[2]);
-          if (lost) break;
+          live = finite3(P[0], P[1], P[2]);
+          if (!live) {
+            store_nan<false>(m, i, n, s - 1, S, out, tri, tri_all, nullptr);
+            if (!GATHER) break;
+          }
         }
 #pragma unroll
         for (int c = 0; c < 3; ++c) X[c] = fx_of(P[c]);
       }
       if (--s < 0) break;
-      f0 = fx_f32(X[0]);
-      f1 = fx_f32(X[1]);
-      f2 = fx_f32(X[2]);
-      t = locate_split(m, PointX{X}, f0, f1, f2, &sp);
-      if (tri_all) tri_all[(int64_t)s * n + i] = t;
+      if (live) {
+        f0 = fx_f32(X[0]);
+        f1 = fx_f32(X[1]);
+        f2 = fx_f32(X[2]);
+        t = locate_split(m, PointX{X}, f0, f1, f2, &sp);
+        if (tri_all) tri_all[(int64_t)s * n + i] = t;
+      }
     }
+    if (!live) continue;
     double p[3] = {(double)X[0], (double)X[1], (double)X[2]};   // the units drop out
     const double inv_n = rsqrt(p[0] * p[0] + p[1] * p[1] + p[2] * p[2]);
 #pragma unroll
     for (int c = 0; c < 3; ++c) p[c] *= inv_n;
-    if (lost || !finite3(p[0], p[1], p[2])) {
+    if (!finite3(p[0], p[1], p[2])) {
       store_nan<false>(m, i, n, s - 1, S, out, tri, tri_all, nullptr);
       continue;
     }
@@ -1100,9 +1159,6 @@ int launch_compose(const MeshView& m, const double* const* coeffs, int S, const 
   bool ff = forms_ff != nullptr;
   for (int k = 0; forms && k < S; ++k)
     if (forms[k] && !(forms_ff && forms_ff[k])) ff = false;
-  // by the argument alone, as the device-driven step chooses (their results
-  // are bitwise equal, also while a run's stack is still empty)
-  const bool any = forms != nullptr;
   const int b = block_for(m, kTuneCompose, kBlock, n);
   const int vj = m.variant[CMM_VARIANT_COMPOSE_JAC], v = m.variant[CMM_VARIANT_COMPOSE];
   auto run = [&](auto list) {
@@ -1114,28 +1170,51 @@ int launch_compose(const MeshView& m, const double* const* coeffs, int S, const 
       list.g[k] = forms && forms[k] && forms_ff ? forms_ff[k] : nullptr;
     }
     auto go = [&](auto kernel) { kernel<<<grid_for(n, b), b, 0, s>>>(m, list, q, n, out, tri, tri_all, jac, perm); };
-    constexpr bool tuned = sizeof(list.p) <= kShortList * sizeof(double*);   // variants for the usual lists only
-    constexpr int J2 = tuned ? 2 : kComposeJacBlocks, J3 = tuned ? 3 : kComposeJacBlocks;
-    constexpr int F2 = tuned ? 2 : kComposeJacBlocksFF, F3 = tuned ? 3 : kComposeJacBlocksFF;
-    constexpr int V6 = tuned ? 6 : kComposeBlocks;
-    if (jac && forms && ff) {
-      if (vj == 2) go(compose_kernel<true, Src, F2, true>);
-      else if (vj == 3) go(compose_kernel<true, Src, F3, true>);
-      else go(compose_kernel<true, Src, kComposeJacBlocksFF, true>);
+    if (jac && forms) {
+      // by the queries that the chip holds at 2, 3 or 4 blocks per SM: below
+      // that the warps are few, and 128 registers with the components unrolled
+      // are faster (level 5, 8 maps, 20,000 queries 39 against 58 us of 4
+      // blocks rolled; 100,000: 91 with 2 blocks, 74 with 3, 79 with 4; 2^20: 654,
+      // 598, 572).  Scattered low floats want the loads in flight of 3 blocks
+      // (2^22 random queries, level 7: 3.88 ms against 4.18 of 4 blocks), but
+      // not while a third wave of blocks would be the larger part (250,000
+      // at level 5: 199 against 189 us).
+      const int v = vj ? vj : n <= 2 * kBlockWave ? 2 : (n <= 3 * kBlockWave || (ff && !perm && n > 8 * kBlockWave)) ? 3 : 4;
+      if (ff) {
+        if (v == 2) go(compose_kernel<true, Src, 2, kFormsFF, false>);
+        else if (v == 3) go(compose_kernel<true, Src, 3, kFormsFF, true>);
+        else go(compose_kernel<true, Src, 4, kFormsFF, true>);
+      } else {
+        if (v == 2) go(compose_kernel<true, Src, 2, kForms, false>);
+        else if (v == 3) go(compose_kernel<true, Src, 3, kForms, true>);
+        else go(compose_kernel<true, Src, 4, kForms, true>);
+      }
     } else if (jac) {
-      if (vj == 2) go(compose_kernel<true, Src, J2>);
-      else if (vj == 3) go(compose_kernel<true, Src, J3>);
+      if (vj == 2) go(compose_kernel<true, Src, 2>);
+      else if (vj == 3) go(compose_kernel<true, Src, 3>);
       else go(compose_kernel<true, Src, kComposeJacBlocks>);
-    } else if (any) {
+    } else if (forms) {
       auto gof = [&](auto kernel) { kernel<<<grid_for(n, b), b, 0, s>>>(m, list, q, n, out, tri, tri_all, perm); };
-      // in caller order the gathers may be scattered: 80 registers hold a
-      // form's nine loads in flight (2^22 random queries 2.53 against 2.95
-      // ms; grouped ones 1.45 against 1.35, a sample grid 287 against 270 us)
-      if (v == 6) gof(compose_forms_kernel<Src, V6>);
-      else if (v == 4 || perm) gof(compose_forms_kernel<Src, kComposeBlocks>);
-      else gof(compose_forms_kernel<Src, kFormsCallerBlocks>);
+      // Own loads pay where a warp's queries share records: with several
+      // queries per triangle, if they are grouped or a map's forms stay in the
+      // L2 (73 MB at level 6, 294 at level 7).  Own against shared fetches:
+      // grouped 250,000 / 600,000 / 2^20 / 2^22 queries at level 7 129 / 254 /
+      // 385 / 1355 against 119 / 247 / 394 / 1504 us, at level 5 92 / 189 / 300 /
+      // 1172 against 100 / 208 / 343 / 1350; caller order, random 250,000 at
+      // level 6 69 against 62, 10^6 sample points there 172 against 198,
+      // 525,000 at level 7 221 against 208.  While 3 blocks per SM hold all
+      // queries 80 registers are faster (60,000 at level 7: 52 / 50 against 61 /
+      // 52).
+      const bool far = (int64_t)m.nt * kFormStride * 8 > kL2Bytes;
+      const bool scattered = perm ? n < 2 * (int64_t)m.nt : (far || n < 4 * (int64_t)m.nt);
+      if (v == 6) gof(compose_forms_kernel<Src, 6, false>);
+      else if (v == 4) gof(compose_forms_kernel<Src, 4, false>);
+      else if (n <= 3 * kBlockWave && n > kBlockWave && far) gof(compose_forms_kernel<Src, 3, true>);
+      else if (n <= 3 * kBlockWave) gof(compose_forms_kernel<Src, 3, false>);
+      else if (scattered) gof(compose_forms_kernel<Src, 4, true>);
+      else gof(compose_forms_kernel<Src, 4, false>);
     } else {
-      if (v == 6) go(compose_kernel<false, Src, V6>);
+      if (v == 6) go(compose_kernel<false, Src, 6>);
       else go(compose_kernel<false, Src, kComposeBlocks>);
     }
   };
@@ -1246,7 +1325,7 @@ int launch_compose_dev(const MeshView& m, const double* const* table, const BveS
   };
   auto gof = [&](auto kernel) { kernel<<<grid_for(n, b), b, 0, s>>>(m, cp, q, n, out, nullptr, nullptr, nullptr); };
   if (ftable)
-    six ? gof(compose_forms_kernel<DevSubmaps, 6>) : gof(compose_forms_kernel<DevSubmaps, kComposeBlocks>);
+    six ? gof(compose_forms_kernel<DevSubmaps, 6, false>) : gof(compose_forms_kernel<DevSubmaps, kComposeBlocks, false>);
   else
     six ? go(compose_kernel<false, DevSubmaps, 6>) : go(compose_kernel<false, DevSubmaps, kComposeBlocks>);
   return check_launch("compose_kernel");

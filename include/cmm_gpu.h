@@ -479,11 +479,11 @@ int cmm_mesh_set_block(cmm_mesh* mesh, int kernel, int threads);
  * autotuner from measured timings; 0 restores the default).  The
  * composition kernels are compiled for several register budgets, named by
  * the resident 256-thread blocks per SM they allow: with Jacobians 2, 3 or
- * 4 (128, 80 or 64 registers a thread; default 4), points only 4 or 6 (64
- * or 40; default 4, but 3 through map forms in the caller's order).  Fewer
- * registers hide more gather latency, more avoid spills.  Applies to lists of
- * at most 32 submaps; longer ones take the default.  Results do not depend on
- * the variant.  No counterpart in the reference. */
+ * 4 (128, 80 or 64 registers a thread), points only 4 or 6 (64 or 40).
+ * Default: 4 through coefficient records; through map forms by the number
+ * and order of the queries.  Fewer registers hide more gather latency, more
+ * avoid spills.  Results do not depend on the variant.  No counterpart in the
+ * reference. */
 #define CMM_VARIANT_COMPOSE_JAC 0
 #define CMM_VARIANT_COMPOSE 1
 int cmm_mesh_set_variant(cmm_mesh* mesh, int knob, int value);

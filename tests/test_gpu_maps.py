@@ -485,3 +485,38 @@ def test_host_pipeline_last_chunk_and_reused_scratch(nat):
         torch.cuda.synchronize()
         assert torch.equal(out[:k], m.compose(cs, dev(q[:k].numpy()))[0].cpu())
     assert m.status(clear=True) == 0
+
+
+@pytest.mark.parametrize("n", [38_913, 77_825, 116_737, 311_297, 327_679, 327_681])
+def test_composition_variants_bitwise_equal(nat, n):
+    """Either side of each rule by which a composition through map forms picks
+    its kernel (own or shared fetches, blocks per SM, rolled components), with
+    and without an order: points, ids of every submap and Jacobians bitwise
+    those of the same queries in calls of 5000, a ragged last warp, queries
+    without an image and a form out of the fixed-point range included."""
+    from cmm_gpu.meshgen import icosahedral_mesh, stencil_frames, random_sphere_points
+    from cmm_gpu.workloads import submap_stack
+    verts, tris = icosahedral_mesh(6)
+    tan, s_pts = stencil_frames(verts)
+    m = nat.Mesh(verts, tris, 6)
+    jets = submap_stack(s_pts, tan, 4, seed=12)
+    jets[2] *= 3.0
+    cs = [m.assemble(dev(j)) for j in jets]
+    fs = [m.assemble_forms(c) for c in cs]
+    fs[1] = None
+    gs = [None if f is None else m.forms_ff(f) for f in fs]
+    q = dev(random_sphere_points(n, seed=n))
+    q[100:100 + 7] = float("nan")
+    q[20_003] = 0.0
+    q[n - 2] *= 1e-3
+    perm = m.query_order(q)
+    for kw in (dict(), dict(want_jac=True), dict(want_jac=True, forms_ff=gs)):
+        def call(x, **k):
+            X, _, ta, J = m.compose(cs, x, want_tri_all=True, forms=fs, **kw, **k)
+            return [X.view(torch.int64), ta.t()] + ([] if J is None else [J.view(torch.int64)])
+        parts = [call(q[i:i + 5000]) for i in range(0, n, 5000)]
+        ref = [torch.cat([p[k] for p in parts]) for k in range(len(parts[0]))]
+        for k in (dict(), dict(perm=perm)):
+            for a, b in zip(call(q, **k), ref):
+                assert torch.equal(a, b)
+    assert m.status(clear=True) == nat.FLAG_NONFINITE
