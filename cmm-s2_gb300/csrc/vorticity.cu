@@ -20,6 +20,7 @@ constexpr double kPi = 3.141592653589793;
 struct VortParams {
   int kind;
   double p[12];
+  float iw, lat[9];   // Gaussian jets: 1 / width and the latitudes in FP32
 };
 
 // zonal jet family (dynamical_fields.py:181-192)
@@ -67,14 +68,17 @@ __device__ double omega0(const VortParams& v, double px, double py, double theta
       const int n = (int)v.p[2];
       // the terms share a sign: those below 2^-60 of the nearest jet's (an
       // exponent larger by 42, from FP32 distances) do not reach the sum, and a
-      // division and an exponential are ~35 FP64 instructions
-      const float latf = to_f32_trunc(lat), iw = __frcp_rn(to_f32_trunc(v.p[1]));
+      // division and an exponential are ~35 FP64 instructions.  A distance is
+      // taken at the far end of its rounding for the nearest jet and at the near
+      // end for one to be left out: a width may be below the latitudes' rounding
+      const float latf = to_f32_trunc(lat);
       float d2[9], dmin = __int_as_float(0x7f800000);
 #pragma unroll
       for (int j = 0; j < 9; ++j) {
-        const float d = (latf - to_f32_trunc(v.p[3 + j])) * iw;
-        d2[j] = d * d;
-        if (j < n) dmin = fminf(dmin, d2[j]);
+        const float d = fabsf(latf - v.lat[j]), e = fmaf(2.4e-7f, fabsf(latf) + fabsf(v.lat[j]), 1e-37f);
+        const float near = fmaxf(d - e, 0.f) * v.iw, far = (d + e) * v.iw;   // NaN - e: 0
+        d2[j] = near * near;
+        if (j < n) dmin = fminf(dmin, far * far);
       }
 #pragma unroll
       for (int j = 0; j < 9; ++j) {
@@ -207,6 +211,8 @@ int launch_vorticity(int kind, const double* params, int nparams, const double* 
   VortParams vp{};
   vp.kind = kind;
   for (int k = 0; k < nparams && k < 12; ++k) vp.p[k] = params[k];
+  vp.iw = 1.f / fabsf((float)vp.p[1]);
+  for (int k = 0; k < 9; ++k) vp.lat[k] = (float)vp.p[3 + k];
   const int b = block_for(vm, kTuneVorticity, 128, Q);
   if (sh && kind == CMM_VORT_NONE && !spline && Q <= kShLanesMaxQ) {
     vorticity_series_kernel<<<grid_for(kShLanes * Q, b), b, 0, s>>>(sh, lmax, vm, rot, X, Q, npr, cos_ring, omega);

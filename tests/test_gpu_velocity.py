@@ -256,3 +256,24 @@ def test_velocity_scales_exactly_and_at_its_limits(nat, nvs):
     out = vm.velocity(vc, 0.0, 0.05, 0.1, 1.5 * x)
     assert float((out / 2.25 - V).abs().max()) < 1e-12 * scale
     assert vm.status() == 0
+
+
+@pytest.mark.parametrize("width", [0.1, 1e-6, 1e-9])
+def test_narrow_gaussian_jets(nat, width):
+    """Jets narrower than the FP32 spacing of their latitudes (6e-8 at 0.75), one
+    on either side of an FP32 value, at points around them: every term that
+    counts is in the sum.  Against numpy on the same coordinates; the
+    colatitude's rounding (3e-16) over the width is an error of that size in
+    d, at most 1 in the slope of exp(-d^2): 1e-15 + 1e-15 / width."""
+    L = 24
+    vm, _ = velmesh(nat, L)
+    lats = np.array([0.75 + 1e-10, 0.75 - 3e-8, -0.4])
+    lat = 0.75 + np.linspace(-5e-8, 5e-8, 2 * L * (L + 1))
+    lat[::7] = lats[0] + width * np.linspace(-2, 2, len(lat[::7]))
+    lat[::11] = -0.4 + width * np.linspace(-2, 2, len(lat[::11]))
+    X = np.stack([np.cos(lat), np.zeros_like(lat), np.sin(lat)], 1)
+    got = host(vm.vorticity(nat.VORT_GAUSSIAN_JETS, [1.0, width, 3.0, *lats], dev(X), 0.0)).reshape(-1)
+    la = np.pi / 2 - np.arctan2(np.sqrt(X[:, 1]**2 + X[:, 0]**2), X[:, 2])
+    ref = np.exp(-((la[:, None] - lats) / width)**2).sum(1)
+    assert np.abs(got - ref).max() < 20 * 2.0**-52 + 1e-15 / width
+    assert vm.status(clear=True) == 0
