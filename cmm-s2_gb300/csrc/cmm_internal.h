@@ -77,7 +77,6 @@ struct MeshView {
   const double* ring_n;
   const double* diag_n;
   double dphi, dthe;
-  int loc_exp;              // every entry of the inverse vertex rows is below 2^loc_exp
   // velocity records (ncomp = 3) in FP32 (cmm_velmesh_set_records):
   // (nt, 64) floats, assembled from the FP32 copy of the factors
   int rec32;

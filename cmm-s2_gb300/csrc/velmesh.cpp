@@ -1,7 +1,6 @@
 // Host-side construction of the MWSS lat-lon velocity mesh
 // (structure_spherical_triangulation, cmm_s2/core/mesh_functions.py:169-318)
 // and the Lagrange time weights of the velocity interpolant.
-#include <algorithm>
 #include <cmath>
 
 #include "cmm_internal.h"
@@ -48,7 +47,6 @@ int build_latlon(int L, const double* theta, const double* phi, const double* gr
   latlon_triangles(L, tv);
   const int nt = (int)tv.size();
   std::vector<double> loc((size_t)nt * kLocStride), asmf((size_t)nt * kAsmStride);
-  double rmax = 1.0;
   for (int t = 0; t < nt; ++t) {
     auto V = [&](int i) { return D3{verts[3 * i], verts[3 * i + 1], verts[3 * i + 2]}; };
     D3 v1 = V(tv[t].x), v2 = V(tv[t].y), v3 = V(tv[t].z);
@@ -57,7 +55,6 @@ int build_latlon(int L, const double* theta, const double* phi, const double* gr
     r[13] = v1.x;
     r[14] = v1.y;
     r[15] = v1.z;
-    for (int k = 0; k < 9; ++k) rmax = std::max(rmax, std::fabs(r[k]));
     assembly_factors(v1, v2, v3, &asmf[(size_t)t * kAsmStride]);
   }
   std::vector<double> vpad(4 * (size_t)nv), gpad(4 * (size_t)M * N);
@@ -147,7 +144,6 @@ int build_latlon(int L, const double* theta, const double* phi, const double* gr
   v.sh_ab = (const double*)m->sh_ab.p;
   v.sh_fm = (const double*)m->sh_fm.p;
   // spacing as the reference computes it (mesh_functions.py:214-215)
-  v.loc_exp = std::ilogb(rmax) + 1;
   v.dphi = std::fabs(phi[1] - phi[0]);
   v.dthe = std::fabs(theta[1] - theta[0]);
   v.phi0_f = (float)phi[0];

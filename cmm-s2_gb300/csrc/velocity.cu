@@ -44,7 +44,7 @@ __device__ __forceinline__ W3 stage(const TimeWeights& tw, int s, const BveState
   return W3{tw.w[s][0], tw.w[s][1], tw.w[s][2]};
 }
 
-// FP64 records in FP64: points off the unit sphere, weights of 2 or more,
+// FP64 records in FP64: points off the unit sphere, weights of 4 or more,
 // ordinates near the ends of the exponent range.
 __device__ __noinline__ void velocity_wide(const MeshView& m, const VelPtrs& vc, int nvs, const W3 w, int t, double x,
                                            double y, double z, double* V) {
@@ -73,24 +73,34 @@ __device__ __noinline__ void velocity_wide(const MeshView& m, const VelPtrs& vc,
 // operations bind the RK4 foot points on GB300 (82 % of the FP64 pipe); here
 // the FP64 pipe forms p - v1 only.  The barycentrics b = R (p - v1) + (1,0,0)
 // carry no cancellation (R p loses the triangle's inverse size, ~1/h, in
-// FP64's last places), the Bernstein weights and each level's six ordinates
-// (relative to the level's largest) go through 2^-58 steps, and the levels are
-// combined in the largest one's scale: every result is within a few 2^-57 of
-// the largest ordinate, where the FP64 sum rounds at 2^-53 per term.
+// FP64's last places) and are within 2^(k-55), 2^k the power of two above the
+// triangle's largest entry of R (one for the mesh, which the polar triangles
+// set, made them 1.5 to 2 times worse than FP64's near the equator: L = 512
+// 8e-14).  The Bernstein weights and each level's six ordinates (relative to
+// the level's largest) go through 2^-58 steps, and the levels are combined in
+// the largest one's scale: from the barycentrics on, a result is within a few
+// 2^-57 of the largest ordinate, where the FP64 sum rounds at 2^-53 per term.
 __device__ __forceinline__ void velocity_fixed(const MeshView& m, const VelPtrs& vc, int nvs, const W3 w, int t,
                                                double x, double y, double z, double* V) {
   const double* L = m.tri_loc + (int64_t)t * kLocStride;   // R (9), norms (4), v1 (3)
   int bad = 0;
   const Limbs d0 = fx_limbs(fx_of(x - __ldg(L + 13))), d1 = fx_limbs(fx_of(y - __ldg(L + 14))),
               d2 = fx_limbs(fx_of(z - __ldg(L + 15)));
-  const int ke = m.loc_exp;   // |R| < 2^ke
+  double R[9];
+  int eR = 0;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) {
+    R[k] = __ldg(L + k);
+    eR = max(eR, fx_exponent(R[k]));
+  }
+  const int ke = eR - 1022;   // |R| < 2^ke, and ke >= 0: a row's norm is at least 1
   long long b[3];
 #pragma unroll
   for (int r = 0; r < 3; ++r) {
     FxSum v{0, 0};
-    v.add(fx_scaled(__ldg(L + 3 * r), 1022 + ke, bad), d0);
-    v.add(fx_scaled(__ldg(L + 3 * r + 1), 1022 + ke, bad), d1);
-    v.add(fx_scaled(__ldg(L + 3 * r + 2), 1022 + ke, bad), d2);
+    v.add(fx_scaled(R[3 * r], eR, bad), d0);
+    v.add(fx_scaled(R[3 * r + 1], eR, bad), d1);
+    v.add(fx_scaled(R[3 * r + 2], eR, bad), d2);
     b[r] = (v.hi << ke) + (v.lo >> (30 - ke));
   }
   b[0] += 1LL << 58;
@@ -118,7 +128,7 @@ __device__ __forceinline__ void velocity_fixed(const MeshView& m, const VelPtrs&
   const Limbs B[6] = {fx_limbs(prod(gV, gV)), fx_limbs(prod(gE, gE)), fx_limbs(prod(gC, gC)),
                       fx_limbs(prod(gV, gE) << 1), fx_limbs(prod(gE, gC) << 1), fx_limbs(prod(gV, gC) << 1)};
   const int* id = kSplitOrd[lo][hi];
-  // the levels' patches times their weights (halved, |w| < 2), in the scale
+  // the levels' patches times their weights (halved, |w| < 4), in the scale
   // 2^(em - 1022) of the largest ordinate so far; one level's code (three
   // unrolled overflow the instruction cache)
   long long U[3] = {0, 0, 0};

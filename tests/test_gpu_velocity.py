@@ -277,3 +277,63 @@ def test_narrow_gaussian_jets(nat, width):
     ref = np.exp(-((la[:, None] - lats) / width)**2).sum(1)
     assert np.abs(got - ref).max() < 20 * 2.0**-52 + 1e-15 / width
     assert vm.status(clear=True) == 0
+
+
+def exact_amplitude(verts, p):
+    """(b_hi - b_mid + e (b_mid - b_lo) + c b_lo)^2 of the points p (n, 3) in the
+    triangles of verts (n, 3, 3): the patch whose ordinates are all 1, in
+    50-digit arithmetic from the vertices."""
+    import decimal
+    ctx = decimal.Context(prec=50)
+    out = []
+    for V, q in zip(verts, p):
+        with decimal.localcontext(ctx):
+            V = [[decimal.Decimal(float(x)) for x in v] for v in V]
+            q = [decimal.Decimal(float(x)) for x in q]
+            det = lambda a, b, c: sum(a[i] * (b[(i + 1) % 3] * c[(i + 2) % 3] - b[(i + 2) % 3] * c[(i + 1) % 3])
+                                      for i in range(3))
+            norm = lambda *vs: sum(sum(x)**2 for x in zip(*vs)).sqrt()
+            D = det(*V)
+            b = [det(q, V[1], V[2]) / D, det(V[0], q, V[2]) / D, det(V[0], V[1], q) / D]
+            lo, mid, hi = sorted(range(3), key=lambda k: b[k])
+            out.append(float((b[hi] - b[mid] + norm(V[hi], V[mid]) * (b[mid] - b[lo]) + norm(*V) * b[lo])**2))
+    return np.array(out)
+
+
+@pytest.mark.parametrize("L,colat", [(512, 1.57), (1024, 1.57), (512, 0.6), (512, 0.02), (128, 1.55), (24, 1.5)])
+def test_velocity_barycentrics_no_worse_than_fp64(nat, L, colat):
+    """The fixed-point evaluation near the equator, where the triangles are
+    largest, and towards the pole, where their inverses are: the patch whose
+    ordinates are all 1 (so its value is the barycentrics' error and nothing
+    else) at 1500 points, largest error against 50 digits no larger than that
+    of the FP64 evaluation, which points of norm 2 take (homogeneous of degree
+    2, exactly a factor of 4)."""
+    vm, verts = velmesh(nat, L)
+    tv = OG.LatLonMesh(L).simplices
+    rng = np.random.default_rng(L)
+    n = 1500
+    th, ph = colat + 0.015 * rng.uniform(-1, 1, n), rng.uniform(0, 2 * np.pi, n)
+    p = np.stack([np.sin(th) * np.cos(ph), np.sin(th) * np.sin(ph), np.cos(th)], 1)
+    ones = vm.new_coeffs()
+    ones[:, :57] = 1.0
+    tri = host(vm.locate(dev(p))[0])
+    ref = exact_amplitude(verts[tv[tri]], p)
+    fixed = host(vm.velocity([ones], 0.0, 0.0, 0.1, dev(p.T)))
+    wide = host(vm.velocity([ones], 0.0, 0.0, 0.1, dev(2 * p.T))) / 4
+    assert np.abs(fixed - ref).max() <= np.abs(wide - ref).max()
+
+
+@pytest.mark.parametrize("w", [2.0, 3.0, 3.9999999, 4.0, 4.0000001, 5.5])
+def test_velocity_weights_either_side_of_the_fixed_range(nat, w):
+    """Two levels at a time whose second weight is w (the fixed-point range
+    ends at 4): the combination of the levels' own velocities, 1e-14 of the
+    largest term (each within 1e-15)."""
+    from cmm_gpu.meshgen import random_sphere_points
+    d = golden("velocity_L8.npz")
+    vm, _ = velmesh(nat, 8)
+    vc = [vm.assemble(dev(v)) for v in d["vals"][:2]]
+    x = dev(np.ascontiguousarray(random_sphere_points(3001, seed=5).T))
+    a, b = (vm.velocity([c], 0.0, 0.0, 0.125, x) for c in vc)
+    got = vm.velocity(vc, 0.0, w * 0.125, 0.125, x)
+    scale = max(float(a.abs().max()), float(b.abs().max())) * w
+    assert float((got - ((1 - w) * a + w * b)).abs().max()) < 1e-14 * scale
