@@ -5,21 +5,21 @@
 //   S_even/odd[t][n] = sum_{l - m even/odd} Pbar_lm(theta_t) A[l][n]
 // over ring pairs t and 12 real columns n (six complex fields).  GB300 has 2
 // FP64 multiply-adds per SM and cycle, so FP64 arithmetic takes 12 L^3 / 4 of
-// them (1.03 ms at L = 512) where the table's bytes need 60 us.  Instead every
-// row of Pbar (over l) and every column of A gets the power of two above its
-// largest entry as its scale, and each entry becomes the integer x 2^53 / scale,
-// rounded (entries of the largest one's binade exactly, the others to half an
-// ulp of it: the size of one FP64 rounding of the sum), cut into six signed
+// them (1.03 ms at L = 512) where the table's bytes need 60 us.  Instead, in
+// each group of 16 degrees of one parity, every row of Pbar (over l) and every
+// column of A gets the power of two above its largest entry as its scale, and
+// each entry becomes the integer x 2^53 / scale, rounded (entries of the largest
+// one's binade exactly, the others to half an ulp of it), cut into six signed
 // digits of 9 bits: integers of at most 256, exact in bf16.  Products of digits
-// i and j belong to level i + j; the levels' sums over 64 degrees are integers
-// accumulated exactly in FP32 in tensor memory (levels 0 to 3 stay within 4 x
-// 64 x 2^16 = 2^24; the lower levels' bound is larger only for digits that are
-// all extreme, and they then round at 2^-52 of the scales' product), and are
-// added up as 64-bit integers.  Levels 7 and up (2^-61 of the scales' product)
-// are left out.  The scheme is known as Ozaki splitting.  Measured: 1032 -> 98 us
-// at L = 512, 167 -> 31 at L = 256, 59 -> 13 at L = 128, results to the same
-// error against 64 bits.
-//
+// i and j belong to level i + j; the levels' sums over a group are integers,
+// accumulated exactly in FP32 in tensor memory (at most 6 x 16 x 2^16 < 2^24),
+// and make one 64-bit integer.  Levels 7 and up (2^-61 of the scales' product)
+// are left out.  The groups' integers are added in 64 bits at the largest scale
+// met.  The scheme is known as Ozaki splitting.  The scales follow the decay of
+// a smooth field's coefficients and the growth of Pbar towards high degrees
+// near the poles: e^(-l/8) at L = 512, first five rings, error relative to the
+// ring's own value at orders 2 and 20: 9e-16 and 3e-15 (FP64 2e-15 and 1e-15);
+// a scale per 64 degrees 4e-14 and 2e-10, one for all degrees 4e-13 and 2e-2.
 // Layouts: both operands as K-major core-matrix images without swizzle in
 // groups of 16 degrees of one parity.  The table (12 bytes per entry) of (m,
 // row block): [even groups, odd groups][6 digits][2 halves of 8 degrees][8-row
@@ -56,9 +56,14 @@ constexpr int kAGroup = 2 * 14 * 128;                      // one degree group o
 constexpr int kPStage = kChunkGroups * kRowGroupBytes * (kRows / 8);
 constexpr int kStage = kPStage + kChunkGroups * kAGroup;   // 110 KiB
 constexpr int kStages = 2;
+constexpr int kMaxGroups = 2 * (kDigitMaxL / 32);          // degree groups of one order
+constexpr int kAccs = 4;                // accumulators, of one degree group each
+constexpr int kScaleBytes = kChunkGroups * (2 * kRows + 4 * kCols);   // a chunk's scales: rows' shorts, columns' ints
+constexpr int kScales = 4;              // chunks of them
+constexpr int kSmemBytes = kStages * kStage + kScales * kScaleBytes;
 constexpr int kAccCols = 16 * kLevels;  // 112 of 128 TMEM columns per accumulator
-constexpr uint32_t kTmemCols = 256;
-constexpr int kNonFinite = 1 << 20;     // column scale of a column with an infinity or NaN
+constexpr uint32_t kTmemCols = 128 * kAccs;
+constexpr int kNonFinite = 1 << 20;     // column scale of a group with an infinity or NaN
 
 struct DigGeometry {
   int L, rows, nblk;      // ring pairs t = 1 .. rows, in nblk blocks
@@ -66,40 +71,41 @@ struct DigGeometry {
 };
 
 // ----------------------------------------------------------- tables, data
-// Block (row block, m): the digit table of its rows from the FP64 table
-// tab[m][l - m][t], one thread per row; scales in pexp[m][t - 1].
+// Block (row block, degree group, m): the digit table of its rows and degrees
+// from the FP64 table tab[m][l - m][t], one thread per row; the rows' scales in
+// pexp, laid out as the table: [m][row block][group][row].
 __global__ void __launch_bounds__(kRows) build_digits_kernel(DigGeometry g, const double* __restrict__ tab,
                                                              unsigned char* __restrict__ out,
-                                                             int* __restrict__ pexp) {
-  const int blk = blockIdx.x, m = blockIdx.y, row = threadIdx.x, L = g.L;
+                                                             short* __restrict__ pexp) {
+  const int blk = blockIdx.x, grp = blockIdx.y, m = blockIdx.z, row = threadIdx.x, L = g.L;
   const int npair = L / 2 + 1, t = 1 + blk * kRows + row, n = L - m;
   const int rg = min(kRows / 8, (g.rows - blk * kRows + 7) / 8), rgt = (g.rows + 7) / 8;
-  if (row >= 8 * rg) return;
+  const int ke = groups16((n + 1) / 2), ko = groups16(n / 2), par = grp >= ke;
+  if (grp >= ke + ko || row >= 8 * rg) return;
   const bool real = t <= g.rows;
   const double* P = tab + tab_off(m, L, npair) + t;
+  const int k0 = par + 32 * (par ? grp - ke : grp);
+  double x[16];
   int e = 1;
-  if (real)
-    for (int k = 0; k < n; ++k) e = max(e, (__double2hiint(P[(int64_t)k * npair]) >> 20) & 2047);
-  const int ke = groups16((n + 1) / 2), ko = groups16(n / 2);
-  unsigned char* base = out + (int64_t)g.gbase[m] * kRowGroupBytes * rgt +
-                        (int64_t)(ke + ko) * kRowGroupBytes * (kRows / 8) * blk + (row >> 3) * 128 + (row & 7) * 16;
-  const int gb = kRowGroupBytes * rg;   // bytes of one degree group of this block
-  for (int q = 0; q < 2 * (ke + ko); ++q) {
-    const int grp = q >> 1, half = q & 1, par = grp >= ke;
-    const int k0 = 16 * (par ? grp - ke : grp) + 8 * half;
+#pragma unroll
+  for (int u = 0; u < 16; ++u) {
+    x[u] = real && k0 + 2 * u < n ? P[(int64_t)(k0 + 2 * u) * npair] : 0.0;
+    e = max(e, (__double2hiint(x[u]) >> 20) & 2047);
+  }
+  unsigned char* o = out + (int64_t)g.gbase[m] * kRowGroupBytes * rgt +
+                     (int64_t)(ke + ko) * kRowGroupBytes * (kRows / 8) * blk + (int64_t)grp * kRowGroupBytes * rg +
+                     (row >> 3) * 128 + (row & 7) * 16;
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
     long long v[8];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int k = par + 2 * (k0 + u);
-      v[u] = real && k < n ? to_fixed(P[(int64_t)k * npair], e) : 0;
-    }
+    for (int u = 0; u < 8; ++u) v[u] = to_fixed(x[8 * half + u], e);
     uint4 d[kDigits];
     digits8(v, d);
-    unsigned char* o = base + (int64_t)grp * gb + half * rg * 128;
 #pragma unroll
-    for (int i = 0; i < kDigits; ++i) *(uint4*)(o + i * 2 * rg * 128) = d[i];
+    for (int i = 0; i < kDigits; ++i) *(uint4*)(o + (2 * i + half) * rg * 128) = d[i];
   }
-  if (real) pexp[(int64_t)m * g.rows + t - 1] = e;
+  pexp[(int64_t)g.gbase[m] * 8 * rgt + (int64_t)(ke + ko) * kRows * blk + grp * 8 * rg + row] = (short)e;
 }
 
 // c[k][l] = sqrt(max(l(l+1) - k(k-1), 0)) / 2, k = 0 .. L+1, and in row L+2
@@ -126,48 +132,48 @@ __global__ void __launch_bounds__(kFieldThreads) velocity_digits_kernel(
     const double* __restrict__ c, const double* __restrict__ tab, unsigned char* __restrict__ tiles,
     int* __restrict__ aexp, double2* __restrict__ S) {
   extern __shared__ double fld[];   // [l - m][kFieldStride]
-  __shared__ int emax[kCols];
+  __shared__ int emax[kMaxGroups][kCols];
   __shared__ double pole[2][kCols];
   const int m = blockIdx.x, L = g.L, n = L - m, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid < kCols) emax[tid] = 1;
+  const int ke = groups16((n + 1) / 2), ko = groups16(n / 2);
   if (psi_out)
     for (int l = tid; l < m; l += kFieldThreads) psi_out[(int64_t)m * L + l] = make_double2(0.0, 0.0);
-  __syncthreads();
-  int e[kCols];
-#pragma unroll
-  for (int k = 0; k < kCols; ++k) e[k] = 0;
-  for (int i = tid; i < n; i += kFieldThreads) {
-    const int l = m + i;
-    const double d = lap ? c[(int64_t)(L + 2) * L + l] : 1.0;
-    double cc[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int q = m - 1 + k;   // q(q-1) is symmetric: order -1 as order 2
-      cc[k] = c[(int64_t)(q < 0 ? 2 : q) * L + l];
-    }
+  for (int i0 = 32 * warp; i0 < n; i0 += kFieldThreads) {   // a warp's degrees: one group of either parity
+    const int i = i0 + lane, l = m + i;
     double2 f[kVelLegendre];
-    velocity_fields_at(a, L, l, m, d, cc, f);
 #pragma unroll
-    for (int k = 0; k < kVelLegendre; ++k) {
-      fld[i * kFieldStride + 2 * k] = f[k].x;
-      fld[i * kFieldStride + 2 * k + 1] = f[k].y;
-      e[2 * k] = max(e[2 * k], (__double2hiint(f[k].x) >> 20) & 2047);
-      e[2 * k + 1] = max(e[2 * k + 1], (__double2hiint(f[k].y) >> 20) & 2047);
+    for (int k = 0; k < kVelLegendre; ++k) f[k] = make_double2(0.0, 0.0);
+    if (i < n) {
+      const double d = lap ? c[(int64_t)(L + 2) * L + l] : 1.0;
+      double cc[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int q = m - 1 + k;   // q(q-1) is symmetric: order -1 as order 2
+        cc[k] = c[(int64_t)(q < 0 ? 2 : q) * L + l];
+      }
+      velocity_fields_at(a, L, l, m, d, cc, f);
+      if (psi_out) psi_out[(int64_t)m * L + l] = f[0];
+#pragma unroll
+      for (int k = 0; k < kVelLegendre; ++k) {
+        fld[i * kFieldStride + 2 * k] = f[k].x;
+        fld[i * kFieldStride + 2 * k + 1] = f[k].y;
+      }
     }
-    if (psi_out) psi_out[(int64_t)m * L + l] = f[0];
-  }
+    const int grp = (lane & 1 ? ke : 0) + i0 / 32;
 #pragma unroll
-  for (int k = 0; k < kCols; ++k) {
-    e[k] = __reduce_max_sync(0xffffffffu, e[k]);
-    if (lane == 0) atomicMax(&emax[k], e[k]);
+    for (int k = 0; k < kCols; ++k) {
+      const int e = max(1, (__double2hiint(k & 1 ? f[k >> 1].y : f[k >> 1].x) >> 20) & 2047);
+      const int ev = __reduce_max_sync(0xffffffffu, lane & 1 ? 0 : e), od = __reduce_max_sync(0xffffffffu, lane & 1 ? e : 0);
+      if (lane < 2 && grp < ke + ko) emax[grp][k] = lane ? od : ev;
+    }
   }
   __syncthreads();
-  if (tid < kCols) aexp[m * kCols + tid] = emax[tid] == 2047 ? kNonFinite : emax[tid];
-  const int ke = groups16((n + 1) / 2), ko = groups16(n / 2);
+  for (int k = tid; k < (ke + ko) * kCols; k += kFieldThreads)
+    aexp[g.gbase[m] * kCols + k] = emax[0][k] == 2047 ? kNonFinite : emax[0][k];
   unsigned char* base = tiles + (int64_t)g.gbase[m] * kAGroup;
   for (int u = tid; u < 2 * (ke + ko) * kCols; u += kFieldThreads) {
     const int col = u % kCols, q = u / kCols, grp = q >> 1, half = q & 1, par = grp >= ke;
-    const int k0 = 16 * (par ? grp - ke : grp) + 8 * half, ec = emax[col];
+    const int k0 = 16 * (par ? grp - ke : grp) + 8 * half, ec = emax[grp][col];
     long long v[8];
 #pragma unroll
     for (int w = 0; w < 8; ++w) {
@@ -210,11 +216,11 @@ __global__ void __launch_bounds__(kFieldThreads) velocity_digits_kernel(
 // ------------------------------------------------------------- synthesis
 // Persistent, one block per SM, over the work items (m, row block) in order
 // of decreasing length, dealt in alternating direction so that each block's
-// share is about the same.  Three roles: warp 4 streams the chunks (up to 64
+// share is about the same.  Three roles: warp 12 streams the chunks (up to 64
 // degrees of one parity: 96 KiB of table, 14 KiB of data) into two stages by
-// bulk copies, warp 5 issues a chunk's MMAs (six per 16 degrees) into one of
-// two accumulators, and warps 0-3, a ring pair per lane, add the levels into
-// 64-bit integers and write an item's spectra at its end.  Bounded by the
+// bulk copies, warp 13 issues six MMAs per group of 16 degrees into one of four
+// accumulators, and warps 0-11, a ring pair and four columns per lane, add the
+// groups' levels to 64-bit integers and write an item's spectra at its end.  Bounded by the
 // table's bytes; copies of one stage are always in flight while the other is
 // multiplied.  Every wait is bounded; a timeout in one role stops all.
 struct DigCursor {
@@ -254,26 +260,19 @@ __device__ __forceinline__ int row_groups(const DigGeometry& g, int blk) {
   return min(kRows / 8, (g.rows - blk * kRows + 7) / 8);
 }
 
-// v 2^p (v zero or normal)
-__device__ __noinline__ double scale_wide(double v, int p) { return ldexp(v, p); }
-__device__ __forceinline__ double scale2(double v, int p) {
-  const int h = __double2hiint(v), e = (h >> 20) & 2047;
-  if (e == 0) return v;
-  if ((unsigned)(e + p - 1) >= 2046u) return scale_wide(v, p);
-  return __hiloint2double(h + p * (1 << 20), __double2loint(v));
-}
-
-constexpr int kSynThreads = 192;
+constexpr int kAddWarps = 12, kAddCols = kCols / 3;
+constexpr int kSynThreads = 32 * (kAddWarps + 2);
 
 __global__ void __launch_bounds__(kSynThreads, 1) synth_digits_kernel(DigGeometry g, int nitems,
                                                                       const unsigned char* __restrict__ ptab,
-                                                                      const int* __restrict__ pexp,
+                                                                      const short* __restrict__ pexp,
                                                                       const unsigned char* __restrict__ tiles,
                                                                       const int* __restrict__ aexp,
                                                                       double2* __restrict__ S,
                                                                       int* __restrict__ status) {
-  extern __shared__ __align__(1024) unsigned char smem[];   // kStages stages of kStage bytes
-  __shared__ __align__(8) uint64_t full[kStages], empty[kStages], acc_full[2], acc_empty[2];
+  extern __shared__ __align__(1024) unsigned char smem[];   // the stages, then the chunks' scales
+  __shared__ __align__(8) uint64_t full[kStages], empty[kStages], acc_full[kAccs], acc_empty[kAccs];
+  __shared__ __align__(8) uint64_t sc_full[kScales], sc_empty[kScales];
   __shared__ uint32_t tmem_base_s;
   __shared__ volatile int abort_s;
   __shared__ int drain_fail_s;
@@ -284,9 +283,13 @@ __global__ void __launch_bounds__(kSynThreads, 1) synth_digits_kernel(DigGeometr
       mbar_init(&full[b], 1);
       mbar_init(&empty[b], 1);
     }
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < kScales; ++b) {
+      mbar_init(&sc_full[b], 1);
+      mbar_init(&sc_empty[b], kAddWarps);
+    }
+    for (int b = 0; b < kAccs; ++b) {
       mbar_init(&acc_full[b], 1);
-      mbar_init(&acc_empty[b], 4);
+      mbar_init(&acc_empty[b], kAddWarps);
     }
     abort_s = 0;
     drain_fail_s = 0;
@@ -305,13 +308,15 @@ __global__ void __launch_bounds__(kSynThreads, 1) synth_digits_kernel(DigGeometr
   const uint32_t tmem = tmem_base_s;
   DigCursor u;
   u.round = 0;
-  if (warp == 4 && lane == 0) {
+  if (warp == kAddWarps && lane == 0) {
     const int rgt = (g.rows + 7) / 8;
     long long j = 0;
     bool ok = dig_item(u, nitems, g);
     while (ok && !abort_s) {
       const int st = (int)(j % kStages);
       if (j >= kStages && !wait_or_abort(&empty[st], (uint32_t)((j / kStages - 1) & 1), &abort_s)) break;
+      const int sc = (int)(j % kScales);
+      if (j >= kScales && !wait_or_abort(&sc_empty[sc], (uint32_t)((j / kScales - 1) & 1), &abort_s)) break;
       int first;
       const int ng = chunk_groups(u, &first), gb = kRowGroupBytes * row_groups(g, u.blk);
       const int64_t base = g.gbase[u.m];
@@ -321,6 +326,12 @@ __global__ void __launch_bounds__(kSynThreads, 1) synth_digits_kernel(DigGeometr
       mbar_expect_tx(&full[st], (uint32_t)(ng * (gb + kAGroup)));
       bulk_g2s(d, sp, (uint32_t)(ng * gb), &full[st]);
       bulk_g2s(d + kPStage, tiles + (base + first) * kAGroup, (uint32_t)(ng * kAGroup), &full[st]);
+      unsigned char* e = smem + kStages * kStage + sc * kScaleBytes;
+      const int rows = 8 * row_groups(g, u.blk);
+      mbar_expect_tx(&sc_full[sc], (uint32_t)(ng * (2 * rows + 4 * kCols)));
+      bulk_g2s(e, aexp + (base + first) * kCols, (uint32_t)(4 * ng * kCols), &sc_full[sc]);
+      bulk_g2s(e + 4 * kChunkGroups * kCols, pexp + base * 8 * rgt + (int64_t)(u.ke + u.ko) * kRows * u.blk + first * rows,
+               (uint32_t)(2 * ng * rows), &sc_full[sc]);
       ++j;
       ok = dig_next(u, nitems, g);
     }
@@ -329,118 +340,160 @@ __global__ void __launch_bounds__(kSynThreads, 1) synth_digits_kernel(DigGeometr
       bool drained = true;
       for (long long k = (j > kStages ? j - kStages : 0); k < j; ++k)
         drained &= mbar_wait(&full[k % kStages], (uint32_t)((k / kStages) & 1));
+      for (long long k = (j > kScales ? j - kScales : 0); k < j; ++k)
+        drained &= mbar_wait(&sc_full[k % kScales], (uint32_t)((k / kScales) & 1));
       if (!drained) drain_fail_s = 1;
     }
-  } else if (warp == 5 && lane == 0) {
+  } else if (warp == kAddWarps + 1 && lane == 0) {
     const uint32_t s0 = smem_u32(smem);
-    long long j = 0;
-    bool committed = false;
-    bool ok = dig_item(u, nitems, g);
-    while (ok && !abort_s) {
-      const int b = (int)(j & 1), st = (int)(j % kStages);
-      if (j >= 2 && !wait_or_abort(&acc_empty[b], (uint32_t)(((j >> 1) - 1) & 1), &abort_s)) break;
+    long long j = 0, k = 0;   // chunks, groups
+    bool ok = dig_item(u, nitems, g), stop = false;
+    while (ok && !stop && !abort_s) {
+      const int st = (int)(j % kStages);
       if (!wait_or_abort(&full[st], (uint32_t)((j / kStages) & 1), &abort_s)) break;
-      tc_fence_after();
       int first;
       const int ng = chunk_groups(u, &first), rg = row_groups(g, u.blk);
-      for (int q = 0; q < ng; ++q) {
+      for (int q = 0; q < ng; ++q, ++k) {
+        const int b = (int)(k % kAccs);
+        if (k >= kAccs && !wait_or_abort(&acc_empty[b], (uint32_t)((k / kAccs - 1) & 1), &abort_s)) {
+          stop = true;
+          break;
+        }
+        tc_fence_after();
         const uint32_t pa = s0 + st * kStage + q * kRowGroupBytes * rg;
         const uint64_t db = smem_desc(s0 + st * kStage + kPStage + q * kAGroup, kAGroup / 2, 128u);
         // rows past the block's last 8-row group read what lies behind it in
         // the stage; their results are not used
         for (int i = 0; i < kDigits; ++i)
           mma_bf16(tmem + b * 128 + 16 * i, smem_desc(pa + i * 2 * rg * 128, (uint32_t)rg * 128u, 128u), db,
-                   mma_idesc(kAccCols - 16 * i), (q > 0 || i > 0) ? 1u : 0u);
+                   mma_idesc(kAccCols - 16 * i), i > 0 ? 1u : 0u);
+        mma_commit(&acc_full[b]);
       }
+      if (stop) break;
       mma_commit(&empty[st]);
-      mma_commit(&acc_full[b]);
-      committed = true;
       ++j;
       ok = dig_next(u, nitems, g);
     }
     // products in flight complete before the tensor memory is released (bounded)
-    if (abort_s && committed) {
-      const long long jl = j - 1;
-      if (!mbar_wait(&empty[jl % kStages], (uint32_t)((jl / kStages) & 1))) drain_fail_s = 1;
-    }
-  } else if (warp < 4) {
-    long long E[kCols], acc[kCols];   // units of 2^-52 of the scales' product
-    float El[kCols], accl[kCols];     // the lower levels, in the same unit
+    if (abort_s && k > 0 && !mbar_wait(&acc_full[(k - 1) % kAccs], (uint32_t)(((k - 1) / kAccs) & 1))) drain_fail_s = 1;
+  } else if (warp < kAddWarps) {
+    constexpr int N = kAddCols;
+    const int quad = warp & 3, col0 = N * (warp >> 2);
+    const uint32_t lanes = tmem + ((uint32_t)(32 * quad) << 16) + (uint32_t)col0;
+    // sums in units of 2^53 2^(ex - 2150) (below 2^62: 32 groups of 2^57), ex the
+    // largest of the groups' exponents so far; the even degrees' beside
+    long long acc[N], E[N];
+    int ex[N], Ex[N];
 #pragma unroll
-    for (int k = 0; k < kCols; ++k) {
-      E[k] = acc[k] = 0;
-      El[k] = accl[k] = 0.f;
+    for (int n = 0; n < N; ++n) {
+      acc[n] = 0;
+      ex[n] = 0;
     }
-    long long j = 0;
-    bool have = dig_item(u, nitems, g);
-    while (have) {
-      const int b = (int)(j & 1);
-      if (!wait_or_abort(&acc_full[b], (uint32_t)((j >> 1) & 1), &abort_s)) break;
+    // a level's sum as an integer, |x| <= 2^22: the bits of 1.5 2^23 + x, less
+    // those of 1.5 2^23 (taken off the group's products at once)
+    constexpr long long kBits = 0x4B400000LL;
+    auto bits = [](float x) { return __float_as_int(__fadd_rn(x, 12582912.f)); };
+    // one group's levels are on their way from tensor memory while the one
+    // before is added (rows past the last ring: never stored)
+    float v[N * kLevels];
+    auto start = [&](unsigned k) {
+      const unsigned b = k % kAccs;
+      if (!warp_wait(&acc_full[b], (k / kAccs) & 1, &abort_s)) return false;
       tc_fence_after();
-      const bool rows_here = 32 * warp < 8 * row_groups(g, u.blk);   // uniform for the warp
-      if (rows_here) {
-        const uint32_t buf = tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)b * 128;
-        long long h[kCols];
+      tmem_start7x4(lanes + b * 128, 16, v);
+      return true;
+    };
+    int i = 0, q = 0;   // group of the item, of the chunk
+    unsigned j = 0;     // chunks
+    bool have = dig_item(u, nitems, g) && start(0);
+    int rows = have ? 8 * row_groups(g, u.blk) : 0;
+#pragma unroll 1
+    for (unsigned k = 0; have; ++k) {   // groups
+      long long h[N];   // the group's products in units of 2^53
+      tmem_wait7x4(v);
 #pragma unroll
-        for (int s = 0; s < kLevels; ++s) {
-          float v[16];
-          tmem_ld16(buf + 16 * s, v);
-#pragma unroll
-          for (int k = 0; k < kCols; ++k) {
-            if (s == 0)
-              h[k] = __float2int_rn(v[k]);
-            else if (s <= 4)
-              h[k] = h[k] * 512 + __float2int_rn(v[k]);
-            else
-              accl[k] = fmaf(v[k], s == 5 ? 1.f / 512.f : 1.f / 262144.f, accl[k]);
-          }
-        }
-#pragma unroll
-        for (int k = 0; k < kCols; ++k) acc[k] += h[k];
+      for (int n = 0; n < N; ++n) {
+        h[n] = mad_wide(bits(v[n]), 1 << 27, -kBits * ((1 << 27) + (1 << 18) + 512 + 1));   // 512^3; 512 and 2 to come
+        h[n] = mad_wide(bits(v[N + n]), 1 << 18, h[n]);
+        h[n] = mad_wide(bits(v[2 * N + n]), 512, h[n]);
+        h[n] = mad_wide(bits(v[3 * N + n]), 1, h[n]);
+        h[n] = mad_wide(__float2int_rn(v[4 * N + n]), 2, h[n] * 1024);
+        h[n] = mad_wide(__float2int_rn(fmaf(v[6 * N + n], 2.f / 262144.f, v[5 * N + n] * (2.f / 512.f))), 1, h[n]);
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[b])) : "memory");
-      if (u.c == u.nce - 1) {   // the even degrees are complete
+      if (lane == 0)
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[k % kAccs])) : "memory");
+      // the group's scales, exponents biased
+      const unsigned sc = j % kScales;
+      if (q == 0 && !warp_wait(&sc_full[sc], (j / kScales) & 1, &abort_s)) break;
+      const unsigned char* scales = smem + kStages * kStage + sc * kScaleBytes;
+      const int pe = ((const short*)(scales + 4 * kChunkGroups * kCols))[q * rows + min(32 * quad + lane, rows - 1)];
+      const int4 ae = *(const int4*)(scales + 4 * (q * kCols + col0));
+      const bool even_end = i + 1 == u.ke, item_end = i + 1 == u.ke + u.ko;
+      const bool chunk_end = even_end || item_end || q + 1 == kChunkGroups;
+      const int m = u.m, t = 1 + u.blk * kRows + 32 * quad + lane;
+      if (chunk_end) {
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&sc_empty[sc])) : "memory");
+        ++j;
+      }
+      q = chunk_end ? 0 : q + 1;
+      ++i;
+      if (item_end) {
+        ++u.round;
+        have = dig_item(u, nitems, g);
+        rows = 8 * row_groups(g, u.blk);
+        i = 0;
+      }
+      have = have && start(k + 1);
+      // at the larger of the two scales, rounded
+      const int e[N] = {pe + ae.x, pe + ae.y, pe + ae.z, pe + ae.w};
+      bool up = false;
 #pragma unroll
-        for (int k = 0; k < kCols; ++k) {
-          E[k] = acc[k];
-          El[k] = accl[k];
-          acc[k] = 0;
-          accl[k] = 0.f;
+      for (int n = 0; n < N; ++n) up = up || e[n] > ex[n];
+      if (__any_sync(0xffffffffu, up)) {
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+          const int d = min(max(e[n] - ex[n], 0), 62);
+          acc[n] = (acc[n] + ((1LL << d) >> 1)) >> d;
+          ex[n] = max(ex[n], e[n]);
         }
       }
-      if (u.c == u.nch - 1) {   // the work item's last chunk: its spectra
-        const int t = 1 + u.blk * kRows + 32 * warp + lane;
-        if (t <= g.rows) {
-          const int pe = pexp[(int64_t)u.m * g.rows + t - 1] - 2096;
-          // value = (hi + lo) 2^54 2^(pe + ae - 2150), (hi + lo) 2^54 the
-          // integers' products, the scales' exponents biased
-          int ae_[kCols];   // all loads before the stores
 #pragma unroll
-          for (int k = 0; k < kCols; ++k) ae_[k] = aexp[u.m * kCols + k];
+      for (int n = 0; n < N; ++n) {
+        const int d = min(ex[n] - e[n], 62);
+        acc[n] += (h[n] + ((1LL << d) >> 1)) >> d;
+      }
+      if (even_end) {   // the even degrees are complete
 #pragma unroll
-          for (int f = 0; f < kVelLegendre; ++f) {
-            double v[2][2];
+        for (int n = 0; n < N; ++n) {
+          E[n] = acc[n];
+          Ex[n] = ex[n];
+          acc[n] = 0;
+          ex[n] = 0;
+        }
+      }
+      if (item_end) {   // the item's spectra
 #pragma unroll
-            for (int r = 0; r < 2; ++r) {
-              const int k = 2 * f + r, ae = ae_[k];
-              v[0][r] = scale2((double)(E[k] + acc[k]) + (double)(El[k] + accl[k]), pe + ae);
-              v[1][r] = scale2((double)(E[k] - acc[k]) + (double)(El[k] - accl[k]), pe + ae);
-              if (ae == kNonFinite) v[0][r] = v[1][r] = __longlong_as_double(0x7ff8000000000000LL);
-            }
-            store_velocity_spectra(S, L, f, t, u.m, make_double2(v[0][0], v[0][1]));
-            if (L - t != t) store_velocity_spectra(S, L, f, L - t, u.m, make_double2(v[1][0], v[1][1]));
+        for (int f = 0; f < N / 2; ++f) {
+          double z[2][2];
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const int n = 2 * f + r;
+            // an integer unit is 2^53 2^(pe - 1075) 2^(ae - 1075)
+            const double ev = fixed_to_double(E[n], Ex[n] - 2097), od = fixed_to_double(acc[n], ex[n] - 2097);
+            z[0][r] = ev + od;
+            z[1][r] = ev - od;
+            if (max(Ex[n], ex[n]) >= kNonFinite) z[0][r] = z[1][r] = __longlong_as_double(0x7ff8000000000000LL);
+            acc[n] = 0;
+            ex[n] = 0;
           }
-        }
-#pragma unroll
-        for (int k = 0; k < kCols; ++k) {
-          E[k] = acc[k] = 0;
-          El[k] = accl[k] = 0.f;
+          const int fld = f + col0 / 2;
+          if (t <= g.rows) store_velocity_spectra(S, L, fld, t, m, make_double2(z[0][0], z[0][1]));
+          if (t <= g.rows && L - t != t) store_velocity_spectra(S, L, fld, L - t, m, make_double2(z[1][0], z[1][1]));
         }
       }
-      ++j;
-      have = dig_next(u, nitems, g);
     }
   }
   tc_fence_before();
@@ -487,12 +540,12 @@ int digit_tables_build(int L, const double* tab, std::shared_ptr<DigitTables>* o
   int rc, dev = 0;
   if ((rc = t->gbase.upload(gb.data(), gb.size() * sizeof(int))) ||
       (rc = t->digits.alloc((size_t)gb[L] * kRowGroupBytes * rgt)) ||
-      (rc = t->pexp.alloc((size_t)L * rows * sizeof(int))) ||
+      (rc = t->pexp.alloc((size_t)gb[L] * 8 * rgt * sizeof(short))) ||
       (rc = t->ladder.alloc((size_t)(L + 3) * L * sizeof(double))))
     return rc;
   cudaError_t e = cudaStreamSynchronize(0);   // the upload, before s reads it
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(synth_digits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStages * kStage);
+    e = cudaFuncSetAttribute(synth_digits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(velocity_digits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              kDigitMaxL * kFieldStride * (int)sizeof(double));
@@ -500,7 +553,8 @@ int digit_tables_build(int L, const double* tab, std::shared_ptr<DigitTables>* o
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&t->sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return cuda_fail(e, "digit_tables_build");
   const DigGeometry g = t->geometry();
-  build_digits_kernel<<<dim3(g.nblk, L), kRows, 0, s>>>(g, tab, (unsigned char*)t->digits.p, (int*)t->pexp.p);
+  build_digits_kernel<<<dim3(g.nblk, gb[1], L), kRows, 0, s>>>(g, tab, (unsigned char*)t->digits.p,
+                                                               (short*)t->pexp.p);
   if ((rc = check("build_digits_kernel"))) return rc;
   ladder_table_kernel<<<dim3((L + 127) / 128, L + 3), 128, 0, s>>>(L, (double*)t->ladder.p);
   if ((rc = check("ladder_table_kernel"))) return rc;
@@ -509,8 +563,9 @@ int digit_tables_build(int L, const double* tab, std::shared_ptr<DigitTables>* o
 }
 
 int digit_workspace(int L, DeviceBuffer* tiles, DeviceBuffer* aexp) {
+  const size_t n = total_groups(L);
   int rc;
-  if ((rc = aexp->alloc((size_t)L * kCols * sizeof(int))) || (rc = tiles->alloc((size_t)total_groups(L) * kAGroup)))
+  if ((rc = aexp->alloc(n * kCols * sizeof(int))) || (rc = tiles->alloc(n * kAGroup)))
     return rc;
   // the padding columns and the zero block are never written; complete before
   // the caller's stream, which may not wait for this one, uses the tiles
@@ -529,8 +584,8 @@ int digit_velocity(const DigitTables& t, const double* tab, const double2* a, bo
       g, a, lap, psi_out, (const double*)t.ladder.p, tab, (unsigned char*)tiles, (int*)aexp, S);
   int rc = check("velocity_digits_kernel");
   if (rc) return rc;
-  synth_digits_kernel<<<std::min(nitems, t.sms), kSynThreads, kStages * kStage, s>>>(
-      g, nitems, (const unsigned char*)t.digits.p, (const int*)t.pexp.p, (const unsigned char*)tiles,
+  synth_digits_kernel<<<std::min(nitems, t.sms), kSynThreads, kSmemBytes, s>>>(
+      g, nitems, (const unsigned char*)t.digits.p, (const short*)t.pexp.p, (const unsigned char*)tiles,
       (const int*)aexp, S, status);
   return check("synth_digits_kernel");
 }

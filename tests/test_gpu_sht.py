@@ -482,3 +482,30 @@ def test_split_velocity_tiles_match_the_field_route(nat, L):
         got, ref = jets[i, 0, 1:-1], smp[i, 1:-1].reshape(-1)
         assert np.abs(got - ref).max() < 1e-6 * scale
     assert tc.status() == 0
+
+
+@pytest.mark.parametrize("L", [128, 200, 512, 1024])
+@pytest.mark.parametrize("m,decay", [(1, 3), (1, 40), (2, 8), (20, 8)])
+def test_digit_synthesis_of_smooth_orders_near_the_poles(nat, L, m, decay):
+    """One order of a smooth field, coefficients e^(-l/decay): near the poles the
+    degrees with the largest Pbar have the smallest coefficients.  The digit
+    synthesis' u_z = i m psi on every ring against the FP64 contraction of the
+    same table (cmm_sht_inverse), relative to the ring's own largest value on
+    rings 1 to 5 and to the field's elsewhere.  Emulated in long double, the
+    digits err by up to 2e-14 of a ring's value (order 2, e^(-l/3); the others
+    3e-15) and FP64 by 3e-15; 5e-14 allows both and the ring transforms."""
+    theta, phi, g, verts, Phi, The = grid(L)
+    rng = np.random.default_rng(L + m)
+    vm = nat.VelMesh(L, theta, phi, g, verts)
+    sht = nat.Sht(L).set_tables(1)
+    l = np.arange(L)
+    psi = np.zeros((L, L), dtype=complex)
+    psi[m, m:] = (np.exp(-l / decay) * rng.choice([-1.0, 1.0], L) * rng.uniform(0.5, 1, L))[m:]
+    jets = torch.empty((3, 4, vm.nv), dtype=torch.float64, device="cuda")
+    nat.check(nat.lib.cmm_sht_velocity(sht.h, vm.h, None, nat._ptr(dev(psi)), nat._ptr(jets), nat._stream()), "velocity")
+    got = jets[2, 0, 1:-1].reshape(L - 1, 2 * L).cpu().numpy()
+    ref = sht.inverse(dev(1j * m * psi)).cpu().numpy()[1:-1]
+    err, own = np.abs(got - ref).max(1), np.abs(ref).max(1)
+    assert (err[:5] <= 5e-14 * own[:5]).all(), (err / own)[:5]
+    assert err.max() <= 5e-14 * own.max()
+    assert sht.status() == 0
