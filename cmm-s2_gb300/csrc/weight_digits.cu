@@ -3,8 +3,12 @@
 // sht_digits.cu describes the scheme): W[m][t][i] = sum_jj Pbar_(m+i)m(odd ring
 // jj) Kp[v][jj][t] + we_t Pbar_(m+i)m(ring t).  Set-up work of a table, L^4 / 16
 // multiply-adds: FP64-bound (about 10 of the 15 ms that a table took at L =
-// 512).  One scale per row (m, i) and per column (v, t); rows of one order and
-// parity in blocks of 128, tiles of 32 columns, 64 jj per accumulation chunk.
+// 512).  Rows of one order and parity in blocks of 128, tiles of 32 columns,
+// chunks of 32 jj, each with a scale per row (m, i) and per column (v, t); the
+// chunks' integers are added at the largest scale met.  (Pbar is largest next
+// to the poles and Kp next to jj = t: with one scale for all jj the weights of
+// low orders erred 2 to 3 times as much as by FP64 sums, so 0.5 to 0.7 times:
+// emulated, L = 256 and 512.)
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 
@@ -25,7 +29,7 @@ using namespace tc;
 
 namespace {
 
-constexpr int kRows = 128, kNT = 32, kChunk = 4, kStages = 4;
+constexpr int kRows = 128, kNT = 32, kChunk = 2, kStages = 4;
 constexpr int kAGroup = kDigits * 2 * 128 * (kRows / 8);   // 16 jj of a row block
 constexpr int kBGroup = 2 * kLevels * kNT / 8 * 128;       // 16 jj of a column tile, zero block last
 constexpr int kStage = kAGroup + kBGroup;
@@ -34,27 +38,33 @@ constexpr uint32_t kTmemCols = 512;
 constexpr int kAddWarps = 8, kThreads = 32 * (kAddWarps + 2), kCols = kNT / 2;
 constexpr int kBatch = 64;                                 // orders whose row digits exist at a time
 
+constexpr int kMaxChunks = kDigitMaxL / 2 / (16 * kChunk);
+
 struct WBlock {
   int m, par, rb;
 };
 
-// Block (tile, v): the column scales and digits of Kp[v][jj][t], t of the tile.
+__host__ __device__ __forceinline__ int chunks_of(int G) { return (G + kChunk - 1) / kChunk; }
+
+// Block (tile, v): the column scales, cexp[chunk][v][t], and digits of
+// Kp[v][jj][t], t of the tile.
 __global__ void __launch_bounds__(256) w_table_kernel(int npo, int npair, int G, const double* __restrict__ Kp,
                                                       unsigned char* __restrict__ out, int* __restrict__ cexp) {
-  __shared__ int emax[kNT];
+  __shared__ int emax[kMaxChunks][kNT];
   const int tile = blockIdx.x, v = blockIdx.y, c = threadIdx.x % kNT, t = tile * kNT + c, ntile = gridDim.x;
   const double* K = Kp + (int64_t)v * npo * npair + t;
-  if (threadIdx.x < kNT) emax[threadIdx.x] = 1;
+  const int nch = chunks_of(G);
+  for (int ch = threadIdx.x / kNT; ch < nch; ch += 256 / kNT) {
+    int e = 1;
+    if (t < npair)
+      for (int k = 16 * kChunk * ch; k < min(npo, 16 * kChunk * (ch + 1)); ++k)
+        e = max(e, (__double2hiint(K[(int64_t)k * npair]) >> 20) & 2047);
+    emax[ch][c] = cexp[(ch * 4 + v) * ntile * kNT + t] = e;
+  }
   __syncthreads();
-  int e = 1;
-  if (t < npair)
-    for (int k = threadIdx.x / kNT; k < npo; k += 256 / kNT) e = max(e, (__double2hiint(K[(int64_t)k * npair]) >> 20) & 2047);
-  atomicMax(&emax[c], e);
-  __syncthreads();
-  e = emax[c];
-  if (threadIdx.x < kNT && t < npair) cexp[v * npair + t] = e;
   unsigned char* base = out + ((int64_t)v * ntile + tile) * G * kBGroup + (c >> 3) * 128 + (c & 7) * 16;
   for (int q = threadIdx.x / kNT; q < 2 * G; q += 256 / kNT) {
+    const int e = emax[q / (2 * kChunk)][c];
     long long x[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
@@ -69,13 +79,13 @@ __global__ void __launch_bounds__(256) w_table_kernel(int npo, int npair, int G,
   }
 }
 
-// Eight rows per block (of row block blockIdx.x / 16): scales and digits of
-// po[m][i][jj], i = 2 r + par.
+// Eight rows per block (of row block blockIdx.x / 16): scales, rexp[block][chunk]
+// [row], and digits of po[m][i][jj], i = 2 r + par.
 __global__ void __launch_bounds__(256) w_rows_kernel(int L, int npo, int G, const WBlock* __restrict__ blocks,
                                                      const double* __restrict__ po, unsigned char* __restrict__ out,
                                                      int* __restrict__ rexp) {
   extern __shared__ double sm[];   // [8][stride]
-  __shared__ int es[8];
+  __shared__ int es[kMaxChunks][8];
   const int b = blockIdx.x >> 4, rg = blockIdx.x & 15, stride = 16 * G + 2;
   const WBlock w = blocks[b];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -83,19 +93,21 @@ __global__ void __launch_bounds__(256) w_rows_kernel(int L, int npo, int G, cons
     const int i = 2 * (w.rb * kRows + rg * 8 + warp) + w.par;
     const bool real = i < L - w.m;
     const double* P = po + tab_off(w.m, L, npo) + (int64_t)i * npo;
-    int e = 1;
-    for (int k = lane; k < 16 * G; k += 32) {
+    static_assert(16 * kChunk == 32, "a chunk is a warp's lanes");
+    const int nch = chunks_of(G);
+    for (int ch = 0; ch < nch; ++ch) {
+      const int k = 32 * ch + lane;
       const double x = real && k < npo ? P[k] : 0.0;
-      sm[warp * stride + k] = x;
-      e = max(e, (__double2hiint(x) >> 20) & 2047);
+      if (k < 16 * G) sm[warp * stride + k] = x;
+      const int e = __reduce_max_sync(0xffffffffu, max(1, (__double2hiint(x) >> 20) & 2047));
+      if (lane == 0) es[ch][warp] = rexp[((int64_t)b * nch + ch) * kRows + rg * 8 + warp] = e;
     }
-    e = __reduce_max_sync(0xffffffffu, e);
-    if (lane == 0) es[warp] = rexp[b * kRows + rg * 8 + warp] = e;
   }
   __syncthreads();
-  const int row = threadIdx.x & 7, e = es[row];
+  const int row = threadIdx.x & 7;
   unsigned char* base = out + (int64_t)b * G * kAGroup + rg * 128 + row * 16;
   for (int q = threadIdx.x >> 3; q < 2 * G; q += 32) {
+    const int e = es[q / (2 * kChunk)][row];
     long long x[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u) x[u] = to_fixed(sm[row * stride + 8 * q + u], e);
@@ -109,7 +121,7 @@ __global__ void __launch_bounds__(256) w_rows_kernel(int L, int npo, int G, cons
 
 // Persistent over the items (row block, column tile); roles as in
 // ring_synthesis_digits_kernel, one sum per output.
-__global__ void __launch_bounds__(kThreads, 1) w_product_kernel(int L, int npo, int G, int ntile, int nitems, int xbit,
+__global__ void __launch_bounds__(kThreads, 1) w_product_kernel(int L, int npo, int G, int ntile, int nitems,
                                                                 const WBlock* __restrict__ blocks,
                                                                 const unsigned char* __restrict__ rows,
                                                                 const int* __restrict__ rexp,
@@ -123,7 +135,7 @@ __global__ void __launch_bounds__(kThreads, 1) w_product_kernel(int L, int npo, 
   __shared__ uint32_t tmem_base_s;
   __shared__ volatile int abort_s;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, npair = L / 2 + 1;
-  const int nch = (G + kChunk - 1) / kChunk;
+  const int nch = chunks_of(G);
   if (tid == 0) {
     for (int b = 0; b < kStages; ++b) {
       mbar_init(&full[b], 1);
@@ -192,45 +204,53 @@ __global__ void __launch_bounds__(kThreads, 1) w_product_kernel(int L, int npo, 
   } else if (warp < kAddWarps) {
     const int q = warp & 3, col0 = kCols * (warp >> 2);
     const uint32_t lanes = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)col0;
-    const int m0 = 1 << (6 + xbit), m1 = 1 << (27 + xbit), m2 = 1 << (18 + xbit), m3 = 512 << xbit, m4 = 1 << xbit;
-    const float f5 = (float)m4 / 512.f, f6 = (float)m4 / 262144.f;
     long long k = 0;
     bool ok = true;
     for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
       const int b = item / ntile, tile = item % ntile;
       const WBlock wb = blocks[b];
       const int r = 32 * q + lane, i = 2 * (wb.rb * kRows + r) + wb.par, nl = L - wb.m;
-      long long a[kCols];
+      const int v = 2 * (wb.m & 1) + wb.par;
+      long long a[kCols];   // in units of 2^53 2^(ex - 2150), below 2^62: 16 chunks of 2^58
+      int ex[kCols];
 #pragma unroll
-      for (int c = 0; c < kCols; ++c) a[c] = 0;
+      for (int c = 0; c < kCols; ++c) {
+        a[c] = 0;
+        ex[c] = 0;
+      }
 #pragma unroll 1
       for (int ch = 0; ch < nch; ++ch, ++k) {
         const int buf = (int)(k & 1);
-        if (!wait_or_abort(&acc_full[buf], (uint32_t)((k >> 1) & 1), &abort_s)) {
+        const int re = rexp[((int64_t)b * nch + ch) * kRows + r];
+        int ce[kCols];
+#pragma unroll
+        for (int c = 0; c < kCols; c += 4) *(int4*)(ce + c) = *(const int4*)(cexp + ((ch * 4 + v) * ntile + tile) * kNT + col0 + c);
+        if (!warp_wait(&acc_full[buf], (uint32_t)((k >> 1) & 1), &abort_s)) {
           ok = false;
           break;
         }
         tc_fence_after();
         const uint32_t at = lanes + (uint32_t)(buf * kAccStride);
+        long long h[kCols];   // the chunk's products in units of 2^53
         float lo[kCols];
 #pragma unroll
         for (int s0 = 0; s0 < kLevels; s0 += 2) {
-          float v[32];
-          tmem_ld2x16(at + kNT * s0, at + kNT * min(s0 + 1, kLevels - 1), v);
+          float x[32];
+          tmem_ld2x16(at + kNT * s0, at + kNT * min(s0 + 1, kLevels - 1), x);
 #pragma unroll
           for (int u = 0; u < 2; ++u) {
             const int s = s0 + u;
 #pragma unroll
             for (int c = 0; c < kCols; ++c) {
-              const float x = v[u * 16 + c];
-              if (s == 0)
-                a[c] = mad_wide(__float2int_rn(x) * m0, 1 << 30, a[c]);
-              else if (s <= 4)
-                a[c] = mad_wide(__float2int_rn(x), s == 1 ? m1 : (s == 2 ? m2 : (s == 3 ? m3 : m4)), a[c]);
+              const float y = x[u * 16 + c];
+              if (s <= 3)
+                h[c] = mad_wide(__float2int_rn(y), s == 0 ? 1 << 27 : (s == 1 ? 1 << 18 : (s == 2 ? 512 : 1)), s ? h[c] : 0);
+              else if (s == 4)
+                h[c] = mad_wide(__float2int_rn(y), 2, h[c] * 1024);
               else if (s == 5)
-                lo[c] = x * f5;
+                lo[c] = y * (2.f / 512.f);
               else if (s == 6)
-                a[c] += __float2int_rn(fmaf(x, f6, lo[c]));
+                h[c] += __float2int_rn(fmaf(y, 2.f / 262144.f, lo[c]));
             }
           }
         }
@@ -238,16 +258,21 @@ __global__ void __launch_bounds__(kThreads, 1) w_product_kernel(int L, int npo, 
         __syncwarp();
         if (lane == 0)
           asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[buf])) : "memory");
+#pragma unroll
+        for (int c = 0; c < kCols; ++c) {   // at the larger of the two scales, rounded
+          const int e = re + ce[c], up = min(max(e - ex[c], 0), 62), dn = min(max(ex[c] - e, 0), 62);
+          a[c] = ((a[c] + ((1LL << up) >> 1)) >> up) + ((h[c] + ((1LL << dn) >> 1)) >> dn);
+          ex[c] = max(ex[c], e);
+        }
       }
       if (!ok || i >= nl) continue;
-      const int v = 2 * (wb.m & 1) + wb.par, e = rexp[b * kRows + r] - 2096 - xbit;
       const int64_t off = tab_off(wb.m, L, npair);
 #pragma unroll
       for (int c = 0; c < kCols; ++c) {
         const int t = tile * kNT + col0 + c;
         if (t < npair)
           W[off + (int64_t)t * nl + i] =
-              fixed_to_double(a[c], e + cexp[v * npair + t]) + pi_L * w[2 * t] * ps[off + (int64_t)i * npair + t];
+              fixed_to_double(a[c], ex[c] - 2097) + pi_L * w[2 * t] * ps[off + (int64_t)i * npair + t];
       }
     }
   }
@@ -283,8 +308,9 @@ int digit_weights(int L, const double* po, const double* ps, const double* Kp, c
   DeviceBuffer db, rows, rexp, table, cexp, fail;
   int rc, dev = 0, sms = 1, failed = 0;
   if ((rc = db.upload(blocks.data(), blocks.size() * sizeof(WBlock))) ||
-      (rc = rows.alloc(most * G * kAGroup)) || (rc = rexp.alloc(most * kRows * sizeof(int))) ||
-      (rc = table.alloc((size_t)4 * ntile * G * kBGroup)) || (rc = cexp.alloc((size_t)4 * npair * sizeof(int))) ||
+      (rc = rows.alloc(most * G * kAGroup)) || (rc = rexp.alloc(most * chunks_of(G) * kRows * sizeof(int))) ||
+      (rc = table.alloc((size_t)4 * ntile * G * kBGroup)) ||
+      (rc = cexp.alloc((size_t)4 * chunks_of(G) * ntile * kNT * sizeof(int))) ||
       (rc = fail.upload(&failed, sizeof(int))))
     return rc;
   cudaError_t e = cudaStreamSynchronize(0);   // the uploads, before s reads them
@@ -303,7 +329,7 @@ int digit_weights(int L, const double* po, const double* ps, const double* Kp, c
     w_rows_kernel<<<n * 16, 256, row_smem, s>>>(L, npo, G, bl, po, (unsigned char*)rows.p, (int*)rexp.p);
     if ((rc = check("w_rows_kernel"))) return rc;
     w_product_kernel<<<std::min(nitems, sms), kThreads, kStages * kStage, s>>>(
-        L, npo, G, ntile, nitems, L <= 512 ? 1 : 0, bl, (const unsigned char*)rows.p, (const int*)rexp.p,
+        L, npo, G, ntile, nitems, bl, (const unsigned char*)rows.p, (const int*)rexp.p,
         (const unsigned char*)table.p, (const int*)cexp.p, ps, w, 3.141592653589793 / L, W,
         (int*)fail.p);
     if ((rc = check("w_product_kernel"))) return rc;
