@@ -345,28 +345,35 @@ int tc_analysis_batch(TcPlan* p, const unsigned char* xtab, double2* const* alm,
 int tc_wait_timeout_probe(long long polls, int* status, cudaStream_t s);
 
 // FP64 velocity synthesis by digits on the tensor cores (sht_digits.cu), L <=
-// kDigitMaxL: the digit table from the FP64 table tab[m][l - m][t] (t =
-// 0..L/2), a plan's own data tiles and column scales, and the fields (from
-// the analysis, lap, or the stream function) -> the nine ring spectra S.
+// kDigitMaxL: the digit table, in digit_tables_bytes of device memory, from the
+// FP64 table tab[m][l - m][t] (t = 0..L/2), and with a plan's own workspace
+// (cleared once) the fields (from the analysis, lap, or the stream function) ->
+// the nine ring spectra S.
 constexpr int kDigitMaxL = 1024;
 struct DigitTables;
-int digit_tables_build(int L, const double* tab, std::shared_ptr<DigitTables>* out, cudaStream_t s);
-int digit_workspace(int L, DeviceBuffer* tiles, DeviceBuffer* aexp);
-int digit_velocity(const DigitTables& t, const double* tab, const double2* a, bool lap, double2* psi_out,
-                   void* tiles, void* aexp, double2* S, int* status, cudaStream_t s);
+size_t digit_tables_bytes(int L);
+int digit_tables_build(int L, const double* tab, void* mem, std::shared_ptr<DigitTables>* out, cudaStream_t s);
+size_t digit_work_bytes(int L);
+int digit_work_clear(int L, void* work, cudaStream_t s);
+int digit_velocity(const DigitTables& t, const double* tab, const double2* a, bool lap, double2* psi_out, void* work,
+                   double2* S, int* status, cudaStream_t s);
 
 // The analysis weights W[m][t][l-m] by digits (weight_digits.cu) from Pbar on the
 // odd fine rings po[m][l-m][jj] and the rings ps[m][l-m][t], their matrix
-// Kp[v][jj][t] and the quadrature weights w; synchronises s.
+// Kp[v][jj][t] and the quadrature weights w, in digit_weights_bytes of scratch;
+// *fail is set where a bounded wait ran out.
+size_t digit_weights_bytes(int L);
 int digit_weights(int L, const double* po, const double* ps, const double* Kp, const double* w, double* W,
-                  cudaStream_t s);
+                  void* scratch, int* fail, cudaStream_t s);
 
 // Inverse ring transforms by digits (ring_digits.cu), L <= kDigitMaxL: tables
-// for `fields` fields of L+1 rings, a plan's own data workspace, and the
-// transform of the spectra S (fields, L+1, L+1; m = L taken as zero) ->
-// x (fields, L+1, 2L).
+// for `fields` fields of L+1 rings in ring_tables_bytes of device memory, a
+// plan's own workspace (cleared once), and the transform of the spectra S
+// (fields, L+1, L+1; m = L taken as zero) -> x (fields, L+1, 2L).
 struct RingTables;
-int ring_tables_build(int L, int fields, std::shared_ptr<RingTables>* out, cudaStream_t s);
-int ring_workspace(int L, int fields, DeviceBuffer* data);
+size_t ring_tables_bytes(int L, int fields);
+int ring_tables_build(int L, int fields, void* mem, std::shared_ptr<RingTables>* out, cudaStream_t s);
+size_t ring_work_bytes(int L, int fields);
+int ring_work_clear(int L, int fields, void* work, cudaStream_t s);
 int ring_inverse(const RingTables& t, int fields, const double2* S, void* data, double* x, int* status, cudaStream_t s);
 }  // namespace cmm

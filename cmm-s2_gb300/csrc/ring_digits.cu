@@ -437,7 +437,7 @@ RingGeometry geometry(int L, int rows, int nt) {
 // Host side ---------------------------------------------------------------
 struct RingTables {
   int L = 0, sms = 1, nt = 32;
-  DeviceBuffer table;
+  const unsigned char* table = nullptr;
 };
 
 // Columns per tile: 32 (the data is read half as often) where that gives every
@@ -447,22 +447,27 @@ static int ring_tile(int L, int fields, int sms) {
   return blocks * ((L / 2 + 31) / 32) >= sms ? 32 : 16;
 }
 
+static int table_bytes(const RingGeometry& g, int nt) { return g.ntile * g.groups() * b_group(nt); }
+
+size_t ring_tables_bytes(int L, int fields) {   // of either tile
+  return std::max(table_bytes(geometry(L, fields * (L + 1), 16), 16), table_bytes(geometry(L, fields * (L + 1), 32), 32));
+}
+
 template <int NT>
-static int ring_tables_nt(RingTables& t, const RingGeometry& g, cudaStream_t s) {
-  int rc = t.table.alloc((size_t)g.ntile * g.groups() * b_group(NT));
-  if (rc) return rc;
-  cudaError_t e = cudaMemsetAsync(t.table.p, 0, t.table.bytes, s);   // the zero block
+static int ring_tables_nt(const RingGeometry& g, unsigned char* table, cudaStream_t s) {
+  cudaError_t e = cudaMemsetAsync(table, 0, table_bytes(g, NT), s);   // the zero block
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(ring_synthesis_digits_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              RingShape<NT>::kSmem);
   if (e != cudaSuccess) return cuda_fail(e, "ring_tables_build");
-  ring_table_kernel<NT><<<dim3(g.groups(), g.ntile), 2 * NT, 0, s>>>(g, (unsigned char*)t.table.p);
+  ring_table_kernel<NT><<<dim3(g.groups(), g.ntile), 2 * NT, 0, s>>>(g, table);
   return check("ring_table_kernel");
 }
 
-int ring_tables_build(int L, int fields, std::shared_ptr<RingTables>* out, cudaStream_t s) {
+int ring_tables_build(int L, int fields, void* mem, std::shared_ptr<RingTables>* out, cudaStream_t s) {
   auto t = std::make_shared<RingTables>();
   t->L = L;
+  t->table = (unsigned char*)mem;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&t->sms, cudaDevAttrMultiProcessorCount, dev);
@@ -472,14 +477,15 @@ int ring_tables_build(int L, int fields, std::shared_ptr<RingTables>* out, cudaS
   if (e != cudaSuccess) return cuda_fail(e, "ring_tables_build");
   t->nt = ring_tile(L, fields, t->sms);
   const RingGeometry g = geometry(L, fields * (L + 1), t->nt);
-  const int rc = t->nt == 32 ? ring_tables_nt<32>(*t, g, s) : ring_tables_nt<16>(*t, g, s);
+  const int rc = t->nt == 32 ? ring_tables_nt<32>(g, (unsigned char*)mem, s) : ring_tables_nt<16>(g, (unsigned char*)mem, s);
   if (rc) return rc;
   *out = std::move(t);
   return CMM_OK;
 }
 
-// data: digits, then rexp, then shift, of `fields` rings per ring index.
-static size_t data_bytes(int L, int fields, size_t* rexp_at, size_t* shift_at) {
+// Workspace of a plan: the data digits, then rexp, then shift.  The rows past
+// the last ring of its block are never written and have to be finite.
+static size_t work_layout(int L, int fields, size_t* rexp_at, size_t* shift_at) {
   const size_t rows = (size_t)fields * (L + 1), blocks = (rows + kRows - 1) / kRows;
   const RingGeometry g = geometry(L, (int)rows, 32);
   *rexp_at = blocks * g.groups() * kAGroup;
@@ -487,24 +493,24 @@ static size_t data_bytes(int L, int fields, size_t* rexp_at, size_t* shift_at) {
   return *shift_at + rows * 2 * kMaxChunks;
 }
 
-int ring_workspace(int L, int fields, DeviceBuffer* data) {
+size_t ring_work_bytes(int L, int fields) {
   size_t a, b;
-  int rc = data->alloc(data_bytes(L, fields, &a, &b));
-  if (rc) return rc;
-  // the rows past the last ring of its block are never written; complete
-  // before the caller's stream, which may not wait for this one, uses them
-  cudaError_t e = cudaMemset(data->p, 0, data->bytes);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(0);
-  if (e == cudaSuccess) return CMM_OK;
-  data->release();
-  return cuda_fail(e, "cudaMemset(ring data)");
+  return (work_layout(L, fields, &a, &b) + 255) / 256 * 256;
+}
+
+int ring_work_clear(int L, int fields, void* work, cudaStream_t s) {
+  size_t a, b;
+  work_layout(L, fields, &a, &b);
+  const size_t block = (size_t)geometry(L, fields * (L + 1), 32).groups() * kAGroup;   // the last one
+  const cudaError_t e = cudaMemsetAsync((unsigned char*)work + a - block, 0, block, s);
+  return e == cudaSuccess ? CMM_OK : cuda_fail(e, "cudaMemsetAsync(ring data)");
 }
 
 int ring_inverse(const RingTables& t, int fields, const double2* S, void* data, double* x, int* status, cudaStream_t s) {
   const int L = t.L, rows = fields * (L + 1);
   const RingGeometry g = geometry(L, rows, t.nt);
   size_t ra, sa;
-  data_bytes(L, fields, &ra, &sa);
+  work_layout(L, fields, &ra, &sa);
   unsigned char* d = (unsigned char*)data;
   int* rexp = (int*)(d + ra);
   unsigned char* shift = d + sa;
@@ -518,10 +524,10 @@ int ring_inverse(const RingTables& t, int fields, const double2* S, void* data, 
   const int xbit = 1.42 * L * 9007199254740992.0 < 9.2e18 ? 1 : 0;
   if (t.nt == 32)
     ring_synthesis_digits_kernel<32><<<grid, kRingThreads, RingShape<32>::kSmem, s>>>(
-        g, nitems, xbit, d, rexp, shift, (const unsigned char*)t.table.p, x, status);
+        g, nitems, xbit, d, rexp, shift, t.table, x, status);
   else
     ring_synthesis_digits_kernel<16><<<grid, kRingThreads, RingShape<16>::kSmem, s>>>(
-        g, nitems, xbit, d, rexp, shift, (const unsigned char*)t.table.p, x, status);
+        g, nitems, xbit, d, rexp, shift, t.table, x, status);
   return check("ring_synthesis_digits_kernel");
 }
 

@@ -10,7 +10,7 @@
 //   3. Legendre analysis with Clenshaw-Curtis weights in cos(theta), exact
 //      for the degree <= 2L-1 products: f_lm = sum_j w_j F'_m(j) Pbar_lm(j).
 //   With Pbar tables 2 and 3 are one contraction with the table of the
-//   combined weights W_lm(t) on the L+1 rings (build_w_kernel).
+//   combined weights W_lm(t) on the L+1 rings (weight_digits.cu).
 // Inverse (pyssht.inverse in project_stream, :84-91): Legendre synthesis on
 // the L+1 rings, then inverse real FFTs (cuFFT Z2D).
 // Pbar_lm are orthonormal with the Condon-Shortley phase and come from the
@@ -463,30 +463,38 @@ constexpr int kTabMaxL = 512;
 constexpr int kTabShared = 1024;   // largest L the analysis kernel's shared arrays hold
 static_assert(kTabShared <= kDigitMaxL, "tables come with the digit tables");
 
-// One thread per (m, ring j): Pbar_{l,m}(theta_{j0 + dj j}), l = m..L-1, j <
-// nj, in the layout [m][l-m][j].
-__global__ void build_pbar_kernel(int L, int nj, int j0, int dj, const double* __restrict__ ct,
-                                  const double* __restrict__ pmm, int pmm_stride, const double* __restrict__ ra,
-                                  const double* __restrict__ rb, double* __restrict__ tab) {
-  const int m = blockIdx.y, j = blockIdx.x * blockDim.x + threadIdx.x;
+// One thread per (m, ring): Pbar_{l,m}, l = m..L-1, in the layout [m][l-m][ring],
+// on the ns rings into ps (blockIdx.z = 0) and on the npo odd fine rings into po.
+// The recurrence factors of the order go through shared memory: read one step
+// after the other, each step waited for them (L = 512: 0.94 ms for both).
+__global__ void __launch_bounds__(128) build_pbar_kernel(int L, const double* __restrict__ ct_rings,
+                                                         const double* __restrict__ pmm_rings,
+                                                         const double* __restrict__ ct_fine,
+                                                         const double* __restrict__ pmm_fine,
+                                                         const double* __restrict__ ra, const double* __restrict__ rb,
+                                                         double* __restrict__ ps, double* __restrict__ po) {
+  extern __shared__ double2 ab[];   // (a, b) of l = m, m + 1, ...
+  const int m = blockIdx.y, j = blockIdx.x * blockDim.x + threadIdx.x, odd = blockIdx.z;
+  const int nj = odd ? (L + 1) / 2 : L / 2 + 1;
+  for (int k = threadIdx.x; k < L - m; k += blockDim.x)
+    ab[k] = make_double2(ra[(int64_t)m * L + m + k], rb[(int64_t)m * L + m + k]);
+  __syncthreads();
   if (j >= nj) return;
-  const double x = ct[j0 + dj * j];
-  double p0 = pmm[(int64_t)m * pmm_stride + j0 + dj * j], p1 = 0.0;
-  double* base = tab + tab_off(m, L, nj);
-  for (int l = m; l < L; ++l) {
-    double P;
-    if (l == m) {
-      P = p0;
-    } else if (l == m + 1) {
-      P = ra[(int64_t)m * L + l] * x * p0;
-      p1 = p0;
-      p0 = P;
-    } else {
-      P = ra[(int64_t)m * L + l] * (x * p0 - rb[(int64_t)m * L + l] * p1);
-      p1 = p0;
-      p0 = P;
-    }
-    base[(int64_t)(l - m) * nj + j] = P;
+  const double x = odd ? ct_fine[2 * j + 1] : ct_rings[j];
+  double p0 = odd ? pmm_fine[(int64_t)m * (2 * L + 1) + 2 * j + 1] : pmm_rings[(int64_t)m * (L + 1) + j], p1 = 0.0;
+  double* out = (odd ? po : ps) + tab_off(m, L, nj) + j;
+  out[0] = p0;
+  if (m + 1 >= L) return;
+  double P = ab[1].x * x * p0;
+  out[nj] = P;
+  p1 = p0;
+  p0 = P;
+#pragma unroll 4
+  for (int k = 2; k < L - m; ++k) {
+    P = ab[k].x * (x * p0 - ab[k].y * p1);
+    p1 = p0;
+    p0 = P;
+    out[(int64_t)k * nj] = P;
   }
 }
 
@@ -505,79 +513,30 @@ __global__ void build_pbar_kernel(int L, int nj, int j0, int dj, const double* _
 // j = 2 jj + 1 <= L (unpaired at j = L), with v = 2 (m odd) + (l-m odd) and s
 // = (-1)^(l-m), the odd fine rings' weight of the pair.
 __global__ void odd_kernel_kernel(int L, const double* __restrict__ w, double* __restrict__ Kp) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x, jj = blockIdx.y, v = blockIdx.z;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, jj = blockIdx.y;
   const int npair = L / 2 + 1, npo = (L + 1) / 2;
   if (t >= npair) return;
-  const double mm = (v & 2) ? -1.0 : 1.0, sl = (v & 1) ? -1.0 : 1.0;
-  auto R = [&](int j) {
-    double s, c, r;
-    sincospi((double)(j - 2 * t) / (4.0 * L), &s, &c);
-    r = c / s;
-    if (t > 0 && t < L) {
-      sincospi((double)(j + 2 * t) / (4.0 * L), &s, &c);
-      r += mm * (c / s);
-    }
-    return ((((j - 1) / 2 - t) & 1) ? -r : r) / (2.0 * L);
-  };
   const int j = 2 * jj + 1;
-  double k = R(j);
-  if (j < L) k += sl * R(2 * L - j);
-  Kp[((int64_t)v * npo + jj) * npair + t] = M_PI / L * w[j] * k;
-}
-
-// W of order m = blockIdx.y from Pbar on the odd fine rings (po, [m][l-m][jj])
-// and on the rings (ps, [m][l-m][t]): 32 degrees of one parity (blockIdx.z
-// & 1) x 64 ring pairs per block, layout [m][t][l-m].  Set-up work, once per
-// table.
-__global__ void __launch_bounds__(256) build_w_kernel(int L, const double* __restrict__ po,
-                                                      const double* __restrict__ ps, const double* __restrict__ Kp,
-                                                      const double* __restrict__ w, double* __restrict__ W) {
-  const int npair = L / 2 + 1, npo = (L + 1) / 2;
-  const int m = blockIdx.y, par = blockIdx.z & 1, i0 = (blockIdx.z >> 1) * 32, t0 = blockIdx.x * 64;
-  const int nl = L - m;
-  if (2 * i0 + par >= nl) return;   // uniform for the block
-  __shared__ double A[32][17], B[16][65];
-  const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;   // ring pair; 8 degrees each
-  const double* P = po + tab_off(m, L, npo);
-  const double* K = Kp + (int64_t)(2 * (m & 1) + par) * npo * npair;
-  double acc[8];
+  const bool mirror = t > 0 && t < L;
+  auto cot = [&](int k) {
+    double s, c;
+    sincospi((double)k / (4.0 * L), &s, &c);
+    return c / s;
+  };
+  // the four cotangents of (j, t) and (2L - j, t), shared by the four v
+  const double n0 = cot(j - 2 * t), n1 = mirror ? cot(j + 2 * t) : 0.0;
+  const double f0 = cot(2 * L - j - 2 * t), f1 = mirror ? cot(2 * L - j + 2 * t) : 0.0;
+  auto R = [&](int q, double a, double b, double mm) {
+    double r = a;
+    if (mirror) r += mm * b;
+    return ((((q - 1) / 2 - t) & 1) ? -r : r) / (2.0 * L);
+  };
 #pragma unroll
-  for (int q = 0; q < 8; ++q) acc[q] = 0.0;
-  // towards the poles Pbar_lm falls off exponentially and grows with l: the
-  // leading tiles of rings where the block's two highest degrees are below
-  // 1e-30 add nothing (about a third of the products)
-  int k_first = 0;
-  const int itop = min(nl - 1, 2 * (i0 + 31) + 1);
-  for (; k_first + 16 < npo; k_first += 16) {
-    const double a = P[(int64_t)itop * npo + k_first + 15], b = itop > 0 ? P[(int64_t)(itop - 1) * npo + k_first + 15] : 0.0;
-    if (!(fabs(a) < 1e-30 && fabs(b) < 1e-30)) break;
-  }
-  for (int k0 = k_first; k0 < npo; k0 += 16) {
-    for (int e = threadIdx.x; e < 32 * 16; e += 256) {
-      const int r = e >> 4, k = e & 15, i = 2 * (i0 + r) + par;
-      A[r][k] = (i < nl && k0 + k < npo) ? P[(int64_t)i * npo + k0 + k] : 0.0;
-    }
-    for (int e = threadIdx.x; e < 16 * 64; e += 256) {
-      const int k = e >> 6, t = e & 63;
-      B[k][t] = (k0 + k < npo && t0 + t < npair) ? K[(int64_t)(k0 + k) * npair + t0 + t] : 0.0;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const double b = B[k][tx];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) acc[q] += A[8 * ty + q][k] * b;
-    }
-    __syncthreads();
-  }
-  const int t = t0 + tx;
-  if (t >= npair) return;
-  const double we = M_PI / L * w[2 * t];   // the even fine ring 2t is ring t
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const int i = 2 * (i0 + 8 * ty + q) + par;
-    if (i < nl)
-      W[tab_off(m, L, npair) + (int64_t)t * nl + i] = acc[q] + we * ps[tab_off(m, L, npair) + (int64_t)i * npair + t];
+  for (int v = 0; v < 4; ++v) {
+    const double mm = (v & 2) ? -1.0 : 1.0, sl = (v & 1) ? -1.0 : 1.0;
+    double k = R(j, n0, n1, mm);
+    if (j < L) k += sl * R(2 * L - j, f0, f1, mm);
+    Kp[((int64_t)v * npo + jj) * npair + t] = M_PI / L * w[j] * k;
   }
 }
 
@@ -1140,12 +1099,13 @@ struct cmm_sht {
   // tables of the FP64 stages (analysis weights w, synthesis Pbar s); plans
   // of one band-limit may hold the same tables (cmm_sht_share_tables)
   struct PbarTables {
-    cmm::DeviceBuffer w, s;
+    cmm::DeviceBuffer mem;                      // of all of them
+    double *w = nullptr, *s = nullptr;
     std::shared_ptr<cmm::DigitTables> digits;   // of s, for the velocity's synthesis
     std::shared_ptr<cmm::RingTables> ring;      // for its ring transforms
   };
   std::shared_ptr<PbarTables> tab;
-  cmm::DeviceBuffer dig_tiles, dig_exp, ring_data;   // this plan's data digits for them
+  cmm::DeviceBuffer dig_work;       // this plan's data digits for them: the rings', then the fields'
   int tab_mode = 0;                 // cmm_sht_set_tables: 0 auto, 1 always, -1 never
   cmm::DeviceBuffer spec, torus, pad, alm, fields, synth, samples, status;
   cmm::TcPlan* tc = nullptr;
@@ -1339,16 +1299,51 @@ static int set_streams(cmm_sht* p, cudaStream_t s) {
 // and 92; 192: 107 and 117; 256: 138 and 172; 512: 466 and 681).
 constexpr int kRingMinL = 160;
 
-// Least L whose analysis weights are made by digits (weight_digits.cu); below,
-// the FP64 contraction takes less time than their set-up.
-constexpr int kDigitWeightsMinL = 256;
+static size_t ring_work(const cmm_sht* p) { return p->L >= kRingMinL ? ring_work_bytes(p->L, kVelSpectra) : 0; }
+static void* field_work(const cmm_sht* p) { return (unsigned char*)p->dig_work.p + ring_work(p); }
 
-// The digit forms' data workspaces of a plan with tables.
-static int ensure_digits(cmm_sht* p) {
-  if (p->dig_tiles.p) return CMM_OK;
-  int rc = CMM_OK;
-  if (p->L >= kRingMinL) rc = ring_workspace(p->L, kVelSpectra, &p->ring_data);
-  return rc ? rc : digit_workspace(p->L, &p->dig_tiles, &p->dig_exp);
+// The digit forms' data workspace of a plan with tables, cleared on s.
+static int ensure_digits(cmm_sht* p, cudaStream_t s) {
+  if (p->dig_work.p) return CMM_OK;
+  DeviceBuffer b;
+  int rc = b.alloc(ring_work(p) + digit_work_bytes(p->L));
+  if (!rc && ring_work(p)) rc = ring_work_clear(p->L, kVelSpectra, b.p, s);
+  if (!rc) rc = digit_work_clear(p->L, (unsigned char*)b.p + ring_work(p), s);
+  if (!rc) std::swap(b.p, p->dig_work.p), std::swap(b.bytes, p->dig_work.bytes);
+  return rc;
+}
+
+// The FP64 tables, enqueued on s: one allocation of the analysis weights, Pbar,
+// the ring table and the digit table.  The digit table is made last: its place
+// holds the build's scratch (Pbar on the odd fine rings, the interpolant's
+// matrix, the weights' digits) until then.  (Separate buffers, freed one by
+// one, and their waits were half of a small plan's first call.)
+static int build_tables(cmm_sht* p, cmm_sht::PbarTables* tab, cudaStream_t s) {
+  const int L = p->L;
+  const int64_t tri = (int64_t)L * (L + 1) / 2;
+  const int ns = L / 2 + 1, npo = (L + 1) / 2;
+  auto aligned = [](size_t n) { return (n + 255) / 256 * 256; };
+  const size_t head = 256, tb = aligned((size_t)tri * ns * 8);
+  const size_t rb_ = L >= kRingMinL ? aligned(ring_tables_bytes(L, kVelSpectra)) : 0;
+  const size_t pob = aligned((size_t)tri * npo * 8), kpb = aligned((size_t)4 * npo * ns * 8);
+  const size_t last = std::max(digit_tables_bytes(L), pob + kpb + digit_weights_bytes(L));
+  int rc = tab->mem.alloc(head + 2 * tb + rb_ + last);
+  if (rc) return rc;
+  unsigned char* mem = (unsigned char*)tab->mem.p;
+  tab->w = (double*)(mem + head);
+  tab->s = (double*)(mem + head + tb);
+  unsigned char *ring = mem + head + 2 * tb, *end = ring + rb_;
+  double *po = (double*)end, *kp = (double*)(end + pob);
+  const double* w = (const double*)p->w_fine.p;
+  build_pbar_kernel<<<dim3((ns + 127) / 128, L, 2), 128, L * sizeof(double2), s>>>(
+      L, (const double*)p->ct_rings.p, (const double*)p->pmm_rings.p, (const double*)p->ct_fine.p,
+      (const double*)p->pmm_fine.p, (const double*)p->ra.p, (const double*)p->rb.p, tab->s, po);
+  if ((rc = check_launch("build_pbar_kernel"))) return rc;
+  odd_kernel_kernel<<<dim3((ns + 127) / 128, npo), 128, 0, s>>>(L, w, kp);
+  if ((rc = check_launch("odd_kernel_kernel"))) return rc;
+  if ((rc = digit_weights(L, po, tab->s, kp, w, tab->w, end + pob + kpb, (int*)mem, s))) return rc;
+  if (rb_ && (rc = ring_tables_build(L, kVelSpectra, ring, &tab->ring, s))) return rc;
+  return digit_tables_build(L, tab->s, end, &tab->digits, s);
 }
 
 // Pbar tables of the FP64 Legendre stages at L <= kTabMaxL, built at their
@@ -1358,7 +1353,7 @@ static int ensure_tables(cmm_sht* p, cudaStream_t s, bool* ok) {
   *ok = false;
   const int L = p->L;
   if (p->tab_mode < 0 || (p->tab_mode == 0 && L > kTabMaxL) || L > kTabShared) return CMM_OK;
-  if (p->tab && p->dig_tiles.p) {
+  if (p->tab && p->dig_work.p) {
     *ok = true;
     return CMM_OK;
   }
@@ -1368,45 +1363,28 @@ static int ensure_tables(cmm_sht* p, cudaStream_t s, bool* ok) {
     return CMM_OK;
   }
   if (cs != cudaStreamCaptureStatusNone) return CMM_OK;
-  int rc;
-  if ((rc = ensure_digits(p))) return rc;
-  if (p->tab) {
-    *ok = true;
-    return CMM_OK;
+  std::shared_ptr<cmm_sht::PbarTables> tab;
+  int rc = CMM_OK, failed = 0;
+  if (!p->tab) {
+    tab = std::make_shared<cmm_sht::PbarTables>();
+    rc = build_tables(p, tab.get(), s);
   }
-  const int64_t tri = (int64_t)L * (L + 1) / 2;
-  const int ns = L / 2 + 1, npo = (L + 1) / 2;
-  auto tab = std::make_shared<cmm_sht::PbarTables>();
-  DeviceBuffer po, kp;   // Pbar on the odd fine rings and their weights, for the build only
-  if ((rc = tab->w.alloc((size_t)tri * ns * 8)) || (rc = tab->s.alloc((size_t)tri * ns * 8)) ||
-      (rc = po.alloc((size_t)tri * npo * 8)) || (rc = kp.alloc((size_t)4 * npo * ns * 8)))
-    return rc;
-  const double *ra = (const double*)p->ra.p, *rb = (const double*)p->rb.p, *w = (const double*)p->w_fine.p;
-  build_pbar_kernel<<<dim3((ns + 127) / 128, L), 128, 0, s>>>(L, ns, 0, 1, (const double*)p->ct_rings.p,
-                                                              (const double*)p->pmm_rings.p, L + 1, ra, rb,
-                                                              (double*)tab->s.p);
-  if ((rc = check_launch("build_pbar_kernel"))) return rc;
-  build_pbar_kernel<<<dim3((npo + 127) / 128, L), 128, 0, s>>>(L, npo, 1, 2, (const double*)p->ct_fine.p,
-                                                               (const double*)p->pmm_fine.p, 2 * L + 1, ra, rb,
-                                                               (double*)po.p);
-  if ((rc = check_launch("build_pbar_kernel"))) return rc;
-  odd_kernel_kernel<<<dim3((ns + 127) / 128, npo, 4), 128, 0, s>>>(L, w, (double*)kp.p);
-  if ((rc = check_launch("odd_kernel_kernel"))) return rc;
-  if (L >= kDigitWeightsMinL) {
-    if ((rc = digit_weights(L, (const double*)po.p, (const double*)tab->s.p, (const double*)kp.p, w, (double*)tab->w.p, s)))
-      return rc;
-  } else {
-    build_w_kernel<<<dim3((ns + 63) / 64, L, 2 * (((L + 1) / 2 + 31) / 32)), 256, 0, s>>>(
-        L, (const double*)po.p, (const double*)tab->s.p, (const double*)kp.p, w, (double*)tab->w.p);
-    if ((rc = check_launch("build_w_kernel"))) return rc;
-  }
-  if ((rc = digit_tables_build(L, (const double*)tab->s.p, &tab->digits, s))) return rc;
-  if (L >= kRingMinL && (rc = ring_tables_build(L, kVelSpectra, &tab->ring, s))) return rc;
+  if (!rc) rc = ensure_digits(p, s);
   // published only once built: a later call of this plan on another
   // stream, unordered with s, must not read a partly written table
-  cudaError_t e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return cuda_fail(e, "build_w_kernel");
-  p->tab = std::move(tab);
+  cudaError_t e = cudaSuccess;
+  if (!rc && tab) e = cudaMemcpyAsync(&failed, tab->mem.p, sizeof(int), cudaMemcpyDeviceToHost, s);
+  const cudaError_t done = cudaStreamSynchronize(s);   // also before anything is freed
+  if (!rc && (e != cudaSuccess || done != cudaSuccess)) rc = cuda_fail(e != cudaSuccess ? e : done, "FP64 tables");
+  if (!rc && failed) {
+    set_last_error("analysis weights: a bounded wait inside the kernel ran out");
+    rc = CMM_ERR_TIMEOUT;
+  }
+  if (rc) {
+    p->dig_work.release();
+    return rc;
+  }
+  if (tab) p->tab = std::move(tab);
   *ok = true;
   return CMM_OK;
 }
@@ -1493,7 +1471,7 @@ int sht_forward(cmm_sht* p, const double* samples, double2* out, cudaStream_t s)
   if ((rc = ensure_tables(p, s, &tab))) return rc;
   if (tab) {
     analysis_w_kernel<<<dim3(L, (L + kTabBlock - 1) / kTabBlock), kTabBlock * kAnaSlices, 0, s>>>(
-        (const double2*)p->spec.p, L, (const double*)p->tab->w.p, out);
+        (const double2*)p->spec.p, L, p->tab->w, out);
     return check_launch("analysis_w_kernel");
   }
   torus_t_kernel<<<g1, b, 0, s>>>((const double2*)p->spec.p, L, M_PI / L, (double2*)p->torus.p);
@@ -1545,9 +1523,9 @@ int sht_inverse(cmm_sht* p, const double2* alm, int nf, double* samples, cudaStr
     const int G = nf == kFields ? 3 : 1;
     dim3 gt(L, (npair + kTabBlock - 1) / kTabBlock, nf / G);
     if (G == 3)
-      synthesis_tab_kernel<3><<<gt, kTabBlock, 0, s>>>(alm, L, (const double*)p->tab->s.p, S);
+      synthesis_tab_kernel<3><<<gt, kTabBlock, 0, s>>>(alm, L, p->tab->s, S);
     else
-      synthesis_tab_kernel<1><<<gt, kTabBlock, 0, s>>>(alm, L, (const double*)p->tab->s.p, S);
+      synthesis_tab_kernel<1><<<gt, kTabBlock, 0, s>>>(alm, L, p->tab->s, S);
     if ((rc = check_launch("synthesis_tab_kernel"))) return rc;
   } else {
   dim3 g(L, (npair + kSynthBlock - 1) / kSynthBlock);
@@ -1619,7 +1597,7 @@ static int velocity_fp64(cmm_sht* p, const cmm_mesh* vm, const double2* a, bool 
   bool tab;
   if ((rc = ensure_tables(p, s, &tab))) return rc;
   if (tab) {
-    rc = digit_velocity(*p->tab->digits, (const double*)p->tab->s.p, a, lap, psi_out, p->dig_tiles.p, p->dig_exp.p, S,
+    rc = digit_velocity(*p->tab->digits, p->tab->s, a, lap, psi_out, field_work(p), S,
                         (int*)p->status.p, s);
     if (rc) return rc;
   } else {
@@ -1636,7 +1614,7 @@ static int velocity_fp64(cmm_sht* p, const cmm_mesh* vm, const double2* a, bool 
     if ((rc = check_launch("synthesis_kernel (velocity)"))) return rc;
   }
   if (tab && p->tab->ring) {
-    rc = ring_inverse(*p->tab->ring, kVelSpectra, S, p->ring_data.p, (double*)p->samples.p, (int*)p->status.p, s);
+    rc = ring_inverse(*p->tab->ring, kVelSpectra, S, p->dig_work.p, (double*)p->samples.p, (int*)p->status.p, s);
     if (rc) return rc;
   } else {
     cufftResult r = cufftExecZ2D(p->ring_inv9, (cufftDoubleComplex*)S, (cufftDoubleReal*)p->samples.p);
@@ -1827,7 +1805,7 @@ int sht_velocity_bwd(cmm_sht* p, const cmm_mesh* vm, const double* gjets, double
     if ((rc = ensure_tables(p, s, &tab))) return rc;
     if (tab) {
       const dim3 gt(L, (L + kTabBlock - 1) / kTabBlock, kFields / 2);
-      legendre_sum_tab_kernel<2><<<gt, kTabBlock, 0, s>>>(Sb, L + 1, L, 2.0, (const double*)p->tab->s.p, Fb, fin,
+      legendre_sum_tab_kernel<2><<<gt, kTabBlock, 0, s>>>(Sb, L + 1, L, 2.0, p->tab->s, Fb, fin,
                                                           fout);
     } else if (npair <= 256)
       legendre_sum_kernel<1><<<gl, 256, 0, s>>>(Sb, L + 1, L, L, nullptr, 2.0, ct, pm, L + 1, ra, rb, Fb, fin, fout);
@@ -1958,7 +1936,9 @@ int sht_share_tables(cmm_sht* p, cmm_sht* src) {
     }
     p->tab = src->tab;
     p->tab_mode = src->tab_mode;
-    return ensure_digits(p);
+    rc = ensure_digits(p, 0);
+    e = cudaStreamSynchronize(0);   // the clears, before a stream that does not wait for this one
+    return rc ? rc : (e == cudaSuccess ? CMM_OK : cuda_fail(e, "cmm_sht_share_tables"));
   }
   if (!src->tc) {
     set_last_error("cmm_sht_share_tables: source plan without split-BF16 tables");
@@ -1983,9 +1963,7 @@ int sht_trim(cmm_sht* p) {
   p->synth.release();
   p->samples.release();
   p->tab.reset();
-  p->dig_tiles.release();
-  p->dig_exp.release();
-  p->ring_data.release();
+  p->dig_work.release();
   return CMM_OK;
 }
 

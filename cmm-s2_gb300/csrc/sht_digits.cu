@@ -518,10 +518,13 @@ int check(const char* what) {
 // Host side ---------------------------------------------------------------
 struct DigitTables {
   int L = 0, sms = 1;
-  DeviceBuffer gbase, digits, pexp, ladder;
+  int* gbase = nullptr;
+  unsigned char* digits = nullptr;
+  short* pexp = nullptr;
+  double* ladder = nullptr;
   DigGeometry geometry() const {
     const int rows = L / 2;
-    return DigGeometry{L, rows, (rows + kRows - 1) / kRows, (const int*)gbase.p};
+    return DigGeometry{L, rows, (rows + kRows - 1) / kRows, gbase};
   }
 };
 
@@ -531,19 +534,27 @@ static int total_groups(int L) {
   return n;
 }
 
-int digit_tables_build(int L, const double* tab, std::shared_ptr<DigitTables>* out, cudaStream_t s) {
+static size_t aligned(size_t n) { return (n + 255) / 256 * 256; }
+static size_t digits_bytes(int L) { return aligned((size_t)total_groups(L) * kRowGroupBytes * ((L / 2 + 7) / 8)); }
+static size_t pexp_bytes(int L) { return aligned((size_t)total_groups(L) * 8 * ((L / 2 + 7) / 8) * sizeof(short)); }
+static size_t ladder_bytes(int L) { return aligned((size_t)(L + 3) * L * sizeof(double)); }
+
+size_t digit_tables_bytes(int L) {
+  return digits_bytes(L) + pexp_bytes(L) + ladder_bytes(L) + (L + 1) * sizeof(int);
+}
+
+int digit_tables_build(int L, const double* tab, void* mem, std::shared_ptr<DigitTables>* out, cudaStream_t s) {
   auto t = std::make_shared<DigitTables>();
   t->L = L;
-  const int rows = L / 2, rgt = (rows + 7) / 8;
+  t->digits = (unsigned char*)mem;
+  t->pexp = (short*)(t->digits + digits_bytes(L));
+  t->ladder = (double*)((unsigned char*)t->pexp + pexp_bytes(L));
+  t->gbase = (int*)((unsigned char*)t->ladder + ladder_bytes(L));
   std::vector<int> gb(L + 1, 0);
   for (int m = 0; m < L; ++m) gb[m + 1] = gb[m] + groups16((L - m + 1) / 2) + groups16((L - m) / 2);
   int rc, dev = 0;
-  if ((rc = t->gbase.upload(gb.data(), gb.size() * sizeof(int))) ||
-      (rc = t->digits.alloc((size_t)gb[L] * kRowGroupBytes * rgt)) ||
-      (rc = t->pexp.alloc((size_t)gb[L] * 8 * rgt * sizeof(short))) ||
-      (rc = t->ladder.alloc((size_t)(L + 3) * L * sizeof(double))))
-    return rc;
-  cudaError_t e = cudaStreamSynchronize(0);   // the upload, before s reads it
+  // from pageable memory: staged before the call returns
+  cudaError_t e = cudaMemcpyAsync(t->gbase, gb.data(), gb.size() * sizeof(int), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(synth_digits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
   if (e == cudaSuccess)
@@ -553,40 +564,35 @@ int digit_tables_build(int L, const double* tab, std::shared_ptr<DigitTables>* o
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&t->sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return cuda_fail(e, "digit_tables_build");
   const DigGeometry g = t->geometry();
-  build_digits_kernel<<<dim3(g.nblk, gb[1], L), kRows, 0, s>>>(g, tab, (unsigned char*)t->digits.p,
-                                                               (short*)t->pexp.p);
+  build_digits_kernel<<<dim3(g.nblk, gb[1], L), kRows, 0, s>>>(g, tab, t->digits, t->pexp);
   if ((rc = check("build_digits_kernel"))) return rc;
-  ladder_table_kernel<<<dim3((L + 127) / 128, L + 3), 128, 0, s>>>(L, (double*)t->ladder.p);
+  ladder_table_kernel<<<dim3((L + 127) / 128, L + 3), 128, 0, s>>>(L, t->ladder);
   if ((rc = check("ladder_table_kernel"))) return rc;
   *out = std::move(t);
   return CMM_OK;
 }
 
-int digit_workspace(int L, DeviceBuffer* tiles, DeviceBuffer* aexp) {
-  const size_t n = total_groups(L);
-  int rc;
-  if ((rc = aexp->alloc(n * kCols * sizeof(int))) || (rc = tiles->alloc(n * kAGroup)))
-    return rc;
-  // the padding columns and the zero block are never written; complete before
-  // the caller's stream, which may not wait for this one, uses the tiles
-  cudaError_t e = cudaMemset(tiles->p, 0, tiles->bytes);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(0);
-  if (e == cudaSuccess) return CMM_OK;
-  tiles->release();
-  return cuda_fail(e, "cudaMemset(digit tiles)");
+// Workspace of a plan: the data tiles, whose padding columns and zero block are
+// never written and have to be zero, then the column scales.
+static size_t tile_bytes(int L) { return aligned((size_t)total_groups(L) * kAGroup); }
+size_t digit_work_bytes(int L) { return tile_bytes(L) + aligned((size_t)total_groups(L) * kCols * sizeof(int)); }
+int digit_work_clear(int L, void* work, cudaStream_t s) {
+  const cudaError_t e = cudaMemsetAsync(work, 0, tile_bytes(L), s);
+  return e == cudaSuccess ? CMM_OK : cuda_fail(e, "cudaMemsetAsync(digit tiles)");
 }
 
-int digit_velocity(const DigitTables& t, const double* tab, const double2* a, bool lap, double2* psi_out,
-                   void* tiles, void* aexp, double2* S, int* status, cudaStream_t s) {
+int digit_velocity(const DigitTables& t, const double* tab, const double2* a, bool lap, double2* psi_out, void* work,
+                   double2* S, int* status, cudaStream_t s) {
   const DigGeometry g = t.geometry();
   const int L = t.L, nitems = L * g.nblk;
-  velocity_digits_kernel<<<L, kFieldThreads, (size_t)L * kFieldStride * sizeof(double), s>>>(
-      g, a, lap, psi_out, (const double*)t.ladder.p, tab, (unsigned char*)tiles, (int*)aexp, S);
+  unsigned char* tiles = (unsigned char*)work;
+  int* aexp = (int*)(tiles + tile_bytes(L));
+  velocity_digits_kernel<<<L, kFieldThreads, (size_t)L * kFieldStride * sizeof(double), s>>>(g, a, lap, psi_out, t.ladder,
+                                                                                            tab, tiles, aexp, S);
   int rc = check("velocity_digits_kernel");
   if (rc) return rc;
-  synth_digits_kernel<<<std::min(nitems, t.sms), kSynThreads, kSmemBytes, s>>>(
-      g, nitems, (const unsigned char*)t.digits.p, (const short*)t.pexp.p, (const unsigned char*)tiles,
-      (const int*)aexp, S, status);
+  synth_digits_kernel<<<std::min(nitems, t.sms), kSynThreads, kSmemBytes, s>>>(g, nitems, t.digits, t.pexp, tiles, aexp, S,
+                                                                              status);
   return check("synth_digits_kernel");
 }
 

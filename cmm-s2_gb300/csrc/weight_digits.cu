@@ -1,19 +1,19 @@
-// The analysis weights' contraction over the odd fine rings (sht.cu,
-// build_w_kernel) by exact digits on the tensor cores (tcgen05, sm_103a;
-// sht_digits.cu describes the scheme): W[m][t][i] = sum_jj Pbar_(m+i)m(odd ring
-// jj) Kp[v][jj][t] + we_t Pbar_(m+i)m(ring t).  Set-up work of a table, L^4 / 16
-// multiply-adds: FP64-bound (about 10 of the 15 ms that a table took at L =
-// 512).  Rows of one order and parity in blocks of 128, tiles of 32 columns,
-// chunks of 32 jj, each with a scale per row (m, i) and per column (v, t); the
+// The analysis weights' contraction over the odd fine rings by exact digits on
+// the tensor cores (tcgen05, sm_103a; sht_digits.cu describes the scheme):
+// W[m][t][i] = sum_jj Pbar_(m+i)m(odd ring jj) Kp[v][jj][t] + we_t
+// Pbar_(m+i)m(ring t).  Set-up work of a table, L^4 / 16 multiply-adds.  Kp
+// depends on the parities v of m and i alone, so that the rows (m, i) of a class
+// v follow each other, order after order, in blocks of 128; tiles of 32
+// columns, chunks of 32 jj, each with a scale per row and per column; the
 // chunks' integers are added at the largest scale met.  (Pbar is largest next
 // to the poles and Kp next to jj = t: with one scale for all jj the weights of
 // low orders erred 2 to 3 times as much as by FP64 sums, so 0.5 to 0.7 times:
-// emulated, L = 256 and 512.)
+// emulated, L = 256 and 512.)  Towards the poles Pbar falls off exponentially:
+// a block leaves out the leading chunks in which all its rows are below 1e-30.
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 
 #include <algorithm>
-#include <vector>
 
 #include "cmm_internal.h"
 #include "device_common.cuh"
@@ -35,21 +35,42 @@ constexpr int kBGroup = 2 * kLevels * kNT / 8 * 128;       // 16 jj of a column 
 constexpr int kStage = kAGroup + kBGroup;
 constexpr int kAccStride = 256;                            // TMEM columns per accumulator (7 x 32 used)
 constexpr uint32_t kTmemCols = 512;
-constexpr int kAddWarps = 8, kThreads = 32 * (kAddWarps + 2), kCols = kNT / 2;
-constexpr int kBatch = 64;                                 // orders whose row digits exist at a time
-
+constexpr int kAddWarps = 16, kThreads = 32 * (kAddWarps + 2), kCols = kNT / (kAddWarps / 4);
+constexpr int kBatch = 288;                                // most row blocks whose digits exist at a time
 constexpr int kMaxChunks = kDigitMaxL / 2 / (16 * kChunk);
-
-struct WBlock {
-  int m, par, rb;
-};
+constexpr int kTiny = 1023 - 100;                          // biased exponent of about 1e-30
 
 __host__ __device__ __forceinline__ int chunks_of(int G) { return (G + kChunk - 1) / kChunk; }
 
+// The classes v = 2 (m odd) + (i odd): order m = 2 k + (v >> 1) has N - k rows,
+// i = (v & 1), (v & 1) + 2, ...
+struct WGeometry {
+  int L, first[5];   // first row block of each class, and the total
+  __host__ __device__ int N(int v) const { return (L - (v >> 1) - (v & 1) + 1) / 2; }
+  __host__ __device__ int rows(int v) const { return N(v) * (N(v) + 1) / 2; }
+  __device__ __forceinline__ int cls(int b) const { return (b >= first[1]) + (b >= first[2]) + (b >= first[3]); }
+  // row r of class v
+  __device__ __forceinline__ void row(int v, int r, int& m, int& i) const {
+    const int n = N(v);
+    const float h = n + 0.5f;
+    int k = min(n - 1, (int)(h - sqrtf(fmaxf(h * h - 2.f * r, 0.f))));
+    auto start = [&](int q) { return q * n - q * (q - 1) / 2; };
+    while (k > 0 && start(k) > r) --k;
+    while (start(k + 1) <= r) ++k;
+    m = 2 * k + (v >> 1);
+    i = 2 * (r - start(k)) + (v & 1);
+  }
+};
+
 // Block (tile, v): the column scales, cexp[chunk][v][t], and digits of
-// Kp[v][jj][t], t of the tile.
+// Kp[v][jj][t], t of the tile, with the zero block.  Also clears the blocks'
+// first chunks (nlead of them) and *fail.
 __global__ void __launch_bounds__(256) w_table_kernel(int npo, int npair, int G, const double* __restrict__ Kp,
-                                                      unsigned char* __restrict__ out, int* __restrict__ cexp) {
+                                                      unsigned char* __restrict__ out, int* __restrict__ cexp,
+                                                      int* __restrict__ lead, int nlead, int* __restrict__ fail) {
+  for (int k = (blockIdx.y * gridDim.x + blockIdx.x) * 256 + threadIdx.x; k < nlead; k += 256 * gridDim.x * gridDim.y)
+    lead[k] = 1 << 30;
+  if (blockIdx.x + blockIdx.y + threadIdx.x == 0) *fail = 0;
   __shared__ int emax[kMaxChunks][kNT];
   const int tile = blockIdx.x, v = blockIdx.y, c = threadIdx.x % kNT, t = tile * kNT + c, ntile = gridDim.x;
   const double* K = Kp + (int64_t)v * npo * npair + t;
@@ -76,32 +97,37 @@ __global__ void __launch_bounds__(256) w_table_kernel(int npo, int npair, int G,
     unsigned char* o = base + (int64_t)(q >> 1) * kBGroup + (q & 1) * (kBGroup / 2);
 #pragma unroll
     for (int j = 0; j < kDigits; ++j) *(uint4*)(o + j * (kNT / 8) * 128) = d[j];
+    *(uint4*)(o + kDigits * (kNT / 8) * 128) = make_uint4(0, 0, 0, 0);
   }
 }
 
-// Eight rows per block (of row block blockIdx.x / 16): scales, rexp[block][chunk]
-// [row], and digits of po[m][i][jj], i = 2 r + par.
-__global__ void __launch_bounds__(256) w_rows_kernel(int L, int npo, int G, const WBlock* __restrict__ blocks,
-                                                     const double* __restrict__ po, unsigned char* __restrict__ out,
-                                                     int* __restrict__ rexp) {
+// Eight rows per block (of row block b0 + blockIdx.x / 16): scales, rexp[block]
+// [chunk][row], digits of po[m][i][jj] and the row block's first chunk.
+__global__ void __launch_bounds__(256) w_rows_kernel(WGeometry g, int npo, int G, int b0, const double* __restrict__ po,
+                                                     unsigned char* __restrict__ out, int* __restrict__ rexp,
+                                                     int* __restrict__ first) {
   extern __shared__ double sm[];   // [8][stride]
   __shared__ int es[kMaxChunks][8];
-  const int b = blockIdx.x >> 4, rg = blockIdx.x & 15, stride = 16 * G + 2;
-  const WBlock w = blocks[b];
+  const int b = blockIdx.x >> 4, rg = blockIdx.x & 15, stride = 16 * G + 2, nch = chunks_of(G);
+  const int v = g.cls(b0 + b);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   {
-    const int i = 2 * (w.rb * kRows + rg * 8 + warp) + w.par;
-    const bool real = i < L - w.m;
-    const double* P = po + tab_off(w.m, L, npo) + (int64_t)i * npo;
+    const int r = (b0 + b - g.first[v]) * kRows + rg * 8 + warp;
+    const bool real = r < g.rows(v);
+    int m = 0, i = 0;
+    if (real) g.row(v, r, m, i);
+    const double* P = po + tab_off(m, g.L, npo) + (int64_t)i * npo;
     static_assert(16 * kChunk == 32, "a chunk is a warp's lanes");
-    const int nch = chunks_of(G);
+    int lead = nch - 1;
     for (int ch = 0; ch < nch; ++ch) {
       const int k = 32 * ch + lane;
       const double x = real && k < npo ? P[k] : 0.0;
       if (k < 16 * G) sm[warp * stride + k] = x;
       const int e = __reduce_max_sync(0xffffffffu, max(1, (__double2hiint(x) >> 20) & 2047));
+      if (e >= kTiny) lead = min(lead, ch);
       if (lane == 0) es[ch][warp] = rexp[((int64_t)b * nch + ch) * kRows + rg * 8 + warp] = e;
     }
+    if (real && lane == 0) atomicMin(first + b, lead);
   }
   __syncthreads();
   const int row = threadIdx.x & 7;
@@ -121,8 +147,8 @@ __global__ void __launch_bounds__(256) w_rows_kernel(int L, int npo, int G, cons
 
 // Persistent over the items (row block, column tile); roles as in
 // ring_synthesis_digits_kernel, one sum per output.
-__global__ void __launch_bounds__(kThreads, 1) w_product_kernel(int L, int npo, int G, int ntile, int nitems,
-                                                                const WBlock* __restrict__ blocks,
+__global__ void __launch_bounds__(kThreads, 1) w_product_kernel(WGeometry g, int npo, int G, int ntile, int nitems,
+                                                                int b0, const int* __restrict__ lead,
                                                                 const unsigned char* __restrict__ rows,
                                                                 const int* __restrict__ rexp,
                                                                 const unsigned char* __restrict__ table,
@@ -134,7 +160,7 @@ __global__ void __launch_bounds__(kThreads, 1) w_product_kernel(int L, int npo, 
   __shared__ __align__(8) uint64_t full[kStages], empty[kStages], acc_full[2], acc_empty[2];
   __shared__ uint32_t tmem_base_s;
   __shared__ volatile int abort_s;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, npair = L / 2 + 1;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, L = g.L, npair = L / 2 + 1;
   const int nch = chunks_of(G);
   if (tid == 0) {
     for (int b = 0; b < kStages; ++b) {
@@ -162,10 +188,10 @@ __global__ void __launch_bounds__(kThreads, 1) w_product_kernel(int L, int npo, 
   if (warp == kAddWarps && lane == 0) {
     long long j = 0;   // groups
     for (int item = blockIdx.x; item < nitems && !abort_s; item += gridDim.x) {
-      const int b = item / ntile, tile = item % ntile, v = 2 * (blocks[b].m & 1) + blocks[b].par;
+      const int b = item / ntile, tile = item % ntile, v = g.cls(b0 + b);
       const unsigned char* A = rows + (int64_t)b * G * kAGroup;
       const unsigned char* B = table + ((int64_t)v * ntile + tile) * G * kBGroup;
-      for (int q = 0; q < G; ++q, ++j) {
+      for (int q = kChunk * lead[b]; q < G; ++q, ++j) {
         const int st = (int)(j % kStages);
         if (j >= kStages && !wait_or_abort(&empty[st], (uint32_t)((j / kStages - 1) & 1), &abort_s)) break;
         unsigned char* d = smem + st * kStage;
@@ -182,7 +208,7 @@ __global__ void __launch_bounds__(kThreads, 1) w_product_kernel(int L, int npo, 
     const uint32_t s0 = smem_u32(smem);
     long long j = 0, k = 0;   // groups, chunks
     for (int item = blockIdx.x; item < nitems && !abort_s; item += gridDim.x)
-      for (int q = 0; q < G; ++q, ++j) {
+      for (int q = kChunk * lead[item / ntile]; q < G; ++q, ++j) {
         const int b = (int)(k & 1), st = (int)(j % kStages), in_chunk = q % kChunk;
         if (in_chunk == 0 && k >= 2 && !wait_or_abort(&acc_empty[b], (uint32_t)(((k >> 1) - 1) & 1), &abort_s)) break;
         if (!wait_or_abort(&full[st], (uint32_t)((j / kStages) & 1), &abort_s)) break;
@@ -207,10 +233,8 @@ __global__ void __launch_bounds__(kThreads, 1) w_product_kernel(int L, int npo, 
     long long k = 0;
     bool ok = true;
     for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
-      const int b = item / ntile, tile = item % ntile;
-      const WBlock wb = blocks[b];
-      const int r = 32 * q + lane, i = 2 * (wb.rb * kRows + r) + wb.par, nl = L - wb.m;
-      const int v = 2 * (wb.m & 1) + wb.par;
+      const int b = item / ntile, tile = item % ntile, v = g.cls(b0 + b);
+      const int r = 32 * q + lane, rc = (b0 + b - g.first[v]) * kRows + r;   // row of the block, of the class
       long long a[kCols];   // in units of 2^53 2^(ex - 2150), below 2^62: 16 chunks of 2^58
       int ex[kCols];
 #pragma unroll
@@ -219,7 +243,7 @@ __global__ void __launch_bounds__(kThreads, 1) w_product_kernel(int L, int npo, 
         ex[c] = 0;
       }
 #pragma unroll 1
-      for (int ch = 0; ch < nch; ++ch, ++k) {
+      for (int ch = lead[b]; ch < nch; ++ch, ++k) {
         const int buf = (int)(k & 1);
         const int re = rexp[((int64_t)b * nch + ch) * kRows + r];
         int ce[kCols];
@@ -232,46 +256,50 @@ __global__ void __launch_bounds__(kThreads, 1) w_product_kernel(int L, int npo, 
         tc_fence_after();
         const uint32_t at = lanes + (uint32_t)(buf * kAccStride);
         long long h[kCols];   // the chunk's products in units of 2^53
-        float lo[kCols];
+        float x[32];
+        tmem_ld4x8(at, at + kNT, at + 2 * kNT, at + 3 * kNT, x);
 #pragma unroll
-        for (int s0 = 0; s0 < kLevels; s0 += 2) {
-          float x[32];
-          tmem_ld2x16(at + kNT * s0, at + kNT * min(s0 + 1, kLevels - 1), x);
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const int s = s0 + u;
-#pragma unroll
-            for (int c = 0; c < kCols; ++c) {
-              const float y = x[u * 16 + c];
-              if (s <= 3)
-                h[c] = mad_wide(__float2int_rn(y), s == 0 ? 1 << 27 : (s == 1 ? 1 << 18 : (s == 2 ? 512 : 1)), s ? h[c] : 0);
-              else if (s == 4)
-                h[c] = mad_wide(__float2int_rn(y), 2, h[c] * 1024);
-              else if (s == 5)
-                lo[c] = y * (2.f / 512.f);
-              else if (s == 6)
-                h[c] += __float2int_rn(fmaf(y, 2.f / 262144.f, lo[c]));
-            }
-          }
+        for (int c = 0; c < kCols; ++c) {
+          h[c] = mad_wide(__float2int_rn(x[c]), 1 << 27, 0);   // 512^3; 512 and 2 to come
+          h[c] = mad_wide(__float2int_rn(x[8 + c]), 1 << 18, h[c]);
+          h[c] = mad_wide(__float2int_rn(x[16 + c]), 512, h[c]) + __float2int_rn(x[24 + c]);
         }
+        tmem_ld4x8(at + 4 * kNT, at + 5 * kNT, at + 6 * kNT, at + 6 * kNT, x);
+#pragma unroll
+        for (int c = 0; c < kCols; ++c)
+          h[c] = mad_wide(__float2int_rn(x[c]), 2, h[c] * 1024) +
+                 __float2int_rn(fmaf(x[16 + c], 2.f / 262144.f, x[8 + c] * (2.f / 512.f)));
         tc_fence_before();
         __syncwarp();
         if (lane == 0)
           asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[buf])) : "memory");
+        // at the larger of the two scales, rounded
+        bool up = false;
 #pragma unroll
-        for (int c = 0; c < kCols; ++c) {   // at the larger of the two scales, rounded
-          const int e = re + ce[c], up = min(max(e - ex[c], 0), 62), dn = min(max(ex[c] - e, 0), 62);
-          a[c] = ((a[c] + ((1LL << up) >> 1)) >> up) + ((h[c] + ((1LL << dn) >> 1)) >> dn);
-          ex[c] = max(ex[c], e);
+        for (int c = 0; c < kCols; ++c) up = up || re + ce[c] > ex[c];
+        if (__any_sync(0xffffffffu, up)) {
+#pragma unroll
+          for (int c = 0; c < kCols; ++c) {
+            const int d = min(max(re + ce[c] - ex[c], 0), 62);
+            a[c] = (a[c] + ((1LL << d) >> 1)) >> d;
+            ex[c] = max(ex[c], re + ce[c]);
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < kCols; ++c) {
+          const int d = min(ex[c] - re - ce[c], 62);
+          a[c] += (h[c] + ((1LL << d) >> 1)) >> d;
         }
       }
-      if (!ok || i >= nl) continue;
-      const int64_t off = tab_off(wb.m, L, npair);
+      if (!ok || rc >= g.rows(v)) continue;
+      int m, i;
+      g.row(v, rc, m, i);
+      const int64_t off = tab_off(m, L, npair);
 #pragma unroll
       for (int c = 0; c < kCols; ++c) {
         const int t = tile * kNT + col0 + c;
         if (t < npair)
-          W[off + (int64_t)t * nl + i] =
+          W[off + (int64_t)t * (L - m) + i] =
               fixed_to_double(a[c], ex[c] - 2097) + pi_L * w[2 * t] * ps[off + (int64_t)i * npair + t];
       }
     }
@@ -292,54 +320,60 @@ int check(const char* what) {
 
 }  // namespace
 
-int digit_weights(int L, const double* po, const double* ps, const double* Kp, const double* w, double* W,
-                  cudaStream_t s) {
-  const int npo = (L + 1) / 2, npair = L / 2 + 1, G = groups16(npo), ntile = (npair + kNT - 1) / kNT;
-  std::vector<WBlock> blocks;
-  std::vector<int> first;   // of each batch of orders
-  size_t most = 0;
-  for (int m = 0; m < L; ++m) {
-    if (m % kBatch == 0) first.push_back((int)blocks.size());
-    for (int par = 0; par < 2; ++par)
-      for (int rb = 0; 2 * rb * kRows + par < L - m; ++rb) blocks.push_back(WBlock{m, par, rb});
+static WGeometry w_geometry(int L) {
+  WGeometry g{L, {0}};
+  for (int v = 0; v < 4; ++v) g.first[v + 1] = g.first[v] + (g.rows(v) + kRows - 1) / kRows;
+  return g;
+}
+
+// Scratch: the row digits of a batch, the table, the scales, the first chunks.
+struct WScratch {
+  size_t rows, table, rexp, cexp, first, total;
+  WScratch(const WGeometry& g, int G, int ntile) {
+    const size_t nb = std::min(kBatch, g.first[4]);
+    auto next = [&](size_t n) {
+      const size_t at = total;
+      total += (n + 255) / 256 * 256;
+      return at;
+    };
+    total = 0;
+    rows = next(nb * G * kAGroup);
+    table = next((size_t)4 * ntile * G * kBGroup);
+    rexp = next(nb * chunks_of(G) * kRows * sizeof(int));
+    cexp = next((size_t)4 * chunks_of(G) * ntile * kNT * sizeof(int));
+    first = next((size_t)g.first[4] * sizeof(int));
   }
-  first.push_back((int)blocks.size());
-  for (size_t b = 0; b + 1 < first.size(); ++b) most = std::max(most, (size_t)(first[b + 1] - first[b]));
-  DeviceBuffer db, rows, rexp, table, cexp, fail;
-  int rc, dev = 0, sms = 1, failed = 0;
-  if ((rc = db.upload(blocks.data(), blocks.size() * sizeof(WBlock))) ||
-      (rc = rows.alloc(most * G * kAGroup)) || (rc = rexp.alloc(most * chunks_of(G) * kRows * sizeof(int))) ||
-      (rc = table.alloc((size_t)4 * ntile * G * kBGroup)) ||
-      (rc = cexp.alloc((size_t)4 * chunks_of(G) * ntile * kNT * sizeof(int))) ||
-      (rc = fail.upload(&failed, sizeof(int))))
-    return rc;
-  cudaError_t e = cudaStreamSynchronize(0);   // the uploads, before s reads them
-  if (e == cudaSuccess) e = cudaMemsetAsync(table.p, 0, table.bytes, s);   // the zero blocks
-  const size_t row_smem = (size_t)8 * (16 * G + 2) * sizeof(double);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(w_product_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStages * kStage);
+};
+
+size_t digit_weights_bytes(int L) {
+  return WScratch(w_geometry(L), groups16((L + 1) / 2), (L / 2 + kNT) / kNT).total;
+}
+
+int digit_weights(int L, const double* po, const double* ps, const double* Kp, const double* w, double* W,
+                  void* scratch, int* fail, cudaStream_t s) {
+  const int npo = (L + 1) / 2, npair = L / 2 + 1, G = groups16(npo), ntile = (npair + kNT - 1) / kNT;
+  const WGeometry g = w_geometry(L);
+  const WScratch at(g, G, ntile);
+  unsigned char* mem = (unsigned char*)scratch;
+  int *rexp = (int*)(mem + at.rexp), *cexp = (int*)(mem + at.cexp), *first = (int*)(mem + at.first);
+  int dev = 0, sms = 1, rc;
+  cudaError_t e =
+      cudaFuncSetAttribute(w_product_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStages * kStage);
   if (e == cudaSuccess) e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return cuda_fail(e, "digit_weights");
-  w_table_kernel<<<dim3(ntile, 4), 256, 0, s>>>(npo, npair, G, Kp, (unsigned char*)table.p, (int*)cexp.p);
+  w_table_kernel<<<dim3(ntile, 4), 256, 0, s>>>(npo, npair, G, Kp, mem + at.table, cexp, first, g.first[4], fail);
   if ((rc = check("w_table_kernel"))) return rc;
-  for (size_t b = 0; b + 1 < first.size(); ++b) {
-    const int n = first[b + 1] - first[b], nitems = n * ntile;
-    const WBlock* bl = (const WBlock*)db.p + first[b];
-    w_rows_kernel<<<n * 16, 256, row_smem, s>>>(L, npo, G, bl, po, (unsigned char*)rows.p, (int*)rexp.p);
+  const int nbatch = (g.first[4] + kBatch - 1) / kBatch, batch = (g.first[4] + nbatch - 1) / nbatch;
+  for (int b = 0; b < g.first[4]; b += batch) {
+    const int n = std::min(batch, g.first[4] - b), nitems = n * ntile;
+    w_rows_kernel<<<n * 16, 256, (size_t)8 * (16 * G + 2) * sizeof(double), s>>>(g, npo, G, b, po, mem + at.rows, rexp,
+                                                                                first + b);
     if ((rc = check("w_rows_kernel"))) return rc;
     w_product_kernel<<<std::min(nitems, sms), kThreads, kStages * kStage, s>>>(
-        L, npo, G, ntile, nitems, bl, (const unsigned char*)rows.p, (const int*)rexp.p,
-        (const unsigned char*)table.p, (const int*)cexp.p, ps, w, 3.141592653589793 / L, W,
-        (int*)fail.p);
+        g, npo, G, ntile, nitems, b, first + b, mem + at.rows, rexp, mem + at.table, cexp, ps, w, 3.141592653589793 / L, W,
+        fail);
     if ((rc = check("w_product_kernel"))) return rc;
-  }
-  e = cudaMemcpyAsync(&failed, fail.p, sizeof(int), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return cuda_fail(e, "w_product_kernel");
-  if (failed) {
-    set_last_error("analysis weights: a bounded wait inside the kernel ran out");
-    return CMM_ERR_TIMEOUT;
   }
   return CMM_OK;
 }

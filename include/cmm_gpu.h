@@ -369,7 +369,7 @@ int cmm_sht_set_schedule(cmm_sht* plan, int schedule);
  * src in CMM_SHT_SPLIT_BF16 mode: `plan` is put in that mode on src's
  * split-bf16 Pbar tables (~4.4 GB at L = 1024).  src in CMM_SHT_FP64 mode:
  * `plan` keeps its precision and takes src's FP64 Pbar tables (built on
- * src first; 0.94 GB at L = 512) and table mode; CMM_ERR_ARG when src's
+ * src first; 0.98 GB at L = 512) and table mode; CMM_ERR_ARG when src's
  * FP64 stages run without tables (cmm_sht_set_tables).  Synchronises. */
 int cmm_sht_share_tables(cmm_sht* plan, cmm_sht* src);
 /* Failure-path self-test: runs the tensor-core kernels' bounded mbarrier
@@ -379,7 +379,7 @@ int cmm_sht_share_tables(cmm_sht* plan, cmm_sht* src);
  * context usable.  No counterpart in the reference. */
 int cmm_sht_timeout_selftest(cmm_sht* plan, long long polls, void* stream);
 /* FP64 Legendre stages from tabulated Pbar_lm (analysis and synthesis as
- * table contractions; 0.94 GB at L = 512, 7.5 GB at L = 1024) instead of
+ * table contractions; 0.98 GB at L = 512, 7.7 GB at L = 1024) instead of
  * the on-the-fly recurrence: mode 0 (default) for L <= 512, 1 for any
  * L <= 1024, -1 never.  The tables are built at the next FP64 stage that
  * runs outside a stream capture, which then synchronises its stream once,

@@ -509,3 +509,22 @@ def test_digit_synthesis_of_smooth_orders_near_the_poles(nat, L, m, decay):
     assert (err[:5] <= 5e-14 * own[:5]).all(), (err / own)[:5]
     assert err.max() <= 5e-14 * own.max()
     assert sht.status() == 0
+
+
+@pytest.mark.parametrize("L", [3, 4, 16, 17, 31, 33, 63, 64, 66, 129, 255, 258, 514, 1024])
+def test_weights_by_digits_match_the_resampling(nat, L):
+    """The analysis from the weight table (digits on the tensor cores) where its
+    tiles end (row blocks of 128 that run on from one order to the next, 32
+    rings per column tile and per scale), on generic samples, against the
+    resampling and recurrence: 1e-12 of the largest coefficient (the
+    recurrences lose about L ulps).  Twice on the table's plan: the first call
+    also makes the table."""
+    rng = np.random.default_rng(L)
+    f = rng.standard_normal((L + 1, 2 * L))
+    f[0], f[-1] = f[0, 0], f[-1, 0]
+    tab, rec = nat.Sht(L).set_tables(1), nat.Sht(L).set_tables(-1)
+    ref = rec.forward(dev(f)).cpu().numpy()
+    a, b = (tab.forward(dev(f)).cpu().numpy() for _ in range(2))
+    np.testing.assert_array_equal(a, b)
+    np.testing.assert_allclose(a, ref, rtol=0, atol=1e-12 * np.abs(ref).max())
+    assert tab.status() == 0
