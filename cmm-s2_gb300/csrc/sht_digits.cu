@@ -393,78 +393,111 @@ __global__ void __launch_bounds__(kSynThreads, 1) synth_digits_kernel(DigGeometr
     // those of 1.5 2^23 (taken off the group's products at once)
     constexpr long long kBits = 0x4B400000LL;
     auto bits = [](float x) { return __float_as_int(__fadd_rn(x, 12582912.f)); };
-    // one group's levels are on their way from tensor memory while the one
-    // before is added (rows past the last ring: never stored)
+    // Two groups of a chunk at a time (one where a parity has an odd number), the
+    // next ones' first levels on their way from tensor memory while these are
+    // added: one by one, the waits and the bookkeeping took as long as the sums.
+    // Rows past the last ring: never stored.
     float v[N * kLevels];
-    auto start = [&](unsigned k) {
-      const unsigned b = k % kAccs;
-      if (!warp_wait(&acc_full[b], (k / kAccs) & 1, &abort_s)) return false;
+    auto start = [&](unsigned k, bool two) {
+      const unsigned last = k + two;
+      if (!warp_wait(&acc_full[last % kAccs], (last / kAccs) & 1, &abort_s)) return false;
       tc_fence_after();
-      tmem_start7x4(lanes + b * 128, 16, v);
+      tmem_start7x4(lanes + k % kAccs * 128, 16, v);
       return true;
     };
-    int i = 0, q = 0;   // group of the item, of the chunk
-    unsigned j = 0;     // chunks
-    bool have = dig_item(u, nitems, g) && start(0);
-    int rows = have ? 8 * row_groups(g, u.blk) : 0;
-#pragma unroll 1
-    for (unsigned k = 0; have; ++k) {   // groups
-      long long h[N];   // the group's products in units of 2^53
+    auto products = [&](long long* h) {   // in units of 2^53
+      const float* x = v;
       tmem_wait7x4(v);
 #pragma unroll
       for (int n = 0; n < N; ++n) {
-        h[n] = mad_wide(bits(v[n]), 1 << 27, -kBits * ((1 << 27) + (1 << 18) + 512 + 1));   // 512^3; 512 and 2 to come
-        h[n] = mad_wide(bits(v[N + n]), 1 << 18, h[n]);
-        h[n] = mad_wide(bits(v[2 * N + n]), 512, h[n]);
-        h[n] = mad_wide(bits(v[3 * N + n]), 1, h[n]);
-        h[n] = mad_wide(__float2int_rn(v[4 * N + n]), 2, h[n] * 1024);
-        h[n] = mad_wide(__float2int_rn(fmaf(v[6 * N + n], 2.f / 262144.f, v[5 * N + n] * (2.f / 512.f))), 1, h[n]);
+        h[n] = mad_wide(bits(x[n]), 1 << 27, -kBits * ((1 << 27) + (1 << 18) + 512 + 1));   // 512^3; 512 and 2 to come
+        h[n] = mad_wide(bits(x[N + n]), 1 << 18, h[n]);
+        h[n] = mad_wide(bits(x[2 * N + n]), 512, h[n]);
+        h[n] = mad_wide(bits(x[3 * N + n]), 1, h[n]);
+        h[n] = mad_wide(__float2int_rn(x[4 * N + n]), 2, h[n] * 1024);
+        h[n] = mad_wide(__float2int_rn(fmaf(x[6 * N + n], 2.f / 262144.f, x[5 * N + n] * (2.f / 512.f))), 1, h[n]);
+      }
+    };
+    int i = 0, q = 0;   // group of the item, of the chunk
+    unsigned j = 0;     // chunks
+    bool have = dig_item(u, nitems, g);
+    bool two = u.ke > 1;
+    have = have && start(0, two);
+    int rows = have ? 8 * row_groups(g, u.blk) : 0;
+#pragma unroll 1
+    for (unsigned k = 0; have;) {   // groups
+      long long h[2][N];
+      products(h[0]);
+      if (two) {
+        tmem_start7x4(lanes + (k + 1) % kAccs * 128, 16, v);
+        products(h[1]);
+      } else {
+#pragma unroll
+        for (int n = 0; n < N; ++n) h[1][n] = 0;
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0)
-        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[k % kAccs])) : "memory");
-      // the group's scales, exponents biased
+      if (lane <= two)
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[(k + lane) % kAccs])) : "memory");
+      // the groups' scales, exponents biased
       const unsigned sc = j % kScales;
       if (q == 0 && !warp_wait(&sc_full[sc], (j / kScales) & 1, &abort_s)) break;
       const unsigned char* scales = smem + kStages * kStage + sc * kScaleBytes;
-      const int pe = ((const short*)(scales + 4 * kChunkGroups * kCols))[q * rows + min(32 * quad + lane, rows - 1)];
-      const int4 ae = *(const int4*)(scales + 4 * (q * kCols + col0));
-      const bool even_end = i + 1 == u.ke, item_end = i + 1 == u.ke + u.ko;
-      const bool chunk_end = even_end || item_end || q + 1 == kChunkGroups;
+      const short* pes = (const short*)(scales + 4 * kChunkGroups * kCols) + q * rows + min(32 * quad + lane, rows - 1);
+      const int4* aes = (const int4*)(scales + 4 * (q * kCols + col0));
+      int e[2][N];
+      {
+        const int pe = pes[0];
+        const int4 a = aes[0];
+        e[0][0] = pe + a.x, e[0][1] = pe + a.y, e[0][2] = pe + a.z, e[0][3] = pe + a.w;
+      }
+      if (two) {
+        const int pe = pes[rows];
+        const int4 a = aes[kCols / 4];
+        e[1][0] = pe + a.x, e[1][1] = pe + a.y, e[1][2] = pe + a.z, e[1][3] = pe + a.w;
+      } else {
+#pragma unroll
+        for (int n = 0; n < N; ++n) e[1][n] = 0;
+      }
+      i += 1 + two;
+      q += 1 + two;
+      k += 1 + two;
+      const bool even_end = i == u.ke, item_end = i == u.ke + u.ko;
+      const bool chunk_end = even_end || item_end || q == kChunkGroups;
       const int m = u.m, t = 1 + u.blk * kRows + 32 * quad + lane;
       if (chunk_end) {
         __syncwarp();
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&sc_empty[sc])) : "memory");
         ++j;
+        q = 0;
       }
-      q = chunk_end ? 0 : q + 1;
-      ++i;
       if (item_end) {
         ++u.round;
         have = dig_item(u, nitems, g);
         rows = 8 * row_groups(g, u.blk);
         i = 0;
       }
-      have = have && start(k + 1);
-      // at the larger of the two scales, rounded
-      const int e[N] = {pe + ae.x, pe + ae.y, pe + ae.z, pe + ae.w};
+      two = (i < u.ke ? u.ke : u.ke + u.ko) - i > 1;
+      have = have && start(k, two);
+      // at the largest of the scales, rounded
       bool up = false;
 #pragma unroll
-      for (int n = 0; n < N; ++n) up = up || e[n] > ex[n];
+      for (int n = 0; n < N; ++n) up = up || max(e[0][n], e[1][n]) > ex[n];
       if (__any_sync(0xffffffffu, up)) {
 #pragma unroll
         for (int n = 0; n < N; ++n) {
-          const int d = min(max(e[n] - ex[n], 0), 62);
+          const int to = max(ex[n], max(e[0][n], e[1][n])), d = min(to - ex[n], 62);
           acc[n] = (acc[n] + ((1LL << d) >> 1)) >> d;
-          ex[n] = max(ex[n], e[n]);
+          ex[n] = to;
         }
       }
 #pragma unroll
-      for (int n = 0; n < N; ++n) {
-        const int d = min(ex[n] - e[n], 62);
-        acc[n] += (h[n] + ((1LL << d) >> 1)) >> d;
-      }
+      for (int w = 0; w < 2; ++w)
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+          const int d = min(ex[n] - e[w][n], 62);
+          acc[n] += (h[w][n] + ((1LL << d) >> 1)) >> d;
+        }
       if (even_end) {   // the even degrees are complete
 #pragma unroll
         for (int n = 0; n < N; ++n) {
