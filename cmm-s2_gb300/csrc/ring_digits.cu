@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(kRingThreads, 1)
         for (int ch = 0; ch < n; ++ch) {
           const int sh = r < g.rows ? shift[(int64_t)r * 2 * kMaxChunks + (type & 1) * kMaxChunks + ch] : 0;
           const int b = (int)(k & 1);
-          if (!wait_or_abort(&acc_full[b], (uint32_t)((k >> 1) & 1), &abort_s)) {
+          if (!warp_wait(&acc_full[b], (uint32_t)((k >> 1) & 1), &abort_s)) {
             ok = false;
             break;
           }

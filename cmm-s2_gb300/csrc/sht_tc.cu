@@ -621,7 +621,7 @@ __global__ void __launch_bounds__(32 * kSynWarps2, 1) synth_tc2_kernel(TcGeometr
     bool have = syn_set(dr, blockIdx.x, nitems, g);
     while (have) {
       const int a = (int)(j & 1);
-      if (!wait_or_abort(&acc_full[a], (uint32_t)((j >> 1) & 1), &abort_s)) break;
+      if (!warp_wait(&acc_full[a], (uint32_t)((j >> 1) & 1), &abort_s)) break;
       tc_fence_after();
       float vE[32], vO[32];
       const uint32_t lanes = (uint32_t)(32 * warp) << 16;
