@@ -1296,9 +1296,10 @@ int launch_query_order(const MeshView& m, const double* q, int64_t n, int32_t* p
   int32_t* key = work;
   int32_t* hist = work + n;
   int32_t* total = hist + (int64_t)kOrderCells * nblk;
-  // bins of the fifth pass: as far as the packed ids leave bits, and for
-  // enough queries
-  int fine = kOrderFine;
+  // bins of the fifth pass: as far as the packed ids leave bits, for enough
+  // queries, and where a cell holds more than one triangle (2^24 queries on a
+  // level-3 mesh: 581 us with the pass, 555 without, for nothing)
+  int fine = m.level > kOrderLevel ? kOrderFine : 0;
   while (fine > 0 && (n < kOrderFineMin || n > (1LL << (32 - 2 * fine)))) --fine;
   order_count_kernel<<<(int)nblk, kOrderBlock, 0, s>>>(m, q, n, per, fine, key, hist);
   int rc = check_launch("order_count_kernel");

@@ -520,3 +520,21 @@ def test_composition_variants_bitwise_equal(nat, n):
             for a, b in zip(call(q, **k), ref):
                 assert torch.equal(a, b)
     assert m.status(clear=True) == nat.FLAG_NONFINITE
+
+
+@pytest.mark.parametrize("level", [3, 4, 5])
+def test_query_order_on_coarse_meshes(nat, level):
+    """cmm_query_order of enough queries for its fifth pass, which meshes whose
+    triangles are no smaller than a cell leave out: a permutation, every cell's
+    queries together (the composition's triangles change at most once per
+    triangle and cell)."""
+    from cmm_gpu.meshgen import icosahedral_mesh, random_sphere_points
+    verts, tris = icosahedral_mesh(level)
+    m = nat.Mesh(verts, tris, level)
+    n = (1 << 20) + 4097
+    q = dev(random_sphere_points(n, seed=level))
+    perm = m.query_order(q).long()
+    assert torch.equal(torch.sort(perm)[0], torch.arange(n, device="cuda"))
+    tri = m.locate(q, want_bcc=False)[0][perm]
+    if level <= 4:
+        assert int((tri[1:] != tri[:-1]).sum()) < 2 * m.nt * 4 ** (4 - level)
