@@ -666,158 +666,226 @@ struct PointX {
 // below FP64's roundings: entries to 2^-59, sums to ~2^-57.  A form with an
 // entry of 2 or more (a map stretching by more than about 2) goes through
 // FP64; a point outside (0.5, 1.4) in squared norm is normalised first.
-//
-// GATHER: a warp fetches its 32 forms together, nine neighbouring lanes' 16
-// bytes a form, through shared memory.  Its loads touch two lines a form
-// where every lane's own nine touch nine times 32, and all are in flight
-// without a register: scattered queries are bound by the lines (2^22 random
-// points through 8 level-7 maps 2.98 ms with own loads at 64 registers, 2.54
-// at 80, 1.82 so; in FP64 2.48).  Grouped queries share lines through the L1,
-// of which the staging takes 144 KB: 1.35 own, 1.48 so.  All lanes of a warp
-// stay in the loop; `live` marks those with a query and a finite image.
-template <class Src, int MINB, bool GATHER>
+
+// The form's nine double2 (in global memory, or GATHER in shared) at X -> X;
+// false, with X unchanged, where an entry is out of range.
+template <bool GATHER>
+__device__ __forceinline__ bool form_fixed(const double2* form, long long* X) {
+  double2 Q[9];   // own: all in flight together where the registers hold them
+  if (!GATHER) {
+#pragma unroll
+    for (int k = 0; k < 9; ++k) Q[k] = __ldg(form + k);
+  }
+  const Limbs x = fx_limbs(X[0]), y = fx_limbs(X[1]), z = fx_limbs(X[2]);
+  auto prod = [](Limbs a, Limbs b) {
+    FxSum v{0, 0};
+    v.add(a, b);
+    return fx_limbs(v.value());
+  };
+  const Limbs xx = prod(x, x), yy = prod(y, y), zz = prod(z, z);
+  const Limbs xy = prod(x, y), xz = prod(x, z), yz = prod(y, z);
+  if (GATHER) {   // the fetches of form_gather
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+  }
+  int bad = 0;
+  long long Y[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const double2 q0 = GATHER ? form[3 * c] : Q[3 * c], q1 = GATHER ? form[3 * c + 1] : Q[3 * c + 1],
+                  q2 = GATHER ? form[3 * c + 2] : Q[3 * c + 2];
+    FxSum r{0, 0};
+    r.add(fx_entry(q0.x, bad), xx);
+    r.add(fx_entry(q0.y, bad), yy);
+    r.add(fx_entry(q1.x, bad), zz);
+    r.add(fx_entry(q1.y, bad), xy);
+    r.add(fx_entry(q2.x, bad), xz);
+    r.add(fx_entry(q2.y, bad), yz);
+    Y[c] = r.value();
+  }
+  if (bad < 0) return false;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) X[c] = Y[c];
+  return true;
+}
+
+// The point back to the unit sphere; false where it has no direction.
+__device__ __forceinline__ bool renormalise(long long* X) {
+  const PointD p = PointX{X}.fp64();
+  const double inv_n = rsqrt(p.x * p.x + p.y * p.y + p.z * p.z);
+  if (!finite3(p.x * inv_n, p.y * inv_n, p.z * inv_n)) return false;
+  X[0] = fx_of(p.x * inv_n);
+  X[1] = fx_of(p.y * inv_n);
+  X[2] = fx_of(p.z * inv_n);
+  return true;
+}
+
+// One submap in FP64: its coefficient records (form null), or a form out of
+// the fixed-point range; false where the image is not finite.
+__device__ __forceinline__ bool form_wide(const MeshView& m, const double* __restrict__ form,
+                                          const double* __restrict__ recs, int t, long long* X) {
+  const PointD u = PointX{X}.fp64();
+  double p[3] = {u.x, u.y, u.z}, P[3];
+  if (form) {
+    for (int c = 0; c < 3; ++c)
+      P[c] = form[6 * c] * p[0] * p[0] + form[6 * c + 1] * p[1] * p[1] + form[6 * c + 2] * p[2] * p[2] +
+             form[6 * c + 3] * p[0] * p[1] + form[6 * c + 4] * p[0] * p[2] + form[6 * c + 5] * p[1] * p[2];
+  } else {
+    record_eval<false>(m, recs, t, p, Pushes{nullptr, 0}, P);
+  }
+  const double r2 = P[0] * P[0] + P[1] * P[1] + P[2] * P[2];
+  if (!(r2 > 0.5 && r2 < 1.4)) {
+    const double inv_n = rsqrt(r2);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) P[c] *= inv_n;
+    if (!finite3(P[0], P[1], P[2])) return false;
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) X[c] = fx_of(P[c]);
+  return true;
+}
+
+// The composed point's normalised coordinates; false where it has none.
+__device__ __forceinline__ bool store_point(const long long* X, double* __restrict__ out) {
+  double p[3] = {(double)X[0], (double)X[1], (double)X[2]};   // the units drop out
+  const double inv_n = rsqrt(p[0] * p[0] + p[1] * p[1] + p[2] * p[2]);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) p[c] *= inv_n;
+  if (!finite3(p[0], p[1], p[2])) return false;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) out[c] = p[c];
+  return true;
+}
+
+__device__ __forceinline__ bool off_sphere(float f0, float f1, float f2) {
+  const float n2 = fmaf(f0, f0, fmaf(f1, f1, f2 * f2));
+  return !(n2 > 0.5f && n2 < 1.4f);
+}
+
+// Every lane loads its own forms.
+template <class Src, int MINB>
 __global__ void __launch_bounds__(kBlock, MINB) compose_forms_kernel(MeshView m, Src cp,
                                                                      const double* __restrict__ q, int64_t n,
                                                                      double* __restrict__ out,
                                                                      int32_t* __restrict__ tri,
                                                                      int32_t* __restrict__ tri_all,
                                                                      const int32_t* __restrict__ perm) {
-  __shared__ double2 stage[GATHER ? 9 * kBlock : 1];
-  const int S = cp.count(), lane = threadIdx.x & 31;
-  for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; GATHER ? j - lane < n : j < n;
+  const int S = cp.count();
+  for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n;
        j += (int64_t)gridDim.x * blockDim.x) {
-    bool live = !GATHER || j < n;
-    int64_t i = j;
-    if (live && perm) i = (int64_t)__ldg(perm + j);
-    if (live && (uint64_t)i >= (uint64_t)n) {   // a bad permutation entry
+    const int64_t i = perm ? (int64_t)__ldg(perm + j) : j;
+    if ((uint64_t)i >= (uint64_t)n) {   // a bad permutation entry
       flag(m, CMM_FLAG_INDEX);
-      if (!GATHER) continue;
-      live = false;
+      continue;
     }
     long long X[3];   // the point, units of 2^-58
     int t;
     Split sp;
-    if (GATHER) {     // of a lane that has no query
-      X[0] = X[1] = X[2] = 0;
-      t = 0;
-      sp = Split{0, 2, 1};
+    {
+      double p[3];
+      if (!load_query(q, i, p)) {
+        store_nan<false>(m, i, n, S - 1, S, out, tri, tri_all, nullptr);
+        continue;
+      }
+      // the first location from the query's own FP64 values
+      t = locate_split(m, PointD{p[0], p[1], p[2]}, to_f32_trunc(p[0]), to_f32_trunc(p[1]), to_f32_trunc(p[2]), &sp);
+      if (tri) tri[i] = t;
+      if (tri_all) tri_all[(int64_t)(S - 1) * n + i] = t;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) X[c] = fx_of(p[c]);
     }
+    bool lost = false;   // no finite image
+    int s = S - 1;
+    float f0 = fx_f32(X[0]), f1 = fx_f32(X[1]), f2 = fx_f32(X[2]);
+    while (true) {
+      if (off_sphere(f0, f1, f2)) {   // rare; the direction, and so the location above, stays
+        lost = !renormalise(X);
+        if (lost) break;
+      }
+      const double* fr = cp.form(s, S);
+      if (fr) fr += (int64_t)t * kFormStride + 18 * kSubIndex[sp.lo][sp.hi];
+      if (!fr || !form_fixed<false>(reinterpret_cast<const double2*>(fr), X)) {
+        lost = !form_wide(m, fr, fr ? nullptr : cp.at(s, S), t, X);
+        if (lost) break;
+      }
+      if (--s < 0) break;
+      f0 = fx_f32(X[0]);
+      f1 = fx_f32(X[1]);
+      f2 = fx_f32(X[2]);
+      t = locate_split(m, PointX{X}, f0, f1, f2, &sp);
+      if (tri_all) tri_all[(int64_t)s * n + i] = t;
+    }
+    if (lost || !store_point(X, out + 3 * i)) store_nan<false>(m, i, n, s - 1, S, out, tri, tri_all, nullptr);
+  }
+}
+
+// A warp fetches its 32 forms together, nine neighbouring lanes' 16 bytes a
+// form, through shared memory.  Its loads touch two lines a form where every
+// lane's own nine touch nine times 32, and all are in flight without a
+// register: scattered queries are bound by the lines (2^22 random points
+// through 8 level-7 maps 2.98 ms with own loads at 64 registers, 2.54 at 80,
+// 1.76 so; in FP64 2.48).  Grouped queries share lines through the L1, of which
+// the staging takes 144 KB: 1.32 own, 1.39 so.  All lanes of a warp stay in the
+// loops; `live` marks those with a query and a finite image so far.
+template <class Src, int MINB>
+__global__ void __launch_bounds__(kBlock, MINB) compose_forms_gather_kernel(MeshView m, Src cp,
+                                                                            const double* __restrict__ q, int64_t n,
+                                                                            double* __restrict__ out,
+                                                                            int32_t* __restrict__ tri,
+                                                                            int32_t* __restrict__ tri_all,
+                                                                            const int32_t* __restrict__ perm) {
+  __shared__ double2 stage[9 * kBlock];
+  double2* warp = stage + 9 * (threadIdx.x & ~31u);
+  const int S = cp.count(), lane = threadIdx.x & 31;
+  for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j - lane < n;
+       j += (int64_t)gridDim.x * blockDim.x) {
+    bool live = j < n;
+    const int64_t i = live && perm ? (int64_t)__ldg(perm + j) : j;
+    if (live && (uint64_t)i >= (uint64_t)n) {   // a bad permutation entry
+      flag(m, CMM_FLAG_INDEX);
+      live = false;
+    }
+    long long X[3] = {0, 0, 0};
+    int t = 0;
+    Split sp{0, 2, 1};
     if (live) {
       double p[3];
       live = load_query(q, i, p);
-      if (!live) {
-        store_nan<false>(m, i, n, S - 1, S, out, tri, tri_all, nullptr);
-        if (!GATHER) continue;
-      } else {
-        // the first location from the query's own FP64 values
+      if (live) {
         t = locate_split(m, PointD{p[0], p[1], p[2]}, to_f32_trunc(p[0]), to_f32_trunc(p[1]), to_f32_trunc(p[2]), &sp);
         if (tri) tri[i] = t;
         if (tri_all) tri_all[(int64_t)(S - 1) * n + i] = t;
 #pragma unroll
         for (int c = 0; c < 3; ++c) X[c] = fx_of(p[c]);
+      } else {
+        store_nan<false>(m, i, n, S - 1, S, out, tri, tri_all, nullptr);
       }
     }
     int s = S - 1;
     float f0 = fx_f32(X[0]), f1 = fx_f32(X[1]), f2 = fx_f32(X[2]);
     while (true) {
-      const float n2 = fmaf(f0, f0, fmaf(f1, f1, f2 * f2));
-      if (live && !(n2 > 0.5f && n2 < 1.4f)) {
-        // rare: back to the unit sphere (the direction, and so the location
-        // above, stays)
-        PointD p = PointX{X}.fp64();
-        const double inv_n = rsqrt(p.x * p.x + p.y * p.y + p.z * p.z);
-        live = finite3(p.x * inv_n, p.y * inv_n, p.z * inv_n);
-        if (live) {
-          X[0] = fx_of(p.x * inv_n);
-          X[1] = fx_of(p.y * inv_n);
-          X[2] = fx_of(p.z * inv_n);
-        } else {
-          store_nan<false>(m, i, n, s - 1, S, out, tri, tri_all, nullptr);
-          if (!GATHER) break;
-        }
-      }
+      bool lost = live && off_sphere(f0, f1, f2) && !renormalise(X);
       const double* fr = cp.form(s, S);
-      bool wide = fr == nullptr;
+      bool wide = !fr;
       if (fr) {
-        const int sub = 18 * kSubIndex[sp.lo][sp.hi];
-        const double2* mine = stage + (GATHER ? 9 * threadIdx.x : 0);
-        double2 Q[9];
-        if (GATHER) {
-          const double2* qf = reinterpret_cast<const double2*>(fr);
-          double2* warp = stage + 9 * (threadIdx.x & ~31u);
-          const int off = (t * kFormStride + sub) / 2;
-          __syncwarp();   // the last map's forms are read
+        const double2* forms = reinterpret_cast<const double2*>(fr);
+        const int off = (t * kFormStride + 18 * kSubIndex[sp.lo][sp.hi]) / 2;
+        __syncwarp();   // the last map's forms are read
 #pragma unroll
-          for (int k = 0; k < 9; ++k) {
-            const int c = 32 * k + lane, r = c / 9;   // double2 c of the warp's, of lane r's form
-            const int o = __shfl_sync(0xffffffffu, off, r) + c - 9 * r;
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(
-                             (unsigned)__cvta_generic_to_shared(warp + c)),
-                         "l"(qf + o)
-                         : "memory");
-          }
-        } else {   // all in flight together where the registers hold them
-          const double2* qf = reinterpret_cast<const double2*>(fr + (int64_t)t * kFormStride + sub);
-#pragma unroll
-          for (int k = 0; k < 9; ++k) Q[k] = __ldg(qf + k);
+        for (int k = 0; k < 9; ++k) {
+          const int c = 32 * k + lane, r = c / 9;   // double2 c of the warp's, of lane r's form
+          const int o = __shfl_sync(0xffffffffu, off, r) + c - 9 * r;
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(warp + c)),
+                       "l"(forms + o)
+                       : "memory");
         }
-        const Limbs x = fx_limbs(X[0]), y = fx_limbs(X[1]), z = fx_limbs(X[2]);
-        auto prod = [](Limbs a, Limbs b) {
-          FxSum v{0, 0};
-          v.add(a, b);
-          return fx_limbs(v.value());
-        };
-        const Limbs xx = prod(x, x), yy = prod(y, y), zz = prod(z, z);
-        const Limbs xy = prod(x, y), xz = prod(x, z), yz = prod(y, z);
-        int bad = 0;
-        long long Y[3];
-        if (GATHER) {
-          asm volatile("cp.async.wait_all;" ::: "memory");
-          __syncwarp();
-        }
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          FxSum r{0, 0};
-          const double2 q0 = GATHER ? mine[3 * c] : Q[3 * c], q1 = GATHER ? mine[3 * c + 1] : Q[3 * c + 1],
-                        q2 = GATHER ? mine[3 * c + 2] : Q[3 * c + 2];
-          r.add(fx_entry(q0.x, bad), xx);
-          r.add(fx_entry(q0.y, bad), yy);
-          r.add(fx_entry(q1.x, bad), zz);
-          r.add(fx_entry(q1.y, bad), xy);
-          r.add(fx_entry(q2.x, bad), xz);
-          r.add(fx_entry(q2.y, bad), yz);
-          Y[c] = r.value();
-        }
-        wide = bad < 0;
-        if (!wide) {
-#pragma unroll
-          for (int c = 0; c < 3; ++c) X[c] = Y[c];
-        }
+        wide = !form_fixed<true>(warp + 9 * lane, X);
+        fr += 2 * (int64_t)off;
       }
-      if (live && wide) {   // in FP64: a coefficient record, or a form out of range
-        const PointD u = PointX{X}.fp64();
-        double p[3] = {u.x, u.y, u.z}, P[3];
-        if (fr) {
-          const double* Q = fr + (int64_t)t * kFormStride + 18 * kSubIndex[sp.lo][sp.hi];
-          for (int c = 0; c < 3; ++c)
-            P[c] = Q[6 * c] * p[0] * p[0] + Q[6 * c + 1] * p[1] * p[1] + Q[6 * c + 2] * p[2] * p[2] +
-                   Q[6 * c + 3] * p[0] * p[1] + Q[6 * c + 4] * p[0] * p[2] + Q[6 * c + 5] * p[1] * p[2];
-        } else {
-          record_eval<false>(m, cp.at(s, S), t, p, Pushes{nullptr, 0}, P);
-        }
-        const double r2 = P[0] * P[0] + P[1] * P[1] + P[2] * P[2];
-        if (!(r2 > 0.5 && r2 < 1.4)) {
-          const double inv_n = rsqrt(r2);
-#pragma unroll
-          for (int c = 0; c < 3; ++c) P[c] *= inv_n;
-          live = finite3(P[0], P[1], P[2]);
-          if (!live) {
-            store_nan<false>(m, i, n, s - 1, S, out, tri, tri_all, nullptr);
-            if (!GATHER) break;
-          }
-        }
-#pragma unroll
-        for (int c = 0; c < 3; ++c) X[c] = fx_of(P[c]);
+      if (live && !lost && wide) lost = !form_wide(m, fr, fr ? nullptr : cp.at(s, S), t, X);
+      if (lost) {
+        store_nan<false>(m, i, n, s - 1, S, out, tri, tri_all, nullptr);
+        live = false;
       }
       if (--s < 0) break;
       if (live) {
@@ -828,18 +896,7 @@ __global__ void __launch_bounds__(kBlock, MINB) compose_forms_kernel(MeshView m,
         if (tri_all) tri_all[(int64_t)s * n + i] = t;
       }
     }
-    if (!live) continue;
-    double p[3] = {(double)X[0], (double)X[1], (double)X[2]};   // the units drop out
-    const double inv_n = rsqrt(p[0] * p[0] + p[1] * p[1] + p[2] * p[2]);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) p[c] *= inv_n;
-    if (!finite3(p[0], p[1], p[2])) {
-      store_nan<false>(m, i, n, s - 1, S, out, tri, tri_all, nullptr);
-      continue;
-    }
-    out[3 * i] = p[0];
-    out[3 * i + 1] = p[1];
-    out[3 * i + 2] = p[2];
+    if (live && !store_point(X, out + 3 * i)) store_nan<false>(m, i, n, s - 1, S, out, tri, tri_all, nullptr);
   }
 }
 
@@ -1198,21 +1255,21 @@ int launch_compose(const MeshView& m, const double* const* coeffs, int S, const 
       // Own loads pay where a warp's queries share records: with several
       // queries per triangle, if they are grouped or a map's forms stay in the
       // L2 (73 MB at level 6, 294 at level 7).  Own against shared fetches:
-      // grouped 250,000 / 600,000 / 2^20 / 2^22 queries at level 7 129 / 254 /
-      // 385 / 1355 against 119 / 247 / 394 / 1504 us, at level 5 92 / 189 / 300 /
-      // 1172 against 100 / 208 / 343 / 1350; caller order, random 250,000 at
-      // level 6 69 against 62, 10^6 sample points there 172 against 198,
-      // 525,000 at level 7 221 against 208.  While 3 blocks per SM hold all
-      // queries 80 registers are faster (60,000 at level 7: 52 / 50 against 61 /
+      // grouped 250,000 / 600,000 / 2^20 / 2^22 queries at level 7 127 / 248 /
+      // 382 / 1324 against 118 / 243 / 385 / 1390 us, at level 5 91 / 186 / 296 /
+      // 1148 against 98 / 204 / 336 / 1310; caller order, random 250,000 at
+      // level 6 69 against 60, 10^6 sample points there 168 against 198,
+      // 525,000 at level 7 221 against 205.  While 3 blocks per SM hold all
+      // queries 80 registers are faster (60,000 at level 7: 51 / 50 against 61 /
       // 52).
       const bool far = (int64_t)m.nt * kFormStride * 8 > kL2Bytes;
       const bool scattered = perm ? n < 2 * (int64_t)m.nt : (far || n < 4 * (int64_t)m.nt);
-      if (v == 6) gof(compose_forms_kernel<Src, 6, false>);
-      else if (v == 4) gof(compose_forms_kernel<Src, 4, false>);
-      else if (n <= 3 * kBlockWave && n > kBlockWave && far) gof(compose_forms_kernel<Src, 3, true>);
-      else if (n <= 3 * kBlockWave) gof(compose_forms_kernel<Src, 3, false>);
-      else if (scattered) gof(compose_forms_kernel<Src, 4, true>);
-      else gof(compose_forms_kernel<Src, 4, false>);
+      if (v == 6) gof(compose_forms_kernel<Src, 6>);
+      else if (v == 4) gof(compose_forms_kernel<Src, 4>);
+      else if (n <= 3 * kBlockWave && n > kBlockWave && far) gof(compose_forms_gather_kernel<Src, 3>);
+      else if (n <= 3 * kBlockWave) gof(compose_forms_kernel<Src, 3>);
+      else if (scattered) gof(compose_forms_gather_kernel<Src, 4>);
+      else gof(compose_forms_kernel<Src, 4>);
     } else {
       if (v == 6) go(compose_kernel<false, Src, 6>);
       else go(compose_kernel<false, Src, kComposeBlocks>);
@@ -1326,7 +1383,7 @@ int launch_compose_dev(const MeshView& m, const double* const* table, const BveS
   };
   auto gof = [&](auto kernel) { kernel<<<grid_for(n, b), b, 0, s>>>(m, cp, q, n, out, nullptr, nullptr, nullptr); };
   if (ftable)
-    six ? gof(compose_forms_kernel<DevSubmaps, 6, false>) : gof(compose_forms_kernel<DevSubmaps, kComposeBlocks, false>);
+    six ? gof(compose_forms_kernel<DevSubmaps, 6>) : gof(compose_forms_kernel<DevSubmaps, kComposeBlocks>);
   else
     six ? go(compose_kernel<false, DevSubmaps, 6>) : go(compose_kernel<false, DevSubmaps, kComposeBlocks>);
   return check_launch("compose_kernel");
