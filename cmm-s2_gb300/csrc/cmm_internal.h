@@ -33,6 +33,7 @@ constexpr int kCoeffStride1 = 24;   // 19 ordinates, padded
 // sub-triangles (kSubIndex) and each component the homogeneous quadratic
 // form P(p) = p^T Q p as (Qxx, Qyy, Qzz, 2Qxy, 2Qxz, 2Qyz), 108 used.
 constexpr int kFormStride = 112;
+constexpr int kMaxLevel = 10;   // finest icosahedral mesh
 // Low floats of a map-form record's float-float split (floats per
 // triangle), for the Jacobian pushes: per sub-triangle (18 floats) and
 // component (6) the symmetric matrix entries Qxx, Qyy, Qzz, Qxy, Qxz, Qyz

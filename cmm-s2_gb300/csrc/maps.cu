@@ -834,6 +834,8 @@ __global__ void __launch_bounds__(kBlock, MINB) compose_forms_gather_kernel(Mesh
                                                                             int32_t* __restrict__ tri,
                                                                             int32_t* __restrict__ tri_all,
                                                                             const int32_t* __restrict__ perm) {
+  // a form's offset is exchanged as an int (in doubles, a level-10 mesh's last triangles would pass 2^31)
+  static_assert((20LL << (2 * kMaxLevel)) * (kFormStride / 2) <= INT32_MAX, "form offsets in double2");
   __shared__ double2 stage[9 * kBlock];
   double2* warp = stage + 9 * (threadIdx.x & ~31u);
   const int S = cp.count(), lane = threadIdx.x & 31;
@@ -869,7 +871,7 @@ __global__ void __launch_bounds__(kBlock, MINB) compose_forms_gather_kernel(Mesh
       bool wide = !fr;
       if (fr) {
         const double2* forms = reinterpret_cast<const double2*>(fr);
-        const int off = (t * kFormStride + 18 * kSubIndex[sp.lo][sp.hi]) / 2;
+        const int off = t * (kFormStride / 2) + 9 * kSubIndex[sp.lo][sp.hi];   // in double2
         __syncwarp();   // the last map's forms are read
 #pragma unroll
         for (int k = 0; k < 9; ++k) {

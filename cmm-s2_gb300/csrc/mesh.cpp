@@ -115,7 +115,8 @@ int64_t tri_key(int a, int b, int c, int64_t nv) {
 }  // namespace
 
 int build_host(const double* verts, int nv, const int32_t* tris, int nt, int level, HostMesh* hm) {
-  if (level < 0 || level > 10) {
+  static_assert(kMaxLevel == 10, "the message below");
+  if (level < 0 || level > kMaxLevel) {
     set_last_error("cmm_mesh_create: level must be in [0, 10]");
     return CMM_ERR_ARG;
   }
