@@ -22,6 +22,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "cmm_internal.h"
 #include "dd.cuh"
@@ -440,6 +441,18 @@ __device__ __forceinline__ void record_eval(const MeshView& m, const double* __r
 // the Jacobians through records 4 %.)
 constexpr int kNoForms = 0, kForms = 1, kFormsFF = 2;
 
+// A form's value in FP64: P_c = p^T Q_c p.
+__device__ __forceinline__ void form_value(const double* __restrict__ q, const double* p, double* P) {
+  const double2* qf = reinterpret_cast<const double2*>(q);
+  const double xx = p[0] * p[0], yy = p[1] * p[1], zz = p[2] * p[2];
+  const double xy = p[0] * p[1], xz = p[0] * p[2], yz = p[1] * p[2];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const double2 q01 = __ldg(qf + 3 * c), q23 = __ldg(qf + 3 * c + 1), q45 = __ldg(qf + 3 * c + 2);
+    P[c] = q01.x * xx + q01.y * yy + q23.x * zz + q23.y * xy + q45.x * xz + q45.y * yz;
+  }
+}
+
 // One submap from its map form: P_c = p^T Q_c p of the sub-triangle's
 // quadratic form (24 FP64 operations for the three components) and the
 // pushes' half derivatives (Q_c p) . w in float-float.  q: the form's 18
@@ -551,7 +564,8 @@ __device__ __forceinline__ void store_jacobian(const double* __restrict__ q, int
 }
 
 // Composition in FP64 with the Jacobian's pushes in float-float: through
-// coefficient records and, with JAC, through map forms.  (The fixed-point
+// coefficient records, through map forms with JAC, and through lists of both
+// with many records.  (The fixed-point
 // evaluation of compose_forms_kernel does not pay with Jacobians: the pushes
 // fill the issue slots that it takes; 2.63 against 2.42 ms per 2^22 queries.)
 // perm (nullable): process the queries in this order (grouped by coarse
@@ -610,8 +624,11 @@ __global__ void __launch_bounds__(kBlock, MINB) compose_kernel(MeshView m, Src c
       if (fr) {
         const int sub = 18 * kSubIndex[sp.lo][sp.hi];
         constexpr bool FF = FORMS == kFormsFF;
-        form_push<FF, ROLL>(fr + (int64_t)t * kFormStride + sub,
-                            FF ? cp.form_ff(s, S) + (int64_t)t * kFormFFStride + sub : nullptr, p, w, P);
+        fr += (int64_t)t * kFormStride + sub;
+        if (JAC)
+          form_push<FF, ROLL>(fr, FF ? cp.form_ff(s, S) + (int64_t)t * kFormFFStride + sub : nullptr, p, w, P);
+        else
+          form_value(fr, p, P);
       } else {
         record_eval<JAC>(m, cp.at(s, S), t, p, w, P);
       }
@@ -727,9 +744,7 @@ __device__ __forceinline__ bool form_wide(const MeshView& m, const double* __res
   const PointD u = PointX{X}.fp64();
   double p[3] = {u.x, u.y, u.z}, P[3];
   if (form) {
-    for (int c = 0; c < 3; ++c)
-      P[c] = form[6 * c] * p[0] * p[0] + form[6 * c + 1] * p[1] * p[1] + form[6 * c + 2] * p[2] * p[2] +
-             form[6 * c + 3] * p[0] * p[1] + form[6 * c + 4] * p[0] * p[2] + form[6 * c + 5] * p[1] * p[2];
+    form_value(form, p, P);
   } else {
     record_eval<false>(m, recs, t, p, Pushes{nullptr, 0}, P);
   }
@@ -745,9 +760,24 @@ __device__ __forceinline__ bool form_wide(const MeshView& m, const double* __res
   return true;
 }
 
+// A first submap without a form (a driver's current map, ahead of its stack) in
+// FP64 from the query's own values -> p its image; false where that is not
+// finite.  Through form_wide, the conversions to fixed point and back around it
+// made one map of the 525,312 sample points at L = 512 81 us instead of 64, and
+// 8,320 points at level 7 23 instead of 15.
+__device__ __forceinline__ bool record_first(const MeshView& m, const double* __restrict__ recs, double* p, int* t) {
+  *t = locate_row_f(m, PointD{p[0], p[1], p[2]}, to_f32_trunc(p[0]), to_f32_trunc(p[1]), to_f32_trunc(p[2]));
+  double P[3];
+  record_eval<false>(m, recs, *t, p, Pushes{nullptr, 0}, P);
+  const double r2 = P[0] * P[0] + P[1] * P[1] + P[2] * P[2];
+  const double sc = r2 > 0.5 && r2 < 1.4 ? 1.0 : rsqrt(r2);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) p[c] = P[c] * sc;
+  return finite3(p[0], p[1], p[2]);
+}
+
 // The composed point's normalised coordinates; false where it has none.
-__device__ __forceinline__ bool store_point(const long long* X, double* __restrict__ out) {
-  double p[3] = {(double)X[0], (double)X[1], (double)X[2]};   // the units drop out
+__device__ __forceinline__ bool store_point(double* p, double* __restrict__ out) {
   const double inv_n = rsqrt(p[0] * p[0] + p[1] * p[1] + p[2] * p[2]);
 #pragma unroll
   for (int c = 0; c < 3; ++c) p[c] *= inv_n;
@@ -756,14 +786,22 @@ __device__ __forceinline__ bool store_point(const long long* X, double* __restri
   for (int c = 0; c < 3; ++c) out[c] = p[c];
   return true;
 }
+__device__ __forceinline__ bool store_point(const long long* X, double* __restrict__ out) {
+  double p[3] = {(double)X[0], (double)X[1], (double)X[2]};   // the units drop out
+  return store_point(p, out);
+}
 
 __device__ __forceinline__ bool off_sphere(float f0, float f1, float f2) {
   const float n2 = fmaf(f0, f0, fmaf(f1, f1, f2 * f2));
   return !(n2 > 0.5f && n2 < 1.4f);
 }
 
-// Every lane loads its own forms.
-template <class Src, int MINB>
+// Every lane loads its own forms.  REC: the first submap has none; the locations
+// then stand at the loop's head, the only copy of their code beside the record's
+// (with one before the loop, as without REC, 981,400 points through 5 level-7
+// maps took 296 us in the shared form, 265 so; without REC the other way round
+// 392 against 377, 2^20 grouped queries).
+template <class Src, int MINB, bool REC>
 __global__ void __launch_bounds__(kBlock, MINB) compose_forms_kernel(MeshView m, Src cp,
                                                                      const double* __restrict__ q, int64_t n,
                                                                      double* __restrict__ out,
@@ -779,7 +817,7 @@ __global__ void __launch_bounds__(kBlock, MINB) compose_forms_kernel(MeshView m,
       continue;
     }
     long long X[3];   // the point, units of 2^-58
-    int t;
+    int t, s = S - 1;
     Split sp;
     {
       double p[3];
@@ -787,18 +825,37 @@ __global__ void __launch_bounds__(kBlock, MINB) compose_forms_kernel(MeshView m,
         store_nan<false>(m, i, n, S - 1, S, out, tri, tri_all, nullptr);
         continue;
       }
-      // the first location from the query's own FP64 values
-      t = locate_split(m, PointD{p[0], p[1], p[2]}, to_f32_trunc(p[0]), to_f32_trunc(p[1]), to_f32_trunc(p[2]), &sp);
-      if (tri) tri[i] = t;
-      if (tri_all) tri_all[(int64_t)(S - 1) * n + i] = t;
+      if (REC) {
+        const bool ok = record_first(m, cp.at(s, S), p, &t);
+        if (tri) tri[i] = t;
+        if (tri_all) tri_all[(int64_t)s * n + i] = t;
+        --s;
+        if (!ok || (s < 0 && !store_point(p, out + 3 * i))) {
+          store_nan<false>(m, i, n, s, S, out, tri, tri_all, nullptr);
+          continue;
+        }
+        if (s < 0) continue;
+      }
+      if (!REC) {   // the first location from the query's own FP64 values
+        t = locate_split(m, PointD{p[0], p[1], p[2]}, to_f32_trunc(p[0]), to_f32_trunc(p[1]), to_f32_trunc(p[2]), &sp);
+        if (tri) tri[i] = t;
+        if (tri_all) tri_all[(int64_t)s * n + i] = t;
+      }
 #pragma unroll
       for (int c = 0; c < 3; ++c) X[c] = fx_of(p[c]);
     }
     bool lost = false;   // no finite image
-    int s = S - 1;
-    float f0 = fx_f32(X[0]), f1 = fx_f32(X[1]), f2 = fx_f32(X[2]);
+    float f0, f1, f2;
+    auto floats = [&] { f0 = fx_f32(X[0]), f1 = fx_f32(X[1]), f2 = fx_f32(X[2]); };
+    auto locate = [&] {
+      floats();
+      t = locate_split(m, PointX{X}, f0, f1, f2, &sp);
+      if (tri_all) tri_all[(int64_t)s * n + i] = t;
+    };
+    if (!REC) floats();
     while (true) {
-      if (off_sphere(f0, f1, f2)) {   // rare; the direction, and so the location above, stays
+      if (REC) locate();
+      if (off_sphere(f0, f1, f2)) {   // rare; the direction, and so the location, stays
         lost = !renormalise(X);
         if (lost) break;
       }
@@ -809,11 +866,7 @@ __global__ void __launch_bounds__(kBlock, MINB) compose_forms_kernel(MeshView m,
         if (lost) break;
       }
       if (--s < 0) break;
-      f0 = fx_f32(X[0]);
-      f1 = fx_f32(X[1]);
-      f2 = fx_f32(X[2]);
-      t = locate_split(m, PointX{X}, f0, f1, f2, &sp);
-      if (tri_all) tri_all[(int64_t)s * n + i] = t;
+      if (!REC) locate();
     }
     if (lost || !store_point(X, out + 3 * i)) store_nan<false>(m, i, n, s - 1, S, out, tri, tri_all, nullptr);
   }
@@ -827,7 +880,7 @@ __global__ void __launch_bounds__(kBlock, MINB) compose_forms_kernel(MeshView m,
 // 1.76 so; in FP64 2.48).  Grouped queries share lines through the L1, of which
 // the staging takes 144 KB: 1.32 own, 1.39 so.  All lanes of a warp stay in the
 // loops; `live` marks those with a query and a finite image so far.
-template <class Src, int MINB>
+template <class Src, int MINB, bool REC>
 __global__ void __launch_bounds__(kBlock, MINB) compose_forms_gather_kernel(MeshView m, Src cp,
                                                                             const double* __restrict__ q, int64_t n,
                                                                             double* __restrict__ out,
@@ -848,24 +901,42 @@ __global__ void __launch_bounds__(kBlock, MINB) compose_forms_gather_kernel(Mesh
       live = false;
     }
     long long X[3] = {0, 0, 0};
-    int t = 0;
+    int t = 0, s = S - 1;
     Split sp{0, 2, 1};
+    double p[3] = {0.0, 0.0, 0.0};
     if (live) {
-      double p[3];
       live = load_query(q, i, p);
+      if (!live) store_nan<false>(m, i, n, s, S, out, tri, tri_all, nullptr);
+    }
+    if (REC) {
       if (live) {
+        live = record_first(m, cp.at(s, S), p, &t);
+        if (tri) tri[i] = t;
+        if (tri_all) tri_all[(int64_t)s * n + i] = t;
+        if (!live || (s == 0 && !store_point(p, out + 3 * i))) store_nan<false>(m, i, n, s - 1, S, out, tri, tri_all, nullptr);
+      }
+      if (--s < 0) continue;
+    }
+    if (live) {
+      if (!REC) {
         t = locate_split(m, PointD{p[0], p[1], p[2]}, to_f32_trunc(p[0]), to_f32_trunc(p[1]), to_f32_trunc(p[2]), &sp);
         if (tri) tri[i] = t;
-        if (tri_all) tri_all[(int64_t)(S - 1) * n + i] = t;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) X[c] = fx_of(p[c]);
-      } else {
-        store_nan<false>(m, i, n, S - 1, S, out, tri, tri_all, nullptr);
+        if (tri_all) tri_all[(int64_t)s * n + i] = t;
       }
+#pragma unroll
+      for (int c = 0; c < 3; ++c) X[c] = fx_of(p[c]);
     }
-    int s = S - 1;
-    float f0 = fx_f32(X[0]), f1 = fx_f32(X[1]), f2 = fx_f32(X[2]);
+    float f0, f1, f2;
+    auto floats = [&] { f0 = fx_f32(X[0]), f1 = fx_f32(X[1]), f2 = fx_f32(X[2]); };
+    auto locate = [&] {
+      if (!live) return;
+      floats();
+      t = locate_split(m, PointX{X}, f0, f1, f2, &sp);
+      if (tri_all) tri_all[(int64_t)s * n + i] = t;
+    };
+    floats();
     while (true) {
+      if (REC) locate();
       bool lost = live && off_sphere(f0, f1, f2) && !renormalise(X);
       const double* fr = cp.form(s, S);
       bool wide = !fr;
@@ -890,13 +961,7 @@ __global__ void __launch_bounds__(kBlock, MINB) compose_forms_gather_kernel(Mesh
         live = false;
       }
       if (--s < 0) break;
-      if (live) {
-        f0 = fx_f32(X[0]);
-        f1 = fx_f32(X[1]);
-        f2 = fx_f32(X[2]);
-        t = locate_split(m, PointX{X}, f0, f1, f2, &sp);
-        if (tri_all) tri_all[(int64_t)s * n + i] = t;
-      }
+      if (!REC) locate();
     }
     if (live && !store_point(X, out + 3 * i)) store_nan<false>(m, i, n, s - 1, S, out, tri, tri_all, nullptr);
   }
@@ -1218,6 +1283,17 @@ int launch_compose(const MeshView& m, const double* const* coeffs, int S, const 
   bool ff = forms_ff != nullptr;
   for (int k = 0; forms && k < S; ++k)
     if (forms[k] && !(forms_ff && forms_ff[k])) ff = false;
+  // points only: lists with records beside a first submap's in FP64, where those
+  // are more than a third of the forms.  The fixed-point kernels convert the point
+  // around each (level 5, 6 records 250,000 points 200 us, 168 in FP64; 3 of 6
+  // level-7 maps 179 and 164; a form costs 15.2 against 20.4 and a record 36
+  // against 29).
+  int with = 0, without = 0;
+  for (int k = 0; forms && k < S; ++k) {
+    with += forms[k] != nullptr;
+    without += !forms[k] && k < S - 1;
+  }
+  const bool mixed = without > 0 && 3 * without > with;
   const int b = block_for(m, kTuneCompose, kBlock, n);
   const int vj = m.variant[CMM_VARIANT_COMPOSE_JAC], v = m.variant[CMM_VARIANT_COMPOSE];
   auto run = [&](auto list) {
@@ -1252,7 +1328,10 @@ int launch_compose(const MeshView& m, const double* const* coeffs, int S, const 
       if (vj == 2) go(compose_kernel<true, Src, 2>);
       else if (vj == 3) go(compose_kernel<true, Src, 3>);
       else go(compose_kernel<true, Src, kComposeJacBlocks>);
-    } else if (forms) {
+    } else if (mixed && with) {
+      if (v == 6) go(compose_kernel<false, Src, 6, kForms>);
+      else go(compose_kernel<false, Src, kComposeBlocks, kForms>);
+    } else if (forms && !mixed && (S > 1 || forms[0])) {
       auto gof = [&](auto kernel) { kernel<<<grid_for(n, b), b, 0, s>>>(m, list, q, n, out, tri, tri_all, perm); };
       // Own loads pay where a warp's queries share records: with several
       // queries per triangle, if they are grouped or a map's forms stay in the
@@ -1261,17 +1340,23 @@ int launch_compose(const MeshView& m, const double* const* coeffs, int S, const 
       // 382 / 1324 against 118 / 243 / 385 / 1390 us, at level 5 91 / 186 / 296 /
       // 1148 against 98 / 204 / 336 / 1310; caller order, random 250,000 at
       // level 6 69 against 60, 10^6 sample points there 168 against 198,
-      // 525,000 at level 7 221 against 205.  While 3 blocks per SM hold all
+      // 525,000 at level 7 221 against 205.  One form behind a record is fetched
+      // as soon by its lane (2^22 random points, level 7: 731 against 762).  While 3 blocks per SM hold all
       // queries 80 registers are faster (60,000 at level 7: 51 / 50 against 61 /
       // 52).
       const bool far = (int64_t)m.nt * kFormStride * 8 > kL2Bytes;
-      const bool scattered = perm ? n < 2 * (int64_t)m.nt : (far || n < 4 * (int64_t)m.nt);
-      if (v == 6) gof(compose_forms_kernel<Src, 6>);
-      else if (v == 4) gof(compose_forms_kernel<Src, 4>);
-      else if (n <= 3 * kBlockWave && n > kBlockWave && far) gof(compose_forms_gather_kernel<Src, 3>);
-      else if (n <= 3 * kBlockWave) gof(compose_forms_kernel<Src, 3>);
-      else if (scattered) gof(compose_forms_gather_kernel<Src, 4>);
-      else gof(compose_forms_kernel<Src, 4>);
+      const bool scattered = (forms[S - 1] || S > 2) && (perm ? n < 2 * (int64_t)m.nt : far || n < 4 * (int64_t)m.nt);
+      auto pick = [&](auto rec) {
+        constexpr bool REC = decltype(rec)::value;
+        if (v == 6) gof(compose_forms_kernel<Src, 6, REC>);
+        else if (v == 4) gof(compose_forms_kernel<Src, 4, REC>);
+        else if (n <= 3 * kBlockWave && n > kBlockWave && far) gof(compose_forms_gather_kernel<Src, 3, REC>);
+        else if (n <= 3 * kBlockWave) gof(compose_forms_kernel<Src, 3, REC>);
+        else if (scattered) gof(compose_forms_gather_kernel<Src, 4, REC>);
+        else gof(compose_forms_kernel<Src, 4, REC>);
+      };
+      if (forms[S - 1]) pick(std::false_type{});
+      else pick(std::true_type{});
     } else {
       if (v == 6) go(compose_kernel<false, Src, 6>);
       else go(compose_kernel<false, Src, kComposeBlocks>);
@@ -1385,7 +1470,7 @@ int launch_compose_dev(const MeshView& m, const double* const* table, const BveS
   };
   auto gof = [&](auto kernel) { kernel<<<grid_for(n, b), b, 0, s>>>(m, cp, q, n, out, nullptr, nullptr, nullptr); };
   if (ftable)
-    six ? gof(compose_forms_kernel<DevSubmaps, 6>) : gof(compose_forms_kernel<DevSubmaps, kComposeBlocks>);
+    six ? gof(compose_forms_kernel<DevSubmaps, 6, true>) : gof(compose_forms_kernel<DevSubmaps, kComposeBlocks, true>);
   else
     six ? go(compose_kernel<false, DevSubmaps, 6>) : go(compose_kernel<false, DevSubmaps, kComposeBlocks>);
   return check_launch("compose_kernel");

@@ -538,3 +538,39 @@ def test_query_order_on_coarse_meshes(nat, level):
     tri = m.locate(q, want_bcc=False)[0][perm]
     if level <= 4:
         assert int((tri[1:] != tri[:-1]).sum()) < 2 * m.nt * 4 ** (4 - level)
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 40_001, 150_001])
+@pytest.mark.parametrize("records", ["-", "r", "rr", "fr", "ffr", "frf", "rfr", "rff", "frrr"])
+def test_lists_of_forms_and_records(nat, n, records):
+    """Points-only compositions of submaps with forms (f) and without (r), in
+    evaluation order from the right (the last is evaluated first): the records
+    ahead of the forms, between them, behind them, alone, and "-" no list; own
+    and shared fetches and the FP64 kernel.  Ids of every submap those of the
+    records alone, points within the bound of forms against records (1e-13);
+    every order of the queries bitwise the same; queries without an image."""
+    from cmm_gpu.meshgen import icosahedral_mesh, stencil_frames, random_sphere_points
+    from cmm_gpu.workloads import submap_stack
+    verts, tris = icosahedral_mesh(5)
+    tan, s_pts = stencil_frames(verts)
+    m = nat.Mesh(verts, tris, 5)
+    S = len(records)
+    cs = [m.assemble(dev(j)) for j in submap_stack(s_pts, tan, S, seed=21)]
+    fs = None if records == "-" else [m.assemble_forms(c) if k == "f" else None for c, k in zip(cs, records)]
+    q = dev(random_sphere_points(n, seed=n))
+    bad = torch.zeros(n, dtype=torch.bool, device="cuda")
+    if n > 40:
+        q[7] = float("nan")
+        q[n - 3] = 0.0
+        bad[7] = bad[n - 3] = True
+        q[11] *= 1e-3
+        q[12] *= 3.0
+    X, _, ta, _ = m.compose(cs, q, want_tri_all=True)
+    Y, _, tb, _ = m.compose(cs, q, want_tri_all=True, forms=fs)
+    assert torch.equal(ta, tb)
+    assert torch.equal(torch.isnan(Y).any(1), bad) and torch.equal(torch.isnan(X).any(1), bad)
+    assert bool((tb[:, bad] == -1).all())
+    assert float((X - Y)[~bad].abs().max()) < 1e-13
+    Z, _, tc, _ = m.compose(cs, q, want_tri_all=True, forms=fs, perm=m.query_order(q))
+    assert torch.equal(Z.view(torch.int64), Y.view(torch.int64)) and torch.equal(tc, tb)
+    m.status(clear=True)
