@@ -699,7 +699,7 @@ int launch_vorticity_bwd(const MeshView& vm, const double* dsh, int lmax, double
     return CMM_ERR_UNSUPPORTED;
   }
   if (gX) {
-    if (dsh && Q <= kShLanesMaxQ)
+    if (dsh && sh_lanes_pay(Q, lmax))
       vorticity_bwd_x_kernel<kShLanes><<<grid_for(kShLanes * Q, kBlock), kBlock, 0, s>>>(vm, dsh, lmax, rot, X, Q, gw,
                                                                                          gX);
     else

@@ -697,9 +697,16 @@ __device__ __forceinline__ void sh_series_n(const MeshView& vm, const double* __
 // order's start values advance four orders at a time, by cos/sin(4 phi) and
 // sin^4(theta).
 constexpr int kShLanes = 4;
-// Points below which the series takes four lanes each: a thread per point then
-// leaves at most 8 warps per SM.
-constexpr int64_t kShLanesMaxQ = 152LL * 8 * 32;
+// Whether the series takes four lanes per point: a thread per point leaves at most
+// a warp per SM; or at most 8, and the degrees are many enough for the shorter
+// chains to outweigh the lanes' own start values, four times a point's work (a
+// thread per point against lanes, us: 9,940 points, degrees to 5 15.1 / 14.4;
+// 18,624 points, 6 17.2 / 21.2, 8 25.4 / 26.8, 10 33.6 / 31.0; 33,024 points, 16
+// 83 / 85, 24 163 / 144; the point gradient alike).
+inline bool sh_lanes_pay(int64_t Q, int lmax) {
+  constexpr int64_t kWarpEach = 152LL * 32;
+  return Q <= kWarpEach || (Q <= 8 * kWarpEach && Q <= 1800LL * lmax);
+}
 
 template <int NS>
 __device__ __forceinline__ void sh_series_lanes(const MeshView& vm, const double* __restrict__ c, int lmax,

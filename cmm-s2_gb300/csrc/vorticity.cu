@@ -214,7 +214,7 @@ int launch_vorticity(int kind, const double* params, int nparams, const double* 
   vp.iw = 1.f / fabsf((float)vp.p[1]);
   for (int k = 0; k < 9; ++k) vp.lat[k] = (float)vp.p[3 + k];
   const int b = block_for(vm, kTuneVorticity, 128, Q);
-  if (sh && kind == CMM_VORT_NONE && !spline && Q <= kShLanesMaxQ) {
+  if (sh && kind == CMM_VORT_NONE && !spline && sh_lanes_pay(Q, lmax)) {
     vorticity_series_kernel<<<grid_for(kShLanes * Q, b), b, 0, s>>>(sh, lmax, vm, rot, X, Q, npr, cos_ring, omega);
     note_launch();
     cudaError_t e = cudaGetLastError();
