@@ -1285,8 +1285,8 @@ static int set_streams(cmm_sht* p, cudaStream_t s) {
     cufftResult r = cufftSetStream(h[k], s);
     if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftSetStream");
   }
-  cufftHandle ht[3] = {p->torus_fwd_t, p->pad_inv_t, p->ring_inv9};
-  for (int k = 0; k < 3; ++k) {
+  cufftHandle ht[2] = {p->torus_fwd_t, p->pad_inv_t};
+  for (int k = 0; k < 2; ++k) {
     cufftResult r = cufftSetStream(ht[k], s);
     if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftSetStream");
   }
@@ -1617,7 +1617,9 @@ static int velocity_fp64(cmm_sht* p, const cmm_mesh* vm, const double2* a, bool 
     rc = ring_inverse(*p->tab->ring, kVelSpectra, S, p->dig_work.p, (double*)p->samples.p, (int*)p->status.p, s);
     if (rc) return rc;
   } else {
-    cufftResult r = cufftExecZ2D(p->ring_inv9, (cufftDoubleComplex*)S, (cufftDoubleReal*)p->samples.p);
+    cufftResult r = cufftSetStream(p->ring_inv9, s);   // not by set_streams: no other call uses it
+    if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftSetStream");
+    r = cufftExecZ2D(p->ring_inv9, (cufftDoubleComplex*)S, (cufftDoubleReal*)p->samples.p);
     if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftExecZ2D(velocity)");
   }
   const int64_t nv = 2 + (int64_t)(L - 1) * 2 * L;
