@@ -50,7 +50,7 @@ METRIC = "map evals/s"
 # the number of queries (the gathers and outputs grow with it): the
 # headline step (queries grouped by coarse cell, map forms and their low
 # floats) ...
-COMPOSE_TRAFFIC_PER_QUERY = (4.9911e9 + 0.9178e9) / (1 << 22)
+COMPOSE_TRAFFIC_PER_QUERY = (4.8678e9 + 0.7849e9) / (1 << 22)
 # ... and in the caller's order (map forms alone).
 COMPOSE_TRAFFIC_PER_QUERY_CALLER = (9.9927e9 + 0.5103e9) / (1 << 22)
 # FP64 instructions (DADD + DMUL + DFMA) per map evaluation (query x
@@ -60,7 +60,7 @@ COMPOSE_TRAFFIC_PER_QUERY_CALLER = (9.9927e9 + 0.5103e9) / (1 << 22)
 # instructions issued per SM per clock, they cost ~13 and ~12 SM cycles
 # per evaluation at their peaks, so the two bind together.
 FP64_INSTR_PER_EVAL = 26.65
-INSTR_PER_EVAL = 1580
+INSTR_PER_EVAL = 1583
 
 
 def peaks():

@@ -1341,9 +1341,11 @@ int launch_compose(const MeshView& m, const double* const* coeffs, int S, const 
       // 1148 against 98 / 204 / 336 / 1310; caller order, random 250,000 at
       // level 6 69 against 60, 10^6 sample points there 168 against 198,
       // 525,000 at level 7 221 against 205.  One form behind a record is fetched
-      // as soon by its lane (2^22 random points, level 7: 731 against 762).  While 3 blocks per SM hold all
-      // queries 80 registers are faster (60,000 at level 7: 51 / 50 against 61 /
-      // 52).
+      // as soon by its lane (2^22 random points, level 7: 731 against 762).  In
+      // the caller's order at level 7 the rule stands for scattered points (8
+      // maps, 2^22: 2980 against 1744 us); a grid's, 2.1 million, take 650 and
+      // 715.  While 3 blocks per SM hold all queries 80 registers are faster
+      // (60,000 at level 7: 51 / 50 against 61 / 52).
       const bool far = (int64_t)m.nt * kFormStride * 8 > kL2Bytes;
       const bool scattered = (forms[S - 1] || S > 2) && (perm ? n < 2 * (int64_t)m.nt : far || n < 4 * (int64_t)m.nt);
       auto pick = [&](auto rec) {

@@ -1296,7 +1296,8 @@ static int set_streams(cmm_sht* p, cudaStream_t s) {
 // Least L whose velocity takes the ring transforms by digits (ring_digits.cu):
 // below, their few work items leave the chip idle and the fast transform is
 // short (velocity inversion at L = 128: 71 us by digits, 66 by the FFT; 160: 93
-// and 92; 192: 107 and 117; 256: 138 and 172; 512: 466 and 681).
+// and 92; 192: 107 and 117; 256: 138 and 172; 512: 466 and 681; the synthesis
+// with one scale per row).
 constexpr int kRingMinL = 160;
 
 static size_t ring_work(const cmm_sht* p) { return p->L >= kRingMinL ? ring_work_bytes(p->L, kVelSpectra) : 0; }
